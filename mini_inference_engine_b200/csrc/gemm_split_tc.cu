@@ -1,0 +1,384 @@
+// y[M, N] = x[M, K] w[N, K]^T (+ bias[N]) for float32 operands, at the precision of float32 products, on the tensor cores of pairs of SMs
+// (the CUDA-core product of csrc/gemm_simt.cu runs where this one does not pay).
+//
+// A float32 number is the sum of three bfloat16 numbers exactly: 8 + 8 + 8 bits of its significand, cut off one after the other
+// (`split`).  Of the nine products of parts six are formed, in float32: the three left out are below 2^-24 of the product, half of what one
+// rounding of a float32 product loses.  The tensor core's own float32 sums are cut off rather than rounded, so
+// a sum stays there for 64 products only (small parts first); every 64-wide chunk of K is taken out of tensor memory and added to a
+// float32 register, rounded to nearest.  Against 64 bits the error is 1.1e-7 at K 2,048 and 1.8e-7 at K 5,632 (2-norm) where one
+// chain of K fused multiply-adds leaves 5.5e-7 and 1.1e-6.
+// A number that is not finite, or a sum that overflows on the way, makes a part infinity minus infinity: an output that is not finite is
+// worked out again as one chain of fused multiply-adds from the operands themselves, so it is what the CUDA-core product gives.
+//
+//   split    [rows, K] float32 -> three bfloat16 planes: bound by memory, 10 bytes a number (11,264 x 2,048: 45 us, 5.1 TB/s).
+//   product  a pair of blocks owns 256 rows of w and BN (64, 128 or 256) tokens; per 64-wide chunk of K each block's stage
+//            holds its half of both operands' three planes (TMA, 128-byte swizzle), 24 cta_group::2 MMAs of K 16 go into one of
+//            two to four accumulators, and eight warps move a finished one into their registers (a thread a row of w, half of the tokens).
+//            Rows of w on the 128-lane side: what a warp stores for a token is 128 contiguous bytes, and a few tokens waste nothing.
+//            The pair runs persistently over (tile, share of K) items; shares meet in `partial` and a last small kernel adds them up in order.
+//
+// Bound: the tensor pipe (6 bfloat16 products for one float32 one: a sixth of its rate) for many tokens, memory (4 bytes of w read, 6
+// written and read again) for few.  2,048 x 11,264 x 2,048: 2,707 us on the CUDA cores -> 415 us (228 TFLOP/s, 252 without the split);
+// 509 x 11,264 x 2,048 1,008 -> 165 us; 509 x 2,048 x 5,632 1,195 -> 90 us; 17 x 2,048 x 2,048 210 -> 28 us.  Chunks of 32 in a deeper ring were slower
+// (550 us at 2,048 tokens): the way from a full accumulator to an empty one costs about 2 us, so what counts is the work per accumulator and their number.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "tcgen05_common.cuh"
+
+typedef __nv_bfloat16 bf16;
+
+#define SP_THREADS 320            // a producer warp, an MMA warp, eight warps that add up
+#define SP_BK 64
+#define SP_MAX_STAGES 3
+#define SP_MAX_ACCS 4
+#define SP_A_PLANE 16384u         // 128 rows of w x 64 x 2 bytes
+
+struct SpParams {
+    float* out; int64_t out_stride;              // [M][out_stride], the first column that of w's first row here
+    const void* bias; int bias_tag;
+    float* partial;                              // [splits][M][N] when splits > 1
+    const float* x; const float* w;              // the operands themselves (an output that is not finite)
+    int M, N, K, k_tiles, splits, k_per_split;
+    int tiles_m, num_items, stages, blocks_w, blocks_x;      // tiles_m: tiles of tokens; blocks: of 128 rows of w, of BN / 2 tokens
+    int* error;
+};
+
+__device__ __forceinline__ void sp_tma_load(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sp_mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void sp_commit(uint64_t* bar) {       // arrives on this barrier in both blocks of the pair
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void sp_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void sp_ld32(uint32_t addr, float* v) {
+    uint32_t r[32];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+                   "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ bool is_finite_f32(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
+// one chain of fused multiply-adds over K, for an output that the parts could not give
+__device__ __noinline__ float sp_chain(const float* __restrict__ x, const float* __restrict__ w, int K) {
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) acc = fmaf(x[k], w[k], acc);
+    return acc;
+}
+
+// --------------------------------------------------------------------------- split
+
+// The top 8 bits of the significand (sign and exponent with them) and what is left; a number that is not finite has no rest.
+__device__ __forceinline__ void cut3(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
+    const uint32_t u = __float_as_uint(v);
+    a = u & 0xffff0000u;
+    if ((u & 0x7f800000u) == 0x7f800000u) { a = (u & 0x007fffffu) ? 0x7fc00000u : a; b = 0u; c = 0u; return; }
+    const float r = v - __uint_as_float(a);                 // exact
+    b = __float_as_uint(r) & 0xffff0000u;
+    c = __float_as_uint(r - __uint_as_float(b));            // exact, at most 8 bits: its lower half is zero
+}
+
+// src [rows, K] -> dst [Kp / 64][row blocks][3 planes][block rows][64]: what one stage of the product reads of one block of rows is one stretch
+// of memory.  A warp takes 4 rows x 64 numbers of K (a thread eight numbers): it reads 256 bytes of a row and writes 512 in a row three times.
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ src, bf16* __restrict__ dst, int rows, int K, int chunks, int block,
+                                                    int row_blocks, bool vec_ok) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, r_in = lane >> 3, piece = lane & 7;
+    const int64_t items = (int64_t)((rows + 3) >> 2) * chunks, step = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += step) {
+        const int g = (int)(it / chunks), kc = (int)(it - (int64_t)g * chunks), row = g * 4 + r_in, k = kc * SP_BK + piece * 8;
+        if (row >= rows) continue;                            // (rows that pad a block hold whatever was there: they feed outputs that are not stored)
+        const float* p = src + (int64_t)row * K + k;
+        float v[8];
+        if (vec_ok && k + 8 <= K) {
+            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+            *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = k + i < K ? p[i] : 0.f;
+        }
+        uint32_t o[3][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t a0, b0, c0, a1, b1, c1;
+            cut3(v[2 * i], a0, b0, c0);
+            cut3(v[2 * i + 1], a1, b1, c1);
+            o[0][i] = (a0 >> 16) | a1; o[1][i] = (b0 >> 16) | b1; o[2][i] = (c0 >> 16) | (c1 & 0xffff0000u);
+        }
+        const int rb = row / block;
+        bf16* d = dst + ((((int64_t)kc * row_blocks + rb) * 3) * block + (row - rb * block)) * SP_BK + piece * 8;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(d + (int64_t)j * block * SP_BK) = make_uint4(o[j][0], o[j][1], o[j][2], o[j][3]);
+    }
+}
+
+// --------------------------------------------------------------------------- product
+
+template <int BN>
+__global__ void __launch_bounds__(SP_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SpParams p) {
+    constexpr int BNH = BN / 2;                                   // tokens a block loads; tokens a thread adds up
+    constexpr uint32_t B_PLANE = BNH * 128u, STAGE = 3 * SP_A_PLANE + 3 * B_PLANE;
+    constexpr int ACCS = 512 / BN < SP_MAX_ACCS ? 512 / BN : SP_MAX_ACCS, TMEM_COLS = ACCS * BN;
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ __align__(8) uint64_t full[SP_MAX_STAGES], empty[SP_MAX_STAGES], acc_full[SP_MAX_ACCS], acc_empty[SP_MAX_ACCS];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+
+    const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int S = p.stages;
+    volatile int* abort_p = &abort_flag;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < SP_MAX_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < SP_MAX_ACCS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }     // eight warps of two blocks
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_slot;
+    pdl_wait();
+
+    // item -> (tile of w, tile of tokens, share of K); tokens fastest, so that the pairs of a wave share panels of w
+    const int tiles = p.num_items / p.splits;
+    if (warp == 0) {
+        int s = 0;
+        uint32_t round = 0;
+        const uint32_t bar0 = cluster_addr(smem_u32(&full[0]), 0);
+        bool ok = true;
+        for (int item = pair; item < p.num_items && ok; item += pairs) {
+            const int tile = item % tiles, k_lo = (item / tiles) * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
+            const int block_w = (tile / p.tiles_m) * 2 + (int)rank, block_x = (tile % p.tiles_m) * 2 + (int)rank;
+            for (int kt = k_lo; kt < k_hi; ++kt) {
+                if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[s], (round - 1) & 1, abort_p))) { ok = false; break; }
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE);
+                    const uint32_t bar = bar0 + (uint32_t)s * 8u, dst = base + (uint32_t)s * STAGE;
+                    const int at_w = (kt * p.blocks_w + block_w) * 384, at_x = (kt * p.blocks_x + block_x) * 3 * BNH;
+                    sp_tma_load(dst, &map_w, bar, 0, at_w);
+                    sp_tma_load(dst + 192 * 128, &map_w, bar, 0, at_w + 192);
+                    sp_tma_load(dst + 3 * SP_A_PLANE, &map_x, bar, 0, at_x);
+                    if constexpr (BN == 256) sp_tma_load(dst + 3 * SP_A_PLANE + 192 * 128, &map_x, bar, 0, at_x + 192);
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ++round; }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const uint32_t idesc = umma_idesc_bf16(256, BN);
+            int s = 0;
+            uint32_t round = 0, chunk = 0;
+            bool ok = true;
+            for (int item = pair; item < p.num_items && ok; item += pairs) {
+                const int k_lo = (item / tiles) * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
+                for (int kt = k_lo; kt < k_hi; ++kt, ++chunk) {
+                    const uint32_t buf = chunk % ACCS, use = chunk / ACCS;
+                    if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use - 1) & 1, abort_p))) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], round & 1, abort_p))) { ok = false; break; }
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t at = base + (uint32_t)s * STAGE;
+                        const uint64_t da = umma_desc_sw128(at), db = umma_desc_sw128(at + 3 * SP_A_PLANE);
+                        const uint32_t d_at = tmem_base + buf * (uint32_t)BN;
+                        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};       // the parts' products, small ones first
+#pragma unroll
+                        for (int t = 0; t < 6; ++t)
+#pragma unroll
+                            for (int ks = 0; ks < SP_BK / 16; ++ks)
+                                sp_mma(d_at, da + (uint64_t)(PA[t] * (SP_A_PLANE >> 4) + ks * 2), db + (uint64_t)(PB[t] * (B_PLANE >> 4) + ks * 2),
+                                       idesc, t > 0 || ks > 0);
+                        sp_commit(&empty[s]);
+                        sp_commit(&acc_full[buf]);
+                    }
+                    __syncwarp();
+                    if (++s == S) { s = 0; ++round; }
+                }
+            }
+        }
+    } else {
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * BNH);
+        const uint32_t acc_empty_leader = cluster_addr(smem_u32(&acc_empty[0]), 0);
+        uint32_t chunk = 0;
+        bool ok = true;
+        for (int item = pair; item < p.num_items && ok; item += pairs) {
+            const int tile = item % tiles, split = item / tiles, k_lo = split * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
+            float acc[BNH];
+#pragma unroll
+            for (int i = 0; i < BNH; ++i) acc[i] = 0.f;
+            for (int kt = k_lo; kt < k_hi; ++kt, ++chunk) {
+                const uint32_t buf = chunk % ACCS, use = chunk / ACCS;
+                if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, abort_p))) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < BNH; c += 32) {
+                    float v[32];
+                    sp_ld32(lane_addr + buf * (uint32_t)BN + (uint32_t)c, v);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) acc[c + i] += v[i];
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) sp_arrive_cluster(acc_empty_leader + buf * 8u);
+            }
+            if (!ok) break;
+            const int n = (tile / p.tiles_m) * 256 + (int)rank * 128 + q * 32 + lane, m0 = (tile % p.tiles_m) * BN + half * BNH;
+            if (n < p.N) {
+                if (p.splits > 1) {
+                    float* o = p.partial + ((int64_t)split * p.M + m0) * p.N + n;
+#pragma unroll
+                    for (int i = 0; i < BNH; ++i) if (m0 + i < p.M) o[(int64_t)i * p.N] = acc[i];
+                } else {
+                    const float b = p.bias ? load_tagged(p.bias, n, p.bias_tag) : 0.f;
+                    float* o = p.out + (int64_t)m0 * p.out_stride + n;
+                    bool fine = true;
+#pragma unroll
+                    for (int i = 0; i < BNH; ++i) {
+                        fine = fine && (m0 + i >= p.M || is_finite_f32(acc[i]));
+                        if (m0 + i < p.M) o[(int64_t)i * p.out_stride] = acc[i] + b;
+                    }
+                    if (!fine)                                     // (looked for again in what was stored: the sums stay in registers)
+                        for (int i = 0; i < BNH && m0 + i < p.M; ++i)
+                            if (!is_finite_f32(o[(int64_t)i * p.out_stride]))
+                                o[(int64_t)i * p.out_stride] = sp_chain(p.x + (int64_t)(m0 + i) * p.K, p.w + (int64_t)n * p.K, p.K) + b;
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (abort_flag) {
+        if (threadIdx.x == 0) atomicExch(p.error, 1);
+        for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    }
+    cluster_sync_all();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+}
+
+// The shares of K added up in order (a thread four columns where N allows).
+template <int V>
+__global__ void __launch_bounds__(256) split_sum_kernel(const SpParams p) {
+    pdl_enter();
+    const int64_t groups = (int64_t)p.M * (p.N / V), per = (int64_t)p.M * p.N;
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= groups) return;
+    const int m = (int)(g / (p.N / V)), n = (int)(g - (int64_t)m * (p.N / V)) * V;
+    const float* src = p.partial + (int64_t)m * p.N + n;
+    float v[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = 0.f;
+    for (int s = 0; s < p.splits; ++s) {
+        float u[V];
+        if constexpr (V == 4) *reinterpret_cast<float4*>(u) = __ldcg(reinterpret_cast<const float4*>(src + s * per));
+        else u[0] = __ldcg(src + s * per);
+#pragma unroll
+        for (int i = 0; i < V; ++i) v[i] += u[i];
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        if (!is_finite_f32(v[i])) v[i] = sp_chain(p.x + (int64_t)m * p.K, p.w + (int64_t)(n + i) * p.K, p.K);
+        if (p.bias) v[i] += load_tagged(p.bias, n + i, p.bias_tag);
+        p.out[(int64_t)m * p.out_stride + n + i] = v[i];
+    }
+}
+
+// --------------------------------------------------------------------------- host side
+
+static int sp_map(CUtensorMap* map, const void* ptr, int64_t rows, int box_rows) {
+    cuuint64_t gdim[2] = {SP_BK, (cuuint64_t)rows};
+    cuuint64_t gstride[1] = {SP_BK * 2};
+    cuuint32_t box[2] = {SP_BK, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
+}
+
+// src [rows, K] float32 -> dst: see split_kernel.  `block` rows a block (a multiple of 8); dst holds ceil(K / 64) * `row_blocks` * 3 * block * 64 numbers, 16-byte
+// aligned, and row_blocks * block >= rows.
+extern "C" int mie_split3(const float* src, void* dst, int rows, int K, int block, int row_blocks, cudaStream_t stream) {
+    if (rows <= 0 || K <= 0) return 0;
+    if (block < 8 || block % 8 || (int64_t)row_blocks * block < rows || (reinterpret_cast<uintptr_t>(dst) & 15)) return MIE_ERR_BAD_ARG;
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && K % 4 == 0;
+    const int chunks = (K + SP_BK - 1) / SP_BK;
+    const int64_t blocks = ((int64_t)((rows + 3) / 4) * chunks + 7) / 8, most = (int64_t)device_sm_count() * 16;
+    return launch_kernel(split_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, stream, src, (bf16*)dst, rows, K, chunks, block, row_blocks, vec);
+}
+
+template <int BN>
+static int sp_launch(const CUtensorMap& mw, const CUtensorMap& mx, SpParams& p, cudaStream_t stream) {
+    constexpr int STAGE = 3 * (int)SP_A_PLANE + 3 * (BN / 2) * 128;
+    p.stages = 226 * 1024 / STAGE < SP_MAX_STAGES ? 226 * 1024 / STAGE : SP_MAX_STAGES;
+    const int smem = p.stages * STAGE + 1024;
+    const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    int pairs = device_sm_count() / 2;
+    if (pairs > p.num_items) pairs = p.num_items;
+    return launch_kernel_cluster(gemm_split_kernel<BN>, dim3(2 * pairs), dim3(SP_THREADS), smem, stream, dim3(2, 1, 1), mw, mx, p);
+}
+
+// y (columns of a matrix with `y_stride` columns) from the planes xs (blocks of bn / 2 rows) and ws (blocks of 128 rows), both an even number of blocks, of
+// x [M, K], w [N, K] float32 row-major.  bn 64, 128 or 256 tokens a tile; splits shares of K (1: no partial); partial [splits][M][N] float32.
+extern "C" int mie_gemm_split(const void* xs, const void* ws, const float* x, const float* w, const void* bias, int bias_tag, float* y,
+                              long long y_stride, float* partial, int M, int N, int K, int bn, int splits, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    const int chunks = (K + SP_BK - 1) / SP_BK, blocks_w = (N + 255) / 256 * 2, blocks_x = bn > 0 ? (M + bn - 1) / bn * 2 : 0;
+    if (K <= 0 || (bn != 64 && bn != 128 && bn != 256) || splits < 1 || splits > chunks || (splits > 1 && !partial)) return MIE_ERR_BAD_ARG;
+    if (((reinterpret_cast<uintptr_t>(xs) | reinterpret_cast<uintptr_t>(ws)) & 127) || (reinterpret_cast<uintptr_t>(partial) & 15)) return MIE_ERR_BAD_ARG;
+    const int64_t rows_w = (int64_t)chunks * blocks_w * 384, rows_x = (int64_t)chunks * blocks_x * 3 * (bn / 2);
+    if (rows_w > 0x7fffffff || rows_x > 0x7fffffff) return MIE_ERR_TOO_LARGE;
+    int rc = tc_setup();
+    if (rc) return rc;
+    CUtensorMap mw, mx;
+    if ((rc = sp_map(&mw, ws, rows_w, 192))) return rc;
+    if ((rc = sp_map(&mx, xs, rows_x, bn == 64 ? 96 : 192))) return rc;
+    SpParams p{};
+    p.out = y; p.out_stride = y_stride; p.bias = bias; p.bias_tag = bias_tag; p.partial = partial; p.x = x; p.w = w;
+    p.M = M; p.N = N; p.K = K; p.k_tiles = chunks; p.blocks_w = blocks_w; p.blocks_x = blocks_x; p.error = g_error_dev;
+    p.k_per_split = (p.k_tiles + splits - 1) / splits;
+    p.splits = (p.k_tiles + p.k_per_split - 1) / p.k_per_split;       // no empty share
+    p.tiles_m = (M + bn - 1) / bn;
+    p.num_items = p.tiles_m * ((N + 255) / 256) * p.splits;
+    rc = bn == 64 ? sp_launch<64>(mw, mx, p, stream) : bn == 128 ? sp_launch<128>(mw, mx, p, stream) : sp_launch<256>(mw, mx, p, stream);
+    if (rc || p.splits == 1) return rc;
+    if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3((unsigned)(((int64_t)M * (N / 4) + 255) / 256)), dim3(256), 0, stream, p);
+    return launch_kernel(split_sum_kernel<1>, dim3((unsigned)(((int64_t)M * N + 255) / 256)), dim3(256), 0, stream, p);
+}
+
+extern "C" int mie_gemm_split_error(void) { return g_error_host ? *g_error_host : 0; }
+extern "C" void mie_gemm_split_clear_error(void) { if (g_error_host) *g_error_host = 0; }

@@ -1,0 +1,90 @@
+"""The float32 product on the tensor cores (``csrc/gemm_split_tc.cu``): which sizes it takes, its plan and its launches.
+
+Both operands are split into three bfloat16 planes in scratch memory, in slabs, so that the scratch is bounded whatever the weight's size."""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from . import build, ops
+from .device import num_sms
+
+MIN_TOKENS = 9                        # Device time against the CUDA-core product, L2 flushed, B200, tokens x outputs x K: 8 x 11,264 x 2,048 82 against 75 us (the
+MIN_K = 128                           # row-streaming kernel reads w once for up to eight tokens), 9 x 2,048 x 2,048 27 : 39, 16 x 11,264 x 2,048 82 : 118,
+MIN_WEIGHT = 1 << 14                  # 17 x 2,048 x 2,048 28 : 214, 509 x 11,264 x 2,048 165 : 1,008, 509 x 2,048 x 5,632 90 : 1,195, 1,000 x 2,560 x 2,048 84 : 517,
+                                      # 2,048 x 11,264 x 2,048 415 : 2,707; small matrices: 64 x 256 x 256 15 : 32, 2,000 x 128 x 128 16 : 40,
+                                      # 64 x 2,048 x 128 15 : 18, 2,000 x 64 x 64 15 : 12 (three launches instead of one)
+W_SLAB_BYTES = 144 << 20              # planes of the weight rows that are in scratch at a time (a slab of 23 M numbers: one
+                                      # gate|up matrix of 2 x 5,632 x 2,048 in one go)
+X_SLAB_BYTES = 48 << 20
+PARTIAL_BYTES = 48 << 20
+
+
+def takes(M: int, N: int, K: int) -> bool:
+    return M >= MIN_TOKENS and K >= MIN_K and N * K >= MIN_WEIGHT
+
+
+def plan(M: int, N: int, K: int) -> tuple:
+    """(tokens a tile, shares of K): the pair with the least estimated time, in cycles.  Measured: a 64-wide chunk of K takes a pair of SMs
+    1,900, 2,250 or 3,850 cycles with 64, 128 or 256 tokens (the 24 MMAs alone 770, 1,540, 3,070: with 256 tokens only two accumulators fit
+    tensor memory, and the way from a full one to an empty one is as long as the MMAs); an item's start and end 3,000; shares of K write and
+    read M x N partial sums each at some 2,500 bytes a cycle, in a launch more."""
+    pairs = max(1, num_sms() // 2)
+    chunks = -(-K // 64)
+    best = None
+    for bn, cycles in ((256, 3850), (128, 2250), (64, 1900)):
+        tiles = -(-M // bn) * -(-N // 256)
+        for splits in (1, 2, 3, 4, 5, 6, 8):
+            if splits > max(1, chunks // 4) or (splits > 1 and splits * M * N * 4 > PARTIAL_BYTES):
+                continue
+            per = -(-chunks // splits)
+            rounds = -(-tiles * splits // pairs)
+            t = rounds * (per * cycles + 3000) + (splits * M * N * 8 / 2500 + 4000 if splits > 1 else 0)
+            if best is None or t < best[0]:
+                best = (t, bn, splits)
+    return best[1], best[2]
+
+
+def _split(lib, t: torch.Tensor, block: int) -> torch.Tensor:
+    """The planes of ``t`` in blocks of ``block`` rows, an even number of them (a pair of SMs takes two)."""
+    rows, K = t.shape
+    blocks = -(-rows // (2 * block)) * 2
+    planes = torch.empty(-(-K // 64) * blocks * 3 * block * 64, dtype=torch.bfloat16, device=t.device)
+    ops._check(lib.mie_split3(ops._ptr(t), ops._ptr(planes), rows, K, block, blocks, ops._stream()), "split3")
+    return planes
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None, force: tuple | None = None) -> torch.Tensor:
+    """out[M, N] = x[M, K] @ w[N, K]^T (+ bias), all float32 and contiguous, at the precision of float32 products."""
+    (M, K), N = x.shape, w.shape[0]
+    ops._need(x.dtype == w.dtype == out.dtype == torch.float32, "the split product takes float32 operands and leaves float32")
+    ops._need(w.shape[1] == K and tuple(out.shape) == (M, N), f"gemm shapes: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    ops._need(x.is_contiguous() and w.is_contiguous() and out.is_contiguous(), "gemm operands must be contiguous")
+    lib = ops.load("gemm_split_tc")
+    Kp = -(-K // 64) * 64
+    w_rows = max(256, W_SLAB_BYTES // (6 * Kp) // 256 * 256)
+    x_rows = max(256, X_SLAB_BYTES // (6 * Kp) // 256 * 256)
+    bn, splits = force or plan(min(M, x_rows), min(N, w_rows), K)
+    xs = _split(lib, x, bn // 2) if M <= x_rows else None
+    for n0 in range(0, N, w_rows):
+        wn = w[n0:n0 + w_rows]
+        ws = _split(lib, wn, 128)
+        for m0 in range(0, M, x_rows):
+            xm = x[m0:m0 + x_rows]
+            xm_planes = xs if xs is not None else _split(lib, xm, bn // 2)
+            m, n = xm.shape[0], wn.shape[0]
+            partial = torch.empty(splits, m, n, dtype=torch.float32, device=x.device) if splits > 1 else None
+            b = bias[n0:n0 + n] if bias is not None else None
+            ops._check(lib.mie_gemm_split(ops._ptr(xm_planes), ops._ptr(ws), ops._ptr(xm), ops._ptr(wn), ops._ptr(b),
+                                          ops.tag(b) if b is not None else 0, ops._ptr(out[m0:m0 + m, n0:n0 + n]), ctypes.c_longlong(N),
+                                          ops._ptr(partial), m, n, K, bn, splits, ops._stream()), f"gemm_split M{m} N{n} K{K}")
+    return out
+
+
+def check_error() -> None:
+    """Raises if a block gave up a bounded wait (call after a synchronise)."""
+    lib = build._libs.get("gemm_split_tc")
+    if lib is not None and lib.mie_gemm_split_error():
+        lib.mie_gemm_split_clear_error()
+        raise ops.KernelError("a block of the float32 tensor-core product gave up waiting on a barrier; its output is not valid")

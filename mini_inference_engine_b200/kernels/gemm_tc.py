@@ -436,6 +436,8 @@ def gemm_pair(x, w: torch.Tensor, out: torch.Tensor | None, bias: torch.Tensor |
 
 def check_error() -> None:
     """Raises if a block of an earlier launch gave up a bounded wait (call after a synchronise)."""
+    from . import gemm_split
+    gemm_split.check_error()
     lib = build._libs.get("gemm_pair_tc")
     if lib is not None and lib.mie_gemm_pair_error():
         lib.mie_gemm_pair_clear_error()

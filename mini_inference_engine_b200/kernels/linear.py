@@ -1,7 +1,8 @@
 """The matrix product y = x W^T (+ b) of every projection, by operand type.
 
-* float32 activations (the true 32-bit mode), or a weight the checkpoint holds in 32 bits:
-  the CUDA-core FMA kernel of ``csrc/gemm_simt.cu``.
+* float32 activations (the true 32-bit mode), or a weight the checkpoint holds in 32 bits: the CUDA-core FMA kernel of
+  ``csrc/gemm_simt.cu``; from nine tokens on, where both are float32, the product on the tensor cores with operands
+  split into three bfloat16 parts (``csrc/gemm_split_tc.cu``), whose error against 64 bits is the smaller one.
 * bfloat16 activations and weights: a tensor-core product.  The reference calls the vendor library
   for these (F.linear, inference_engine/model.py:172,178,180,181,185).  ``auto`` (the default) uses
   this package's tcgen05 kernel (``csrc/gemm_tcgen05.cu``) where it is the faster one -- few tokens,
@@ -14,7 +15,7 @@ from __future__ import annotations
 
 import torch
 
-from . import gemm_tc, ops
+from . import gemm_split, gemm_tc, ops
 
 _bf16_backend = "auto"
 AUTO_MAX_TOKENS = 32          # up to this many tokens ``auto`` takes the tcgen05 kernel.  Whole decode step, TinyLlama-1.1B
@@ -118,6 +119,8 @@ def linear(x, w: torch.Tensor, bias, out_dtype: torch.dtype) -> torch.Tensor:
     if isinstance(x, gemm_tc.DeferredNorm):          # only handed out where splits_k_on_tcgen05 said yes
         return gemm_tc.gemm(x, w, out, bias)
     if x.dtype == torch.float32 or w.dtype == torch.float32 or _bf16_backend == "simt":
+        if x.dtype == w.dtype == out_dtype == torch.float32 and x.is_cuda and gemm_split.takes(M, N, x.shape[1]):
+            return gemm_split.gemm_split(x, w, out, bias)
         return ops.gemm_simt(x, w, out, bias)
     if uses_tcgen05(x, w, out_dtype) and gemm_tc.supports(x, w, out):
         return gemm_tc.gemm(x, w, out, bias)

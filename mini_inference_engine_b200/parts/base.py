@@ -153,7 +153,7 @@ class StreamUpdated:
 
 class Runtime:
     """Device, activation type and the matrix product for that type.  ``float32`` runs every
-    product on CUDA cores in true 32-bit; ``bfloat16`` uses the tensor-core product for 16-bit
+    product at the precision of true 32-bit; ``bfloat16`` uses the tensor-core product for 16-bit
     weights and the CUDA-core one for a matrix that the checkpoint holds in 32 bits."""
 
     def __init__(self, device, dtype: torch.dtype):
@@ -182,7 +182,7 @@ class Runtime:
     def product_sources(self, *weights) -> set:
         """The kernel sources behind ``linear`` for these weights."""
         if self.dtype == torch.float32 or any(w is not None and w.dtype == torch.float32 for w in weights):
-            return {"gemm_simt"} if self.dtype == torch.float32 else {"gemm_simt"} | self._tc_sources()
+            return {"gemm_simt", "gemm_split_tc"} if self.dtype == torch.float32 else {"gemm_simt"} | self._tc_sources()
         return self._tc_sources()
 
     @staticmethod
