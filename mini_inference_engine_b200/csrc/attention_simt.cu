@@ -53,7 +53,7 @@ paged_attention_kernel(const T* __restrict__ q, int64_t q_stride, const T* __res
                        const int* __restrict__ row_q_len, const int* __restrict__ row_ctx_len,
                        int num_rows, TO* __restrict__ out, int num_heads, int num_kv_heads,
                        int head_dim, int page_size, int page_shift, float scale, int window,
-                       int keep, int QT, int HG, int min_q_len, int64_t num_pages, int* report, const ScoreMods mods) {
+                       int keep, int QT, int HG, int min_q_len, int below, int64_t num_pages, int* report, const ScoreMods mods) {
     extern __shared__ __align__(16) float smem[];
     __shared__ int s_row, s_q0;
     const int D = head_dim, DP = head_dim + 4;
@@ -66,7 +66,7 @@ paged_attention_kernel(const T* __restrict__ q, int64_t q_stride, const T* __res
     if (threadIdx.x < 32) {
         int tile, tiles;
         const int found = warp_find_row(row_q_len, num_rows, (int)blockIdx.x,
-                                        [&](int ql) { return ql >= min_q_len ? (ql + QT - 1) / QT : 0; },   // shorter rows belong to another kernel
+                                        [&](int ql) { return ql >= min_q_len && ql < below ? (ql + QT - 1) / QT : 0; },   // other rows belong to another kernel
                                         tile, tiles);
         if (threadIdx.x == 0) { s_row = found; s_q0 = tile * QT; }
     }
@@ -177,14 +177,14 @@ static size_t att_smem_bytes(int head_dim) {
     return sizeof(float) * ((size_t)ATT_WARPS * head_dim + 2 * (size_t)ATT_KEYS * (head_dim + 4));
 }
 
-// Rows with fewer than `min_q_len` new tokens are skipped (another kernel serves them).
+// Rows with fewer than `min_q_len` new tokens, or `below` and more, are skipped (another kernel serves them).
 // q: [num_tokens, ...] with `q_stride` elements between tokens and heads packed [H, D] at the row
 // start; out: [num_tokens, H, D] contiguous; caches: [pages, H_kv, page_size, D].
 extern "C" int mie_paged_attention(const void* q, int64_t q_stride, const void* k_cache, const void* v_cache,
                                    const int* block_tables, int table_stride, const int* row_q_start,
                                    const int* row_q_len, const int* row_ctx_len, int num_rows,
                                    int num_tokens, void* out, int act_tag, int num_heads, int num_kv_heads,
-                                   int head_dim, int page_size, float scale, int window, int keep, int min_q_len,
+                                   int head_dim, int page_size, float scale, int window, int keep, int min_q_len, int below,
                                    long long num_pages, int out_f32, float softcap, const float* sink, const float* dist_bias,
                                    int dist_len, const float* slope, cudaStream_t stream) {
     if (num_rows <= 0 || num_tokens <= 0) return 0;
@@ -208,21 +208,21 @@ extern "C" int mie_paged_attention(const void* q, int64_t q_stride, const void* 
         return launch_kernel(paged_attention_kernel<float, float>, grid, dim3(ATT_WARPS * 32), smem, stream,
             (const float*)q, q_stride, (const float*)k_cache, (const float*)v_cache, block_tables, table_stride,
             row_q_start, row_q_len, row_ctx_len, num_rows, (float*)out, num_heads, num_kv_heads, head_dim,
-            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, (int64_t)num_pages, g_range_report, mods);
+            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, below, (int64_t)num_pages, g_range_report, mods);
     } else if (act_tag == MIE_BF16 && out_f32) {             // bfloat16 operands, the output left in float32
         e = cudaFuncSetAttribute(paged_attention_kernel<bf16, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         return launch_kernel(paged_attention_kernel<bf16, float>, grid, dim3(ATT_WARPS * 32), smem, stream,
             (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, table_stride,
             row_q_start, row_q_len, row_ctx_len, num_rows, (float*)out, num_heads, num_kv_heads, head_dim,
-            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, (int64_t)num_pages, g_range_report, mods);
+            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, below, (int64_t)num_pages, g_range_report, mods);
     } else if (act_tag == MIE_BF16) {
         e = cudaFuncSetAttribute(paged_attention_kernel<bf16, bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         return launch_kernel(paged_attention_kernel<bf16, bf16>, grid, dim3(ATT_WARPS * 32), smem, stream,
             (const bf16*)q, q_stride, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, table_stride,
             row_q_start, row_q_len, row_ctx_len, num_rows, (bf16*)out, num_heads, num_kv_heads, head_dim,
-            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, (int64_t)num_pages, g_range_report, mods);
+            page_size, page_shift, scale, window, keep, QT, HG, min_q_len, below, (int64_t)num_pages, g_range_report, mods);
     }
     return MIE_ERR_BAD_ARG;
 }

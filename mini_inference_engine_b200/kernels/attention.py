@@ -1,6 +1,7 @@
 """Chooses the attention kernels for a step.
 
-float32 (the true 32-bit path): the CUDA-core kernel serves every row.
+float32 (the true 32-bit path): two CUDA-core kernels, one for rows with many new tokens and heads of up to 128
+(``csrc/attention_f32.cu``), one for the rest.
 bfloat16: rows with one new token go to the tensor-core decode kernel (context split across
 blocks), rows with more go to a prefill kernel -- the tcgen05 one for head sizes 64 and 128, the
 mma.sync one for the other multiples of 16 up to 128; head sizes beyond those kernels fall back to
@@ -57,6 +58,23 @@ def rotates_in_decode(dtype, head_dim: int, ctx) -> bool:
             and decode_only(ctx))
 
 
+F32_MIN_PAIRS = 16          # a row with fewer pairs would leave three quarters of a 64-pair tile empty; the other kernel gives each of its pairs a warp
+
+
+def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size, scale, window, mods, keep):
+    """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles of 64 pairs, shorter ones one pair a warp.  Where the host does
+    not know the rows' lengths (a captured step) each of the two kernels takes the rows that are its own."""
+    min_q_len = max(2, -(-F32_MIN_PAIRS // (num_heads // num_kv_heads)))
+    q_lens = ctx.host.get("q_len")
+    long = None if q_lens is None else [n for n in q_lens if n >= min_q_len]
+    sizes = (ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, page_size, scale, window)
+    if long is None or len(long) < len(q_lens):
+        ops.paged_attention(*args, *sizes, mods=mods, keep=keep, below=min_q_len)
+    if long is None or long:
+        ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)))
+    return out
+
+
 def attention(qkv, ctx, cache, out, num_heads, num_kv_heads, head_dim, scale, window, rope=None, q_stride=None, mods=None,
               keep: int = 0):
     """``rope`` = (cos, sin): ``qkv`` is unrotated and the cache rows of the new tokens are unwritten; only
@@ -82,6 +100,8 @@ def attention(qkv, ctx, cache, out, num_heads, num_kv_heads, head_dim, scale, wi
                              "in steps of 32 up to 128)")
         return ops.decode_attention(*args, out, num_heads, num_kv_heads, head_dim, cache.page_size, scale, window,
                                     max_ctx=ctx.max_ctx_len, rope=rope)
+    if not fast and _backend == "auto" and ops.attention_f32_takes(qkv, cache.k, cache.v, out, head_dim):
+        return _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, cache.page_size, scale, window, mods, keep)
     if not fast:
         return ops.paged_attention(*args, ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, cache.page_size,
                                    scale, window, mods=mods, keep=keep)

@@ -402,10 +402,10 @@ _NO_MODS = ScoreMods()
 def paged_attention(q: torch.Tensor, q_stride: int, k_cache, v_cache, block_tables, row_q_start, row_q_len,
                     row_ctx_len, num_tokens: int, out: torch.Tensor, num_heads: int, num_kv_heads: int,
                     head_dim: int, page_size: int, scale: float, window: int | None = None,
-                    min_q_len: int = 1, mods: ScoreMods | None = None, keep: int = 0) -> torch.Tensor:
+                    min_q_len: int = 1, mods: ScoreMods | None = None, keep: int = 0, below: int = 1 << 30) -> torch.Tensor:
     """Causal attention of every new token over its request's pages (CUDA-core kernel, float32 or
     bfloat16).  ``q`` holds [H, D] at the start of each token row of ``q_stride`` elements.  Rows
-    with fewer than ``min_q_len`` new tokens are left alone.  ``keep``: with a window, the first that many keys stay in sight too."""
+    with fewer than ``min_q_len`` new tokens, or with ``below`` and more, are left alone.  ``keep``: with a window, the first that many keys stay in sight too."""
     _need(head_dim % 16 == 0 and 16 <= head_dim <= 256,
           f"head_dim {head_dim}: this kernel takes multiples of 16 from 16 to 256")
     _need(num_heads % num_kv_heads == 0, "query heads must be a multiple of kv heads")
@@ -421,10 +421,36 @@ def paged_attention(q: torch.Tensor, q_stride: int, k_cache, v_cache, block_tabl
                                    _ptr(block_tables), block_tables.shape[1], _ptr(row_q_start), _ptr(row_q_len),
                                    _ptr(row_ctx_len), rows, num_tokens, _ptr(out), tag(q), num_heads,
                                    num_kv_heads, head_dim, page_size, ctypes.c_float(scale),
-                                   int(window or 0), int(keep), int(min_q_len), ctypes.c_longlong(k_cache.shape[0]),
+                                   int(window or 0), int(keep), int(min_q_len), int(below), ctypes.c_longlong(k_cache.shape[0]),
                                    int(out.dtype == torch.float32 and q.dtype != torch.float32), *(mods or _NO_MODS).args(num_heads),
                                    _stream()),
            "paged_attention")
+    return out
+
+
+def attention_f32_takes(q, k_cache, v_cache, out, head_dim: int) -> bool:
+    """Whether ``attention_f32`` serves these operands (everything float32, heads of up to 128, 16-byte rows of the caches and the output)."""
+    return (q.dtype == k_cache.dtype == v_cache.dtype == out.dtype == torch.float32 and head_dim % 16 == 0 and 16 <= head_dim <= 128
+            and all(t.data_ptr() % 16 == 0 for t in (k_cache, v_cache, out)))
+
+
+def attention_f32(q: torch.Tensor, q_stride: int, k_cache, v_cache, block_tables, row_q_start, row_q_len, row_ctx_len, num_tokens: int,
+                  out: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, scale: float, window: int | None = None,
+                  min_q_len: int = 1, mods: ScoreMods | None = None, keep: int = 0, work=None) -> torch.Tensor:
+    """``paged_attention`` in float32 for rows with ``min_q_len`` new tokens or more: 64 (token, head) pairs a block.  ``work`` = (rows, tokens):
+    how many such rows there are and their tokens in sum, where the caller knows."""
+    _need(attention_f32_takes(q, k_cache, v_cache, out, head_dim), "attention_f32: float32 operands with 16-byte rows, heads of 16 to 128 in steps of 16")
+    _need(num_heads % num_kv_heads == 0, "query heads must be a multiple of kv heads")
+    for t, n in ((block_tables, "block_tables"), (row_q_start, "row_q_start"), (row_q_len, "row_q_len"), (row_ctx_len, "row_ctx_len")):
+        _i32(t, n)
+    _need(out.is_contiguous(), "attention output must be contiguous")
+    rows, tokens = work if work is not None else (row_q_len.numel(), num_tokens)
+    tiles = tokens * (num_heads // num_kv_heads) // 64 + rows               # every row's last tile may be partly filled
+    lib = load("attention_f32")
+    _check(lib.mie_attention_f32(_ptr(q), ctypes.c_int64(q_stride), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), block_tables.shape[1],
+                                 _ptr(row_q_start), _ptr(row_q_len), _ptr(row_ctx_len), row_q_len.numel(), tiles, _ptr(out), num_heads, num_kv_heads,
+                                 head_dim, page_size, ctypes.c_float(scale), int(window or 0), int(keep), int(min_q_len),
+                                 ctypes.c_longlong(k_cache.shape[0]), *(mods or _NO_MODS).args(num_heads), _stream()), "attention_f32")
     return out
 
 

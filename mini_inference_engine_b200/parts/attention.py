@@ -66,7 +66,7 @@ class Attention(Mixer):
         import torch as _torch
         names = self.rt.product_sources(self.w_qkv, self.w_o) | self.position.kernel_sources()
         if self.rt.dtype == _torch.float32 or self.head_dim > 128:
-            names.add("attention_simt")
+            names |= {"attention_simt"} | ({"attention_f32"} if self.rt.dtype == _torch.float32 and self.head_dim <= 128 else set())
         if self.rt.dtype != _torch.float32 and self.head_dim <= 128:
             names |= {"attention_decode", "attention_prefill_tc" if self.head_dim in (64, 128) else "attention_prefill"}
         return names
@@ -275,7 +275,7 @@ def _padded_rows(parts, multiple: int = 8):
 
 def _attention_sources(rt, padded: int, keep: int = 0) -> set:
     if rt.dtype == torch.float32 or padded > 128:
-        return {"attention_simt"}
+        return {"attention_simt"} | ({"attention_f32"} if rt.dtype == torch.float32 and padded <= 128 else set())
     return {"attention_decode_kept" if keep else "attention_decode", "attention_prefill_tc" if padded in (64, 128) else "attention_prefill"}
 
 
