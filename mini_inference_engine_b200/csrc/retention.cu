@@ -10,7 +10,8 @@
 // are computed once and serve all heads.  The state lives in `state[slot, h, c, d]` (value column c, key dimension
 // d: transposed, so that the threads that share a column read neighbouring words).
 //
-// A request's new tokens are cut into chunks of RET_L.  The recurrence is linear in S, so a chunk's effect on the
+// Rows of more than RET_L new tokens with key sizes of up to 128 in steps of 4 go to decay_chunk.cu (chunks as matrix products); what follows serves
+// the others.  A request's new tokens are cut into chunks of RET_L.  The recurrence is linear in S, so a chunk's effect on the
 // state is (gamma^len, the state it builds from zero), and the chunks of a long portion run side by side:
 //   pass 0   every chunk j but the last of a row of two or more: the state it builds from zero     -> scratch[j + 1]
 //   combine  per such row, in order: scratch[0] = the request's state, scratch[j + 1] += gamma^RET_L * scratch[j]
@@ -34,7 +35,22 @@
 
 // `act` 1: q and k pass silu first (a linear attention over activated projections).  `q_scale` multiplies q; `k_tok`
 // (optional, [T, H] float32) is one more factor on a token's key per head (a write gate folded into the key).
-template <typename T>
+// VEC entries go together (4 where sizes and alignment allow, else 1): a thread takes VEC entries of a head or, where they rotate, VEC pairs;
+// entries are read before the token's cosines are there.  2,048 tokens of 8 heads of 128: 34 us one entry a thread, 12 us four.
+template <typename T, int VEC> __device__ __forceinline__ void load_vec(const T* p, float* v) {
+    if constexpr (VEC == 1) v[0] = to_f32<T>(*p);
+    else if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+    else {
+        const uint2 u = *reinterpret_cast<const uint2*>(p);
+        v[0] = __uint_as_float(u.x << 16); v[1] = __uint_as_float(u.x & 0xffff0000u);
+        v[2] = __uint_as_float(u.y << 16); v[3] = __uint_as_float(u.y & 0xffff0000u);
+    }
+}
+template <int VEC> __device__ __forceinline__ void store_vec(float* p, const float* v) {
+    if constexpr (VEC == 1) *p = v[0];
+    else *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(v);
+}
+template <typename T, int VEC>
 __global__ void retention_prepare_kernel(const T* __restrict__ qkv, int64_t stride, const int* __restrict__ positions,
                                          const float* __restrict__ freq, float k_scale, float* __restrict__ qr,
                                          float* __restrict__ kr, int H, int D, int rot, int act, float q_scale,
@@ -42,33 +58,59 @@ __global__ void retention_prepare_kernel(const T* __restrict__ qkv, int64_t stri
     extern __shared__ float cs[];                 // cos [rot/2], sin [rot/2]
     pdl_enter();
     const int t = blockIdx.x, half = rot >> 1;
-    const float pos = (float)positions[t];
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        const float a = pos * freq[i];
-        cs[i] = cosf(a);
-        cs[half + i] = sinf(a);
-    }
-    __syncthreads();
     const T* src = qkv + (int64_t)t * stride;
-    for (int i = threadIdx.x; i < H * D; i += blockDim.x) {
-        const int d = i % D;
-        float qo = to_f32<T>(src[i]), ko = to_f32<T>(src[H * D + i]);
-        if (act) { qo = qo / (1.0f + expf(-qo)); ko = ko / (1.0f + expf(-ko)); }
-        if (d < rot) {
-            const int j = d < half ? d : d - half;
-            const int pi = d < half ? i + half : i - half;
-            const float c = cs[j], sn = cs[half + j];
-            const float qp = to_f32<T>(src[pi]), kp = to_f32<T>(src[H * D + pi]);
-            qo = d < half ? qo * c - qp * sn : qo * c + qp * sn;
-            ko = d < half ? ko * c - kp * sn : ko * c + kp * sn;
+    // a head's work: half / VEC pairs of pieces, then (D - rot) / VEC pieces
+    const int pairs = half / VEC, pieces = pairs + (D - rot) / VEC, items = 2 * H * pieces;       // (q's, then k's)
+    int i = threadIdx.x;
+    float a[VEC], b[VEC];
+    auto place = [&](int it, int& h, int& d, bool& key) {
+        key = it >= H * pieces;
+        const int j = key ? it - H * pieces : it;
+        h = j / pieces;
+        const int p = j - h * pieces;
+        d = p < pairs ? p * VEC : rot + (p - pairs) * VEC;
+    };
+    auto fetch = [&](int it) {
+        int h, d; bool key;
+        place(it, h, d, key);
+        const T* p = src + (key ? H * D : 0) + h * D + d;
+        load_vec<T, VEC>(p, a);
+        if (d < half) load_vec<T, VEC>(p + half, b);
+    };
+    if (i < items) fetch(i);
+    if (half) {
+        const float pos = (float)positions[t];
+        for (int j = threadIdx.x; j < half; j += blockDim.x) {
+            const float x = pos * freq[j];
+            cs[j] = cosf(x);
+            cs[half + j] = sinf(x);
         }
-        qr[(int64_t)t * H * D + i] = qo * q_scale;
-        kr[(int64_t)t * H * D + i] = ko * (k_tok ? k_scale * k_tok[(int64_t)t * H + i / D] : k_scale);
+        __syncthreads();
+    }
+    for (; i < items;) {
+        int h, d; bool key;
+        place(i, h, d, key);
+        const float scale = key ? (k_tok ? k_scale * k_tok[(int64_t)t * H + h] : k_scale) : q_scale;
+        float* to = (key ? kr : qr) + ((int64_t)t * H + h) * D + d;
+        float o[VEC], o2[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            if (act) a[e] = a[e] / (1.0f + expf(-a[e]));
+            if (d < half) {
+                const float c = cs[d + e], sn = cs[half + d + e];
+                o[e] = (a[e] * c - b[e] * sn) * scale;
+                o2[e] = (b[e] * c + a[e] * sn) * scale;
+            } else o[e] = a[e] * scale;
+        }
+        store_vec<VEC>(to, o);
+        if (d < half) store_vec<VEC>(to + half, o2);
+        i += blockDim.x;
+        if (i < items) fetch(i);
     }
 }
 
 // Which (row, chunk) has number `index`, counting every row's chunks (numbering 1: max(1, ceil(len / RET_L)) a row) or
-// only the chunks of rows that have two or more (numbering 0: these have a scratch slot each).  Returns the row (-1: none), the chunk within the row, the row's
+// only the chunks of rows that have two or more (numbering 0: these have a scratch slot each) or only rows of one (numbering 2).  Returns the row (-1: none), the chunk within the row, the row's
 // count in that numbering, and how many chunks of numbering 0 lie in front of the row.  Asked by whole warps.
 __device__ __forceinline__ int find_chunk(const int* __restrict__ row_q_len, int num_rows, int index, int numbering,
                                           int& within, int& items, int& before0) {
@@ -78,7 +120,7 @@ __device__ __forceinline__ int find_chunk(const int* __restrict__ row_q_len, int
         const int r = base + lane;
         const int n1 = r < num_rows ? max(1, (row_q_len[r] + RET_L - 1) / RET_L) : 0;
         const int n0 = n1 > 1 ? n1 : 0;
-        const int n = numbering ? n1 : n0;
+        const int n = numbering == 2 ? (n1 == 1 ? 1 : 0) : numbering ? n1 : n0;
         int incl = n, incl0 = n0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -107,7 +149,7 @@ __global__ void retention_chunk_kernel(const float* __restrict__ qr, const float
                                        const float* __restrict__ decay, float* __restrict__ state,
                                        float* __restrict__ scratch, float* __restrict__ out, int num_rows, int H, int D, int Dv,
                                        int CW, int slices, const float* __restrict__ tok_decay, float* __restrict__ chunk_decay,
-                                       int Dv_in, int v_act) {
+                                       int Dv_in, int v_act, int numbering) {
     // `tok_decay` (optional, [T, H]): the decay of every token instead of one per head; pass 0 then leaves the product of
     // a chunk's decays in `chunk_decay` for the combine.  `Dv_in` < Dv: v has Dv_in columns a head and the state's column
     // Dv_in is fed with ones (the sum of the keys under the same decays: a normalizer).  `v_act`: v passes silu.
@@ -119,7 +161,7 @@ __global__ void retention_chunk_kernel(const float* __restrict__ qr, const float
     float* a_s = v_s + RET_TT * CW;          // [RET_TT] the tokens' decays
     pdl_enter();
     int within, items, before0;
-    const int r = find_chunk(row_q_len, num_rows, (int)blockIdx.y, PASS, within, items, before0);
+    const int r = find_chunk(row_q_len, num_rows, (int)blockIdx.y, numbering, within, items, before0);
     if (r < 0 || (PASS == 0 && within == items - 1)) return;          // nobody needs what a row's last chunk builds from zero
     const int h = blockIdx.x / slices, slice = blockIdx.x - h * slices;
     const int q_len = row_q_len[r], q_start = row_q_start[r];
@@ -290,15 +332,17 @@ __global__ void head_rms_gate_kernel(const float* __restrict__ o, const T* __res
 // The general entry.  `rows_in` holds [ q: H x D | k: H x D | v: H x Dv_in | ... ] per token.  `act`: q, k and v pass silu
 // (no rotation then).  `tok_decay` / `k_tok` (optional, float32 [T, H]): a decay and a factor on the key per token and head,
 // in place of `decay` [H].  `ones`: the state and the output have one more column per head, Dv_in + 1 in all, fed with ones.
+// `kinds` 0: every row; 1: q and k of all rows are prepared, and the rows of one chunk are run (decay_chunk.cu runs the others); 2: q and k are
+// prepared and nothing else.
 // state [slots, H, Dv, D], out [T, H, Dv] with Dv = Dv_in + ones; `chunk_decay`: scratch of (scratch_chunks + 1) * H floats.
 extern "C" int mie_decay_scan(const void* qkv, int tag, long long stride, const int* positions, const int* row_q_start,
                               const int* row_q_len, const int* state_slots, const float* decay, const float* freq,
                               float q_scale, float k_scale, const float* tok_decay, const float* k_tok, int act, int ones,
                               float* state, float* qr, float* kr, float* scratch, long long scratch_chunks, float* chunk_decay,
-                              float* out, int num_tokens, int num_rows, int max_q_len, int H, int D, int Dv_in, int rot,
+                              float* out, int num_tokens, int num_rows, int max_q_len, int H, int D, int Dv_in, int rot, int kinds,
                               cudaStream_t stream) {
     if (num_rows <= 0 || num_tokens <= 0) return 0;
-    if (H <= 0 || D <= 0 || Dv_in <= 0 || rot < 0 || rot > D || (rot & 1) || (act && rot) || (!decay && !tok_decay) || ones < 0 || ones > 1)
+    if (kinds < 0 || kinds > 2 || H <= 0 || D <= 0 || Dv_in <= 0 || rot < 0 || rot > D || (rot & 1) || (act && rot) || (!decay && !tok_decay) || ones < 0 || ones > 1)
         return MIE_ERR_BAD_ARG;
     const int Dv = Dv_in + ones;
     int P = 1;
@@ -323,25 +367,29 @@ extern "C" int mie_decay_scan(const void* qkv, int tag, long long stride, const 
     const Cut cut0 = cut(Dv >= 2 * (256 / P) ? 2 : 1), cut1 = cut(1);
     // chunks the step can have at most: every row one, and one more per RET_L tokens; those of rows with two or more
     // (such a row has more than RET_L tokens): two per RET_L tokens
-    const int chunks1 = num_rows + num_tokens / RET_L, chunks0 = max_q_len > RET_L ? 2 * (num_tokens / RET_L) : 0;
+    const int chunks1 = kinds ? num_rows : num_rows + num_tokens / RET_L, chunks0 = kinds == 0 && max_q_len > RET_L ? 2 * (num_tokens / RET_L) : 0;
     if (chunks0 > scratch_chunks) return MIE_ERR_BAD_ARG;
     if (chunks0 > 0 && tok_decay && !chunk_decay) return MIE_ERR_BAD_ARG;
     float* cdec = tok_decay ? chunk_decay : nullptr;
     const int prep_threads = H * D >= 1024 ? 256 : 128;
+    const size_t quad = tag == MIE_F32 ? 16 : 8;
+    const bool vec4 = D % 4 == 0 && rot % 8 == 0 && reinterpret_cast<uintptr_t>(qkv) % quad == 0 && stride % 4 == 0 &&
+                      ((reinterpret_cast<uintptr_t>(qr) | reinterpret_cast<uintptr_t>(kr)) & 15) == 0;
     int rc;
 #define RET_PASS(T, PASS, PP, ny)                                                                                             \
     ((PASS == 0 && cut0.NC == 2) ? RET_PASS_N(T, 0, PP, 2, ny, cut0) : RET_PASS_N(T, PASS, PP, 1, ny, (PASS == 0 ? cut0 : cut1)))
 #define RET_PASS_N(T, PASS, PP, NN, ny, CUT)                                                                                  \
     launch_kernel(retention_chunk_kernel<T, PASS, PP, NN>, dim3(H * CUT.slices, ny), dim3(CUT.threads), CUT.smem, stream, qr, \
                   kr, (const T*)qkv + 2 * H * D, (int64_t)stride, row_q_start, row_q_len, state_slots, decay, state, scratch, \
-                  out, num_rows, H, D, Dv, CUT.CW, CUT.slices, tok_decay, cdec, Dv_in, act)
+                  out, num_rows, H, D, Dv, CUT.CW, CUT.slices, tok_decay, cdec, Dv_in, act, PASS == 0 ? 0 : kinds == 0 ? 1 : 2)
 #define RET_PASS_P(T, PASS, ny)                                                                                               \
     (P == 1 ? RET_PASS(T, PASS, 1, ny) : P == 2 ? RET_PASS(T, PASS, 2, ny) : P == 4 ? RET_PASS(T, PASS, 4, ny)                \
      : P == 8 ? RET_PASS(T, PASS, 8, ny) : P == 16 ? RET_PASS(T, PASS, 16, ny) : RET_PASS(T, PASS, 32, ny))
 #define RET_LAUNCH(T)                                                                                                         \
-    rc = launch_kernel(retention_prepare_kernel<T>, dim3(num_tokens), dim3(prep_threads), (size_t)rot * sizeof(float), stream, \
-                       (const T*)qkv, (int64_t)stride, positions, freq, k_scale, qr, kr, H, D, rot, act, q_scale, k_tok);     \
-    if (rc) return rc;                                                                                                        \
+    rc = launch_kernel(vec4 ? retention_prepare_kernel<T, 4> : retention_prepare_kernel<T, 1>, dim3(num_tokens), dim3(prep_threads), \
+                       (size_t)rot * sizeof(float), stream, (const T*)qkv, (int64_t)stride, positions, freq, k_scale, qr, kr, H, D,  \
+                       rot, act, q_scale, k_tok);                                                                             \
+    if (rc || kinds == 2) return rc;                                                                                          \
     if (chunks0 > 0) {                                                                                                        \
         rc = RET_PASS_P(T, 0, chunks0);                                                                                       \
         if (rc) return rc;                                                                                                    \
@@ -357,16 +405,6 @@ extern "C" int mie_decay_scan(const void* qkv, int tag, long long stride, const 
 #undef RET_PASS
 #undef RET_PASS_N
     return MIE_ERR_BAD_ARG;
-}
-
-extern "C" int mie_retention_scan(const void* qkv, int tag, long long stride, const int* positions, const int* row_q_start,
-                                  const int* row_q_len, const int* state_slots, const float* decay, const float* freq,
-                                  float k_scale, float* state, float* qr, float* kr, float* scratch, long long scratch_chunks,
-                                  float* out, int num_tokens, int num_rows, int max_q_len, int H, int D, int Dv, int rot,
-                                  cudaStream_t stream) {
-    return mie_decay_scan(qkv, tag, stride, positions, row_q_start, row_q_len, state_slots, decay, freq, 1.0f, k_scale, nullptr, nullptr,
-                          0, 0, state, qr, kr, scratch, scratch_chunks, nullptr, out, num_tokens, num_rows, max_q_len, H, D, Dv, rot,
-                          stream);
 }
 
 extern "C" int mie_retention_chunk_tokens() { return RET_L; }

@@ -35,7 +35,7 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--shared", "-Xcompiler", "-fP
 SOURCES = ("embedding", "norm", "rope_cache", "attention_simt", "attention_f32", "attention_decode", "attention_decode_kept", "attention_decode_static", "attention_prefill",
            "attention_prefill_tc",
            "activation", "gemm_simt", "gemm_split_tc", "gemm_tcgen05", "gemm_chain", "gemm_pair_tc",
-           "sampling", "norm_group", "qk_norm_rope", "retention", "linear_recurrence",
+           "sampling", "norm_group", "qk_norm_rope", "retention", "decay_chunk", "linear_recurrence",
            "hyper_norm", "latent_kv", "diff_attention", "delta_rule", "delta_chunk", "delta_head", "moe", "stream_update", "layer_norm", "sandwich_norm")
 
 _libs: dict[str, ctypes.CDLL] = {}

@@ -893,11 +893,11 @@ def turn_heads(attn: torch.Tensor, positions, freq: torch.Tensor, out: torch.Ten
 # --------------------------------------------------------------------------- retention
 
 def retention_scan(qkv: torch.Tensor, positions, row_q_start, row_q_len, state_slots, decay, freq, state, out, *,
-                   num_heads: int, dim: int, vdim: int, rot: int, k_scale: float, max_q_len: int) -> torch.Tensor:
+                   num_heads: int, dim: int, vdim: int, rot: int, k_scale: float, max_q_len: int, q_lens=None) -> torch.Tensor:
     """S <- decay_h S + k v^T, o = S^T q for every new token of every row, from and to ``state`` [slots, H, vdim, dim]
     float32; q and k are rotated (angle = position x ``freq``) and k scaled first.  ``qkv`` rows hold
     [q: H x dim | k: H x dim | v: H x vdim | ...]; ``out`` [T, H * vdim] float32.  Rows longer than a chunk are cut
-    into chunks that run side by side (``max_q_len``: the longest row the launch may meet)."""
+    into chunks (``max_q_len``: the longest row the launch may meet; ``q_lens``: all rows' lengths, where the host knows them)."""
     T = qkv.shape[0]
     _need(qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.shape[1] >= num_heads * (2 * dim + vdim), "qkv rows must hold q, k and v")
     _need(state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (num_heads, vdim, dim),
@@ -908,21 +908,55 @@ def retention_scan(qkv: torch.Tensor, positions, row_q_start, row_q_len, state_s
     for t, n in ((positions, "positions"), (row_q_start, "row_q_start"), (row_q_len, "row_q_len"), (state_slots, "state_slots")):
         _i32(t, n)
     _need(positions.numel() == T, "one position per token")
+    return _decay_rows(qkv, positions, row_q_start, row_q_len, state_slots, state, out, num_heads, dim, vdim, vdim, max_q_len, decay, None, None, False,
+                       1.0, k_scale, freq, rot, q_lens)
+
+
+DECAY_CHUNK_TOKENS = 64        # rows of more new tokens than this go in chunks as matrix products
+
+
+def decay_chunks_take(dim: int) -> bool:
+    return dim % 4 == 0 and dim <= 128
+
+
+def _decay_rows(rows_in, positions, row_q_start, row_q_len, state_slots, state, out, H, D, vdim, dv, max_q_len, decay, tok_decay, k_tok, act, q_scale,
+                k_scale, freq, rot, q_lens):
+    """The recurrence behind ``retention_scan`` and ``decay_scan``: rows of up to 64 new tokens token by token, longer ones in chunks as matrix
+    products (token by token in chunks side by side where the key size is beyond those kernels).  ``q_lens``: the rows' lengths where the host
+    knows them (a captured step does not: then both run, each on the rows that are its own)."""
+    T, rows = rows_in.shape[0], row_q_len.numel()
     lib = load("retention")
-    chunk = lib.mie_retention_chunk_tokens()
-    chunks = 2 * (T // chunk) if max_q_len > chunk else 0
-    scratch = _workspace(qkv.device, "retention_chunks", chunks * num_heads * vdim * dim, torch.float32) if chunks else None
-    qr = torch.empty(2, T, num_heads * dim, dtype=torch.float32, device=qkv.device)
-    _check(lib.mie_retention_scan(_ptr(qkv), tag(qkv), ctypes.c_longlong(qkv.stride(0)), _ptr(positions), _ptr(row_q_start),
-                                  _ptr(row_q_len), _ptr(state_slots), _ptr(decay), _ptr(freq), ctypes.c_float(k_scale),
-                                  _ptr(state), _ptr(qr[0]), _ptr(qr[1]), _ptr(scratch), ctypes.c_longlong(chunks), _ptr(out), T,
-                                  row_q_len.numel(), int(max_q_len), num_heads, dim, vdim, rot, _stream()), "retention_scan")
+    chunk = DECAY_CHUNK_TOKENS
+    chunked = max_q_len > chunk and decay_chunks_take(D)
+    long = [n for n in q_lens if n > chunk] if q_lens is not None else None
+    kinds = 0
+    chunks, scratch, cdec = 0, None, None
+    if chunked:
+        kinds = 2 if long is not None and len(long) == rows else 1
+    elif max_q_len > chunk:
+        chunks = 2 * (T // chunk)
+        scratch = _workspace(rows_in.device, "retention_chunks", chunks * H * dv * D, torch.float32)
+        cdec = _workspace(rows_in.device, "retention_chunk_decay", (chunks + 1) * H, torch.float32) if tok_decay is not None else None
+    qr = torch.empty(2, T, H * D, dtype=torch.float32, device=rows_in.device)
+    _check(lib.mie_decay_scan(_ptr(rows_in), tag(rows_in), ctypes.c_longlong(rows_in.stride(0)), _ptr(positions), _ptr(row_q_start),
+                              _ptr(row_q_len), _ptr(state_slots), _ptr(decay), _ptr(freq), ctypes.c_float(q_scale), ctypes.c_float(k_scale),
+                              _ptr(tok_decay), _ptr(k_tok), int(act), int(dv > vdim), _ptr(state), _ptr(qr[0]), _ptr(qr[1]), _ptr(scratch),
+                              ctypes.c_longlong(chunks), _ptr(cdec), _ptr(out), T, rows, int(max_q_len), H, D, vdim, rot, kinds, _stream()), "decay_scan")
+    if chunked:
+        dc = load("decay_chunk")
+        chunks = sum(-(-n // chunk) for n in long) if long is not None else 2 * (T // chunk)     # (a row of two chunks has more than 64 tokens)
+        states = torch.empty(chunks * H * dv * D, dtype=torch.float32, device=rows_in.device)
+        work = torch.empty(chunks * H * dc.mie_decay_chunk_floats(), dtype=torch.float32, device=rows_in.device)
+        v = rows_in[:, 2 * H * D:]
+        _check(dc.mie_decay_chunks(_ptr(qr[0]), _ptr(qr[1]), _ptr(v), tag(v), ctypes.c_longlong(v.stride(0)), _ptr(row_q_start), _ptr(row_q_len),
+                                   _ptr(state_slots), rows, _ptr(decay), _ptr(tok_decay), _ptr(state), _ptr(states), _ptr(work), chunks, _ptr(out), H, D,
+                                   vdim, dv, int(act), _stream()), "decay_chunks")
     return out
 
 
 def decay_scan(rows_in: torch.Tensor, positions, row_q_start, row_q_len, state_slots, state, out, *, num_heads: int, dim: int, vdim: int,
                max_q_len: int, decay=None, tok_decay=None, k_tok=None, act: bool = False, ones: bool = False, q_scale: float = 1.0,
-               k_scale: float = 1.0, freq=None, rot: int = 0) -> torch.Tensor:
+               k_scale: float = 1.0, freq=None, rot: int = 0, q_lens=None) -> torch.Tensor:
     """The general form of ``retention_scan``: S <- a S + k v^T, o = S^T q per head with a = ``decay`` [H] or, per token,
     ``tok_decay`` [T, H]; ``k_tok`` [T, H] is one more factor on a token's key; ``act``: q, k and v pass silu (no rotation
     then); ``ones``: the state and the output have a column more per head, fed with ones instead of a value (the decayed sum
@@ -946,18 +980,8 @@ def decay_scan(rows_in: torch.Tensor, positions, row_q_start, row_q_len, state_s
     for t_, n in ((positions, "positions"), (row_q_start, "row_q_start"), (row_q_len, "row_q_len"), (state_slots, "state_slots")):
         _i32(t_, n)
     _need(positions.numel() == T, "one position per token")
-    lib = load("retention")
-    chunk = lib.mie_retention_chunk_tokens()
-    chunks = 2 * (T // chunk) if max_q_len > chunk else 0
-    scratch = _workspace(rows_in.device, "retention_chunks", chunks * num_heads * dv * dim, torch.float32) if chunks else None
-    cdec = _workspace(rows_in.device, "retention_chunk_decay", (chunks + 1) * num_heads, torch.float32) if chunks and tok_decay is not None else None
-    qr = torch.empty(2, T, num_heads * dim, dtype=torch.float32, device=rows_in.device)
-    _check(lib.mie_decay_scan(_ptr(rows_in), tag(rows_in), ctypes.c_longlong(rows_in.stride(0)), _ptr(positions), _ptr(row_q_start),
-                              _ptr(row_q_len), _ptr(state_slots), _ptr(decay), _ptr(freq), ctypes.c_float(q_scale), ctypes.c_float(k_scale),
-                              _ptr(tok_decay), _ptr(k_tok), int(act), int(ones), _ptr(state), _ptr(qr[0]), _ptr(qr[1]), _ptr(scratch),
-                              ctypes.c_longlong(chunks), _ptr(cdec), _ptr(out), T, row_q_len.numel(), int(max_q_len), num_heads, dim,
-                              vdim, rot, _stream()), "decay_scan")
-    return out
+    return _decay_rows(rows_in, positions, row_q_start, row_q_len, state_slots, state, out, num_heads, dim, vdim, dv, max_q_len, decay, tok_decay, k_tok,
+                       act, q_scale, k_scale, freq, rot, q_lens)
 
 
 def gate_scan(z: torch.Tensor, bias_i, bias_f, cap: float, row_q_start, row_q_len, state_slots, m_state: torch.Tensor, num_heads: int):

@@ -47,7 +47,7 @@ class MatrixMemory(Mixer):
         return (StateNeed((self.num_heads, self.vdim + 1, self.dim), torch.float32), StateNeed((self.num_heads,), torch.float32))
 
     def kernel_sources(self):
-        return {"retention"} | self.rt.product_sources(self.w_in, self.w_gates, self.w_o)
+        return {"retention", "decay_chunk"} | self.rt.product_sources(self.w_in, self.w_gates, self.w_o)
 
     def forward(self, x, ctx, cache):
         H, D, Dv, T = self.num_heads, self.dim, self.vdim, ctx.num_tokens
@@ -59,7 +59,7 @@ class MatrixMemory(Mixer):
         keep, write, m = ops.gate_scan(z, self.b_i, self.b_f, self.gate_cap, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, m_state, H)
         o = self.rt.empty(T, H * (Dv + 1), dtype=torch.float32)
         ops.decay_scan(proj, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o, num_heads=H, dim=D, vdim=Dv,
-                       max_q_len=ctx.max_q_len, tok_decay=keep, k_tok=write, ones=True, q_scale=D ** -0.5)
+                       max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), tok_decay=keep, k_tok=write, ones=True, q_scale=D ** -0.5)
         gated = self.rt.empty(T, H * Dv)
         at = 2 * H * D + H * Dv
         ops.group_norm_gate(o, proj[:, at:at + H * Dv], gated, groups=H, size=Dv, eps=self.eps, weight=self.norm, m=m)

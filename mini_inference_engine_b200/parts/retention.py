@@ -48,7 +48,7 @@ class Retention(Mixer):
         return StateNeed((self.num_heads, self.vdim, self.dim), torch.float32)
 
     def kernel_sources(self):
-        return {"retention"} | self.rt.product_sources(self.w_qkvg, self.w_o)
+        return {"retention", "decay_chunk"} | self.rt.product_sources(self.w_qkvg, self.w_o)
 
     def forward(self, x, ctx, cache):
         H, D, Dv = self.num_heads, self.dim, self.vdim
@@ -56,7 +56,7 @@ class Retention(Mixer):
         o = self.rt.empty(ctx.num_tokens, H * Dv, dtype=torch.float32)
         ops.retention_scan(qkvg, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, self.decay_t, self.freq,
                            cache.state, o, num_heads=H, dim=D, vdim=Dv, rot=self.rot_dims, k_scale=D ** -0.5,
-                           max_q_len=ctx.max_q_len)
+                           max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"))
         gated = self.rt.empty(ctx.num_tokens, H * Dv)
         ops.head_rms_gate(o, qkvg[:, 2 * H * D + H * Dv:], gated, H, Dv, self.eps)
         return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)
@@ -96,14 +96,14 @@ class LightningAttention(Mixer):
         return StateNeed((self.num_heads, self.vdim, self.dim), torch.float32)
 
     def kernel_sources(self):
-        return {"retention"} | self.rt.product_sources(self.w_qkvg, self.w_o)
+        return {"retention", "decay_chunk"} | self.rt.product_sources(self.w_qkvg, self.w_o)
 
     def forward(self, x, ctx, cache):
         H, D, Dv = self.num_heads, self.dim, self.vdim
         qkvg = self.rt.linear(x, self.w_qkvg)
         o = self.rt.empty(ctx.num_tokens, H * Dv, dtype=torch.float32)
         ops.decay_scan(qkvg, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, cache.state, o, num_heads=H, dim=D,
-                       vdim=Dv, max_q_len=ctx.max_q_len, decay=self.decay_t, act=True)
+                       vdim=Dv, max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), decay=self.decay_t, act=True)
         gated = self.rt.empty(ctx.num_tokens, H * Dv)
         at = 2 * H * D + H * Dv
         ops.group_norm_gate(o, qkvg[:, at:at + H * Dv], gated, groups=1, size=H * Dv, eps=self.eps, weight=self.norm)
