@@ -1,4 +1,4 @@
-// The gated delta rule with one decay per head over long portions, in chunks of 64 tokens (delta_rule.cu walks token by token).
+// The gated delta rule over long portions, in chunks of 64 tokens (delta_rule.cu walks token by token), with one decay per head or one per head and key channel.
 //
 // Within a chunk, with G_i the sum of the log decays up to token i, S the state in front of the chunk and
 //   A_ij = beta_i exp(G_i - G_j) (k_i . k_j)  for j < i,      P_ij = exp(G_i - G_j) (q_i . k_j)  for j <= i,
@@ -14,6 +14,11 @@
 //   chunk_scan   a block per (row, head, 16 value columns) walks the row's chunks: its slice of the state stays in registers (and in shared
 //                memory for the products that read it); keys and queries of the next chunk arrive by asynchronous copies while
 //                this one is computed.
+//
+// With a decay per channel G_i is a vector: e^{G_i} multiplies k_i and q_i, e^{G_C - G_i} the k_i that the state takes, and the entries of A and P are
+// sums over channels with a factor each.  channel_prep (a block per (chunk, head)) writes these keys and queries out, so the scan only reads other operands.  Between blocks of 16
+// tokens the factor e^{G_i - G_j} is e^{G_i - G_r} e^{G_r - G_j} with r the last token in front of i's block: two products of a matrix, no exponent
+// positive, whatever the decays; within a block it is the product of the tokens' own decays, carried from token to token.
 //
 // Rows with fewer than `min_len` new tokens are left to delta_rule.cu.  Chunks count from the start of a row's portion.
 #include "common.cuh"
@@ -36,10 +41,19 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
     return r;
 }
 __device__ __forceinline__ float sum2(unsigned long long v) { const float2 f = unpack2(v); return f.x + f.y; }
+template <bool B> struct Flag { static constexpr bool value = B; };
 struct Quad { unsigned long long lo, hi; };                    // four consecutive floats as two pairs
 __device__ __forceinline__ Quad quad(const float* p) {
     const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
     return Quad{v.x, v.y};
+}
+// entries m .. m + 3 of which only those up to r count: the others, whatever they are (a later token's may not be finite), become zero
+__device__ __forceinline__ Quad up_to(Quad b, int m, int r) {
+    if (m + 1 > r) b.lo &= 0xffffffffull;
+    if (m > r) b.lo = 0ull;
+    if (m + 3 > r) b.hi &= 0xffffffffull;
+    if (m + 2 > r) b.hi = 0ull;
+    return b;
 }
 // 16 (or 4) bytes from global to shared memory; zeros where `on` is false (nothing is read then)
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool on) {
@@ -71,7 +85,61 @@ struct ChunkScratch {           // per (chunk, head): T diag(beta) [64, 64], P [
     }
 };
 
+struct ChannelScratch {         // per (chunk, head): T diag(beta) [64, 64], P [64, 64], then rows of D: e^G k [64], e^G q [64], e^{G_C - G} k [64], e^{G_C} [1]
+    float* tb; float* p; float* kt; float* qt; float* ke; float* ec;
+    __device__ __forceinline__ ChannelScratch(float* base, int64_t item, int D) {
+        tb = base + item * (2 * CH * CH + (3 * CH + 1) * D);
+        p = tb + CH * CH;
+        kt = p + CH * CH;
+        qt = kt + CH * D;
+        ke = qt + CH * D;
+        ec = ke + CH * D;
+    }
+};
+
 __device__ __forceinline__ int chunks_of(int n, int min_len) { return n >= min_len ? (n + CH - 1) / CH : 0; }
+
+// T = (I + A)^-1 for A [64][CHP] with entries below the diagonal only, by the whole block (a barrier in front and behind); X: 3 x 256 floats.
+__device__ __forceinline__ void unit_triangular_inverse(const float* A, float* T, float* X) {
+    // diagonal blocks: a column of the inverse a thread, by substitution, in registers
+    if (threadIdx.x < 64) {
+        float t[16];
+        const int db = (threadIdx.x >> 4) * 16, dc = threadIdx.x & 15;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float v = i == dc ? 1.f : 0.f;
+#pragma unroll
+            for (int m = 0; m < i; ++m) v = fmaf(-A[(db + i) * CHP + db + m], t[m], v);
+            t[i] = v;
+            T[(db + i) * CHP + db + dc] = v;
+        }
+    }
+    __syncthreads();
+    // the blocks below: T_ij = -T_ii (sum over j <= m < i of A_im T_mj), one diagonal of blocks after the other
+    for (int w = 1; w < 4; ++w) {
+        const int n = (4 - w) * 256;                       // entries of the blocks (i, i - w)
+        for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+            const int bi = w + (idx >> 8), bj = bi - w, r = (idx >> 4) & 15, c = idx & 15;
+            float v = 0.f;
+            for (int mb = bj * 16; mb < bi * 16; mb += 16) {
+                float part = 0.f;
+#pragma unroll
+                for (int m = 0; m < 16; ++m) part = fmaf(A[(bi * 16 + r) * CHP + mb + m], T[(mb + m) * CHP + bj * 16 + c], part);
+                v += part;
+            }
+            X[idx] = v;
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+            const int bi = w + (idx >> 8), bj = bi - w, r = (idx >> 4) & 15, c = idx & 15;
+            float v = 0.f;
+#pragma unroll
+            for (int m = 0; m < 16; ++m) v = fmaf(T[(bi * 16 + r) * CHP + bi * 16 + m], X[(idx & ~255) + m * 16 + c], v);
+            T[(bi * 16 + r) * CHP + bj * 16 + c] = -v;
+        }
+        __syncthreads();
+    }
+}
 
 template <int DT>
 __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
@@ -162,44 +230,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* _
             A[i * CHP + j] = j < i ? be[i] * f * KK[i * CHP + j] : 0.f;
         }
         __syncthreads();
-        // diagonal blocks: a column of the inverse a thread, by substitution, in registers
-        if (threadIdx.x < 64) {
-            float t[16];
-            const int db = (threadIdx.x >> 4) * 16, dc = threadIdx.x & 15;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float v = i == dc ? 1.f : 0.f;
-#pragma unroll
-                for (int m = 0; m < i; ++m) v = fmaf(-A[(db + i) * CHP + db + m], t[m], v);
-                t[i] = v;
-                T[(db + i) * CHP + db + dc] = v;
-            }
-        }
-        __syncthreads();
-        // the blocks below: T_ij = -T_ii (sum over j <= m < i of A_im T_mj), one diagonal of blocks after the other
-        for (int w = 1; w < 4; ++w) {
-            const int n = (4 - w) * 256;                       // entries of the blocks (i, i - w)
-            for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
-                const int bi = w + (idx >> 8), bj = bi - w, r = (idx >> 4) & 15, c = idx & 15;
-                float v = 0.f;
-                for (int mb = bj * 16; mb < bi * 16; mb += 16) {
-                    float part = 0.f;
-#pragma unroll
-                    for (int m = 0; m < 16; ++m) part = fmaf(A[(bi * 16 + r) * CHP + mb + m], T[(mb + m) * CHP + bj * 16 + c], part);
-                    v += part;
-                }
-                X[idx] = v;
-            }
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
-                const int bi = w + (idx >> 8), bj = bi - w, r = (idx >> 4) & 15, c = idx & 15;
-                float v = 0.f;
-#pragma unroll
-                for (int m = 0; m < 16; ++m) v = fmaf(T[(bi * 16 + r) * CHP + bi * 16 + m], X[(idx & ~255) + m * 16 + c], v);
-                T[(bi * 16 + r) * CHP + bj * 16 + c] = -v;
-            }
-            __syncthreads();
-        }
+        unit_triangular_inverse(A, T, X);
         for (int idx = threadIdx.x; idx < CH * CH; idx += blockDim.x) {
             const int i = idx >> 6, j = idx & 63;
             out.tb[idx] = j <= i ? T[i * CHP + j] * be[j] : 0.f;
@@ -207,7 +238,204 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* _
     }
 }
 
+// The sums over the lanes of v[0 .. 31], one a lane: lane l gets that of v[l].
+__device__ __forceinline__ float transposed_sums(float (&v)[32], int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+#define CP_THREADS 512
+
+// 170 KB: one block of 16 warps on an SM.  1,500 tokens of 16 heads of 128: 136 us with a load of the decays in every step of the walk within a block, 75 us with
+// a block's decays read ahead and all columns of a row summed over the lanes at once.
 template <int DT>
+__global__ void __launch_bounds__(CP_THREADS) delta_channel_prep_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
+                                                                        const float* __restrict__ decay, const float* __restrict__ log_decay,
+                                                                        const int* __restrict__ row_q_start, const int* __restrict__ row_q_len, int num_rows,
+                                                                        int min_len, float* __restrict__ scratch, int H, int G, int D) {
+    constexpr int DP = DT + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* K = sm;                                             // [64][DP]; then e^(sum from the block's first token) k
+    float* Q = K + CH * DP;                                    // ... q
+    float* R = Q + CH * DP;                                    // log decays, then e^(sum from the next token to the block's last) k: no exponent is the difference of two larger ones
+    float* KK = R + CH * DP;                                   // [64][CHP]: A before beta
+    float* QK = KK + CH * CHP;                                 // P
+    float* tot = QK + CH * CHP;                                // [4][DT]: the log decays of whole blocks
+    float* Y = tot + 4 * DT;                                   // [4 quarters of the channels][KK, QK][64][16]: the blocks on the diagonal
+    float* A = KK;
+    float* T = K;                                              // (the keys and queries are not read after the products)
+    float* X = Q;
+    __shared__ float be[CH];
+    __shared__ int s_row, s_chunk;
+    pdl_enter();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        int within, items;
+        const int r = warp_find_row(row_q_len, num_rows, (int)blockIdx.x, [&](int n) { return chunks_of(n, min_len); }, within, items);
+        if (lane == 0) { s_row = r; s_chunk = within; }
+    }
+    __syncthreads();
+    if (s_row < 0) return;
+    const int h = blockIdx.y, g = h / (H / G);
+    const int t0 = row_q_start[s_row] + s_chunk * CH, count = min(CH, row_q_len[s_row] - s_chunk * CH);
+    copy_rows<DT>(K, kn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
+    copy_rows<DT>(Q, qn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
+    copy_rows<DT>(R, log_decay + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);       // (tokens beyond the row's end decay nothing and write nothing)
+    copy_commit();
+    if (threadIdx.x < CH) be[threadIdx.x] = threadIdx.x < count ? beta[(int64_t)(t0 + threadIdx.x) * H + h] : 0.f;
+    // within a block of 16 tokens: a warp a block and a quarter of the channels; the factor of every column is carried from row to row
+    constexpr int PER = DT / 128 > 0 ? DT / 128 : 1;           // (DT 64: half of the lanes have a channel)
+    const int blk = warp >> 2, d = ((warp & 3) * 32 + lane) * PER;
+    const bool on = d < DT && d < D;
+    float w[16];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) w[i] = on && 16 * blk + i < count ? decay[((int64_t)(t0 + 16 * blk + i) * H + h) * D + d] : 1.f;
+    copy_wait<0>();
+    __syncthreads();
+    {
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float k = on ? K[(16 * blk + i) * DP + d] : 0.f, q = on ? Q[(16 * blk + i) * DP + d] : 0.f;
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (j < i) f[j] *= w[i];
+                if (j == i) f[j] = k;
+                v[j] = j <= i ? k * f[j] : 0.f;
+                v[16 + j] = j <= i ? q * f[j] : 0.f;
+            }
+            const float sum = transposed_sums(v, lane);        // lane j: k_i . k_j, lane 16 + j: q_i . k_j over this warp's channels
+            Y[(((warp & 3) * 2 + (lane >> 4)) * CH + 16 * blk + i) * 16 + (lane & 15)] = sum;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * CH * CH; i += CP_THREADS) {
+        const int which = i >> 12, r = (i >> 6) & 63, c = i & 63;
+        const float* y = Y + (which * CH + r) * 16 + (c & 15);
+        (which ? QK : KK)[r * CHP + c] = (r >> 4) == (c >> 4) ? (y[0] + y[2 * CH * 16]) + (y[4 * CH * 16] + y[6 * CH * 16]) : 0.f;
+    }
+    // sums of log decays; keys and queries with their factors, into scratch memory and, for the products between blocks, in place
+    const ChannelScratch out(scratch, (int64_t)blockIdx.x * H + h, D);
+    for (int c = threadIdx.x; c < 4 * DT; c += CP_THREADS) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s += R[((c / DT) * 16 + i) * DP + c % DT];
+        tot[c] = s;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < 4 * DT; c += CP_THREADS) {
+        const int b = c / DT, e = c % DT;
+        if (e >= D) {
+            for (int i = 16 * b; i < 16 * b + 16; ++i) R[i * DP + e] = 0.f;
+            continue;
+        }
+        float before = 0.f, behind = 0.f, x[16], k[16];
+        for (int m = 0; m < b; ++m) before += tot[m * DT + e];
+        for (int m = b + 1; m < 4; ++m) behind += tot[m * DT + e];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { x[i] = R[(16 * b + i) * DP + e]; k[i] = K[(16 * b + i) * DP + e]; }
+        float run = 0.f;
+        const float all_behind = expf(behind), all_before = expf(before);
+#pragma unroll
+        for (int i = 15; i >= 0; --i) {
+            const int at = 16 * b + i;
+            const float back = expf(run);
+            R[at * DP + e] = k[i] * back;
+            out.ke[at * D + e] = k[i] * back * all_behind;
+            run += x[i];
+        }
+        run = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int at = 16 * b + i;
+            run += x[i];
+            const float fwd = expf(run), q = Q[at * DP + e];
+            K[at * DP + e] = k[i] * fwd;
+            Q[at * DP + e] = q * fwd;
+            out.kt[at * D + e] = k[i] * fwd * all_before;
+            out.qt[at * D + e] = q * fwd * all_before;
+            if (at == CH - 1) out.ec[e] = expf(before + run);
+        }
+    }
+    __syncthreads();
+    // between blocks: a warp a pair of blocks and half of the channels; the keys and the queries of block bi against the keys of block bj
+    float part[4][4];
+    const int pair = warp >> 1, bi = pair < 1 ? 1 : pair < 3 ? 2 : 3, bj = pair < 1 ? 0 : pair < 3 ? pair - 1 : pair - 3;
+    const int r = lane >> 2, c = lane & 3;
+    if (warp < 12) {
+        unsigned long long acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        const int d0 = (warp & 1) * (DT / 2);
+#pragma unroll 2
+        for (int dd = d0; dd < d0 + DT / 2; dd += 4) {
+            float4 m = make_float4(1.f, 1.f, 1.f, 1.f);        // the blocks between the two
+            if (bi - bj > 1) {
+                float4 s = *reinterpret_cast<const float4*>(tot + (bj + 1) * DT + dd);
+                if (bi - bj > 2) {
+                    const float4 t = *reinterpret_cast<const float4*>(tot + (bj + 2) * DT + dd);
+                    s = make_float4(s.x + t.x, s.y + t.y, s.z + t.z, s.w + t.w);
+                }
+                m = make_float4(expf(s.x), expf(s.y), expf(s.z), expf(s.w));
+            }
+            Quad a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float4 x = *reinterpret_cast<const float4*>((i < 2 ? K : Q) + (16 * bi + r + 8 * (i & 1)) * DP + dd);
+                a[i].lo = pack2(x.x * m.x, x.y * m.y);
+                a[i].hi = pack2(x.z * m.z, x.w * m.w);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const Quad y = quad(R + (16 * bj + c + 4 * j) * DP + dd);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { fma2(acc[i][j], a[i].lo, y.lo); fma2(acc[i][j], a[i].hi, y.hi); }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] = sum2(acc[i][j]);
+    }
+    for (int half = 0; half < 2; ++half) {
+        if (warp < 12 && (warp & 1) == half) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float* to = (i < 2 ? KK : QK) + (16 * bi + r + 8 * (i & 1)) * CHP + 16 * bj + c + 4 * j;
+                    *to = half ? *to + part[i][j] : part[i][j];
+                }
+        }
+        __syncthreads();
+    }
+    for (int idx = threadIdx.x; idx < CH * CH; idx += CP_THREADS) {
+        const int i = idx >> 6, j = idx & 63;
+        out.p[idx] = QK[i * CHP + j];
+        A[i * CHP + j] = j < i ? be[i] * KK[i * CHP + j] : 0.f;
+    }
+    __syncthreads();
+    unit_triangular_inverse(A, T, X);
+    for (int idx = threadIdx.x; idx < CH * CH; idx += CP_THREADS) {
+        const int i = idx >> 6, j = idx & 63;
+        out.tb[idx] = j <= i ? T[i * CHP + j] * be[j] : 0.f;
+    }
+}
+
+// CHANNEL: a decay per channel -- the operands come with their factors from channel_prep, and the keys that the state takes replace the others in
+// shared memory once the products with the state are done with those.
+template <int DT, bool CHANNEL>
 __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
                                                                const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
                                                                const int* __restrict__ state_slots, int min_len, const float* __restrict__ scratch,
@@ -260,15 +488,24 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
             float* st = KQ + (c & 1) * STAGE;
             const int64_t tf = t0 + c * CH;
             const int count = min(CH, n - c * CH);
-            copy_rows<DT>(st, kn + (tf * G + g) * D, (int64_t)G * D, D, count);
-            copy_rows<DT>(st + CH * DP, qn + (tf * G + g) * D, (int64_t)G * D, D, count);
+            if constexpr (CHANNEL) {
+                const ChannelScratch in(const_cast<float*>(scratch), (first + c) * H + h, D);
+                copy_rows<DT>(st, in.kt, D, D, CH);
+                copy_rows<DT>(st + CH * DP, in.qt, D, D, CH);
+            } else {
+                copy_rows<DT>(st, kn + (tf * G + g) * D, (int64_t)G * D, D, count);
+                copy_rows<DT>(st + CH * DP, qn + (tf * G + g) * D, (int64_t)G * D, D, count);
+            }
             float* v = st + 2 * CH * DP;
             for (int i = threadIdx.x; i < CH * COLS; i += 256) {
                 const int t = i >> 4, j = i & 15;
                 const bool on = t < count && j0 + j < Dv;
                 copy4(v + i, on ? vn + ((tf + t) * H + h) * Dv + j0 + j : vn, on);
             }
-            if (threadIdx.x < 32) {
+            if constexpr (CHANNEL) {
+                const float* ec = ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).ec;
+                if (threadIdx.x < DT / 4) copy16(v + CH * COLS + threadIdx.x * 4, threadIdx.x * 4 < D ? ec + threadIdx.x * 4 : ec, threadIdx.x * 4 < D);
+            } else if (threadIdx.x < 32) {
                 const float* eg = ChunkScratch(const_cast<float*>(scratch), (first + c) * H + h).eg;      // e^G and e^{G_C - G} lie side by side
                 copy16(v + CH * COLS + threadIdx.x * 4, eg + threadIdx.x * 4, true);
             }
@@ -276,11 +513,12 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
         copy_commit();
     };
     auto issue_squares = [&](int c) {
-        const ChunkScratch in(const_cast<float*>(scratch), (first + c) * H + h);
+        const float* tb = CHANNEL ? ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).tb
+                                  : ChunkScratch(const_cast<float*>(scratch), (first + c) * H + h).tb;
         for (int i = threadIdx.x; i < CH * CH / 4; i += 256) {
             const int r = i >> 4, m = (i & 15) * 4;
-            copy16(TB + r * CHP + m, in.tb + i * 4, true);
-            copy16(P + r * CHP + m, in.p + i * 4, true);
+            copy16(TB + r * CHP + m, tb + i * 4, true);
+            copy16(P + r * CHP + m, tb + CH * CH + i * 4, true);
         }
         copy_commit();
     };
@@ -294,8 +532,8 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
         copy_wait<0>();                                        // keys and queries of this chunk
         __syncthreads();                                       // ... of every thread; S of the chunk before; TB and P are free
         issue_squares(c);
-        issue_keys(c + 1);
-        const float* st = KQ + (c & 1) * STAGE;
+        if constexpr (!CHANNEL) issue_keys(c + 1);
+        float* st = KQ + (c & 1) * STAGE;
         const float* V = st + 2 * CH * DP;
         const float* eg = V + CH * COLS;
         const float* er = eg + CH;
@@ -318,7 +556,7 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = r1 + 4 * i;
-                const float e = eg[r];
+                const float e = CHANNEL ? 1.f : eg[r];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     o[i][k] = e * sum2(acc[i][k]);
@@ -326,46 +564,59 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
                 }
             }
         }
-        copy_wait<1>();                                        // TB and P of this chunk
+        if constexpr (CHANNEL) {
+            __syncthreads();                                   // the keys are done with: those that the state takes come in their place
+            copy_rows<DT>(st, ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).ke, D, D, CH);
+            copy_commit();
+            issue_keys(c + 1);
+            copy_wait<2>();
+        } else copy_wait<1>();                                 // TB and P of this chunk
         __syncthreads();
         {
             unsigned long long u[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
             const int end = rw * 8 + 8;                        // no row of the warp reads beyond its diagonal
-#pragma unroll 2
-            for (int m = 0; m < end; m += 4) {
+            auto add = [&](int m, auto diagonal) {
                 const Quad b0 = quad(R + c1 * CHP + m), b1 = quad(R + (c1 + 8) * CHP + m);
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const Quad a = quad(TB + (r2 + 4 * i) * CHP + m);
-                    fma2(u[i][0], a.lo, b0.lo); fma2(u[i][0], a.hi, b0.hi);
-                    fma2(u[i][1], a.lo, b1.lo); fma2(u[i][1], a.hi, b1.hi);
+                    const Quad x = diagonal.value ? up_to(b0, m, r2 + 4 * i) : b0, y = diagonal.value ? up_to(b1, m, r2 + 4 * i) : b1;
+                    fma2(u[i][0], a.lo, x.lo); fma2(u[i][0], a.hi, x.hi);
+                    fma2(u[i][1], a.lo, y.lo); fma2(u[i][1], a.hi, y.hi);
                 }
-            }
+            };
+#pragma unroll 2
+            for (int m = 0; m < end - 8; m += 4) add(m, Flag<false>{});
+            add(end - 8, Flag<true>{});
+            add(end - 4, Flag<true>{});
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int r = r2 + 4 * i;
-                const float e = er[r];
+                const float e = CHANNEL ? 1.f : er[r];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     const float v = sum2(u[i][k]);
                     U[(c1 + 8 * k) * CHP + r] = v;
-                    UE[(c1 + 8 * k) * CHP + r] = e * v;
+                    if constexpr (!CHANNEL) UE[(c1 + 8 * k) * CHP + r] = e * v;
                 }
             }
         }
+        if constexpr (CHANNEL) copy_wait<1>();                 // the keys that the state takes
         __syncthreads();
         if (half == 0) {
             // the state: its columns times the chunk's whole decay, plus keys times U
-            const float total = eg[CH - 1];
-            const unsigned long long tt = pack2(total, total);
+            unsigned long long t_lo, t_hi;
+            if constexpr (CHANNEL) { const Quad e = quad(eg + d4); t_lo = e.lo; t_hi = e.hi; }
+            else t_lo = t_hi = pack2(eg[CH - 1], eg[CH - 1]);
+            const float* taken = CHANNEL ? U : UE;
             unsigned long long n_lo[JT], n_hi[JT];
 #pragma unroll
-            for (int jj = 0; jj < JT; ++jj) { n_lo[jj] = n_hi[jj] = 0ull; fma2(n_lo[jj], s_lo[jj], tt); fma2(n_hi[jj], s_hi[jj], tt); }
+            for (int jj = 0; jj < JT; ++jj) { n_lo[jj] = n_hi[jj] = 0ull; fma2(n_lo[jj], s_lo[jj], t_lo); fma2(n_hi[jj], s_hi[jj], t_hi); }
 #pragma unroll 2
             for (int i = 0; i < CH; i += 4) {
                 float4 u[JT];
 #pragma unroll
-                for (int jj = 0; jj < JT; ++jj) u[jj] = *reinterpret_cast<const float4*>(UE + (jl + 4 * jj) * CHP + i);
+                for (int jj = 0; jj < JT; ++jj) u[jj] = *reinterpret_cast<const float4*>(taken + (jl + 4 * jj) * CHP + i);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const Quad key = quad(st + (i + k) * DP + d4);
@@ -389,16 +640,20 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
             const int end = (warp & 3) * 16 + 16;
-#pragma unroll 2
-            for (int m = 0; m < end; m += 4) {
+            auto add = [&](int m, auto diagonal) {
                 const Quad b0 = quad(U + c1 * CHP + m), b1 = quad(U + (c1 + 8) * CHP + m);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const Quad a = quad(P + (r1 + 4 * i) * CHP + m);
-                    fma2(acc[i][0], a.lo, b0.lo); fma2(acc[i][0], a.hi, b0.hi);
-                    fma2(acc[i][1], a.lo, b1.lo); fma2(acc[i][1], a.hi, b1.hi);
+                    const Quad x = diagonal.value ? up_to(b0, m, r1 + 4 * i) : b0, y = diagonal.value ? up_to(b1, m, r1 + 4 * i) : b1;
+                    fma2(acc[i][0], a.lo, x.lo); fma2(acc[i][0], a.hi, x.hi);
+                    fma2(acc[i][1], a.lo, y.lo); fma2(acc[i][1], a.hi, y.hi);
                 }
-            }
+            };
+#pragma unroll 2
+            for (int m = 0; m < end - 16; m += 4) add(m, Flag<false>{});
+#pragma unroll
+            for (int m = 16; m > 0; m -= 4) add(end - m, Flag<true>{});
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int t = c * CH + r1 + 4 * i;
@@ -422,37 +677,50 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
 }
 
 template <int DT>
-static int launch_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* log_decay, const int* row_q_start,
+static int launch_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* log_decay, const int* row_q_start,
                          const int* row_q_len, const int* state_slots, float* state, float* out, float* scratch, int max_chunks, int num_rows,
                          int min_len, int H, int G, int D, int Dv, cudaStream_t stream) {
-    const size_t prep = (size_t)(2 * CH * (DT + 4) + 2 * CH * CHP + 3 * 256) * sizeof(float);      // two blocks on an SM
     const size_t scan = (size_t)(2 * (2 * CH * (DT + 4) + CH * COLS + 2 * CH) + 2 * CH * CHP + COLS * (DT + 4) + 3 * COLS * CHP) * sizeof(float);
+    const dim3 scan_grid(num_rows, H, (Dv + COLS - 1) / COLS);
+    if (decay) {                                               // a decay per channel
+        const size_t prep = (size_t)(3 * CH * (DT + 4) + 2 * CH * CHP + 4 * DT + 8 * CH * 16) * sizeof(float);
+        cudaError_t e = cudaFuncSetAttribute(delta_channel_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
+        if (e != cudaSuccess) return (int)e;
+        const int rc = launch_kernel(delta_channel_prep_kernel<DT>, dim3(max_chunks, H), dim3(CP_THREADS), prep, stream, qn, kn, beta, decay, log_decay, row_q_start,
+                                     row_q_len, num_rows, min_len, scratch, H, G, D);
+        if (rc) return rc;
+        return launch_kernel(delta_chunk_scan_kernel<DT, true>, scan_grid, dim3(256), scan, stream, qn, kn, vn, row_q_start, row_q_len, state_slots, min_len,
+                             (const float*)scratch, state, out, H, G, D, Dv);
+    }
+    const size_t prep = (size_t)(2 * CH * (DT + 4) + 2 * CH * CHP + 3 * 256) * sizeof(float);      // two blocks on an SM
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
     if (e != cudaSuccess) return (int)e;
     const int rc = launch_kernel(delta_chunk_prep_kernel<DT>, dim3(max_chunks, G), dim3(256), prep, stream, qn, kn, beta, log_decay, row_q_start,
                                  row_q_len, num_rows, min_len, scratch, H, G, D);
     if (rc) return rc;
-    return launch_kernel(delta_chunk_scan_kernel<DT>, dim3(num_rows, H, (Dv + COLS - 1) / COLS), dim3(256), scan, stream, qn, kn, vn, row_q_start,
-                         row_q_len, state_slots, min_len, (const float*)scratch, state, out, H, G, D, Dv);
+    return launch_kernel(delta_chunk_scan_kernel<DT, false>, scan_grid, dim3(256), scan, stream, qn, kn, vn, row_q_start, row_q_len, state_slots, min_len,
+                         (const float*)scratch, state, out, H, G, D, Dv);
 }
 
 // Floats of scratch memory for one (chunk, head); tokens a chunk.
-extern "C" int mie_delta_chunk_floats(void) { return 2 * CH * CH + 2 * CH; }
+extern "C" int mie_delta_chunk_floats(int per_channel, int D) { return 2 * CH * CH + (per_channel ? (3 * CH + 1) * D : 2 * CH); }
 extern "C" int mie_delta_chunk_tokens(void) { return CH; }
 
-// qn, kn: float32 [T, G, D]; vn, out: [T, H, Dv]; beta, log_decay (not positive): [T, H]; state [slots, H, Dv, D].  D a multiple of 4 up to
-// 128, everything 16-byte aligned.  max_chunks: no fewer than the chunks of all rows with min_len tokens or more; scratch holds
+// qn, kn: float32 [T, G, D]; vn, out: [T, H, Dv]; beta [T, H]; log_decay (not positive) [T, H] with `decay` null, or [T, H, D] with `decay` [T, H, D] its
+// exponential; state [slots, H, Dv, D].  D a multiple of 4 up to 128, everything 16-byte aligned.  max_chunks: no fewer than the chunks of all rows with min_len tokens or more; scratch holds
 // max_chunks * H times mie_delta_chunk_floats() floats.
-extern "C" int mie_delta_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* log_decay,
+extern "C" int mie_delta_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* log_decay,
                                 const int* row_q_start, const int* row_q_len, const int* state_slots, float* state, float* out, float* scratch,
                                 int max_chunks, int num_rows, int min_len, int H, int G, int D, int Dv, cudaStream_t stream) {
     if (num_rows <= 0 || max_chunks <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || D % 4 || Dv <= 0 || min_len < 1) return MIE_ERR_BAD_ARG;
     if (D > 128 || H > 65535) return MIE_ERR_TOO_LARGE;
+    if (decay && ((reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(log_decay)) & 15)) return MIE_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(scratch)) & 15)
         return MIE_ERR_BAD_ARG;
     if (D <= 64)
-        return launch_chunks<64>(qn, kn, vn, beta, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
-    return launch_chunks<128>(qn, kn, vn, beta, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
+        return launch_chunks<64>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
+    return launch_chunks<128>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
 }

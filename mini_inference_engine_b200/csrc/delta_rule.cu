@@ -46,7 +46,8 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int64_t stride,
                                      const int* __restrict__ state_slots, const float* __restrict__ a_log,
                                      const float* __restrict__ dt_bias, float* __restrict__ qn, float* __restrict__ kn,
                                      float* __restrict__ vn, float* __restrict__ beta, float* __restrict__ decay,
-                                     float* __restrict__ kq, int H, int G, int D, int Dv, int K, float q_scale, float unit_eps) {
+                                     float* __restrict__ log_decay, float* __restrict__ kq, int H, int G, int D, int Dv, int K, float q_scale,
+                                     float unit_eps) {
     pdl_enter();
     const int t = blockIdx.x;
     const int row = token_row[t];
@@ -92,7 +93,9 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int64_t stride,
     for (int h = threadIdx.x; h < H; h += blockDim.x) beta[(int64_t)t * H + h] = 1.0f / (1.0f + expf(-to_f32<T>(bl[h])));
     for (int i = threadIdx.x; i < H * D; i += blockDim.x) {
         const float rate = expf(a_log[i / D]);
-        decay[(int64_t)t * H * D + i] = expf(-rate * softplus_f(low[(int64_t)t * low_stride + i] + dt_bias[i]));
+        const float l = -rate * softplus_f(low[(int64_t)t * low_stride + i] + dt_bias[i]);
+        decay[(int64_t)t * H * D + i] = expf(l);
+        if (log_decay) log_decay[(int64_t)t * H * D + i] = fmaxf(l, -100.f);
     }
     __syncthreads();                                   // q and k of this token, written above by other warps of the block
     for (int g = warp; g < G; g += nw) {               // k . q per key head: the same for every value column of the recurrence
@@ -340,7 +343,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const TG* __r
 extern "C" int mie_delta_prepare(const void* proj, int tag, long long stride, const float* low, long long low_stride, const float* taps,
                                  const float* conv_state, const int* token_row, const int* row_q_start, const int* state_slots,
                                  const float* a_log, const float* dt_bias, float* qn, float* kn, float* vn, float* beta, float* decay,
-                                 float* kq, int num_tokens, int H, int G, int D, int Dv, int K, float q_scale, float unit_eps,
+                                 float* log_decay, float* kq, int num_tokens, int H, int G, int D, int Dv, int K, float q_scale, float unit_eps,
                                  cudaStream_t stream) {
     if (num_tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || Dv <= 0 || K < 1) return MIE_ERR_BAD_ARG;
@@ -349,11 +352,11 @@ extern "C" int mie_delta_prepare(const void* proj, int tag, long long stride, co
     if (tag == MIE_F32)
         return launch_kernel(delta_prepare_kernel<float>, dim3(num_tokens), dim3(threads), 0, stream, (const float*)proj, (int64_t)stride,
                              low, (int64_t)low_stride, taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias, qn, kn, vn,
-                             beta, decay, kq, H, G, D, Dv, K, q_scale, unit_eps);
+                             beta, decay, log_decay, kq, H, G, D, Dv, K, q_scale, unit_eps);
     else if (tag == MIE_BF16)
         return launch_kernel(delta_prepare_kernel<bf16>, dim3(num_tokens), dim3(threads), 0, stream, (const bf16*)proj, (int64_t)stride,
                              low, (int64_t)low_stride, taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias, qn, kn, vn,
-                             beta, decay, kq, H, G, D, Dv, K, q_scale, unit_eps);
+                             beta, decay, log_decay, kq, H, G, D, Dv, K, q_scale, unit_eps);
     return MIE_ERR_BAD_ARG;
 }
 

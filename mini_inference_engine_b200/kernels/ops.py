@@ -1233,11 +1233,12 @@ def diff_combine(maps: torch.Tensor, gate, out: torch.Tensor, *, num_heads: int,
 # --------------------------------------------------------------------------- gated delta rule
 
 def delta_prepare(proj: torch.Tensor, low: torch.Tensor, taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias,
-                  qn, kn, vn, beta, decay, kq, *, num_heads: int, num_kv_heads: int, dim: int, vdim: int, unit_eps: float) -> None:
+                  qn, kn, vn, beta, decay, kq, *, num_heads: int, num_kv_heads: int, dim: int, vdim: int, unit_eps: float, log_decay=None) -> None:
     """From rows [q: G x dim | k: G x dim | v: H x vdim | beta logits: H | ...] of the input projection and float32 rows
     [a: H x dim | ...] of the low-rank one: convolution over time + silu of q, k, v (float32 taps [channels, K], older inputs
     from ``conv_state`` [slots, K - 1, channels]), q and k unit vectors per head (q times dim^-1/2), beta = sigmoid,
-    decay = exp(-exp(a_log[h]) softplus(a + dt_bias)), kq = k . q per key head.  All outputs float32."""
+    decay = exp(-exp(a_log[h]) softplus(a + dt_bias)), kq = k . q per key head; ``log_decay``: the exponent besides (none below -100).
+    All outputs float32."""
     T = proj.shape[0]
     H, G, D, Dv = num_heads, num_kv_heads, dim, vdim
     C = 2 * G * D + H * Dv
@@ -1249,14 +1250,14 @@ def delta_prepare(proj: torch.Tensor, low: torch.Tensor, taps, conv_state, token
           "convolution state must be float32 [slots, K - 1, channels]")
     _f32(a_log, "A_log", H)
     _f32(dt_bias, "dt_bias", H * D)
-    for t, n in ((qn, G * D), (kn, G * D), (vn, H * Dv), (beta, H), (decay, H * D), (kq, G)):
+    for t, n in ((qn, G * D), (kn, G * D), (vn, H * Dv), (beta, H), (decay, H * D), (kq, G)) + (((log_decay, H * D),) if log_decay is not None else ()):
         _need(t.dtype == torch.float32 and t.is_contiguous() and t.shape == (T, n), "outputs must be float32 [T, n]")
     for t, n in ((token_row, "token_row"), (row_q_start, "row_q_start"), (state_slots, "state_slots")):
         _i32(t, n)
     lib = load("delta_rule")
     _check(lib.mie_delta_prepare(_ptr(proj), tag(proj), ctypes.c_longlong(proj.stride(0)), _ptr(low), ctypes.c_longlong(low.stride(0)),
                                  _ptr(taps), _ptr(conv_state), _ptr(token_row), _ptr(row_q_start), _ptr(state_slots), _ptr(a_log),
-                                 _ptr(dt_bias), _ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(decay), _ptr(kq), T, H, G, D, Dv, K,
+                                 _ptr(dt_bias), _ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(decay), _ptr(log_decay), _ptr(kq), T, H, G, D, Dv, K,
                                  ctypes.c_float(D ** -0.5), ctypes.c_float(unit_eps), _stream()), "delta_prepare")
 
 
@@ -1366,14 +1367,15 @@ def delta_chunks_take(dim: int) -> bool:
 
 
 def delta_chunks(qn, kn, vn, beta, log_decay, row_q_start, row_q_len, state_slots, state, out, *, num_heads: int, num_kv_heads: int, dim: int,
-                 vdim: int, min_len: int, work=None) -> torch.Tensor:
-    """``delta_scan`` with one decay per head, in chunks of 64 tokens, for the rows with ``min_len`` new tokens or more (the others are left
-    alone).  ``log_decay`` [T, H] float32, not positive.  ``work`` = (rows, tokens) of those rows where the caller knows."""
+                 vdim: int, min_len: int, work=None, decay=None) -> torch.Tensor:
+    """``delta_scan`` in chunks of 64 tokens, for the rows with ``min_len`` new tokens or more (the others are left
+    alone).  ``log_decay`` float32, not positive: [T, H], or [T, H * dim] with ``decay`` [T, H * dim] its exponential.  ``work`` = (rows, tokens) of those rows where the caller knows."""
     T = qn.shape[0]
     H, G, D, Dv = num_heads, num_kv_heads, dim, vdim
     _need(delta_chunks_take(D), f"keys of {D}: the chunked kernel takes multiples of 4 up to 128")
     _need(state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (H, Dv, D), "state must be float32 [slots, H, vdim, dim]")
-    for t, n in ((qn, G * D), (kn, G * D), (vn, H * Dv), (beta, H), (log_decay, H), (out, H * Dv)):
+    A = D if decay is not None else 1
+    for t, n in ((qn, G * D), (kn, G * D), (vn, H * Dv), (beta, H), (log_decay, H * A), (out, H * Dv)) + (((decay, H * D),) if decay is not None else ()):
         _need(t.dtype == torch.float32 and t.is_contiguous() and t.shape == (T, n), "operands must be float32 [T, n]")
     for t, n in ((row_q_start, "row_q_start"), (row_q_len, "row_q_len"), (state_slots, "state_slots")):
         _i32(t, n)
@@ -1381,8 +1383,8 @@ def delta_chunks(qn, kn, vn, beta, log_decay, row_q_start, row_q_len, state_slot
     rows, tokens = work if work is not None else (row_q_len.numel(), T)
     size = lib.mie_delta_chunk_tokens()
     chunks = tokens // size + min(rows, tokens // max(1, min_len))
-    scratch = _workspace(qn.device, "delta_chunks", chunks * H * lib.mie_delta_chunk_floats(), torch.float32)
-    _check(lib.mie_delta_chunks(_ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(log_decay), _ptr(row_q_start), _ptr(row_q_len), _ptr(state_slots),
+    scratch = torch.empty(chunks * H * lib.mie_delta_chunk_floats(int(decay is not None), D), dtype=torch.float32, device=qn.device)
+    _check(lib.mie_delta_chunks(_ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(decay), _ptr(log_decay), _ptr(row_q_start), _ptr(row_q_len), _ptr(state_slots),
                                 _ptr(state), _ptr(out), _ptr(scratch), chunks, row_q_len.numel(), int(min_len), H, G, D, Dv, _stream()), "delta_chunks")
     return out
 

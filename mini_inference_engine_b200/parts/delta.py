@@ -10,7 +10,7 @@ mean square, multiplied by a weight shared by the heads and by sigmoid(W_g2 W_g1
 
 Products: q|k|v|beta of the input are one, the two low-rank down-projections (a1|g1) one, and their up-projections one
 block-diagonal product that leaves float32.  The convolution, activations, unit norms and decays are one kernel, the
-recurrence one, the head norm and gate one.  Two states (a tuple of needs): S [heads, vdim, dim] and the
+recurrence is one token by token and two in chunks, the head norm and gate are one.  Two states (a tuple of needs): S [heads, vdim, dim] and the
 convolution's last taps - 1 inputs."""
 from __future__ import annotations
 
@@ -20,6 +20,10 @@ from ..kernels import ops
 from ..weights.loader import TensorSpec
 from .attention import _padded_rows
 from .base import Mixer, StateNeed, register_part
+
+
+CHANNEL_CHUNKED_FROM = 112      # new tokens from which a row's recurrence goes in chunks (the line of one decay per head, see CHUNKED_FROM: the scans are the same; 1,500 tokens
+                                # in rows of 500 and 1,000, 16 heads of 128 x 128: 427 us token by token, 302 us in chunks, preparation included)
 
 
 class ChannelDelta(Mixer):
@@ -76,7 +80,7 @@ class ChannelDelta(Mixer):
         return (StateNeed((self.num_heads, self.vdim, self.dim), torch.float32), StateNeed((self.taps - 1, C), torch.float32))
 
     def kernel_sources(self):
-        return {"delta_rule"} | self.rt.product_sources(self.w_in, self.w_low, self.w_up, self.w_o)
+        return {"delta_rule", "delta_chunk"} | self.rt.product_sources(self.w_in, self.w_low, self.w_up, self.w_o)
 
     def forward(self, x, ctx, cache):
         H, G, D, Dv, T = self.num_heads, self.num_kv_heads, self.dim, self.vdim, ctx.num_tokens
@@ -85,13 +89,22 @@ class ChannelDelta(Mixer):
         low = self.rt.linear(self.rt.linear(x, self.w_low), self.w_up, None, out_dtype=torch.float32)     # [a: H x D | gate: H x Dv]
         f32 = lambda n: self.rt.empty(T, n, dtype=torch.float32)
         qn, kn, vn, beta, decay, kq = f32(G * D), f32(G * D), f32(H * Dv), f32(H), f32(H * D), f32(G)
+        sizes = dict(num_heads=H, num_kv_heads=G, dim=D, vdim=Dv)
+        # (as in HeadDelta: where the host does not know the rows' lengths each of the two kernels takes the rows that are its own)
+        chunked = ops.delta_chunks_take(D) and ctx.max_q_len >= CHANNEL_CHUNKED_FROM
+        q_lens = ctx.host.get("q_len")
+        long = [n for n in q_lens if n >= CHANNEL_CHUNKED_FROM] if chunked and q_lens is not None else None
+        log_decay = f32(H * D) if chunked else None
         ops.delta_prepare(proj, low, self.conv, conv_state, ctx.token_row, ctx.row_q_start, ctx.state_slots, self.a_log, self.dt_bias,
-                          qn, kn, vn, beta, decay, kq, num_heads=H, num_kv_heads=G, dim=D, vdim=Dv, unit_eps=self.unit_eps)
+                          qn, kn, vn, beta, decay, kq, unit_eps=self.unit_eps, log_decay=log_decay, **sizes)
         if self.taps > 1:
             ops.conv_state_update(proj, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, conv_state)
         o = f32(H * Dv)
-        ops.delta_scan(qn, kn, vn, beta, decay, kq, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o, num_heads=H,
-                       num_kv_heads=G, dim=D, vdim=Dv)
+        rows = (ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o)
+        if chunked:
+            ops.delta_chunks(qn, kn, vn, beta, log_decay, *rows, min_len=CHANNEL_CHUNKED_FROM, work=(len(long), sum(long)) if long else None, decay=decay, **sizes)
+        if long is None or len(long) < len(q_lens):
+            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHANNEL_CHUNKED_FROM if chunked else 1 << 30, **sizes)
         gated = self.rt.empty(T, H * Dv)
         ops.head_norm_gate(o, low[:, H * D:], self.norm, gated, H, Dv, self.eps)
         return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)
