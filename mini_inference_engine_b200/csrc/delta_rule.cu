@@ -106,6 +106,153 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int64_t stride,
     }
 }
 
+// The same for four taps and sizes in steps of four channels (key heads of up to 128): a warp takes a head's q and k, or 128 channels of v or of the decays, of RUN
+// consecutive tokens, four channels a lane; the tokens' inputs are asked for together and pass through a window in registers, so an input is read once, not once
+// a tap.  Bound by memory: 1,500 tokens of 16 heads of 128 (58 MB) 94 us a token a block, two bytes at a time -> 45 us (runs of four 46, of two 56).
+template <typename T> struct Raw4;
+template <> struct Raw4<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void get(float* x) const { x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+};
+template <> struct Raw4<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void get(float* x) const {
+        x[0] = __uint_as_float(v.x << 16); x[1] = __uint_as_float(v.x & 0xffff0000u);
+        x[2] = __uint_as_float(v.y << 16); x[3] = __uint_as_float(v.y & 0xffff0000u);
+    }
+};
+// Four channels from `c` on: their taps and the three inputs in front of the next token.
+template <typename T> struct Window4 {
+    float w[4][4], x[3][4];                      // taps [channel][back 3 .. 0], inputs [oldest first][channel]
+    __device__ __forceinline__ void taps(const float* t, int c) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(w[e]) = *reinterpret_cast<const float4*>(t + (int64_t)(c + e) * 4);
+    }
+    __device__ __forceinline__ void start(const T* proj, int64_t stride, const float* st, int C, int t, int local, int c) {
+#pragma unroll
+        for (int back = 3; back > 0; --back) {
+            if (back <= local) { Raw4<T> r; r.load(proj + (int64_t)(t - back) * stride + c); r.get(x[3 - back]); }
+            else *reinterpret_cast<float4*>(x[3 - back]) = *reinterpret_cast<const float4*>(st + (int64_t)(3 - (back - local)) * C + c);
+        }
+    }
+    __device__ __forceinline__ void step(const Raw4<T>& raw, float* y) {
+        float in[4];
+        raw.get(in);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float a = fmaf(w[e][3], in[e], fmaf(w[e][2], x[2][e], fmaf(w[e][1], x[1][e], fmaf(w[e][0], x[0][e], 0.f))));
+            y[e] = a / (1.0f + expf(-a));
+            x[0][e] = x[1][e]; x[1][e] = x[2][e]; x[2][e] = in[e];
+        }
+    }
+};
+template <typename T, int RUN>
+__global__ void __launch_bounds__(256) delta_prepare_runs_kernel(const T* __restrict__ proj, int64_t stride, const float* __restrict__ low, int64_t low_stride,
+                                                                 const float* __restrict__ taps, const float* __restrict__ conv_state,
+                                                                 const int* __restrict__ token_row, const int* __restrict__ row_q_start,
+                                                                 const int* __restrict__ state_slots, const float* __restrict__ a_log,
+                                                                 const float* __restrict__ dt_bias, float* __restrict__ qn, float* __restrict__ kn,
+                                                                 float* __restrict__ vn, float* __restrict__ beta, float* __restrict__ decay,
+                                                                 float* __restrict__ log_decay, float* __restrict__ kq, int num_tokens, int H, int G, int D,
+                                                                 int Dv, float q_scale, float unit_eps) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, C = 2 * G * D + H * Dv, pieces_v = (H * Dv + 127) / 128, pieces_d = (H * D + 127) / 128;
+    int unit = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int t0 = blockIdx.x * RUN, n = min(RUN, num_tokens - t0);
+    if (unit >= G + pieces_v + pieces_d + 1) return;
+    if (unit < G + pieces_v) {
+        const bool keys = unit < G;
+        const int at = keys ? lane * 4 : (unit - G) * 128 + lane * 4;      // within the head, or within v
+        const bool on = at < (keys ? D : H * Dv);
+        const int c0 = keys ? unit * D + at : 2 * G * D + at, c1 = keys ? (G + unit) * D + at : c0;
+        Raw4<T> raw0[RUN], raw1[RUN];
+        Window4<T> a, b;
+        if (on) {
+#pragma unroll
+            for (int i = 0; i < RUN; ++i)
+                if (i < n) { raw0[i].load(proj + (int64_t)(t0 + i) * stride + c0); if (keys) raw1[i].load(proj + (int64_t)(t0 + i) * stride + c1); }
+            a.taps(taps, c0);
+            if (keys) b.taps(taps, c1);
+        }
+        int row = -1;
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) {
+            if (i >= n) break;
+            const int t = t0 + i, r = token_row[t];
+            if (r != row) {
+                row = r;
+                const float* st = conv_state + (int64_t)state_slots[r] * 3 * C;
+                const int local = t - row_q_start[r];
+                if (on) a.start(proj, stride, st, C, t, local, c0);
+                if (on && keys) b.start(proj, stride, st, C, t, local, c1);
+            }
+            float q[4] = {0.f, 0.f, 0.f, 0.f}, k[4] = {0.f, 0.f, 0.f, 0.f};
+            if (on) a.step(raw0[i], q);
+            if (!keys) {
+                if (on) *reinterpret_cast<float4*>(vn + (int64_t)t * H * Dv + at) = make_float4(q[0], q[1], q[2], q[3]);
+                continue;
+            }
+            if (on) b.step(raw1[i], k);
+            float qq = 0.f, kk = 0.f, qk = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { qq = fmaf(q[e], q[e], qq); kk = fmaf(k[e], k[e], kk); qk = fmaf(q[e], k[e], qk); }
+            qq = warp_sum(qq);
+            kk = warp_sum(kk);
+            qk = warp_sum(qk);
+            const float qs = q_scale / sqrtf(qq + unit_eps), ks = 1.0f / sqrtf(kk + unit_eps);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { q[e] *= qs; k[e] *= ks; }
+            const int64_t to = ((int64_t)t * G + unit) * D + at;
+            if (on) {
+                *reinterpret_cast<float4*>(qn + to) = make_float4(q[0], q[1], q[2], q[3]);
+                *reinterpret_cast<float4*>(kn + to) = make_float4(k[0], k[1], k[2], k[3]);
+            }
+            if (lane == 0) kq[(int64_t)t * G + unit] = qk * qs * ks;
+        }
+        return;
+    }
+    unit -= G + pieces_v;
+    if (unit < pieces_d) {
+        const int at = unit * 128 + lane * 4;
+        if (at >= H * D) return;
+        const float rate = expf(a_log[at / D]);                // (four channels of one head: D is a multiple of 4)
+        const float4 bias = *reinterpret_cast<const float4*>(dt_bias + at);
+        float4 x[RUN];
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) if (i < n) x[i] = *reinterpret_cast<const float4*>(low + (int64_t)(t0 + i) * low_stride + at);
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) {
+            if (i >= n) break;
+            const float4 l = make_float4(-rate * softplus_f(x[i].x + bias.x), -rate * softplus_f(x[i].y + bias.y), -rate * softplus_f(x[i].z + bias.z),
+                                         -rate * softplus_f(x[i].w + bias.w));
+            const int64_t to = (int64_t)(t0 + i) * H * D + at;
+            *reinterpret_cast<float4*>(decay + to) = make_float4(expf(l.x), expf(l.y), expf(l.z), expf(l.w));
+            if (log_decay) *reinterpret_cast<float4*>(log_decay + to) = make_float4(fmaxf(l.x, -100.f), fmaxf(l.y, -100.f), fmaxf(l.z, -100.f), fmaxf(l.w, -100.f));
+        }
+        return;
+    }
+    for (int i = 0; i < n; ++i)
+        for (int h = lane; h < H; h += 32) beta[(int64_t)(t0 + i) * H + h] = 1.0f / (1.0f + expf(-to_f32<T>(proj[(int64_t)(t0 + i) * stride + C + h])));
+}
+
+template <typename T>
+static int launch_prepare_runs(const T* proj, long long stride, const float* low, long long low_stride, const float* taps, const float* conv_state,
+                               const int* token_row, const int* row_q_start, const int* state_slots, const float* a_log, const float* dt_bias, float* qn,
+                               float* kn, float* vn, float* beta, float* decay, float* log_decay, float* kq, int num_tokens, int H, int G, int D, int Dv,
+                               float q_scale, float unit_eps, cudaStream_t stream) {
+    const int units = G + (H * Dv + 127) / 128 + (H * D + 127) / 128 + 1, ny = (units + 7) / 8;
+    // runs of eight tokens where that leaves a block for every SM twice over, else of one (decoding: every token is another request's anyway)
+    if ((int64_t)((num_tokens + 7) / 8) * ny >= 2 * device_sm_count())
+        return launch_kernel(delta_prepare_runs_kernel<T, 8>, dim3((num_tokens + 7) / 8, ny), dim3(256), 0, stream, proj, (int64_t)stride, low, (int64_t)low_stride,
+                             taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias, qn, kn, vn, beta, decay, log_decay, kq, num_tokens, H, G, D, Dv,
+                             q_scale, unit_eps);
+    return launch_kernel(delta_prepare_runs_kernel<T, 1>, dim3(num_tokens, ny), dim3(256), 0, stream, proj, (int64_t)stride, low, (int64_t)low_stride, taps,
+                         conv_state, token_row, row_q_start, state_slots, a_log, dt_bias, qn, kn, vn, beta, decay, log_decay, kq, num_tokens, H, G, D, Dv, q_scale,
+                         unit_eps);
+}
+
 // The convolution state of every row after the step: row i of the new state is the input at q_len - (K - 1) + i of the
 // portion, or, where the portion is shorter than that reaches back, a row of the old state.  One thread per channel
 // walks the rows upwards, so the move is safe in place.
@@ -347,6 +494,18 @@ extern "C" int mie_delta_prepare(const void* proj, int tag, long long stride, co
                                  cudaStream_t stream) {
     if (num_tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || Dv <= 0 || K < 1) return MIE_ERR_BAD_ARG;
+    const int piece = tag == MIE_F32 ? 16 : 8;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(low) | reinterpret_cast<uintptr_t>(taps) | reinterpret_cast<uintptr_t>(conv_state) |
+                          reinterpret_cast<uintptr_t>(dt_bias) | reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn) |
+                          reinterpret_cast<uintptr_t>(vn) | reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(log_decay);
+    if (K == 4 && D % 4 == 0 && D <= 128 && (H * Dv) % 4 == 0 && stride % 4 == 0 && low_stride % 4 == 0 && all % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(proj) % piece == 0 && (tag == MIE_F32 || tag == MIE_BF16)) {
+        if (tag == MIE_F32)
+            return launch_prepare_runs<float>((const float*)proj, stride, low, low_stride, taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias,
+                                              qn, kn, vn, beta, decay, log_decay, kq, num_tokens, H, G, D, Dv, q_scale, unit_eps, stream);
+        return launch_prepare_runs<bf16>((const bf16*)proj, stride, low, low_stride, taps, conv_state, token_row, row_q_start, state_slots, a_log, dt_bias, qn, kn,
+                                         vn, beta, decay, log_decay, kq, num_tokens, H, G, D, Dv, q_scale, unit_eps, stream);
+    }
     const int units = 2 * G + H;
     const int threads = units >= 8 ? 256 : (units >= 4 ? 128 : 64);
     if (tag == MIE_F32)

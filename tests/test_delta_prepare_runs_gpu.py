@@ -1,0 +1,34 @@
+"""The channel delta rule's preparation four channels a lane, in runs of tokens, against the kernel that takes a token a block: rows that begin and end
+inside a run, inputs older than the portion, head sizes with idle lanes, both types."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows", [[1], [1] * 9, [3, 1, 2, 8, 17, 5], [700, 900], [4000]])
+@pytest.mark.parametrize("H,G,D,V", [(2, 2, 128, 128), (4, 2, 64, 32), (3, 1, 20, 12), (16, 16, 128, 128)])
+def test_runs_against_tokens(dt, rows, H, G, D, V):
+    from mini_inference_engine_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(len(rows) + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    T, C = sum(rows), 2 * G * D + H * V
+    if T > 1000 and H == 16:
+        rows, T = [300, 260], 560
+    proj, low = rnd(T, -(-(C + H) // 8) * 8).to(dt), rnd(T, H * D + 4)
+    taps, conv, a_log, bias = rnd(C, 4) * 0.5, rnd(len(rows) + 1, 3, C), rnd(H), rnd(H * D)
+    lens = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    starts = torch.cumsum(lens, 0, dtype=torch.int32) - lens
+    token_row = torch.repeat_interleave(torch.arange(len(rows), dtype=torch.int32, device="cuda"), lens)
+    slots = torch.tensor([len(rows) - i for i in range(len(rows))], dtype=torch.int32, device="cuda")
+    results = []
+    for shift in (0, 1):                                        # taps that do not start on 16 bytes: the kernel with a token a block
+        t = torch.empty(C * 4 + 4, device="cuda")[shift:shift + C * 4].view(C, 4).copy_(taps)
+        outs = [torch.zeros(T, n, device="cuda") for n in (G * D, G * D, H * V, H, H * D, G, H * D)]
+        ops.delta_prepare(proj, low, t, conv, token_row, starts, slots, a_log, bias, *outs[:6], num_heads=H, num_kv_heads=G, dim=D, vdim=V, unit_eps=1e-6,
+                          log_decay=outs[6])
+        results.append(outs)
+    torch.cuda.synchronize()
+    for a, b in zip(*results):                                  # (sums of squares over a head in another order: a few units in the last place)
+        assert torch.isfinite(a).all() and (a - b).abs().max() <= 2e-6 * b.abs().max()
