@@ -17,11 +17,10 @@
 //
 // The reference does this with a library attention call per prompt portion
 // (inference_engine/model.py:146-158).  A block works through its key tiles one after the other
-// (S, softmax, PV); two blocks share an SM at head_dim 64 (256 TMEM columns and 97 KB of shared
-// memory each), so one block's softmax runs under the other's products.  When a launch has more
-// query tiles than the GPU runs at a time, a block takes two tiles of a row one after the other,
-// the j-th from the end and the j-th from the start: under the causal mask every such pair has the
-// same number of key tiles, so the blocks end together instead of leaving a tail of long ones.
+// (S, softmax, PV); two blocks share an SM (256 TMEM columns and 97 KB of shared memory each: 128 keys a tile at head_dim 64, 64 keys
+// at head_dim 128), so one block's softmax runs under the other's products.  Tiles go longest first over all heads; where that fills the GPU
+// better, a block takes two tiles of a row one after the other, the j-th from the end and the j-th from the start: under the causal mask every
+// such pair has the same number of key tiles.  Small launches with heads of 128 take 128 keys a tile and an SM alone (launch_fa).
 //
 // Roles: warp 0 = TMA producer (one lane), warp 1 = TMEM owner + MMA issuer (one lane), warps 2..5 =
 // softmax and epilogue.  Barriers: q_full, kv_full[2] / kv_empty[2] (two key/value stages; kv_empty
@@ -108,7 +107,9 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // maximum settles); an instance for each combination, so that the plain softmax keeps its instruction count and the others test nothing per element.  A sink
 // joins the sum in every instance (it costs a term at a row's start).  KEEP: the instance for a window or block that keeps the
 // first keys in sight (p.keep).
-template <int D, int MODS, bool KEEP>
+// BN: keys a tile.  Heads of 64 take 128.  Heads of 128 have an instance with 64 (one query tile in shared memory, 256 tensor-memory columns: two blocks
+// on an SM, one's softmax under the other's products) and one with 128 (two query tiles, an SM alone); launch_fa says which runs when.
+template <int D, int MODS, bool KEEP, int BN>
 __global__ void __launch_bounds__(FA_THREADS, MODS & 3 ? 1 : 2)   // two blocks per SM: at most 168 registers (the instances with
                                                                   // a cap or a bias table need more and take an SM alone)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv activation [tokens, q_stride], box {64, 128}
@@ -116,10 +117,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                             const __grid_constant__ CUtensorMap map_v,
                             const FaParams p) {
     constexpr int PARTS = D / 64;                               // 64-column sub-tiles (128 bytes = one swizzle row)
-    constexpr uint32_t SUB_BYTES = 128 * 64 * 2;                // one [128 rows x 64] sub-tile
-    constexpr uint32_t Q_BYTES = PARTS * SUB_BYTES, KV_BYTES = PARTS * SUB_BYTES;
-    constexpr uint32_t TMEM_S = 0, TMEM_P = 128, TMEM_O = 192;  // column offsets: S 128 cols, P 64 cols (bf16 pairs), O D cols
-    constexpr uint32_t TMEM_COLS = D == 64 ? 256 : 512;
+    constexpr uint32_t SUB_BYTES = 128 * 64 * 2, KV_SUB = BN * 64 * 2;      // one [128 rows x 64] sub-tile of queries, one [BN x 64] of keys
+    constexpr uint32_t Q_BYTES = PARTS * SUB_BYTES, KV_BYTES = PARTS * KV_SUB;
+    constexpr int QS = BN == 128 ? 2 : 1;                       // query tiles in shared memory
+    constexpr uint32_t TMEM_S = 0, TMEM_P = BN, TMEM_O = BN == 128 ? 192 : 128;  // column offsets: S BN cols, P BN / 2 cols (bf16 pairs), O D cols
+    constexpr uint32_t TMEM_COLS = D == 128 && BN == 128 ? 512 : 256;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t q_full[2], kv_full[2], kv_empty[2], s_full, p_full, o_full;
     __shared__ uint32_t tmem_base_slot;
@@ -129,8 +131,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
     unsigned char* tiles = smem_dyn + (base - smem_u32(smem_dyn));
     // layout: Q of the first query tile | Q of the second | K stage 0 | V stage 0 | K stage 1 | V stage 1
     auto q_addr = [&](int u) { return base + (uint32_t)u * Q_BYTES; };
-    auto k_addr = [&](int s) { return base + 2 * Q_BYTES + (uint32_t)s * 2 * KV_BYTES; };
-    auto v_addr = [&](int s) { return base + 2 * Q_BYTES + (uint32_t)s * 2 * KV_BYTES + KV_BYTES; };
+    auto k_addr = [&](int s) { return base + QS * Q_BYTES + (uint32_t)s * 2 * KV_BYTES; };
+    auto v_addr = [&](int s) { return base + QS * Q_BYTES + (uint32_t)s * 2 * KV_BYTES + KV_BYTES; };
 
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -145,7 +147,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
     // below that every tile has a block of its own and the longest one is the critical path.
     if (warp == 0) {
         int pair, tiles_r;
-        const int r = warp_find_row(p.row_q_len, p.num_rows, (int)blockIdx.x, [&](int ql) {
+        const int r = warp_find_row(p.row_q_len, p.num_rows, (int)blockIdx.y, [&](int ql) {
             const int t = ql >= p.min_q_len ? (ql + FA_BM - 1) / FA_BM : 0;
             return p.pair ? (t + 1) / 2 : t;
         }, pair, tiles_r);
@@ -174,7 +176,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
     }
     // key/value rows that no copy fills (beyond the context) must hold finite values: 0 * NaN is NaN
     for (uint32_t i = threadIdx.x * 16; i < 4 * KV_BYTES; i += FA_THREADS * 16)
-        *reinterpret_cast<uint4*>(tiles + 2 * Q_BYTES + i) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(tiles + QS * Q_BYTES + i) = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the TMA unit must see the zeros before it overwrites them
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(TMEM_COLS) : "memory");
@@ -190,10 +192,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
 
     if (row >= 0) {
         const int q_len = p.row_q_len[row], ctx = p.row_ctx_len[row], q_start = p.row_q_start[row];
-        const int head = blockIdx.y;
+        const int head = blockIdx.x;
         const int kvh = head / (p.num_heads / p.num_kv_heads);
         const int nsub = s_nsub;
-        // the geometry of query tile u: first query's position, rows, key range in tiles of FA_BN keys
+        // the geometry of query tile u: first query's position, rows, key range in tiles of BN keys
         struct Sub { int q0, pos0, nq, k_hi, k_lo, kbeg, kept, ntiles; };
         Sub sb[2];
 #pragma unroll
@@ -204,14 +206,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
             g.nq = min(FA_BM, q_len - g.q0);
             g.k_hi = g.pos0 + g.nq;                              // one past the last key any query here reads
             g.k_lo = mask_first_key(g.pos0, p.window);
-            g.kbeg = g.k_lo & ~(FA_BN - 1);
-            g.kept = KEEP ? mask_kept_tiles(p.keep, g.kbeg, FA_BN) : 0;     // tiles of kept keys in front of the window's
-            g.ntiles = u < nsub ? g.kept + (g.k_hi - g.kbeg + FA_BN - 1) / FA_BN : 0;
+            g.kbeg = g.k_lo & ~(BN - 1);
+            g.kept = KEEP ? mask_kept_tiles(p.keep, g.kbeg, BN) : 0;     // tiles of kept keys in front of the window's
+            g.ntiles = u < nsub ? g.kept + (g.k_hi - g.kbeg + BN - 1) / BN : 0;
         }
         const int nA = sb[0].ntiles, G = nA + sb[1].ntiles;      // key tiles of the first query tile, and of both
         // Key tiles are counted through both query tiles (g = 0 .. G-1): stages and barrier phases go on
         // from the first query tile to the second without a break.
-        const int rows_per_copy = min(p.page_size, FA_BN);       // one TMA copy = one page (or a 128-row piece of it)
+        const int rows_per_copy = min(p.page_size, BN);       // one TMA copy = one page (or a 128-row piece of it)
 
         if (warp == 0) {
             // The producer warp: lane c issues the copies of page c of a tile, and fetches the page id
@@ -228,12 +230,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
             }
             auto key0_of = [&](int g) {
                 const int t = g < nA ? g : g - nA, kept = g < nA ? sb[0].kept : sb[1].kept;
-                if (MODS & 4) return (g < nA ? sb[0].kbeg + (nA - 1) * FA_BN : sb[1].kbeg + (G - nA - 1) * FA_BN) - t * FA_BN;
-                return t < kept ? t * FA_BN : (g < nA ? sb[0].kbeg : sb[1].kbeg) + (t - kept) * FA_BN;
+                if (MODS & 4) return (g < nA ? sb[0].kbeg + (nA - 1) * BN : sb[1].kbeg + (G - nA - 1) * BN) - t * BN;
+                return t < kept ? t * BN : (g < nA ? sb[0].kbeg : sb[1].kbeg) + (t - kept) * BN;
             };
             auto copies_of = [&](int g) {
                 const int key0 = key0_of(g), hi = g < nA ? sb[0].k_hi : sb[1].k_hi;
-                return (min(key0 + FA_BN, hi) - key0 + rows_per_copy - 1) / rows_per_copy;
+                return (min(key0 + BN, hi) - key0 + rows_per_copy - 1) / rows_per_copy;
             };
             auto page_of = [&](int g) {                           // lane's page id in key tile g (0 if it has no copy there)
                 if (g >= G || lane >= copies_of(g)) return 0;
@@ -257,19 +259,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                     const int src_row = (page * p.num_kv_heads + kvh) * p.page_size + (key & (p.page_size - 1));
 #pragma unroll
                     for (int part = 0; part < PARTS; ++part) {
-                        const uint32_t off = part * SUB_BYTES + (uint32_t)lane * rows_per_copy * 128u;
+                        const uint32_t off = part * KV_SUB + (uint32_t)lane * rows_per_copy * 128u;
                         tma_load_2d(tiles + (k_addr(s) - base) + off, &map_k, &kv_full[s], part * 64, src_row);
                         tma_load_2d(tiles + (v_addr(s) - base) + off, &map_v, &kv_full[s], part * 64, src_row);
                     }
                 }
             }
         } else if (warp == 1) {
-            // Head size 64: the whole warp walks this loop and an elected lane issues, so that what feeds the
-            // tensor-core instructions stays uniform across the warp (issued from a loop that one lane ran alone, an
-            // MMA cost that lane 90 - 150 cycles): 49.8 -> 45.1 us at 2,048 tokens, 531 -> 496 us at 8,192.  Head size
-            // 128 (one block on an SM, twice the exponent-free work per score): one lane alone, the 32 polling lanes
-            // cost the softmax warps more than the issue gains (964 -> 1,027 us at 8,192 tokens with the whole warp).
-            constexpr bool WARP_ISSUE = D == 64;
+            // The whole warp walks this loop and an elected lane issues, so that what feeds the tensor-core instructions stays
+            // uniform across the warp (issued from a loop that one lane ran alone, an MMA cost that lane 90 - 150 cycles): heads of 64, 49.8 ->
+            // 45.1 us at 2,048 tokens, 531 -> 496 us at 8,192.  Heads of 128 that have an SM alone (twice the exponent-free work per
+            // score): one lane, the 32 polling lanes cost the softmax warps more than the issue gains (964 -> 1,027 us at
+            // 8,192 tokens with the whole warp).
+            constexpr bool WARP_ISSUE = !(D == 128 && BN == 128);
             if (WARP_ISSUE || lane == 0) {
                 const bool issuer = WARP_ISSUE ? elect_one() : true;
                 auto wait_for = [&](uint64_t* bar, uint32_t parity) {
@@ -277,24 +279,24 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                 };
                 auto converge = [&]() { if (WARP_ISSUE) __syncwarp(); };
                 // S: M 128, N 128, both operands K-major.  PV: M 128, N D, B (values) MN-major.
-                const uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN);
+                const uint32_t idesc_s = umma_idesc_bf16(FA_BM, BN);
                 const uint32_t idesc_o = umma_idesc_bf16(FA_BM, D) | (1u << 16);
                 // One thread issues every MMA, and between two of them it can do little: the descriptors
                 // of all operand slices are formed once, here, so that an MMA costs its own instruction.
-                constexpr int KS = D / 16, KV = FA_BN / 16;
+                constexpr int KS = D / 16, KV = BN / 16;
                 uint64_t dq[2][KS], dk[2][KS], dv[2][KV];
 #pragma unroll
                 for (int ks = 0; ks < KS; ++ks) {
-                    const uint32_t off = (ks / 4) * SUB_BYTES + (ks % 4) * 32;
+                    const uint32_t off = (ks / 4) * SUB_BYTES + (ks % 4) * 32, off_k = (ks / 4) * KV_SUB + (ks % 4) * 32;
                     dq[0][ks] = umma_desc_sw128(q_addr(0) + off);
-                    dq[1][ks] = umma_desc_sw128(q_addr(1) + off);
-                    dk[0][ks] = umma_desc_sw128(k_addr(0) + off);
-                    dk[1][ks] = umma_desc_sw128(k_addr(1) + off);
+                    dq[1][ks] = umma_desc_sw128(q_addr(QS - 1) + off);
+                    dk[0][ks] = umma_desc_sw128(k_addr(0) + off_k);
+                    dk[1][ks] = umma_desc_sw128(k_addr(1) + off_k);
                 }
 #pragma unroll
                 for (int kk = 0; kk < KV; ++kk) {                  // 16 keys per MMA: 8 TMEM columns of P, 2 atoms of V
-                    dv[0][kk] = umma_desc_sw128_mn(v_addr(0) + kk * 2048, SUB_BYTES);
-                    dv[1][kk] = umma_desc_sw128_mn(v_addr(1) + kk * 2048, SUB_BYTES);
+                    dv[0][kk] = umma_desc_sw128_mn(v_addr(0) + kk * 2048, KV_SUB);
+                    dv[1][kk] = umma_desc_sw128_mn(v_addr(1) + kk * 2048, KV_SUB);
                 }
                 auto issue_s = [&](int g) {                        // scores of key tile g against its query tile
                     const bool second = g >= nA, st = g & 1;
@@ -376,9 +378,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                     ok = __all_sync(0xffffffffu, mbar_wait(&s_full, g & 1, abort_p));     // the warp goes on or gives up as one
                     if (!ok) break;
                     tc_fence_after();
-                    const int key0 = (MODS & 4) ? kbeg + (ntiles - 1 - t) * FA_BN : t < kept ? t * FA_BN : kbeg + (t - kept) * FA_BN;
+                    const int key0 = (MODS & 4) ? kbeg + (ntiles - 1 - t) * BN : t < kept ? t * BN : kbeg + (t - kept) * BN;
                     // masks are needed only where the tile touches the diagonal, the window's edge or the range's start
-                    bool need_mask = key0 + FA_BN - 1 > pos0 || key0 < k_lo || (p.window != 0 && key0 < mask_first_key(pos0 + FA_BM - 1, p.window));
+                    bool need_mask = key0 + BN - 1 > pos0 || key0 < k_lo || (p.window != 0 && key0 < mask_first_key(pos0 + FA_BM - 1, p.window));
                     // A key is read if lo <= key <= hi or, with kept keys, if it is below `also`: a tile in front of the window's holds kept
                     // keys only (earlier than every query), a tile of the window may begin with some.  The bounds are the row's, worked out
                     // once: inside the loops over elements the mask's rule (a block's start is a division) costs more than all else there.
@@ -386,7 +388,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                     if (KEEP) {
                         const bool front = t < kept;
                         if (front) { lo = 0; hi = p.keep - 1; also = 0; }
-                        if (front) need_mask = key0 + FA_BN > p.keep;
+                        if (front) need_mask = key0 + BN > p.keep;
                     }
                     // The row of S comes out of TMEM in four chunks of 32 columns; the load of the next chunk is
                     // in flight while the current one is worked on.
@@ -397,13 +399,17 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                         tmem_ld32_async(lane_addr + TMEM_S + 32, cb);
                         body(0, ca);
                         tmem_ld_wait(cb);
-                        tmem_ld32_async(lane_addr + TMEM_S + 64, ca);
-                        body(1, cb);
-                        tmem_ld_wait(ca);
-                        tmem_ld32_async(lane_addr + TMEM_S + 96, cb);
-                        body(2, ca);
-                        tmem_ld_wait(cb);
-                        body(3, cb);
+                        if constexpr (BN == 64) {
+                            body(1, cb);
+                        } else {
+                            tmem_ld32_async(lane_addr + TMEM_S + 64, ca);
+                            body(1, cb);
+                            tmem_ld_wait(ca);
+                            tmem_ld32_async(lane_addr + TMEM_S + 96, cb);
+                            body(2, ca);
+                            tmem_ld_wait(cb);
+                            body(3, cb);
+                        }
                     };
                     auto masked = [&](int key) {
                         return key > hi || (key < lo && (!KEEP || key >= also));
@@ -949,20 +955,48 @@ static int make_map_2d(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_
 
 static int g_fa_pp_mode = -1;
 
+template <int D, int MODS, bool KEEP, int BN>
+static int launch_fa_tile(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p, int tiles, int rows, cudaStream_t stream) {
+    constexpr int PARTS = D / 64;
+    const size_t smem = (size_t)PARTS * 64 * 2 * ((BN == 128 ? 2 : 1) * 128 + 4 * BN) + 1024;     // query tiles, two stages of keys and values
+    cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, MODS, KEEP, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    // heads fastest: the longest tiles of all heads start first
+    const dim3 grid(p.num_heads, p.pair ? (tiles + rows + 1) / 2 : tiles);
+    if (grid.y > 65535) return MIE_ERR_TOO_LARGE;
+    return launch_kernel(prefill_attention_tc_kernel<D, MODS, KEEP, BN>, grid, dim3(FA_THREADS), smem, stream, mq, mk, mv, p);
+}
+
+// Keys a tile that launch_fa will choose for these sizes: the tensor maps' boxes must be as high.
+static int fa_keys(int head_dim, int mods, int num_heads, int work_tokens, int work_rows) {
+    const int64_t blocks = (int64_t)((work_tokens + FA_BM - 1) / FA_BM + work_rows - 1) * num_heads;
+    return head_dim == 128 && (mods & 3) == 0 && blocks > 2 * (int64_t)device_sm_count() ? 64 : 128;
+}
+
+// tiles <= tokens / 128 + rows (of the rows that this kernel serves, where the caller knows them).  Whether a block takes one tile or a pair of equal
+// total length, and for heads of 128 how many keys a tile: device time in a graph, one pass after the other, us.
+//   Heads of 64, two blocks on an SM (296 places).  Pairs are all as long as the longest tile and one more, so they pay only where one round of
+//   them fills nearly every place; else tiles alone, longest first, fill the GPU evenly (32 heads, alone : in pairs): 1,152 tokens 22 : 30,
+//   1,400 27 : 33, 1,600 33 : 37, 1,800 40.5 : 40.3, 2,048 44.4 : 42.4, 3,000 85 : 104; rows of 333 and 667 tokens 18 : 25.
+//   Heads of 128: tiles of 128 keys with an SM alone are the faster ones (a launch of few blocks waits for its longest), tiles of 64 with two blocks on an
+//   SM the more per second.  More blocks than 296 (32 heads, 128 keys and pairs : 64 keys): 1,500 tokens 71 : 45, 2,048 88 : 65, 8,192 980 : 767, rows of
+//   645 tokens on 1,500 and of 1,292 138 : 73; fewer: 1,000 tokens 29 : 33, 2,048 tokens of 16 heads 45 : 59, 4,096 of 8 heads 76 : 108.
 template <int D, int MODS, bool KEEP>
 static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p, int work_tokens,
                      int work_rows, cudaStream_t stream) {
-    const size_t smem = (size_t)(D / 64) * 128 * 64 * 2 * 6 + 1024;     // 2 x Q + 2 x (K + V)
-    cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, MODS, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    // tiles <= tokens / 128 + rows (of the rows that this kernel serves, where the caller knows them); a block takes
-    // one tile, or a pair of them (at most (tiles + rows) / 2 pairs) once the tiles of all heads are more than the
-    // GPU runs at a time
     const int tiles = (work_tokens + FA_BM - 1) / FA_BM + work_rows;
+    const int64_t sms = device_sm_count(), blocks = (int64_t)((work_tokens + FA_BM - 1) / FA_BM + work_rows - 1) * p.num_heads;
     FaParams pp = p;
-    pp.pair = (int64_t)tiles * p.num_heads > (int64_t)device_sm_count() * (D == 64 ? 2 : 1);
-    const dim3 grid(pp.pair ? (tiles + work_rows + 1) / 2 : tiles, p.num_heads);
-    return launch_kernel(prefill_attention_tc_kernel<D, MODS, KEEP>, grid, dim3(FA_THREADS), smem, stream, mq, mk, mv, pp);
+    if constexpr (D == 128) {
+        if constexpr ((MODS & 3) == 0)
+            if (fa_keys(D, MODS, p.num_heads, work_tokens, work_rows) == 64) return launch_fa_tile<D, MODS, KEEP, 64>(mq, mk, mv, pp, tiles, work_rows, stream);
+        pp.pair = (int64_t)tiles * p.num_heads > sms;
+    } else if constexpr ((MODS & 3) != 0) {
+        pp.pair = (int64_t)tiles * p.num_heads > 2 * sms;          // (these instances have an SM alone)
+    } else {
+        pp.pair = work_rows == 1 && blocks <= 4 * sms && blocks * 10 > 33 * sms;
+    }
+    return launch_fa_tile<D, MODS, KEEP, 128>(mq, mk, mv, pp, tiles, work_rows, stream);
 }
 
 // q: the fused qkv activation [num_tokens, q_stride] bfloat16 (query head h at columns h*D ..), caches
@@ -1001,7 +1035,7 @@ extern "C" int mie_prefill_attention_tc(const void* q, int64_t q_stride, const v
     if (mods > 4) return MIE_ERR_BAD_ARG;              // a slope with a cap or a bias: the mma.sync kernel takes those
     p.check_pages = num_pages; p.report = g_range_report;
     CUtensorMap mq, mk, mv;
-    const int box_rows = page_size < FA_BN ? page_size : FA_BN;
+    const int keys = fa_keys(head_dim, mods, num_heads, work_tokens, work_rows), box_rows = page_size < keys ? page_size : keys;
     const uint64_t cache_rows = (uint64_t)num_pages * num_kv_heads * page_size;
     if ((rc = make_map_2d(&mq, q, (uint64_t)num_tokens, (uint64_t)q_stride, (uint64_t)q_stride, FA_BM))) return rc;
     if ((rc = make_map_2d(&mk, k_cache, cache_rows, (uint64_t)head_dim, (uint64_t)head_dim, box_rows))) return rc;
