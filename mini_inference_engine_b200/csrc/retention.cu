@@ -431,78 +431,98 @@ extern "C" int mie_head_rms_gate(const float* o, const void* g, int tag, long lo
 //   i_t = cap tanh((zi_t + bi) / cap)          f_t = logsigmoid(cap tanh((zf_t + bf) / cap))        (cap <= 0: no cap)
 //   m_t = max(f_t + m_{t-1}, i_t)              keep_t = exp(f_t + m_{t-1} - m_t)      write_t = exp(i_t - m_t)
 // z [T, 2H] float32 holds [zi: H | zf: H] per token; m_state [slots, H] carries m between steps (0 for a fresh request).
-// A warp per (row, head) takes 32 tokens at a time: with L_j the sum of f over the tile up to token j and m_c the maximum carried
+// A warp takes 32 tokens at a time: with L_j the sum of f over the tile up to token j and m_c the maximum carried
 // into the tile, m_j - L_j = max(m_c, max over s <= j of (i_s - L_s)), so a prefix sum and a prefix maximum by shuffles give all 32
 // maxima at once, and the sums never run over more than a tile (no large numbers are subtracted from one another).
-__global__ void gate_scan_kernel(const float* __restrict__ z, const float* __restrict__ bi, const float* __restrict__ bf, float cap,
+// A block per (row, head): a long row is cut into a segment for each of its 16 warps.  What a segment does to the maximum carried into it
+// is m -> max(m + sum of f, the maximum it builds from nothing); every warp works that out for its own segment first, takes the maximum through the segments
+// in front of it, and then writes its tokens' factors.  2,048 tokens of 8 heads: 36 us with one warp a row and head, XX us.
+#define GATE_WARPS 16
+__global__ void __launch_bounds__(GATE_WARPS * 32) gate_scan_kernel(const float* __restrict__ z, const float* __restrict__ bi, const float* __restrict__ bf, float cap,
                                  const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
                                  const int* __restrict__ state_slots, float* __restrict__ m_state, float* __restrict__ keep,
                                  float* __restrict__ write, float* __restrict__ m_out, int num_rows, int H) {
+    __shared__ float seg_sum[GATE_WARPS], seg_max[GATE_WARPS];
     pdl_enter();
-    const int lane = threadIdx.x & 31;
-    const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= num_rows * H) return;
-    const int r = item / H, h = item - r * H;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int r = blockIdx.x / H, h = blockIdx.x - r * H;
     const int start = row_q_start[r], len = row_q_len[r];
+    const int tiles = (len + 31) / 32, per = (tiles + warps - 1) / warps, t_lo = warp * per * 32, t_hi = min(len, t_lo + per * 32);
     float* ms = m_state + (int64_t)state_slots[r] * H + h;
-    float m_c = *ms;
+    const float m_row = *ms;
     const float b_i = bi ? bi[h] : 0.f, b_f = bf ? bf[h] : 0.f, inv = cap > 0.f ? 1.0f / cap : 0.f;
-    // four tiles' pre-activations are loaded before the first of them is scanned: the loads of a tile would otherwise stand
-    // in front of every tile's chain
-    for (int t00 = 0; t00 < len; t00 += 128) {
-        float zi4[4], zf4[4];
+    // the segment's tokens from the maximum m_c carried into it; returns the maximum behind them and leaves the sum of f in f_sum
+    auto walk = [&](float m_c, bool store, float& f_sum) {
+        f_sum = 0.f;
+        // four tiles' pre-activations are loaded before the first of them is scanned: the loads of a tile would otherwise stand
+        // in front of every tile's chain
+        for (int t00 = t_lo; t00 < t_hi; t00 += 128) {
+            float zi4[4], zf4[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int tt = t00 + 32 * k + lane;
-            const int64_t t = start + tt;
-            zi4[k] = tt < len ? z[t * 2 * H + h] : 0.f;
-            zf4[k] = tt < len ? z[t * 2 * H + H + h] : 0.f;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int t0 = t00 + 32 * k;
-            if (t0 >= len) break;
-            const bool ok = t0 + lane < len;
-            const int64_t t = start + t0 + lane;
-            float gi = -INFINITY, f = 0.f;                         // lanes beyond the row: nothing is written, nothing forgotten
-            if (ok) {
-                float zi = zi4[k] + b_i, zf = zf4[k] + b_f;
-                if (cap > 0.f) { zi = cap * tanhf(zi * inv); zf = cap * tanhf(zf * inv); }
-                gi = zi;
-                f = fminf(zf, 0.f) - log1pf(expf(-fabsf(zf)));     // log sigmoid
+            for (int k = 0; k < 4; ++k) {
+                const int tt = t00 + 32 * k + lane;
+                const int64_t t = start + tt;
+                zi4[k] = tt < t_hi ? z[t * 2 * H + h] : 0.f;
+                zf4[k] = tt < t_hi ? z[t * 2 * H + H + h] : 0.f;
             }
-            float L = f;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, L, o); if (lane >= o) L += up; }
-            const float own = gi - L;
-            float a = own;
+            for (int k = 0; k < 4; ++k) {
+                const int t0 = t00 + 32 * k;
+                if (t0 >= t_hi) break;
+                const bool ok = t0 + lane < t_hi;
+                const int64_t t = start + t0 + lane;
+                float gi = -INFINITY, f = 0.f;                     // lanes beyond the row: nothing is written, nothing forgotten
+                if (ok) {
+                    float zi = zi4[k] + b_i, zf = zf4[k] + b_f;
+                    if (cap > 0.f) { zi = cap * tanhf(zi * inv); zf = cap * tanhf(zf * inv); }
+                    gi = zi;
+                    f = fminf(zf, 0.f) - log1pf(expf(-fabsf(zf)));     // log sigmoid
+                }
+                float L = f;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, a, o); if (lane >= o) a = fmaxf(a, up); }
-            // u_j = m_j - L_j never falls, and f_j + m_{j-1} - m_j = u_{j-1} - u_j: where a token only forgets, its keep factor is
-            // exactly 1, and where it sets the maximum, its write factor is; no difference of large sums enters a factor that the
-            // state multiplies up over many tokens
-            const float u = fmaxf(m_c, a);
-            float u_prev = __shfl_up_sync(0xffffffffu, u, 1);
-            if (lane == 0) u_prev = m_c;
-            const float m = L + u;
-            if (ok) {
-                keep[t * H + h] = expf(u_prev - u);
-                write[t * H + h] = expf(own - u);
-                m_out[t * H + h] = m;
+                for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, L, o); if (lane >= o) L += up; }
+                const float own = gi - L;
+                float a = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, a, o); if (lane >= o) a = fmaxf(a, up); }
+                // u_j = m_j - L_j never falls, and f_j + m_{j-1} - m_j = u_{j-1} - u_j: where a token only forgets, its keep factor is
+                // exactly 1, and where it sets the maximum, its write factor is; no difference of large sums enters a factor that the
+                // state multiplies up over many tokens
+                const float u = fmaxf(m_c, a);
+                float u_prev = __shfl_up_sync(0xffffffffu, u, 1);
+                if (lane == 0) u_prev = m_c;
+                const float m = L + u;
+                if (ok && store) {
+                    keep[t * H + h] = expf(u_prev - u);
+                    write[t * H + h] = expf(own - u);
+                    m_out[t * H + h] = m;
+                }
+                const int end = min(31, t_hi - t0 - 1);
+                m_c = __shfl_sync(0xffffffffu, m, end);
+                f_sum += __shfl_sync(0xffffffffu, L, end);
             }
-            m_c = __shfl_sync(0xffffffffu, m, min(31, len - t0 - 1));
         }
+        return m_c;
+    };
+    float m_in = m_row, sum;
+    if (tiles > per) {                                             // more than one segment
+        const float built = walk(-INFINITY, false, sum);
+        if (lane == 0) { seg_sum[warp] = sum; seg_max[warp] = built; }
+        __syncthreads();                                           // (every thread is past its read of *ms, too)
+        for (int s = 0; s < warp && s * per < tiles; ++s) m_in = fmaxf(m_in + seg_sum[s], seg_max[s]);
     }
-    if (lane == 0) *ms = m_c;
+    if (t_lo >= len) return;
+    const float m_end = walk(m_in, true, sum);
+    if (t_hi == len && lane == 0) *ms = m_end;
 }
 
 extern "C" int mie_gate_scan(const float* z, const float* bi, const float* bf, float cap, const int* row_q_start, const int* row_q_len,
-                             const int* state_slots, float* m_state, float* keep, float* write, float* m_out, int num_rows, int H,
+                             const int* state_slots, float* m_state, float* keep, float* write, float* m_out, int max_q_len, int num_rows, int H,
                              cudaStream_t stream) {
     if (num_rows <= 0) return 0;
     if (H <= 0) return MIE_ERR_BAD_ARG;
-    const int items = num_rows * H, warps = 2;
-    return launch_kernel(gate_scan_kernel, dim3((items + warps - 1) / warps), dim3(warps * 32), 0, stream, z, bi, bf, cap, row_q_start,
+    // one warp where no row has more than a tile (a launch bound by its start)
+    return launch_kernel(gate_scan_kernel, dim3(num_rows * H), dim3(max_q_len > 32 ? GATE_WARPS * 32 : 32), 0, stream, z, bi, bf, cap, row_q_start,
                          row_q_len, state_slots, m_state, keep, write, m_out, num_rows, H);
 }
 
@@ -523,21 +543,39 @@ __global__ void group_norm_gate_kernel(const float* __restrict__ o, int stride, 
     const int64_t t = item / groups;
     const int g = (int)(item - t * groups);
     const float* src = o + item * stride;
+    const T* gt = gate ? gate + t * g_stride + (int64_t)g * size : nullptr;
+    // the weight of entry i: its place in the row modulo w_len (a division an entry only where w_len is neither the group's size nor the row's)
+    const bool plain_w = w && (w_len == size || w_len >= groups * size);
+    const float* wp = plain_w && w_len != size ? w + g * size : w;
+    auto finish = [&](int i, float v, float zz) {
+        if (w) v *= plain_w ? wp[i] : w[(g * size + i) % w_len];
+        if (gt) v *= gate_silu ? zz / (1.0f + expf(-zz)) : 1.0f / (1.0f + expf(-zz));
+        out[(t * groups + g) * size + i] = from_f32<T>(v);
+    };
     float scale = 1.f;
+    if (size <= 512) {                                             // a group stays in registers between its two uses, and all its loads are out together
+        float v[16], zz[16];
+        const float nrm = normalizer ? src[size] : 0.f, mm = normalizer ? m[item] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int i = lane + 32 * k;
+            v[k] = i < size ? src[i] : 0.f;
+            zz[k] = gt && i < size ? to_f32<T>(gt[i]) : 0.f;
+        }
+        if (normalizer) scale = 1.0f / (fmaxf(fabsf(nrm), expf(-mm)) + 1e-6f);
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) { const float x = v[k] * scale; ss += x * x; }
+        const float s = scale / sqrtf(warp_sum(ss) / (float)size + eps);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) if (lane + 32 * k < size) finish(lane + 32 * k, v[k] * s, zz[k]);
+        return;
+    }
     if (normalizer) scale = 1.0f / (fmaxf(fabsf(src[size]), expf(-m[item])) + 1e-6f);
     float ss = 0.f;
     for (int i = lane; i < size; i += 32) { const float v = src[i] * scale; ss += v * v; }
     const float s = scale / sqrtf(warp_sum(ss) / (float)size + eps);
-    const T* gt = gate ? gate + t * g_stride + (int64_t)g * size : nullptr;
-    for (int i = lane; i < size; i += 32) {
-        float v = src[i] * s;
-        if (w) v *= w[(g * size + i) % w_len];
-        if (gt) {
-            const float zz = to_f32<T>(gt[i]);
-            v *= gate_silu ? zz / (1.0f + expf(-zz)) : 1.0f / (1.0f + expf(-zz));
-        }
-        out[(t * groups + g) * size + i] = from_f32<T>(v);
-    }
+    for (int i = lane; i < size; i += 32) finish(i, src[i] * s, gt ? to_f32<T>(gt[i]) : 0.f);
 }
 
 extern "C" int mie_group_norm_gate(const float* o, int stride, const float* m, const float* w, int w_len, const void* gate, int tag,

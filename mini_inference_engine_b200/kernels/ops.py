@@ -984,11 +984,11 @@ def decay_scan(rows_in: torch.Tensor, positions, row_q_start, row_q_len, state_s
                        act, q_scale, k_scale, freq, rot, q_lens)
 
 
-def gate_scan(z: torch.Tensor, bias_i, bias_f, cap: float, row_q_start, row_q_len, state_slots, m_state: torch.Tensor, num_heads: int):
+def gate_scan(z: torch.Tensor, bias_i, bias_f, cap: float, row_q_start, row_q_len, state_slots, m_state: torch.Tensor, num_heads: int, max_q_len=None):
     """Exponential gates with a running maximum, token by token per row and head: from z [T, 2H] float32 = [input | forget]
     pre-activations, i = cap tanh((zi + bias_i) / cap), f = logsigmoid(cap tanh((zf + bias_f) / cap)) (``cap`` 0: no cap),
     m_t = max(f + m_{t-1}, i), keep = exp(f + m_{t-1} - m_t), write = exp(i - m_t).  ``m_state`` [slots, H] float32 carries m.
-    Returns (keep, write, m), float32 [T, H] each."""
+    ``max_q_len``: the longest row the launch may meet, where the caller knows.  Returns (keep, write, m), float32 [T, H] each."""
     T = z.shape[0]
     _need(z.dtype == torch.float32 and z.is_contiguous() and z.shape == (T, 2 * num_heads), "gate pre-activations must be float32 [T, 2H]")
     _need(m_state.dtype == torch.float32 and m_state.is_contiguous() and tuple(m_state.shape[1:]) == (num_heads,), "m state must be float32 [slots, H]")
@@ -999,8 +999,8 @@ def gate_scan(z: torch.Tensor, bias_i, bias_f, cap: float, row_q_start, row_q_le
         _i32(t_, n)
     keep, write, m = (torch.empty(T, num_heads, dtype=torch.float32, device=z.device) for _ in range(3))
     _check(load("retention").mie_gate_scan(_ptr(z), _ptr(bias_i), _ptr(bias_f), ctypes.c_float(cap), _ptr(row_q_start), _ptr(row_q_len),
-                                           _ptr(state_slots), _ptr(m_state), _ptr(keep), _ptr(write), _ptr(m), row_q_len.numel(),
-                                           num_heads, _stream()), "gate_scan")
+                                           _ptr(state_slots), _ptr(m_state), _ptr(keep), _ptr(write), _ptr(m), int(T if max_q_len is None else max_q_len),
+                                           row_q_len.numel(), num_heads, _stream()), "gate_scan")
     return keep, write, m
 
 

@@ -56,7 +56,7 @@ class MatrixMemory(Mixer):
         z = self.rt.linear(x, self.w_gates, None, out_dtype=torch.float32)
         if z.shape[1] != 2 * H:
             z = z[:, :2 * H].contiguous()
-        keep, write, m = ops.gate_scan(z, self.b_i, self.b_f, self.gate_cap, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, m_state, H)
+        keep, write, m = ops.gate_scan(z, self.b_i, self.b_f, self.gate_cap, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, m_state, H, ctx.max_q_len)
         o = self.rt.empty(T, H * (Dv + 1), dtype=torch.float32)
         ops.decay_scan(proj, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o, num_heads=H, dim=D, vdim=Dv,
                        max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), tok_decay=keep, k_tok=write, ones=True, q_scale=D ** -0.5)
