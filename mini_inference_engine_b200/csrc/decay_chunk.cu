@@ -7,10 +7,9 @@
 // so a token costs 2 D Dv multiply-adds and half a chunk's of Q K^T and P V, out of shared memory in tiles of registers, where token by token it costs
 // 5 D Dv in two passes, with a shared-memory read for every one or two.  Products of decays are products (no logarithms: a decay may be 0).  Float32 on the CUDA cores throughout.
 //
-//   scores   a block per (chunk, head): P = Q K^T * M (lower triangle) and G into scratch memory.
-//   states   a block per (chunk, head, 64 value columns): what the chunk adds to the state -> states[chunk].
+//   local    a block per (chunk, head, half of the value columns): P = Q K^T * M (lower triangle) and G into scratch memory, and what the chunk adds to the state -> states[chunk].
 //   combine  per row in order: states[chunk] becomes the state in front of the chunk; the state after the last goes to the request's slot.
-//   output   a block per (chunk, head, 128 value columns).
+//   output   a block per (chunk, head, 64 value columns).
 //
 // Rows of one chunk are left to retention.cu.  q and k come prepared (rotated or activated, scaled) as float32 from its first kernel.  Bound: the
 // CUDA cores' multiply-adds.
@@ -52,11 +51,6 @@ __device__ __forceinline__ float dc_value(const DcParams& p, int64_t token, int 
     return p.v_act ? v / (1.0f + expf(-v)) : v;
 }
 
-// The decay of the chunk's token i (tokens beyond the row's end decay nothing).
-__device__ __forceinline__ float dc_decay(const DcParams& p, int t0, int count, int i, int h) {
-    return i >= count ? 1.f : p.tok_decay ? p.tok_decay[(int64_t)(t0 + i) * p.H + h] : p.decay[h];
-}
-
 // Which chunk this block has: its row, its number in the row; the blocks count chunks of rows of two or more.
 __device__ __forceinline__ bool dc_find(const DcParams& p, int* s_row, int* s_chunk) {
     if (threadIdx.x < 32) {
@@ -68,24 +62,24 @@ __device__ __forceinline__ bool dc_find(const DcParams& p, int* s_row, int* s_ch
     return *s_row >= 0;
 }
 
-// P and G of a (chunk, head): 64 x 64 entries, the blocks of 16 x 16 above the diagonal left out.
-template <int DT>
-__global__ void __launch_bounds__(256, 2) decay_scores_kernel(const DcParams p) {
+template <typename T, int DT>
+__global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, int halves) {
     constexpr int DP = DT + 4;
     extern __shared__ __align__(16) float sm[];
     float* Q = sm;                                     // [64][DP]
     float* K = Q + DC_L * DP;                          // [64][DP]
-    float* M = K + DC_L * DP;                          // [64][DC_P]: products of decays
+    float* M = K + DC_L * DP;                          // [64][DC_P]: products of decays; then a tile of values [64 tokens][DC_P]
     __shared__ float a[DC_L], G[DC_L];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
     if (!dc_find(p, &s_row, &s_chunk)) return;
     pdl_wait();
-    const int h = blockIdx.y, H = p.H, D = p.D;
+    const int h = blockIdx.y, H = p.H, D = p.D, half = blockIdx.z;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     dc_rows<DT>(K, p.k + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
-    dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
-    if (threadIdx.x < DC_L) a[threadIdx.x] = dc_decay(p, t0, count, threadIdx.x, h);
+    if (half == 0) dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
+    if (threadIdx.x < DC_L)
+        a[threadIdx.x] = threadIdx.x >= count ? 1.f : p.tok_decay ? p.tok_decay[(int64_t)(t0 + threadIdx.x) * H + h] : p.decay[h];
     __syncthreads();
     if (threadIdx.x < DC_L) {                          // a column of M a thread
         const int j = threadIdx.x;
@@ -103,118 +97,97 @@ __global__ void __launch_bounds__(256, 2) decay_scores_kernel(const DcParams p) 
     dc_wait_all();
     __syncthreads();
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float* out = dc_scratch(p, blockIdx.x, h);
-    float s[4][4];
+    if (half == 0) {
+        float* out = dc_scratch(p, blockIdx.x, h);
+        float s[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
 #pragma unroll 4
-    for (int d = 0; d < DT; d += 4) {
-        float4 kk[4];
+        for (int d = 0; d < DT; d += 4) {
+            float4 kk[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * DP + d);
+            for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * DP + d);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * DP + d);
+            for (int i = 0; i < 4; ++i) {
+                const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * DP + d);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (j > i) continue;               // wholly above the diagonal
-                s[i][j] = fmaf(qq.x, kk[j].x, s[i][j]);
-                s[i][j] = fmaf(qq.y, kk[j].y, s[i][j]);
-                s[i][j] = fmaf(qq.z, kk[j].z, s[i][j]);
-                s[i][j] = fmaf(qq.w, kk[j].w, s[i][j]);
+                for (int j = 0; j < 4; ++j) {
+                    if (j > i) continue;               // wholly above the diagonal
+                    s[i][j] = fmaf(qq.x, kk[j].x, s[i][j]);
+                    s[i][j] = fmaf(qq.y, kk[j].y, s[i][j]);
+                    s[i][j] = fmaf(qq.z, kk[j].z, s[i][j]);
+                    s[i][j] = fmaf(qq.w, kk[j].w, s[i][j]);
+                }
             }
         }
-    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = ty + 16 * i, c = tx + 16 * j;
-            out[r * DC_L + c] = c <= r ? s[i][j] * M[r * DC_P + c] : 0.f;
-        }
-    if (threadIdx.x < DC_L) out[DC_L * DC_L + threadIdx.x] = G[threadIdx.x];
-}
-
-// What a (chunk, head) adds to 64 columns of the state: a thread 8 columns x 8 (DT 64: 4) entries of the key, so that shared memory gives a byte a
-// multiply-add (a 4 x 8 tile is bound by those reads).
-template <typename T, int DT>
-__global__ void __launch_bounds__(128, 4) decay_states_kernel(const DcParams p) {
-    constexpr int DP = DT + 4, E = DT / 64;
-    extern __shared__ __align__(16) float sm[];
-    float* K = sm;                                     // [64][DP]: keys with what is left of them at the chunk's end
-    float* V = K + DC_L * DP;                          // [64][DC_P]
-    __shared__ float a[DC_L], left[DC_L];
-    __shared__ int s_row, s_chunk;
-    pdl_launch_dependents();
-    if (!dc_find(p, &s_row, &s_chunk)) return;
-    pdl_wait();
-    const int h = blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
-    const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
-    dc_rows<DT>(K, p.k + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
-    if (threadIdx.x < DC_L) a[threadIdx.x] = dc_decay(p, t0, count, threadIdx.x, h);
-#pragma unroll 8
-    for (int i = threadIdx.x; i < DC_L * 64; i += 128) {
-        const int t = i >> 6, c = i & 63;
-        V[t * DC_P + c] = t < count && c0 + c < p.Dv_in ? dc_value<T>(p, t0 + t, h, c0 + c) : 0.f;
+            for (int j = 0; j < 4; ++j) {
+                const int r = ty + 16 * i, c = tx + 16 * j;
+                out[r * DC_L + c] = c <= r ? s[i][j] * M[r * DC_P + c] : 0.f;
+            }
+        if (threadIdx.x < DC_L) out[DC_L * DC_L + threadIdx.x] = G[threadIdx.x];
     }
+    // keys with what is left of them at the chunk's end (in place: the scores are done with them once every thread is here)
+    const float w_mine = M[(count - 1) * DC_P + (threadIdx.x & 63)];
     __syncthreads();
-    if (threadIdx.x < 32) {                            // products of the decays behind a token, two tokens a lane
-        const float a1 = a[2 * threadIdx.x + 1];
-        float run = a[2 * threadIdx.x] * a1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const float down = __shfl_down_sync(0xffffffffu, run, o); if (threadIdx.x + o < 32) run *= down; }
-        float behind = __shfl_down_sync(0xffffffffu, run, 1);
-        if (threadIdx.x == 31) behind = 1.f;
-        left[2 * threadIdx.x + 1] = behind;
-        left[2 * threadIdx.x] = a1 * behind;
-    }
-    dc_wait_all();
+    if (threadIdx.x < DC_L) a[threadIdx.x] = threadIdx.x < count ? w_mine : 0.f;
     __syncthreads();
-    for (int i = threadIdx.x; i < DC_L * (DT / 4); i += 128) {
+    for (int i = threadIdx.x; i < DC_L * (DT / 4); i += 256) {
         const int r = i / (DT / 4);
         float4* at = reinterpret_cast<float4*>(K + r * DP + (i - r * (DT / 4)) * 4);
         float4 v = *at;
-        const float w = left[r];
+        const float w = a[r];
         v.x *= w; v.y *= w; v.z *= w; v.w *= w;
         *at = v;
     }
-    __syncthreads();
+    // the state's columns, 64 at a time: column 4 ty + c, entries 4 tx + 64 e .. + 3
     float* to = p.states + ((int64_t)blockIdx.x * H + h) * (int64_t)p.Dv * D;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;      // columns 4 ty + c and 32 + 4 ty + c, entries 4 tx + 64 e .. + 3
-    float s[8][4 * E];
+    constexpr int E = DT / 64;
+    const int tiles = (p.Dv_in + 63) / 64, per = (tiles + halves - 1) / halves;
+    for (int tile = half * per; tile < min(tiles, (half + 1) * per); ++tile) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < DC_L * 64; i += 256) {
+            const int t = i >> 6, c = i & 63, col = tile * 64 + c;
+            M[t * DC_P + c] = t < count && col < p.Dv_in ? dc_value<T>(p, t0 + t, h, col) : 0.f;
+        }
+        __syncthreads();
+        float s[4][4 * E];
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int e = 0; e < 4 * E; ++e) s[c][e] = 0.f;
+            for (int e = 0; e < 4 * E; ++e) s[c][e] = 0.f;
 #pragma unroll 4
-    for (int t = 0; t < DC_L; ++t) {
-        const float4 v0 = *reinterpret_cast<const float4*>(V + t * DC_P + 4 * ty), v1 = *reinterpret_cast<const float4*>(V + t * DC_P + 32 + 4 * ty);
-        const float vc[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        for (int t = 0; t < DC_L; ++t) {
+            const float4 vv = *reinterpret_cast<const float4*>(M + t * DC_P + 4 * ty);
+            const float vc[4] = {vv.x, vv.y, vv.z, vv.w};
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const float4 kk = *reinterpret_cast<const float4*>(K + t * DP + 64 * e + 4 * tx);
+            for (int e = 0; e < E; ++e) {
+                const float4 kk = *reinterpret_cast<const float4*>(K + t * DP + 64 * e + 4 * tx);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                s[c][4 * e] = fmaf(vc[c], kk.x, s[c][4 * e]);
-                s[c][4 * e + 1] = fmaf(vc[c], kk.y, s[c][4 * e + 1]);
-                s[c][4 * e + 2] = fmaf(vc[c], kk.z, s[c][4 * e + 2]);
-                s[c][4 * e + 3] = fmaf(vc[c], kk.w, s[c][4 * e + 3]);
+                for (int c = 0; c < 4; ++c) {
+                    s[c][4 * e] = fmaf(vc[c], kk.x, s[c][4 * e]);
+                    s[c][4 * e + 1] = fmaf(vc[c], kk.y, s[c][4 * e + 1]);
+                    s[c][4 * e + 2] = fmaf(vc[c], kk.z, s[c][4 * e + 2]);
+                    s[c][4 * e + 3] = fmaf(vc[c], kk.w, s[c][4 * e + 3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int col = tile * 64 + 4 * ty + c;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const int d = 64 * e + 4 * tx;
+                if (col < p.Dv_in && d < D)
+                    *reinterpret_cast<float4*>(to + (int64_t)col * D + d) = make_float4(s[c][4 * e], s[c][4 * e + 1], s[c][4 * e + 2], s[c][4 * e + 3]);
             }
         }
     }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const int col = c0 + (c >> 2) * 32 + 4 * ty + (c & 3);
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int d = 64 * e + 4 * tx;
-            if (col < p.Dv_in && d < D)
-                *reinterpret_cast<float4*>(to + (int64_t)col * D + d) = make_float4(s[c][4 * e], s[c][4 * e + 1], s[c][4 * e + 2], s[c][4 * e + 3]);
-        }
-    }
-    if (blockIdx.z == 0 && p.Dv > p.Dv_in && threadIdx.x < D) {      // the column fed with ones: the sum of the keys
+    if (half == 0 && p.Dv > p.Dv_in && threadIdx.x < D) {      // the column fed with ones: the sum of the keys
         float sum = 0.f;
         for (int t = 0; t < DC_L; ++t) sum += K[t * DP + threadIdx.x];
         to[(int64_t)p.Dv_in * D + threadIdx.x] = sum;
@@ -254,139 +227,99 @@ __global__ void __launch_bounds__(128) decay_combine_kernel(const DcParams p) {
     *reinterpret_cast<float4*>(end) = cur;
 }
 
-// 64 tokens x 128 columns a block, 8 x 8 a thread (a byte of shared memory a multiply-add): one product over the key's entries and then the chunk's
-// tokens, [Q | P] [S ; V], in slices of 32 through two buffers -- keys, states and P by asynchronous copies, the values through registers.
-#define DO_K 32
-#define DO_P 36                 // stride of a row of 32
-template <typename T>
-__global__ void __launch_bounds__(128, 3) decay_output_kernel(const DcParams p) {
-    extern __shared__ __align__(16) float sm[];        // two buffers of A [64][DO_P] | B [128][DO_P], or of B the values [32][128]
-    constexpr int A_FLOATS = DC_L * DO_P, STAGE = A_FLOATS + 128 * DO_P;
+template <typename T, int DT>
+__global__ void __launch_bounds__(256, 2) decay_output_kernel(const DcParams p) {
+    constexpr int DP = DT + 4;
+    extern __shared__ __align__(16) float sm[];
+    float* Q = sm;                                     // [64][DP]
+    float* S = Q + DC_L * DP;                          // the state's columns [64][DP]
+    float* P = S + 64 * DP;                            // [64][DC_P]
+    float* VT = P + DC_L * DC_P;                       // values, a column a row [64][DC_P]
     __shared__ float G[DC_L];
+    __shared__ __align__(16) float n[DT];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
     if (!dc_find(p, &s_row, &s_chunk)) return;
     pdl_wait();
-    const int h = blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 128;
+    const int h = blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     const float* from = p.states + ((int64_t)blockIdx.x * H + h) * (int64_t)p.Dv * D;
-    const float* q = p.q + ((int64_t)t0 * H + h) * D;
     const float* pg = dc_scratch(p, blockIdx.x, h);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, nq = (D + DO_K - 1) / DO_K, col = c0 + threadIdx.x;
+    const bool ones = blockIdx.z == 0 && p.Dv > p.Dv_in;
+    dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
+    dc_rows<DT>(S, from + (int64_t)c0 * D, D, D, min(64, p.Dv_in - c0));
+    for (int i = threadIdx.x; i < DC_L * (DC_L / 4); i += 256) dc_copy16(P + (i >> 4) * DC_P + (i & 15) * 4, pg + i * 4, true);
     if (threadIdx.x < DC_L) G[threadIdx.x] = pg[DC_L * DC_L + threadIdx.x];
-    float next[DO_K];                                  // the values of this thread's column in the slice that comes
-    auto issue = [&](int sl) {
-        if (sl < nq + 2) {
-            float* A = sm + (sl & 1) * STAGE;
-            float* B = A + A_FLOATS;
-            const int k0 = sl < nq ? sl * DO_K : (sl - nq) * DO_K;
+    if (ones && threadIdx.x < DT) n[threadIdx.x] = threadIdx.x < D ? from[(int64_t)p.Dv_in * D + threadIdx.x] : 0.f;
+    for (int i = threadIdx.x; i < DC_L * 64; i += 256) {
+        const int t = i >> 6, c = i & 63;
+        VT[c * DC_P + t] = t < count && c0 + c < p.Dv_in ? dc_value<T>(p, t0 + t, h, c0 + c) : 0.f;
+    }
+    dc_wait_all();
+    __syncthreads();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float o[4][4];
 #pragma unroll
-            for (int i = threadIdx.x; i < DC_L * (DO_K / 4); i += 128) {
-                const int r = i >> 3, k = k0 + (i & 7) * 4;
-                const bool on = sl >= nq || (r < count && k < D);
-                dc_copy16(A + r * DO_P + (i & 7) * 4, sl >= nq ? pg + r * DC_L + k : on ? q + (int64_t)r * H * D + k : q, on);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < DT; d += 4) {
+        float4 ss[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss[j] = *reinterpret_cast<const float4*>(S + (tx + 16 * j) * DP + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * DP + d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                o[i][j] = fmaf(qq.x, ss[j].x, o[i][j]);
+                o[i][j] = fmaf(qq.y, ss[j].y, o[i][j]);
+                o[i][j] = fmaf(qq.z, ss[j].z, o[i][j]);
+                o[i][j] = fmaf(qq.w, ss[j].w, o[i][j]);
             }
-            if (sl < nq) {
-#pragma unroll
-                for (int i = threadIdx.x; i < 128 * (DO_K / 4); i += 128) {
-                    const int r = i >> 3, k = k0 + (i & 7) * 4;
-                    const bool on = c0 + r < p.Dv_in && k < D;
-                    dc_copy16(B + r * DO_P + (i & 7) * 4, on ? from + (int64_t)(c0 + r) * D + k : from, on);
-                }
-            } else {
-#pragma unroll
-                for (int t = 0; t < DO_K; ++t) next[t] = k0 + t < count && col < p.Dv_in ? dc_value<T>(p, t0 + k0 + t, h, col) : 0.f;
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    float o[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
-    issue(0);
-    for (int sl = 0; sl < nq + 2; ++sl) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        issue(sl + 1);
-        const float* A = sm + (sl & 1) * STAGE;
-        const float* B = A + A_FLOATS;
-        if (sl < nq) {
-#pragma unroll
-            for (int k = 0; k < DO_K; k += 4) {
-                float4 b[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * DO_P + k);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 x = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * DO_P + k);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        o[i][j] = fmaf(x.x, b[j].x, o[i][j]);
-                        o[i][j] = fmaf(x.y, b[j].y, o[i][j]);
-                        o[i][j] = fmaf(x.z, b[j].z, o[i][j]);
-                        o[i][j] = fmaf(x.w, b[j].w, o[i][j]);
-                    }
-                }
-            }
-            if (sl == nq - 1) {                        // what the state gave, with the decays since the chunk's start
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float g = G[ty + 8 * i];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) o[i][j] *= g;
-                }
-            }
-        } else {
-            const int k0 = (sl - nq) * DO_K;
-#pragma unroll 2
-            for (int k = 0; k < DO_K; k += 4) {
-                float b[4][8];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) b[e][j] = B[(k + e) * 128 + tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = ty + 8 * i - k0 - k;         // tokens of this group that row i sees: those up to r
-                    if (r < 0) continue;                       // (later tokens: their values, whatever they are, do not enter)
-                    const float4 x = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * DO_P + k);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        o[i][j] = fmaf(x.x, b[0][j], o[i][j]);
-                        if (r >= 1) o[i][j] = fmaf(x.y, b[1][j], o[i][j]);
-                        if (r >= 2) o[i][j] = fmaf(x.z, b[2][j], o[i][j]);
-                        if (r >= 3) o[i][j] = fmaf(x.w, b[3][j], o[i][j]);
-                    }
-                }
-            }
-        }
-        if (sl + 1 >= nq && sl + 1 < nq + 2) {         // (nobody reads that buffer until the next barrier)
-            float* B2 = sm + ((sl + 1) & 1) * STAGE + A_FLOATS;
-#pragma unroll
-            for (int t = 0; t < DO_K; ++t) B2[t * 128 + threadIdx.x] = next[t];
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = ty + 8 * i;
+    for (int i = 0; i < 4; ++i) {
+        const float g = G[ty + 16 * i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i][j] *= g;
+    }
+    for (int t = 0; t < DC_L; t += 4) {
+        float4 vv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) vv[j] = *reinterpret_cast<const float4*>(VT + (tx + 16 * j) * DC_P + t);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = ty + 16 * i;
+            if (t > r) continue;                       // (later tokens: their values, whatever they are, do not enter)
+            const float4 pp = *reinterpret_cast<const float4*>(P + r * DC_P + t);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                o[i][j] = fmaf(pp.x, vv[j].x, o[i][j]);
+                if (t + 1 <= r) o[i][j] = fmaf(pp.y, vv[j].y, o[i][j]);
+                if (t + 2 <= r) o[i][j] = fmaf(pp.z, vv[j].z, o[i][j]);
+                if (t + 3 <= r) o[i][j] = fmaf(pp.w, vv[j].w, o[i][j]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
         if (r >= count) continue;
         float* to = p.out + ((int64_t)(t0 + r) * H + h) * p.Dv;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) if (c0 + tx + 16 * j < p.Dv_in) to[c0 + tx + 16 * j] = o[i][j];
+        for (int j = 0; j < 4; ++j) if (c0 + tx + 16 * j < p.Dv_in) to[c0 + tx + 16 * j] = o[i][j];
     }
-    if (blockIdx.z == 0 && p.Dv > p.Dv_in) {           // the column fed with ones, n . q: two lanes a token
-        const int r = threadIdx.x >> 1, part = threadIdx.x & 1;
+    if (ones) {                                        // n . q: four lanes a token
+        const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
         float dot = 0.f, sum = 0.f;
-        if (r < count)
-            for (int d = 4 * part; d < D; d += 8) {
-                const float4 x = *reinterpret_cast<const float4*>(q + (int64_t)r * H * D + d), n = *reinterpret_cast<const float4*>(from + (int64_t)p.Dv_in * D + d);
-                dot = fmaf(x.x, n.x, dot); dot = fmaf(x.y, n.y, dot); dot = fmaf(x.z, n.z, dot); dot = fmaf(x.w, n.w, dot);
-            }
-        for (int t = part; t <= r; t += 2) sum += pg[r * DC_L + t];
+        for (int d = part; d < DT; d += 4) dot = fmaf(Q[r * DP + d], n[d], dot);
+        for (int t = part; t <= r; t += 4) sum += P[r * DC_P + t];
         float v = fmaf(G[r], dot, sum);
         v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
         if (part == 0 && r < count) p.out[((int64_t)(t0 + r) * H + h) * p.Dv + p.Dv_in] = v;
     }
 }
@@ -405,23 +338,20 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(states) |
          reinterpret_cast<uintptr_t>(scratch)) & 15) return MIE_ERR_BAD_ARG;
     const DcParams p{q, k, v, v_stride, row_q_start, row_q_len, state_slots, num_rows, decay, tok_decay, state, states, scratch, out, H, D, Dv_in, Dv, v_act};
+    const int halves = Dv_in > 64 ? 2 : 1;
     const int64_t quads = (int64_t)H * Dv * D / 4;
     int rc;
 #define DC_LAUNCH(T, DT)                                                                                                                  \
     {                                                                                                                                     \
-        const int smem_p = (2 * DC_L * (DT + 4) + DC_L * DC_P) * 4, smem_s = (DC_L * (DT + 4) + DC_L * DC_P) * 4;                         \
-        const int smem_o = 2 * (DC_L + 128) * DO_P * 4;                                                                                   \
-        cudaError_t e = cudaFuncSetAttribute(decay_scores_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_p);               \
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_states_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s);  \
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_output_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_o);      \
+        const int smem_l = (2 * DC_L * (DT + 4) + DC_L * DC_P) * 4, smem_o = ((DC_L + 64) * (DT + 4) + 2 * DC_L * DC_P) * 4;              \
+        cudaError_t e = cudaFuncSetAttribute(decay_local_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l);             \
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_output_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_o);  \
         if (e != cudaSuccess) return (int)e;                                                                                              \
-        rc = launch_kernel(decay_scores_kernel<DT>, dim3(chunks, H), dim3(256), smem_p, stream, p);                                       \
-        if (rc) return rc;                                                                                                                \
-        rc = launch_kernel(decay_states_kernel<T, DT>, dim3(chunks, H, (Dv_in + 63) / 64), dim3(128), smem_s, stream, p);                 \
+        rc = launch_kernel(decay_local_kernel<T, DT>, dim3(chunks, H, halves), dim3(256), smem_l, stream, p, halves);                     \
         if (rc) return rc;                                                                                                                \
         rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), num_rows), dim3(128), 0, stream, p);               \
         if (rc) return rc;                                                                                                                \
-        return launch_kernel(decay_output_kernel<T>, dim3(chunks, H, (Dv_in + 127) / 128), dim3(128), smem_o, stream, p);                 \
+        return launch_kernel(decay_output_kernel<T, DT>, dim3(chunks, H, (Dv_in + 63) / 64), dim3(256), smem_o, stream, p);               \
     }
     if (v_tag == MIE_F32) { if (D <= 64) DC_LAUNCH(float, 64) else DC_LAUNCH(float, 128) }
     if (v_tag == MIE_BF16) { if (D <= 64) DC_LAUNCH(bf16, 64) else DC_LAUNCH(bf16, 128) }
