@@ -984,6 +984,43 @@ def decay_scan(rows_in: torch.Tensor, positions, row_q_start, row_q_len, state_s
                        act, q_scale, k_scale, freq, rot, q_lens)
 
 
+def decay_step_takes(rows_in, state, dim: int, rot: int, vdim: int) -> bool:
+    """Whether ``decay_step`` serves these operands (four entries at a time)."""
+    return (dim % 4 == 0 and dim <= 128 and rot % 8 == 0 and vdim < 8192 and rows_in.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
+            and rows_in.data_ptr() % (4 * rows_in.element_size()) == 0)
+
+
+def decay_step(rows_in: torch.Tensor, positions, row_q_start, state_slots, state, out=None, *, num_heads: int, dim: int, vdim: int, decay=None, tok_decay=None,
+               k_tok=None, act: bool = False, ones: bool = False, q_scale: float = 1.0, k_scale: float = 1.0, freq=None, rot: int = 0, gate=None, gated=None,
+               eps: float = 0.0) -> torch.Tensor:
+    """``decay_scan`` for a step whose rows all have one new token, in one launch.  With ``gated`` [T, H * vdim] (of the rows' type) each head's outputs are divided by
+    their root mean square, multiplied by silu of ``gate`` [T, H * vdim] (a column slice will do) and written there instead of ``out``."""
+    T, dv = rows_in.shape[0], vdim + int(ones)
+    _need(rows_in.dim() == 2 and rows_in.stride(1) == 1 and rows_in.shape[1] >= num_heads * (2 * dim + vdim), "rows must hold q, k and v")
+    _need(decay_step_takes(rows_in, state, dim, rot, vdim), "decay_step takes keys, rows and states in steps of four entries, keys of up to 128")
+    _need(state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (num_heads, dv, dim), "state must be float32 [slots, H, vdim (+ 1), dim]")
+    _need((decay is None) != (tok_decay is None), "a decay per head or per token and head, not both")
+    if decay is not None:
+        _need(decay.dtype == torch.float32 and decay.numel() == num_heads, "one float32 decay per head")
+    for t_, n in ((tok_decay, "tok_decay"), (k_tok, "k_tok")):
+        if t_ is not None:
+            _need(t_.dtype == torch.float32 and t_.is_contiguous() and t_.shape == (T, num_heads), f"{n} must be float32 [T, H]")
+    _need(rot == 0 or (freq is not None and freq.dtype == torch.float32 and freq.numel() * 2 == rot and not act), "one float32 frequency per rotated pair; no rotation of activated q, k")
+    for t_, n in ((positions, "positions"), (row_q_start, "row_q_start"), (state_slots, "state_slots")):
+        _i32(t_, n)
+    _need(row_q_start.numel() == T == positions.numel(), "one new token a row")
+    if gated is not None:
+        _need(gated.dtype == rows_in.dtype == gate.dtype and gated.is_contiguous() and gated.shape == (T, num_heads * vdim) == gate.shape and gate.stride(1) == 1
+              and not ones, "gate and gated must be [T, H * vdim] of the rows' type")
+    else:
+        _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape == (T, num_heads * dv), "out must be float32 [T, H * (vdim (+ 1))]")
+    _check(load("retention").mie_decay_step(_ptr(rows_in), tag(rows_in), ctypes.c_longlong(rows_in.stride(0)), _ptr(positions), _ptr(row_q_start), _ptr(state_slots),
+                                            _ptr(decay), _ptr(freq), ctypes.c_float(q_scale), ctypes.c_float(k_scale), _ptr(tok_decay), _ptr(k_tok), int(act),
+                                            _ptr(state), _ptr(out), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(gated),
+                                            ctypes.c_float(eps), T, num_heads, dim, vdim, dv, rot, _stream()), "decay_step")
+    return gated if gated is not None else out
+
+
 def gate_scan(z: torch.Tensor, bias_i, bias_f, cap: float, row_q_start, row_q_len, state_slots, m_state: torch.Tensor, num_heads: int, max_q_len=None):
     """Exponential gates with a running maximum, token by token per row and head: from z [T, 2H] float32 = [input | forget]
     pre-activations, i = cap tanh((zi + bias_i) / cap), f = logsigmoid(cap tanh((zf + bias_f) / cap)) (``cap`` 0: no cap),

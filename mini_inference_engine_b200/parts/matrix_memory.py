@@ -17,6 +17,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import ops
+from ..kernels.attention import decode_only
 from ..weights.loader import TensorSpec
 from .attention import _padded_rows
 from .base import Mixer, StateNeed, register_part
@@ -58,8 +59,12 @@ class MatrixMemory(Mixer):
             z = z[:, :2 * H].contiguous()
         keep, write, m = ops.gate_scan(z, self.b_i, self.b_f, self.gate_cap, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, m_state, H, ctx.max_q_len)
         o = self.rt.empty(T, H * (Dv + 1), dtype=torch.float32)
-        ops.decay_scan(proj, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o, num_heads=H, dim=D, vdim=Dv,
-                       max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), tok_decay=keep, k_tok=write, ones=True, q_scale=D ** -0.5)
+        if decode_only(ctx) and ops.decay_step_takes(proj, state, D, 0, Dv):
+            ops.decay_step(proj, ctx.positions, ctx.row_q_start, ctx.state_slots, state, o, num_heads=H, dim=D, vdim=Dv, tok_decay=keep, k_tok=write, ones=True,
+                           q_scale=D ** -0.5)
+        else:
+            ops.decay_scan(proj, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o, num_heads=H, dim=D, vdim=Dv,
+                           max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), tok_decay=keep, k_tok=write, ones=True, q_scale=D ** -0.5)
         gated = self.rt.empty(T, H * Dv)
         at = 2 * H * D + H * Dv
         ops.group_norm_gate(o, proj[:, at:at + H * Dv], gated, groups=H, size=Dv, eps=self.eps, weight=self.norm, m=m)

@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import ops
+from ..kernels.attention import decode_only
 from ..weights.loader import TensorSpec
 from .base import Mixer, StateNeed, register_part
 from .rope import rotary_frequencies
@@ -53,6 +54,11 @@ class Retention(Mixer):
     def forward(self, x, ctx, cache):
         H, D, Dv = self.num_heads, self.dim, self.vdim
         qkvg = self.rt.linear(x, self.w_qkvg)
+        if decode_only(ctx) and ops.decay_step_takes(qkvg, cache.state, D, self.rot_dims, Dv):
+            gated = self.rt.empty(ctx.num_tokens, H * Dv)
+            ops.decay_step(qkvg, ctx.positions, ctx.row_q_start, ctx.state_slots, cache.state, num_heads=H, dim=D, vdim=Dv, decay=self.decay_t,
+                           k_scale=D ** -0.5, freq=self.freq, rot=self.rot_dims, gate=qkvg[:, 2 * H * D + H * Dv:2 * H * D + 2 * H * Dv], gated=gated, eps=self.eps)
+            return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)
         o = self.rt.empty(ctx.num_tokens, H * Dv, dtype=torch.float32)
         ops.retention_scan(qkvg, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, self.decay_t, self.freq,
                            cache.state, o, num_heads=H, dim=D, vdim=Dv, rot=self.rot_dims, k_scale=D ** -0.5,
@@ -102,8 +108,11 @@ class LightningAttention(Mixer):
         H, D, Dv = self.num_heads, self.dim, self.vdim
         qkvg = self.rt.linear(x, self.w_qkvg)
         o = self.rt.empty(ctx.num_tokens, H * Dv, dtype=torch.float32)
-        ops.decay_scan(qkvg, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, cache.state, o, num_heads=H, dim=D,
-                       vdim=Dv, max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), decay=self.decay_t, act=True)
+        if decode_only(ctx) and ops.decay_step_takes(qkvg, cache.state, D, 0, Dv):
+            ops.decay_step(qkvg, ctx.positions, ctx.row_q_start, ctx.state_slots, cache.state, o, num_heads=H, dim=D, vdim=Dv, decay=self.decay_t, act=True)
+        else:
+            ops.decay_scan(qkvg, ctx.positions, ctx.row_q_start, ctx.row_q_len, ctx.state_slots, cache.state, o, num_heads=H, dim=D,
+                           vdim=Dv, max_q_len=ctx.max_q_len, q_lens=ctx.host.get("q_len"), decay=self.decay_t, act=True)
         gated = self.rt.empty(ctx.num_tokens, H * Dv)
         at = 2 * H * D + H * Dv
         ops.group_norm_gate(o, qkvg[:, at:at + H * Dv], gated, groups=1, size=H * Dv, eps=self.eps, weight=self.norm)
