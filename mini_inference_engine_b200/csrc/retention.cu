@@ -525,8 +525,6 @@ extern "C" int mie_decay_scan(const void* qkv, int tag, long long stride, const 
     return MIE_ERR_BAD_ARG;
 }
 
-extern "C" int mie_retention_chunk_tokens() { return RET_L; }
-
 extern "C" int mie_head_rms_gate(const float* o, const void* g, int tag, long long g_stride, void* out, int num_tokens, int H,
                                  int Dv, float eps, cudaStream_t stream) {
     if (num_tokens <= 0) return 0;
