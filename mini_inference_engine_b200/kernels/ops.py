@@ -1605,10 +1605,30 @@ def moe_glu(gu: torch.Tensor, num_experts: int, activation: str, *, ids=None, wt
     return act
 
 
-def grouped_linear(rows: torch.Tensor, b: torch.Tensor, ends: torch.Tensor) -> torch.Tensor:
+def grouped_linear(rows: torch.Tensor, b: torch.Tensor, ends: torch.Tensor, relu2_weight: torch.Tensor | None = None) -> torch.Tensor:
     """The product of row ranges with a matrix each: rows [R, K] bfloat16 sorted by group, b [groups, K, N] (any strides
-    with one unit stride per matrix), ends int32 [groups] one past each group's last row -> [R, N] bfloat16.  The library's
-    grouped product (float32 accumulation), as the plain products of prompt-sized steps are the library's."""
+    with one unit stride per matrix), ends int32 [groups] one past each group's last row -> [R, N] bfloat16 (float32 accumulation; rows behind the
+    last group's are left as they are).  ``relu2_weight`` float32 [R]: row r is relu(product)^2 times entry r.  Operands that ``grouped_fits`` names on
+    pairs of SMs (``csrc/gemm_pair_tc.cu``), others by the library's grouped product."""
     _need(rows.is_cuda and rows.dtype == torch.bfloat16 == b.dtype and rows.is_contiguous() and ends.dtype == torch.int32,
           "grouped product: bfloat16 rows and matrices on the device, int32 ends")
-    return torch._grouped_mm(rows, b, offs=ends)          # (not counted in ``launches``: that counts this package's own kernels)
+    if not grouped_fits(rows, b, ends):
+        up = torch._grouped_mm(rows, b, offs=ends)        # (not counted in ``launches``: that counts this package's own kernels)
+        return up if relu2_weight is None else moe_act_rows(up, relu2_weight, "relu2")
+    groups, K, N = b.shape
+    R = rows.shape[0]
+    if relu2_weight is not None:
+        _f32(relu2_weight, "row weights")
+        _need(relu2_weight.numel() == R, "one weight per row")
+    out = torch.empty(R, N, dtype=torch.bfloat16, device=rows.device)
+    _check(load("gemm_pair_tc").mie_gemm_grouped(_ptr(rows), _ptr(b), ctypes.c_longlong(b.stride(2)), ctypes.c_longlong(b.stride(0)), _ptr(ends), groups,
+                                                 _ptr(relu2_weight), _ptr(out), R, N, K, _stream()), "grouped_linear")
+    return out
+
+
+def grouped_fits(rows: torch.Tensor, b: torch.Tensor, ends: torch.Tensor) -> bool:
+    """Whether the package's grouped product takes these operands: matrices with K innermost, sizes and strides in whole 16-byte pieces."""
+    groups, K, N = b.shape
+    return (b.stride(1) == 1 and 0 < groups <= 1024 and ends.is_contiguous() and ends.numel() == groups and rows.shape[1] == K
+            and K > 0 and K % 8 == 0 and N % 8 == 0 and all(b.stride(i) > 0 and b.stride(i) % 8 == 0 for i in (0, 2))
+            and max(b.stride(0), b.stride(2)) % min(b.stride(0), b.stride(2)) == 0 and rows.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)

@@ -160,7 +160,7 @@ class RoutedExperts(FeedForward):
     and one kernel between them.  A handful of tokens (no more (token, expert) pairs than experts): every pair streams
     its own expert's rows and no others, so a decoding step reads only the experts that were chosen.  Many tokens in
     bfloat16 where a token uses at most half of the experts: the pairs are sorted by expert and both products run expert
-    by expert over those rows (the library's grouped product), so no expert computes for a token that did not choose it."""
+    by expert over those rows (one launch a product, on pairs of SMs), so no expert computes for a token that did not choose it."""
 
     def __init__(self, hidden_size: int, num_experts: int, top: int, expert_size: int, activation: str = "relu2", gated: bool = False,
                  score: str = "top_softmax", correction: bool = False, groups: int = 1, keep: int = 1, identity: int = 0, shared=None,
@@ -239,7 +239,7 @@ class RoutedExperts(FeedForward):
 
     def kernel_sources(self):
         shared = self.shared.kernel_sources() if self.shared is not None else set()
-        return {"moe", "gemm_simt"} | self.rt.product_sources(self.w_up, self.w_down) | shared      # (gemm_simt: the router of a very wide model)
+        return {"moe", "gemm_simt"} | ({"gemm_pair_tc"} if self.grouped else set()) | self.rt.product_sources(self.w_up, self.w_down) | shared      # (gemm_simt: the router of a very wide model)
 
     def forward(self, x, ctx):
         """The chosen experts and the shared expert depend on nothing of one another.  For a handful of tokens both are short
@@ -290,9 +290,12 @@ class RoutedExperts(FeedForward):
             ends, place, row_weight = ops.moe_sort(ids, wts, self.outputs)      # identity experts sort behind the last expert's rows
             ends = ends[:self.num_experts]
             rows = ops.moe_gather(x, place, self.top)
-            up = ops.grouped_linear(rows, self.b_up, ends)
-            hid = (ops.moe_glu(up, 1, self.activation, row_weight=row_weight, limit=self.limit) if self.gated
-                   else ops.moe_act_rows(up, row_weight, self.activation))
+            if not self.gated and self.activation == "relu2":                # the activation rides in the product's epilogue
+                hid = ops.grouped_linear(rows, self.b_up, ends, relu2_weight=row_weight)
+            else:
+                up = ops.grouped_linear(rows, self.b_up, ends)
+                hid = (ops.moe_glu(up, 1, self.activation, row_weight=row_weight, limit=self.limit) if self.gated
+                       else ops.moe_act_rows(up, row_weight, self.activation))
             down = ops.grouped_linear(hid, self.b_down, ends)
             return ops.moe_combine(down, place, self.top, torch.empty(T, self.hidden_size, dtype=torch.float32, device=x.device),
                                    ids if self.identity else None, self.num_experts)
