@@ -331,7 +331,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 // tile's rows beyond its group's end belong to the next group: they are computed and not stored.  w comes through a map of three dimensions
 // (K, N, group), so that a group's last columns and last k-tile end in zeros and not in its neighbour's weights, wherever the groups lie (stacked, or
 // side by side along K).  Epilogue: bfloat16, or bfloat16(row_weight[r] relu(y)^2), a row factor and the activation without a pass of their own.
-// 4,096 rows in 16 groups: 2,048 x 960 XX us (the library's grouped product 45 us, and 7 us for the activation behind it), 960 x 2,048 XX us (45 us).
+// Bound: the tensor cores, about a third of whose work is the groups' last tiles.  4,096 rows in 16 groups, 2,048 x 2,112 and back: 46 us a product (the
+// library's 45 us and 2 us of its preparation, and 7 us for the activation between the two).  Weights as the MMA's rows with 64 to 256 of x as
+// its columns, last tiles last, was slower: 50 us, the last tiles read their weights from memory again.
 #define GG_MAX_GROUPS 1024
 
 struct GgParams {
