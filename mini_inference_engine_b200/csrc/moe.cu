@@ -189,6 +189,46 @@ __device__ __forceinline__ void route_by_rule(const float* zt, int* ids, float* 
     }
 }
 
+// Modes 0 and 2 for one token by a whole warp (up to 32 choices, lane k keeps the k-th): route_by_rule outcome for outcome and bit for bit, the
+// sums in the order of the choices.
+__device__ __forceinline__ void route_top_warp(const float* zt, int* ids, float* wts, int n, int top, const RouteRule& rr, float* rest, int lane) {
+    const unsigned full = 0xffffffffu;
+    float prev_v = INFINITY, first = 0.f, sum = 0.f, mine = 0.f;
+    int prev_i = -1, chosen = 0;
+    for (int k = 0; k < top; ++k) {
+        float best = -INFINITY;
+        int bi = -1;
+        for (int e = lane; e < n; e += 32) {
+            const float v = zt[e];
+            const bool after_prev = v < prev_v || (v == prev_v && e > prev_i);
+            if (after_prev && (bi < 0 || v > best)) { best = v; bi = e; }
+        }
+#pragma unroll
+        for (int off = 16; off; off >>= 1) {
+            const float ob = __shfl_xor_sync(full, best, off);
+            const int oi = __shfl_xor_sync(full, bi, off);
+            if (oi >= 0 && (bi < 0 || ob > best || (ob == best && oi < bi))) { best = ob; bi = oi; }
+        }
+        if (bi < 0) { bi = 0; best = -INFINITY; }              // logits that are not numbers: keep the ids in range
+        if (k == 0) first = best;
+        const float p = rr.mode == 2 ? 1.0f / (1.0f + expf(-zt[bi])) : expf(best - first);
+        sum += p;
+        if (lane == k) { mine = p; chosen = bi; }
+        prev_v = best;
+        prev_i = bi;
+    }
+    if (rr.mode != 2) mine /= sum;
+    if (lane < top) { ids[lane] = chosen; wts[lane] = mine; }
+    if (rest) {
+        float idw = 0.f;
+        for (int k = 0; k < top; ++k) {
+            const float w = __shfl_sync(full, mine, k);
+            if (__shfl_sync(full, chosen, k) >= rr.real) idw += w;
+        }
+        if (lane == 0) *rest = idw;
+    }
+}
+
 __global__ void moe_route_kernel(const float* __restrict__ z, int* __restrict__ ids, float* __restrict__ wts, int num_tokens, int E,
                                  int top, RouteRule rr) {
     pdl_enter();
@@ -208,79 +248,102 @@ static __host__ __device__ inline int router_segments(int E, int h, int warps) {
     return S;
 }
 
-// A block per ROUTER_TOKENS tokens: their inputs into shared memory as float32, a warp per (output, column segment) in turn
-// for the logits of all of them (the output's row is read once a block), the segments' sums added in their order, then a
-// warp per token for the scores and, by the second rule, the choice (by the first rule a thread per token chooses).  `logits`
-// (optional) receives z.
-template <typename TA>
-__global__ void __launch_bounds__(ROUTER_THREADS)
+// A block per TOKENS tokens: their inputs into shared memory as float32, a warp per (two outputs, column segment) in turn for the
+// logits of all of them (the outputs' rows are read once a block, an input once for two outputs), the segments' sums added in their order, then a
+// warp per token for the scores and the choice (a thread per token chooses more than 32).  `logits` (optional) receives z.
+// Bound: issue slots and shared-memory reads.  1,024 tokens of 2,048, sixteen outputs: 17.9 us with an output an item and eight tokens' worth of
+// predicated-off work in blocks of four, 12.4 us.
+template <typename TA, int TOKENS>
+__global__ void __launch_bounds__(ROUTER_THREADS, 2)
 moe_router_kernel(const TA* __restrict__ x, const float* __restrict__ w, int* __restrict__ ids, float* __restrict__ wts,
-                  float* __restrict__ logits, int num_tokens, int h, int E, int top, int tpb, int S, RouteRule rr) {
-    extern __shared__ __align__(16) float rs[];               // x [tpb, h], then z [tpb, E], then the segments' sums [S, tpb, E]
-    float* z = rs + (size_t)tpb * h;
-    float* zp = z + (size_t)tpb * E;
+                  float* __restrict__ logits, int num_tokens, int h, int E, int top, int S, RouteRule rr) {
+    extern __shared__ __align__(16) float rs[];               // x [TOKENS, h], then z [TOKENS, E], then the segments' sums [S, TOKENS, E]
+    float* z = rs + (size_t)TOKENS * h;
+    float* zp = z + (size_t)TOKENS * E;
     pdl_enter();
-    const int t0 = blockIdx.x * tpb, nt = min(tpb, num_tokens - t0);
+    const int t0 = blockIdx.x * TOKENS, nt = min(TOKENS, num_tokens - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const bool vec = (h & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    const int seg = ((h + S - 1) / S + 127) / 128 * 128;      // columns a segment, whole 128-column steps
+    const int items = (E + 1) / 2 * S;
+    // 512 columns of the two rows of an item, eight 16-byte loads a lane; the first are asked for before the inputs are on their way to shared memory
+    float4 a[2][4];
+    auto fetch = [&](int item, int base) {
+        const int e = item / S * 2, end = min(h, (item % S + 1) * seg);
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = base + lane * 4 + 128 * u;
+                a[o][u] = e + o < E && c < end ? *reinterpret_cast<const float4*>(w + (int64_t)(e + o) * h + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+    };
+    if (vec && warp < items) fetch(warp, warp % S * seg);
     const TA* xb = x + (int64_t)t0 * h;
     if (sizeof(TA) == 2 && (h & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {      // eight inputs a load
         for (int c = threadIdx.x * 8; c < nt * h; c += blockDim.x * 8) {
             const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(xb) + c);
             const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
-            const float2 a = __bfloat1622float2(p[0]), b = __bfloat1622float2(p[1]), c2 = __bfloat1622float2(p[2]), d = __bfloat1622float2(p[3]);
-            *reinterpret_cast<float4*>(rs + c) = make_float4(a.x, a.y, b.x, b.y);
-            *reinterpret_cast<float4*>(rs + c + 4) = make_float4(c2.x, c2.y, d.x, d.y);
+            const float2 a0 = __bfloat1622float2(p[0]), a1 = __bfloat1622float2(p[1]), a2 = __bfloat1622float2(p[2]), a3 = __bfloat1622float2(p[3]);
+            *reinterpret_cast<float4*>(rs + c) = make_float4(a0.x, a0.y, a1.x, a1.y);
+            *reinterpret_cast<float4*>(rs + c + 4) = make_float4(a2.x, a2.y, a3.x, a3.y);
         }
     } else {
         for (int c = threadIdx.x; c < nt * h; c += blockDim.x) rs[c] = to_f32<TA>(xb[c]);
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const bool vec = (h & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-    const int seg = ((h + S - 1) / S + 127) / 128 * 128;      // columns a segment, whole 128-column steps
-    for (int item = warp; item < E * S; item += nw) {
-        const int e = item / S, s = item - e * S;
+    // (the last block's tokens may be fewer: what lies in the others' places is multiplied too and not used)
+    for (int item = warp; item < items; item += nw) {
+        const int e = item / S * 2, s = item % S;
         const int c_begin = s * seg, c_end = min(h, c_begin + seg);
-        const float* row = w + (int64_t)e * h;
-        float acc[ROUTER_TOKENS];
+        float acc[2][TOKENS];
 #pragma unroll
-        for (int i = 0; i < ROUTER_TOKENS; ++i) acc[i] = 0.f;
+        for (int i = 0; i < TOKENS; ++i) acc[0][i] = acc[1][i] = 0.f;
         if (vec) {
-            for (int c0 = c_begin + lane * 4; c0 < c_end; c0 += 512) {           // four 16-byte loads of the row in flight
-                float4 a[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    a[u] = c0 + 128 * u < c_end ? *reinterpret_cast<const float4*>(row + c0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int base = c_begin; base < c_end; base += 512) {
+                if (item != warp || base != c_begin) fetch(item, base);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int c = c0 + 128 * u;
-                    if (c >= c_end) break;
+                    const int c = base + lane * 4 + 128 * u;
+                    if (base + 128 * u >= c_end) break;
+                    if (c < c_end) {
 #pragma unroll
-                    for (int i = 0; i < ROUTER_TOKENS; ++i)
-                        if (i < nt) {
+                        for (int i = 0; i < TOKENS; ++i) {
                             const float4 b = *reinterpret_cast<const float4*>(rs + (size_t)i * h + c);
-                            acc[i] = fmaf(a[u].x, b.x, acc[i]); acc[i] = fmaf(a[u].y, b.y, acc[i]);
-                            acc[i] = fmaf(a[u].z, b.z, acc[i]); acc[i] = fmaf(a[u].w, b.w, acc[i]);
+#pragma unroll
+                            for (int o = 0; o < 2; ++o) {
+                                acc[o][i] = fmaf(a[o][u].x, b.x, acc[o][i]); acc[o][i] = fmaf(a[o][u].y, b.y, acc[o][i]);
+                                acc[o][i] = fmaf(a[o][u].z, b.z, acc[o][i]); acc[o][i] = fmaf(a[o][u].w, b.w, acc[o][i]);
+                            }
                         }
+                    }
                 }
             }
         } else {
+            const float* row = w + (int64_t)e * h;
+            const float* row2 = e + 1 < E ? row + h : row;
             for (int c = c_begin + lane; c < c_end; c += 32) {
-                const float a = row[c];
+                const float w0 = row[c], w1 = row2[c];
 #pragma unroll
-                for (int i = 0; i < ROUTER_TOKENS; ++i)
-                    if (i < nt) acc[i] = fmaf(a, rs[(size_t)i * h + c], acc[i]);
+                for (int i = 0; i < TOKENS; ++i) {
+                    const float b = rs[(size_t)i * h + c];
+                    acc[0][i] = fmaf(w0, b, acc[0][i]);
+                    acc[1][i] = fmaf(w1, b, acc[1][i]);
+                }
             }
         }
 #pragma unroll
-        for (int i = 0; i < ROUTER_TOKENS; ++i) {
-            const float v = warp_sum(acc[i]);
-            if (lane == 0 && i < nt) zp[((size_t)s * tpb + i) * E + e] = v;
-        }
+        for (int i = 0; i < TOKENS; ++i)
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const float v = warp_sum(acc[o][i]);
+                if (lane == 0 && i < nt && e + o < E) zp[((size_t)s * TOKENS + i) * E + e + o] = v;
+            }
     }
     __syncthreads();
     for (int c = threadIdx.x; c < nt * E; c += blockDim.x) {
         float v = zp[c];
-        for (int s = 1; s < S; ++s) v += zp[(size_t)s * tpb * E + c];
+        for (int s = 1; s < S; ++s) v += zp[(size_t)s * TOKENS * E + c];
         z[c] = v;
     }
     __syncthreads();
@@ -301,6 +364,11 @@ moe_router_kernel(const TA* __restrict__ x, const float* __restrict__ w, int* __
             route_scored_warp(z + i * E, ids + (int64_t)(t0 + i) * top, wts + (int64_t)(t0 + i) * top, E, top, rr,
                               rr.rest ? rr.rest + t0 + i : nullptr, lane);
         }
+        return;
+    }
+    if (top <= 32) {
+        for (int i = warp; i < nt; i += nw)
+            route_top_warp(z + i * E, ids + (int64_t)(t0 + i) * top, wts + (int64_t)(t0 + i) * top, E, top, rr, rr.rest ? rr.rest + t0 + i : nullptr, lane);
         return;
     }
     if (threadIdx.x < nt)
@@ -704,15 +772,16 @@ extern "C" int mie_moe_router(const void* x, int tag, const float* w, int* ids, 
     while (tpb > 1 && (num_tokens + tpb - 1) / tpb < device_sm_count()) tpb >>= 1;      // ... or would leave SMs without a block
     const size_t smem = (size_t)tpb * (h + (S + 1) * E) * sizeof(float);
     if (smem > 200 * 1024) return MIE_ERR_TOO_LARGE;
-    const int blocks = (num_tokens + tpb - 1) / tpb;
-    cudaError_t e;
-    if (tag == MIE_F32) {
-        if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(moe_router_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return (int)e;
-        return launch_kernel(moe_router_kernel<float>, dim3(blocks), dim3(threads), smem, stream, (const float*)x, w, ids, wts, logits, num_tokens, h, E, top, tpb, S, rr);
-    } else if (tag == MIE_BF16) {
-        if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(moe_router_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return (int)e;
-        return launch_kernel(moe_router_kernel<bf16>, dim3(blocks), dim3(threads), smem, stream, (const bf16*)x, w, ids, wts, logits, num_tokens, h, E, top, tpb, S, rr);
-    }
+    auto launch = [&](auto kernel, auto* in) {
+        const cudaError_t e = smem > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+        if (e != cudaSuccess) return (int)e;
+        return launch_kernel(kernel, dim3((num_tokens + tpb - 1) / tpb), dim3(threads), smem, stream, in, w, ids, wts, logits, num_tokens, h, E, top, S, rr);
+    };
+#define ROUTER(T) (tpb == 8 ? launch(moe_router_kernel<T, 8>, (const T*)x) : tpb == 4 ? launch(moe_router_kernel<T, 4>, (const T*)x)  \
+                   : tpb == 2 ? launch(moe_router_kernel<T, 2>, (const T*)x) : launch(moe_router_kernel<T, 1>, (const T*)x))
+    if (tag == MIE_F32) return ROUTER(float);
+    if (tag == MIE_BF16) return ROUTER(bf16);
+#undef ROUTER
     return MIE_ERR_BAD_ARG;
 }
 
