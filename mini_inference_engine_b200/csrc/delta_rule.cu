@@ -534,10 +534,77 @@ extern "C" int mie_conv_state_update(const void* x, int tag, long long stride, c
     return MIE_ERR_BAD_ARG;
 }
 
+// Rows of one new token, where the caller knows that the scan has no others: the scan's lanes, operations and order without its
+// ring -- a lane asks for its pieces of four columns, of k, q and the decays at once, and a block needs no shared memory, so that the whole launch is resident.
+// Bound: the states' way through memory and one round trip.  Sixteen rows of 16 heads of 128 x 128 beside a portion: 17.6 -> 7.3 us.
+#define SINGLE_COLS 4        // columns a group of 16 lanes
+template <int R, bool ONE>
+__global__ void __launch_bounds__(128) delta_single_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
+                                                           const float* __restrict__ beta, const float* __restrict__ decay, const float* __restrict__ kq,
+                                                           const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
+                                                           const int* __restrict__ state_slots, float* __restrict__ state, float* __restrict__ out, int H,
+                                                           int G, int Dv) {
+    constexpr int L = 16, D = L * R;
+    pdl_enter();
+    const int row = blockIdx.x, h = blockIdx.y, kh = h / (H / G), l = threadIdx.x % L;
+    const int j0 = blockIdx.z * (128 / L * SINGLE_COLS) + threadIdx.x / L;
+    const int n = row_q_len[row], slot = state_slots[row];
+    const int64_t t = row_q_start[row];
+    if (n != 1) return;
+    float* sp = state + ((int64_t)slot * H + h) * Dv * D;
+    float s[SINGLE_COLS][R], k[R], q[R], g[ONE ? 1 : R], v[SINGLE_COLS];
+#pragma unroll
+    for (int c = 0; c < SINGLE_COLS; ++c) {
+        const int j = min(j0 + c * (128 / L), Dv - 1);
+#pragma unroll
+        for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(s[c] + r) = *reinterpret_cast<const float4*>(sp + (int64_t)j * D + 4 * (l + L * (r >> 2)));
+        v[c] = vn[(t * H + h) * Dv + j];
+    }
+#pragma unroll
+    for (int r = 0; r < R; r += 4) {
+        const int i = 4 * (l + L * (r >> 2));
+        *reinterpret_cast<float4*>(k + r) = *reinterpret_cast<const float4*>(kn + (t * G + kh) * D + i);
+        *reinterpret_cast<float4*>(q + r) = *reinterpret_cast<const float4*>(qn + (t * G + kh) * D + i);
+        if constexpr (!ONE) *reinterpret_cast<float4*>(g + r) = *reinterpret_cast<const float4*>(decay + (t * H + h) * D + i);
+    }
+    const float one = ONE ? decay[t * H + h] : 1.f, b = beta[t * H + h], kqt = kq[t * G + kh];
+#pragma unroll
+    for (int c = 0; c < SINGLE_COLS; ++c) {
+        const int j = j0 + c * (128 / L);
+        float r1 = 0.f, r2 = 0.f, r1b = 0.f, r2b = 0.f;
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+            if constexpr (!ONE) {
+                s[c][r] *= g[r];
+                s[c][r + 1] *= g[r + 1];
+            }
+            r1 = fmaf(s[c][r], k[r], r1);
+            r1b = fmaf(s[c][r + 1], k[r + 1], r1b);
+            r2 = fmaf(s[c][r], q[r], r2);
+            r2b = fmaf(s[c][r + 1], q[r + 1], r2b);
+        }
+        r1 += r1b;
+        r2 += r2b;
+#pragma unroll
+        for (int o = L >> 1; o > 0; o >>= 1) {
+            r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+            r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+        }
+        if (j < Dv) {
+            const float u = b * (v[c] - one * r1);
+#pragma unroll
+            for (int r = 0; r < R; ++r) s[c][r] = fmaf(k[r], u, one * s[c][r]);
+            if (l == 0) out[(t * H + h) * Dv + j] = fmaf(u, kqt, one * r2);
+#pragma unroll
+            for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(sp + (int64_t)j * D + 4 * (l + L * (r >> 2))) = *reinterpret_cast<const float4*>(s[c] + r);
+        }
+    }
+}
+
 template <int R, bool ONE>
 static int launch_scan(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* kq,
                        const int* row_q_start, const int* row_q_len, const int* state_slots, float* state, float* out, int num_rows,
-                       int H, int G, int D, int Dv, int below, cudaStream_t stream) {
+                       int H, int G, int D, int Dv, int below, int singles, cudaStream_t stream) {
     int L = 1;
     while (L * R < D) L <<= 1;
     if (L > 32) return MIE_ERR_TOO_LARGE;
@@ -554,6 +621,10 @@ static int launch_scan(const float* qn, const float* kn, const float* vn, const 
     const size_t smem = (size_t)DELTA_BATCHES * tb * slot_bytes;
     const bool vec = D == L * R && D % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn) | (ONE ? 0 : reinterpret_cast<uintptr_t>(decay))) & 15) == 0;
+    if constexpr (R <= 8)
+        if (singles && vec && L == 16 && below > 1 && (reinterpret_cast<uintptr_t>(state) & 15) == 0)
+            return launch_kernel(delta_single_kernel<R, ONE>, dim3(num_rows, H, (Dv + 8 * SINGLE_COLS - 1) / (8 * SINGLE_COLS)), dim3(128), 0, stream, qn, kn, vn,
+                                 beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, H, G, Dv);
     // the vectorised kernel with the lanes a column as a constant for the common key sizes (64 and 128: 16 lanes), else at run time
     auto kernel = !vec ? delta_scan_kernel<R, false, 0, ONE> : (L == 16 ? delta_scan_kernel<R, true, 16, ONE> : delta_scan_kernel<R, true, 0, ONE>);
     if (smem > 48 * 1024) {
@@ -564,14 +635,15 @@ static int launch_scan(const float* qn, const float* kn, const float* vn, const 
                          state_slots, state, out, H, G, D, Dv, L, cols, tb, slot_floats, below);
 }
 
+// singles: every row with fewer than `below` new tokens has exactly one.
 extern "C" int mie_delta_scan(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* kq,
                               const int* row_q_start, const int* row_q_len, const int* state_slots, float* state, float* out,
-                              int num_rows, int H, int G, int D, int Dv, int A, int below, cudaStream_t stream) {
+                              int num_rows, int H, int G, int D, int Dv, int A, int below, int singles, cudaStream_t stream) {
     if (num_rows <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || D <= 0 || Dv <= 0 || (A != 1 && A != D)) return MIE_ERR_BAD_ARG;
     // entries of a column a lane: the fewest for which sixteen lanes hold a column (thirty-two for the longest keys)
-#define SCAN(R) (A == 1 ? launch_scan<R, true>(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, num_rows, H, G, D, Dv, below, stream)  \
-                        : launch_scan<R, false>(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, num_rows, H, G, D, Dv, below, stream))
+#define SCAN(R) (A == 1 ? launch_scan<R, true>(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, num_rows, H, G, D, Dv, below, singles, stream)  \
+                        : launch_scan<R, false>(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, num_rows, H, G, D, Dv, below, singles, stream))
     if (D <= 64) return SCAN(4);
     if (D <= 128) return SCAN(8);
     if (D <= DELTA_MAX_KEY) return SCAN(16);

@@ -1312,10 +1312,10 @@ def conv_state_update(x: torch.Tensor, row_q_start, row_q_len, state_slots, conv
 
 
 def delta_scan(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots, state, out, *, num_heads: int, num_kv_heads: int,
-               dim: int, vdim: int, below: int = 1 << 30) -> torch.Tensor:
+               dim: int, vdim: int, below: int = 1 << 30, singles: bool = False) -> torch.Tensor:
     """S <- decay S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q for every new token of every row, from and to
     ``state`` [slots, H, vdim, dim] float32.  ``decay`` [T, H * dim], or [T, H]: one per head.  ``out`` [T, H * vdim] float32.  Rows with
-    ``below`` new tokens or more are left alone (``delta_chunks``)."""
+    ``below`` new tokens or more are left alone (``delta_chunks``).  ``singles``: the caller knows that all others have exactly one."""
     T = qn.shape[0]
     H, G, D, Dv = num_heads, num_kv_heads, dim, vdim
     A = decay.shape[1] // H
@@ -1327,7 +1327,7 @@ def delta_scan(qn, kn, vn, beta, decay, kq, row_q_start, row_q_len, state_slots,
         _i32(t, n)
     lib = load("delta_rule")
     _check(lib.mie_delta_scan(_ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(decay), _ptr(kq), _ptr(row_q_start), _ptr(row_q_len),
-                              _ptr(state_slots), _ptr(state), _ptr(out), row_q_len.numel(), H, G, D, Dv, A, int(below), _stream()), "delta_scan")
+                              _ptr(state_slots), _ptr(state), _ptr(out), row_q_len.numel(), H, G, D, Dv, A, int(below), int(singles), _stream()), "delta_scan")
     return out
 
 

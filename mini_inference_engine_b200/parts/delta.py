@@ -17,9 +17,16 @@ from __future__ import annotations
 import torch
 
 from ..kernels import ops
+from ..kernels.attention import _row_kinds, decode_only
 from ..weights.loader import TensorSpec
 from .attention import _padded_rows
 from .base import Mixer, StateNeed, register_part
+
+
+def _singles(ctx, long) -> bool:
+    """Whether the rows that are left to the scan have one new token each: known on the host, and no row of more than one is shorter than the chunked ones."""
+    kinds = _row_kinds(ctx)
+    return kinds is not None and kinds[1] == len(long or ())
 
 
 CHANNEL_CHUNKED_FROM = 112      # new tokens from which a row's recurrence goes in chunks (the line of one decay per head, see CHUNKED_FROM: the scans are the same; 1,500 tokens
@@ -104,7 +111,7 @@ class ChannelDelta(Mixer):
         if chunked:
             ops.delta_chunks(qn, kn, vn, beta, log_decay, *rows, min_len=CHANNEL_CHUNKED_FROM, work=(len(long), sum(long)) if long else None, decay=decay, **sizes)
         if long is None or len(long) < len(q_lens):
-            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHANNEL_CHUNKED_FROM if chunked else 1 << 30, **sizes)
+            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHANNEL_CHUNKED_FROM if chunked else 1 << 30, singles=_singles(ctx, long), **sizes)
         gated = self.rt.empty(T, H * Dv)
         ops.head_norm_gate(o, low[:, H * D:], self.norm, gated, H, Dv, self.eps)
         return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)
@@ -162,7 +169,6 @@ class HeadDelta(Mixer):
         return {"delta_rule", "delta_chunk", "delta_head"} | self.rt.product_sources(self.w_in, self.w_o)
 
     def forward(self, x, ctx, cache):
-        from ..kernels.attention import decode_only
         H, G, D, Dv, T = self.num_heads, self.num_kv_heads, self.dim, self.vdim, ctx.num_tokens
         state, ring = cache.parts[0].state, cache.parts[1].state
         sizes = dict(num_heads=H, num_kv_heads=G, dim=D, vdim=Dv)
@@ -186,7 +192,7 @@ class HeadDelta(Mixer):
         if chunked:
             ops.delta_chunks(qn, kn, vn, beta, log_decay, *rows, min_len=CHUNKED_FROM, work=(len(long), sum(long)) if long else None, **sizes)
         if long is None or len(long) < len(q_lens):
-            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHUNKED_FROM if chunked else 1 << 30, **sizes)
+            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHUNKED_FROM if chunked else 1 << 30, singles=_singles(ctx, long), **sizes)
         at = 2 * G * D + H * Dv
         ops.head_norm_gate(o, proj[:, at:at + H * Dv], self.norm, gated, H, Dv, self.eps, silu=True)
         return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)
