@@ -65,3 +65,30 @@ def test_modified_scores_in_large_launches(what):
     mods = ops.ScoreMods(3.0 if what == "cap" else 0.0, torch.randn(H, generator=g).cuda() if what == "sink" else None,
                          torch.randn(H, 90, generator=g).cuda() if what == "bias" else None, (torch.rand(H, generator=g) * 0.1).cuda() if what == "slope" else None)
     close(*both([(1400, 1500)], H, 8, 128, 16, mods=mods))
+
+
+@pytest.mark.parametrize("n", [300, 800, 1500])
+def test_fewer_keys_a_tile_lose_no_precision(n):
+    """The same heads in a launch of few blocks (128 keys a tile) and, each thirty-two times, in one of many (64 keys): the error against 64 bits is no larger."""
+    from mini_inference_engine_b200.kernels import ops
+    G, D, page, copies = 4, 128, 16, 32
+    g = torch.Generator().manual_seed(n)
+    pages = -(-n // page)
+    k, v = (torch.randn(pages, G, page, D, generator=g).bfloat16().cuda() for _ in "kv")
+    q = torch.randn(n, G, D, generator=g).bfloat16().cuda() * 1.5
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    table = torch.arange(pages, dtype=torch.int32, device="cuda").view(1, -1)
+    flat = lambda t: t.permute(1, 0, 2, 3).reshape(G, -1, D)[:, :n].double()
+    scores = q.double().permute(1, 0, 2) @ flat(k).transpose(1, 2) * D ** -0.5
+    scores = scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), -float("inf"))
+    want = (torch.softmax(scores, -1) @ flat(v)).permute(1, 0, 2)
+    errors = []
+    for times in (1, copies):
+        H = G * times
+        qs = q.repeat_interleave(times, 1).reshape(n, H * D).contiguous()
+        out = torch.empty(n, H, D, device="cuda")
+        ops.prefill_attention_tc(qs, H * D, k, v, table, i32(0), i32(n), i32(n), n, out, H, G, D, page, D ** -0.5, 0, work=(1, n))
+        torch.cuda.synchronize()
+        ops.check_tc_errors()
+        errors.append((out.view(n, G, times, D)[:, :, 0].double() - want).norm().item())
+    assert errors[1] <= errors[0]
