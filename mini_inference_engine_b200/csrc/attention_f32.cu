@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(THREADS, DT == 64 ? 3 : 2) f32_attention_kerne
     }
     __syncthreads();
     const int r = s_row;
+    pdl_wait();                                       // (a block without work waits too: see common.cuh)
     if (r < 0) return;
-    pdl_wait();
     const int q_len = p.row_q_len[r], ctx_len = p.row_ctx_len[r], q_start = p.row_q_start[r], pair0 = s_tile * F32_PAIRS;
     if (ctx_len > p.table_stride * p.page_size) {
         if (threadIdx.x == 0) range_report(p.report, MIE_RANGE_POSITION, MIE_K_ATTENTION_SIMT, r, ctx_len);

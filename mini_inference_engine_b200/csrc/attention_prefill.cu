@@ -61,8 +61,8 @@ prefill_attention_kernel(const PrefillParams p) {
     }
     __syncthreads();
     const int row = s_row;
+    pdl_wait();                                                    // (a block without work waits too: see common.cuh)
     if (row < 0) return;
-    pdl_wait();
     const int q0 = s_q0;
     const int q_len = p.row_q_len[row], ctx = p.row_ctx_len[row], q_start = p.row_q_start[row];
     const int head = blockIdx.y;

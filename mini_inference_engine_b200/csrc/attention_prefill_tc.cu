@@ -163,7 +163,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
         }
     }
     __syncthreads();
-    if (s_row < 0) return;
+    if (s_row < 0) {
+        pdl_wait();                                              // a block without work waits too: see common.cuh
+        return;
+    }
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -625,7 +628,10 @@ prefill_attention_pp_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
     }
     __syncthreads();
-    if (s_row < 0) return;
+    if (s_row < 0) {
+        pdl_wait();                                              // a block without work waits too: see common.cuh
+        return;
+    }
 
     if (threadIdx.x == 0) {
         abort_flag = 0;

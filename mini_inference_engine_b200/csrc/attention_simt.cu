@@ -72,8 +72,8 @@ paged_attention_kernel(const T* __restrict__ q, int64_t q_stride, const T* __res
     }
     __syncthreads();
     const int r = s_row;
+    pdl_wait();                                 // (a block without work waits too: see common.cuh)
     if (r < 0) return;
-    pdl_wait();
     const int q0 = s_q0;
     const int q_len = row_q_len[r], ctx_len = row_ctx_len[r], q_start = row_q_start[r];
     if (ctx_len > table_stride * page_size) {      // more positions than the row's block table covers: reported, row left alone

@@ -72,8 +72,9 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
     __shared__ float a[DC_L], G[DC_L];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
-    if (!dc_find(p, &s_row, &s_chunk)) return;
-    pdl_wait();
+    const bool mine = dc_find(p, &s_row, &s_chunk);
+    pdl_wait();                                        // (a block without work waits too: see common.cuh)
+    if (!mine) return;
     const int h = blockIdx.y, H = p.H, D = p.D, half = blockIdx.z;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     dc_rows<DT>(K, p.k + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
@@ -239,8 +240,9 @@ __global__ void __launch_bounds__(256, 2) decay_output_kernel(const DcParams p) 
     __shared__ __align__(16) float n[DT];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
-    if (!dc_find(p, &s_row, &s_chunk)) return;
-    pdl_wait();
+    const bool mine = dc_find(p, &s_row, &s_chunk);
+    pdl_wait();                                        // (a block without work waits too: see common.cuh)
+    if (!mine) return;
     const int h = blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     const float* from = p.states + ((int64_t)blockIdx.x * H + h) * (int64_t)p.Dv * D;
