@@ -1,9 +1,10 @@
 // y[M, N] = x[M, K] w[N, K]^T (+ bias[N]) for float32 operands, at the precision of float32 products, on the tensor cores of pairs of SMs
 // (the CUDA-core product of csrc/gemm_simt.cu runs where this one does not pay).
 //
-// A float32 number is the sum of three bfloat16 numbers exactly: 8 + 8 + 8 bits of its significand, cut off one after the other
-// (`split`).  Of the nine products of parts six are formed, in float32: the three left out are below 2^-24 of the product, half of what one
-// rounding of a float32 product loses.  The tensor core's own float32 sums are cut off rather than rounded, so
+// A float32 number is the sum of three bfloat16 numbers exactly: the nearest one, the nearest to what is left, and the rest (`split`); the second is at most
+// 2^-8 of the number, the third 2^-17.  Of the nine products of parts six are formed, in float32: the three left out are at most 2^-24 of the product
+// together, as much as one rounding of a float32 product may lose, and of either sign.  (Parts cut off towards zero would leave out up to 2^-21, always of the
+// product's sign, so that a sum of products of one sign never lost it again.)  The tensor core's own float32 sums are cut off rather than rounded, so
 // a sum stays there for 64 products only (small parts first); every 64-wide chunk of K is taken out of tensor memory and added to a
 // float32 register, rounded to nearest.  Against 64 bits the error is 1.1e-7 at K 2,048 and 1.8e-7 at K 5,632 (2-norm) where one
 // chain of K fused multiply-adds leaves 5.5e-7 and 1.1e-6.
@@ -88,14 +89,18 @@ __device__ __noinline__ float sp_chain(const float* __restrict__ x, const float*
 
 // --------------------------------------------------------------------------- split
 
-// The top 8 bits of the significand (sign and exponent with them) and what is left; a number that is not finite has no rest.
+// The nearest bfloat16 number (8 bits of the significand); the one towards zero where rounding would leave the range.
+__device__ __forceinline__ float top_part(float v) {
+    const uint32_t u = __float_as_uint(v), r = (u + 0x7fffu + ((u >> 16) & 1u)) & 0xffff0000u;
+    return __uint_as_float((r & 0x7f800000u) == 0x7f800000u ? u & 0xffff0000u : r);
+}
+// A number as its nearest bfloat16 number, the nearest to what is left, and the rest, which is one too; a number that is not finite has no rest.
 __device__ __forceinline__ void cut3(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
     const uint32_t u = __float_as_uint(v);
-    a = u & 0xffff0000u;
-    if ((u & 0x7f800000u) == 0x7f800000u) { a = (u & 0x007fffffu) ? 0x7fc00000u : a; b = 0u; c = 0u; return; }
-    const float r = v - __uint_as_float(a);                 // exact
-    b = __float_as_uint(r) & 0xffff0000u;
-    c = __float_as_uint(r - __uint_as_float(b));            // exact, at most 8 bits: its lower half is zero
+    b = c = 0u;
+    if ((u & 0x7f800000u) == 0x7f800000u) { a = (u & 0x007fffffu) ? 0x7fc00000u : u; return; }
+    const float fa = top_part(v), r = v - fa, fb = top_part(r);            // the differences are exact
+    a = __float_as_uint(fa); b = __float_as_uint(fb); c = __float_as_uint(r - fb);       // (at most 7 bits: c's lower half is zero)
 }
 
 // src [rows, K] -> dst [Kp / 64][row blocks][3 planes][block rows][64]: what one stage of the product reads of one block of rows is one stretch

@@ -37,6 +37,26 @@ def test_any_sizes(M, N, K, spread):
         check(got, x, w, b)
 
 
+@pytest.mark.parametrize("K", [128, 512, 2048])
+@pytest.mark.parametrize("kind", ["equal", "just above", "just below", "one sign", "both signs"])
+def test_no_further_from_64_bits_than_float32_sums(kind, K):
+    """Significands whose parts are as large as they get, products of one sign, whose errors add up, and ordinary numbers: the 2-norm of the error is no larger
+    than that of chains of fused multiply-adds, or than half a unit in the last place of the results, which both sides lose at the end."""
+    from mini_inference_engine_b200.kernels import gemm_split, ops
+    M, N = 200, 320
+    g = torch.Generator(device="cuda").manual_seed(K)
+    few = lambda *s: torch.randint(0, 8, s, generator=g, device="cuda").float() * 2.0 ** -23
+    make = {"equal": lambda *s: torch.full(s, 1.0 + 2.0 ** -7 - 2.0 ** -23, device="cuda"), "just above": lambda *s: 1.0 + 2.0 ** -8 - few(*s),
+            "just below": lambda *s: 1.0 - 2.0 ** -9 - few(*s) / 2, "one sign": lambda *s: 1.0 + torch.rand(*s, generator=g, device="cuda"),
+            "both signs": lambda *s: torch.randn(*s, generator=g, device="cuda")}[kind]
+    x, w = make(M, K), make(N, K)
+    want = x.double() @ w.double().t()
+    off = lambda t: ((t.double() - want).norm() / want.norm()).item()
+    split, chain = off(gemm_split.gemm_split(x, w, torch.empty(M, N, device="cuda"))), off(ops.gemm_simt(x, w, torch.empty(M, N, device="cuda")))
+    print(f"{kind}, K {K}: split {split:.3g}, fused multiply-adds {chain:.3g}")
+    assert split <= max(chain, 2.0 ** -24)
+
+
 @pytest.mark.parametrize("bn", [64, 128, 256])
 @pytest.mark.parametrize("splits", [1, 3, 8])
 def test_every_tile_and_share_of_k(bn, splits):
