@@ -8,7 +8,7 @@
 // a sum stays there for 64 products only (small parts first); every 64-wide chunk of K is taken out of tensor memory and added to a
 // float32 register, rounded to nearest.  Against 64 bits the error is 1.1e-7 at K 2,048 and 1.8e-7 at K 5,632 (2-norm) where one
 // chain of K fused multiply-adds leaves 5.5e-7 and 1.1e-6.
-// A number that is not finite, or a sum that overflows on the way, makes a part infinity minus infinity: an output that is not finite is
+// A number that is not finite, one too small for its parts, or a sum that overflows on the way makes the sum of the parts infinite or NaN: an output that is not finite is
 // worked out again as one chain of fused multiply-adds from the operands themselves, so it is what the CUDA-core product gives.
 //
 //   split    [rows, K] float32 -> three bfloat16 planes: bound by memory, 10 bytes a number (11,264 x 2,048: 45 us, 5.1 TB/s).
@@ -94,13 +94,17 @@ __device__ __forceinline__ float top_part(float v) {
     const uint32_t u = __float_as_uint(v), r = (u + 0x7fffu + ((u >> 16) & 1u)) & 0xffff0000u;
     return __uint_as_float((r & 0x7f800000u) == 0x7f800000u ? u & 0xffff0000u : r);
 }
-// A number as its nearest bfloat16 number, the nearest to what is left, and the rest, which is one too; a number that is not finite has no rest.
+// A part that is neither zero nor a normal number: bfloat16 may hold less of it than there is (its last bit is 2^-133, float32's 2^-149).
+__device__ __forceinline__ bool too_small(uint32_t u) { return (u & 0x7f800000u) == 0u && (u & 0x007fffffu) != 0u; }
+// A number as its nearest bfloat16 number, the nearest to what is left, and the rest, which is one too; a number that is not finite has no rest.  One so small
+// (below 2^-102) that a part leaves the normal numbers goes on as NaN, and its outputs with it: they are then worked out from the operands.
 __device__ __forceinline__ void cut3(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
     const uint32_t u = __float_as_uint(v);
     b = c = 0u;
     if ((u & 0x7f800000u) == 0x7f800000u) { a = (u & 0x007fffffu) ? 0x7fc00000u : u; return; }
     const float fa = top_part(v), r = v - fa, fb = top_part(r);            // the differences are exact
     a = __float_as_uint(fa); b = __float_as_uint(fb); c = __float_as_uint(r - fb);       // (at most 7 bits: c's lower half is zero)
+    if (too_small(a) || too_small(b) || too_small(c)) { a = 0x7fc00000u; b = c = 0u; }
 }
 
 // src [rows, K] -> dst [Kp / 64][row blocks][3 planes][block rows][64]: what one stage of the product reads of one block of rows is one stretch

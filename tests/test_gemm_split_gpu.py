@@ -96,6 +96,18 @@ def test_numbers_that_are_not_finite_or_overflow(force):
     assert ((got - want).abs()[fine] <= 1e-4 * 512 ** 0.5).all()
 
 
+@pytest.mark.parametrize("down,up", [(-104, 90), (-113, 100), (-120, 110), (-128, 115), (-140, 120)])
+def test_numbers_below_the_range_of_their_parts(down, up):
+    """Operands down to float32's last bit, times large ones: nothing of them is lost."""
+    from mini_inference_engine_b200.kernels import gemm_split
+    x, w, _ = operands(70, 300, 512, 7)
+    x[5] = 0.0
+    x[9, ::2] = 0.0
+    x, w = x * 2.0 ** down, w * 2.0 ** up
+    check(gemm_split.gemm_split(x, w, torch.empty(70, 300, device="cuda")), x, w, None)
+    check(gemm_split.gemm_split(w, x, torch.empty(300, 70, device="cuda"), force=(64, 2)), w, x, None)
+
+
 def test_the_runtime_takes_it_for_prompts_in_float32():
     from mini_inference_engine_b200.kernels import gemm_split
     from mini_inference_engine_b200.kernels.linear import linear
