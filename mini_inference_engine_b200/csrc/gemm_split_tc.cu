@@ -9,7 +9,8 @@
 // float32 register, rounded to nearest.  Against 64 bits the error is 1.1e-7 at K 2,048 and 1.8e-7 at K 5,632 (2-norm) where one
 // chain of K fused multiply-adds leaves 5.5e-7 and 1.1e-6.
 // A number that is not finite, one too small for its parts, or a sum that overflows on the way makes the sum of the parts infinite or NaN: an output that is not finite is
-// worked out again as one chain of fused multiply-adds from the operands themselves, so it is what the CUDA-core product gives.
+// worked out again as one chain of fused multiply-adds from the operands themselves, so it is what the CUDA-core product gives: by the whole block, once its
+// tiles are done and nothing waits for it, 64 x 64 outputs at a time (`sp_again`).
 //
 //   split    [rows, K] float32 -> three bfloat16 planes: bound by memory, 10 bytes a number (11,264 x 2,048: 45 us, 5.1 TB/s).
 //   product  a pair of blocks owns 256 rows of w and BN (64, 128 or 256) tokens; per 64-wide chunk of K each block's stage
@@ -80,11 +81,59 @@ __device__ __forceinline__ void sp_ld32(uint32_t addr, float* v) {
 
 __device__ __forceinline__ bool is_finite_f32(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
-// one chain of fused multiply-adds over K, for an output that the parts could not give
-__device__ __noinline__ float sp_chain(const float* __restrict__ x, const float* __restrict__ w, int K) {
-    float acc = 0.f;
-    for (int k = 0; k < K; ++k) acc = fmaf(x[k], w[k], acc);
-    return acc;
+// The outputs of tokens m0 .. m0 + mc and rows n0 .. n0 + nc of w that are not finite, worked out again from the operands themselves by the whole block (256 threads or
+// more), one chain of fused multiply-adds each: 64 x 64 outputs a step, 32 of K at a time through `sm` (2 x 64 x 33 floats), four by four a thread; what is
+// finite stays as it is, and a thread whose outputs all are only helps with the loads.
+#define SP_AGAIN_FLOATS (2 * 64 * 33)
+__device__ __noinline__ void sp_again(const SpParams& p, float* sm, int m0, int mc, int n0, int nc) {
+    float* xs = sm;
+    float* ws = sm + 64 * 33;
+    const int tid = threadIdx.x, ty = (tid >> 4) * 4, tx = tid & 15;
+    const int m_end = min(m0 + mc, p.M), n_end = min(n0 + nc, p.N);
+    for (int mt = m0; mt < m_end; mt += 64)
+        for (int nt = n0; nt < n_end; nt += 64) {
+            uint32_t again = 0;
+            float* o = p.out + (int64_t)(mt + ty) * p.out_stride + nt + tx;
+            if (tid < 256) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (mt + ty + i < m_end && nt + tx + 16 * j < n_end && !is_finite_f32(o[i * p.out_stride + 16 * j])) again |= 1u << (4 * i + j);
+            }
+            if (!__syncthreads_or(again != 0)) continue;
+            float acc[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+            for (int k0 = 0; k0 < p.K; k0 += 32) {
+                for (int i = tid; i < 64 * 32; i += blockDim.x) {
+                    const int r = i >> 5, k = i & 31;
+                    xs[r * 33 + k] = mt + r < m_end && k0 + k < p.K ? p.x[(int64_t)(mt + r) * p.K + k0 + k] : 0.f;
+                    ws[r * 33 + k] = nt + r < n_end && k0 + k < p.K ? p.w[(int64_t)(nt + r) * p.K + k0 + k] : 0.f;
+                }
+                __syncthreads();
+                if (again) {
+                    const int n = min(32, p.K - k0);
+                    for (int k = 0; k < n; ++k) {
+                        float a[4], b[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) { a[i] = xs[(ty + i) * 33 + k]; b[i] = ws[(tx + 16 * i) * 33 + k]; }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                    }
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if ((again >> (4 * i + j)) & 1) o[i * p.out_stride + 16 * j] = acc[i][j] + (p.bias ? load_tagged(p.bias, nt + tx + 16 * j, p.bias_tag) : 0.f);
+        }
 }
 
 // --------------------------------------------------------------------------- split
@@ -145,14 +194,14 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ sr
 
 template <int BN>
 __global__ void __launch_bounds__(SP_THREADS, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SpParams p) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SpParams p) {
     constexpr int BNH = BN / 2;                                   // tokens a block loads; tokens a thread adds up
     constexpr uint32_t B_PLANE = BNH * 128u, STAGE = 3 * SP_A_PLANE + 3 * B_PLANE;
     constexpr int ACCS = 512 / BN < SP_MAX_ACCS ? 512 / BN : SP_MAX_ACCS, TMEM_COLS = ACCS * BN;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) uint64_t full[SP_MAX_STAGES], empty[SP_MAX_STAGES], acc_full[SP_MAX_ACCS], acc_empty[SP_MAX_ACCS];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, again;                             // again: an output of this block is not finite
 
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -163,7 +212,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        abort_flag = 0;
+        abort_flag = again = 0;
         for (int s = 0; s < SP_MAX_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < SP_MAX_ACCS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }     // eight warps of two blocks
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -278,10 +327,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                         fine = fine && (m0 + i >= p.M || is_finite_f32(acc[i]));
                         if (m0 + i < p.M) o[(int64_t)i * p.out_stride] = acc[i] + b;
                     }
-                    if (!fine)                                     // (looked for again in what was stored: the sums stay in registers)
-                        for (int i = 0; i < BNH && m0 + i < p.M; ++i)
-                            if (!is_finite_f32(o[(int64_t)i * p.out_stride]))
-                                o[(int64_t)i * p.out_stride] = sp_chain(p.x + (int64_t)(m0 + i) * p.K, p.w + (int64_t)n * p.K, p.K) + b;
+                    if (!fine) again = 1;
                 }
             }
         }
@@ -292,37 +338,46 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (abort_flag) {
         if (threadIdx.x == 0) atomicExch(p.error, 1);
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    } else if (again) {                                            // (every copy has arrived and every MMA has read it: the stages' memory is free)
+        float* sm = reinterpret_cast<float*>(smem_dyn + (base - smem_u32(smem_dyn)));
+        for (int item = pair; item < p.num_items; item += pairs)
+            sp_again(p, sm, (item % p.tiles_m) * BN, BN, (item / p.tiles_m) * 256 + (int)rank * 128, 128);
     }
     cluster_sync_all();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
 
-// The shares of K added up in order (a thread four columns where N allows).
+// The shares of K added up in order: a block 64 columns of 4 V tokens, a thread V columns next to one another.
 template <int V>
-__global__ void __launch_bounds__(256) split_sum_kernel(const SpParams p) {
+__global__ void __launch_bounds__(256) split_sum_kernel(const __grid_constant__ SpParams p) {
+    __shared__ float sm[SP_AGAIN_FLOATS];
     pdl_enter();
-    const int64_t groups = (int64_t)p.M * (p.N / V), per = (int64_t)p.M * p.N;
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= groups) return;
-    const int m = (int)(g / (p.N / V)), n = (int)(g - (int64_t)m * (p.N / V)) * V;
-    const float* src = p.partial + (int64_t)m * p.N + n;
-    float v[V];
+    constexpr int TOKENS = 4 * V;
+    const int tiles_n = (p.N + 63) / 64, m0 = (int)(blockIdx.x / tiles_n) * TOKENS, n0 = (int)(blockIdx.x % tiles_n) * 64;
+    const int m = m0 + threadIdx.x / (64 / V), n = n0 + threadIdx.x % (64 / V) * V;
+    bool fine = true;
+    if (m < p.M && n < p.N) {
+        const int64_t per = (int64_t)p.M * p.N;
+        const float* src = p.partial + (int64_t)m * p.N + n;
+        float v[V];
 #pragma unroll
-    for (int i = 0; i < V; ++i) v[i] = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-        float u[V];
-        if constexpr (V == 4) *reinterpret_cast<float4*>(u) = __ldcg(reinterpret_cast<const float4*>(src + s * per));
-        else u[0] = __ldcg(src + s * per);
+        for (int i = 0; i < V; ++i) v[i] = 0.f;
+        for (int s = 0; s < p.splits; ++s) {
+            float u[V];
+            if constexpr (V == 4) *reinterpret_cast<float4*>(u) = __ldcg(reinterpret_cast<const float4*>(src + s * per));
+            else u[0] = __ldcg(src + s * per);
 #pragma unroll
-        for (int i = 0; i < V; ++i) v[i] += u[i];
+            for (int i = 0; i < V; ++i) v[i] += u[i];
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            fine = fine && is_finite_f32(v[i]);
+            if (p.bias) v[i] += load_tagged(p.bias, n + i, p.bias_tag);
+            p.out[(int64_t)m * p.out_stride + n + i] = v[i];
+        }
     }
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        if (!is_finite_f32(v[i])) v[i] = sp_chain(p.x + (int64_t)m * p.K, p.w + (int64_t)(n + i) * p.K, p.K);
-        if (p.bias) v[i] += load_tagged(p.bias, n + i, p.bias_tag);
-        p.out[(int64_t)m * p.out_stride + n + i] = v[i];
-    }
+    if (__syncthreads_or(!fine)) sp_again(p, sm, m0, TOKENS, n0, 64);
 }
 
 // --------------------------------------------------------------------------- host side
@@ -385,8 +440,9 @@ extern "C" int mie_gemm_split(const void* xs, const void* ws, const float* x, co
     p.num_items = p.tiles_m * ((N + 255) / 256) * p.splits;
     rc = bn == 64 ? sp_launch<64>(mw, mx, p, stream) : bn == 128 ? sp_launch<128>(mw, mx, p, stream) : sp_launch<256>(mw, mx, p, stream);
     if (rc || p.splits == 1) return rc;
-    if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3((unsigned)(((int64_t)M * (N / 4) + 255) / 256)), dim3(256), 0, stream, p);
-    return launch_kernel(split_sum_kernel<1>, dim3((unsigned)(((int64_t)M * N + 255) / 256)), dim3(256), 0, stream, p);
+    const unsigned tiles_n = (unsigned)((N + 63) / 64);
+    if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3(tiles_n * (unsigned)((M + 15) / 16)), dim3(256), 0, stream, p);
+    return launch_kernel(split_sum_kernel<1>, dim3(tiles_n * (unsigned)((M + 3) / 4)), dim3(256), 0, stream, p);
 }
 
 extern "C" int mie_gemm_split_error(void) { return g_error_host ? *g_error_host : 0; }

@@ -96,6 +96,43 @@ def test_numbers_that_are_not_finite_or_overflow(force):
     assert ((got - want).abs()[fine] <= 1e-4 * 512 ** 0.5).all()
 
 
+@pytest.mark.parametrize("what", ["nan", "inf", "overflow", "a column"])
+@pytest.mark.parametrize("force", [(64, 1), (256, 1), (128, 3)])
+def test_many_outputs_that_are_not_finite(what, force):
+    """A step of such numbers is what the CUDA-core product leaves, and takes no more than a few times that product's time (seen: 2.3 to 4 times, and 7 times with
+    tiles that only a third of the SMs have; an output after the other in a thread took many more times)."""
+    from mini_inference_engine_b200.kernels import gemm_split, gemm_tc, ops
+    M, N, K = 640, 2048, 1024
+    x, w, bias = operands(M, N, K, 3)
+    if what == "nan":
+        x.fill_(float("nan"))
+    elif what == "inf":
+        x[:] = float("inf")
+    elif what == "overflow":
+        x, w = x.abs() * 1e20 + 1e20, w.abs() * 1e19 + 1e19
+    else:
+        w[:, 17] = -float("inf")
+    got, want = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    split, plain = lambda: gemm_split.gemm_split(x, w, got, bias, force=force), lambda: ops.gemm_simt(x, w, want, bias)
+    times = []
+    for fn in (split, plain):
+        fn()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        for _ in range(3):
+            fn()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) / 3)
+    gemm_tc.check_error()
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(got), kind(want))
+    assert not torch.isfinite(want).any()
+    print(f"{what}, {force}: {times[0]:.3f} ms, the CUDA-core product {times[1]:.3f} ms")
+    assert times[0] <= 16 * times[1]
+
+
 @pytest.mark.parametrize("down,up", [(-104, 90), (-113, 100), (-120, 110), (-128, 115), (-140, 120)])
 def test_numbers_below_the_range_of_their_parts(down, up):
     """Operands down to float32's last bit, times large ones: nothing of them is lost."""
