@@ -134,7 +134,8 @@ __device__ __forceinline__ void unit_triangular_inverse(const float* A, float* T
             const int bi = w + (idx >> 8), bj = bi - w, r = (idx >> 4) & 15, c = idx & 15;
             float v = 0.f;
 #pragma unroll
-            for (int m = 0; m < 16; ++m) v = fmaf(T[(bi * 16 + r) * CHP + bi * 16 + m], X[(idx & ~255) + m * 16 + c], v);
+            for (int m = 0; m < 16; ++m)                       // (the inverse ends at its diagonal; a later token's sums, which may not be finite, are not read)
+                v = fmaf(T[(bi * 16 + r) * CHP + bi * 16 + m], m <= r ? X[(idx & ~255) + m * 16 + c] : 0.f, v);
             T[(bi * 16 + r) * CHP + bj * 16 + c] = -v;
         }
         __syncthreads();

@@ -44,14 +44,16 @@ def exact(rows, q, k, v, beta, log, slots, state, H, G):
     return o, S_all
 
 
-def run(rows, q, k, v, beta, log, starts, lens, slots, state, H, G, D, V, min_len=1, known=True, token_by_token=False):
+def run(rows, q, k, v, beta, log, starts, lens, slots, state, H, G, D, V, min_len=1, known=True, token_by_token=False, a_head=False):
     from mini_inference_engine_b200.kernels import ops
     T = sum(rows)
     state, out = state.clone(), torch.zeros(T, H * V, device="cuda")
     flat = lambda t: t.reshape(T, -1).contiguous()
     sizes = dict(num_heads=H, num_kv_heads=G, dim=D, vdim=V)
     decay = torch.exp(log)
-    if token_by_token:
+    if a_head:                                                # one decay per head: the first channel's
+        ops.delta_chunks(flat(q), flat(k), flat(v), beta, log[:, :, 0].contiguous(), starts, lens, slots, state, out, min_len=min_len, **sizes)
+    elif token_by_token:
         kq = flat((q * k).sum(-1))
         ops.delta_scan(flat(q), flat(k), flat(v), beta, flat(decay), kq, starts, lens, slots, state, out, **sizes)
     else:
@@ -92,14 +94,15 @@ def test_short_rows_are_left_alone(known):
         assert (out[lo:hi] - ref[lo:hi]).abs().max() <= 1e-5 * ref.abs().max()
 
 
-def test_a_token_that_is_not_finite_spoils_only_what_follows():
+@pytest.mark.parametrize("a_head", [False, True])
+@pytest.mark.parametrize("at", [0, 15, 64, 75, 85, 103, 112, 127, 139])
+@pytest.mark.parametrize("what", ["key", "value"])
+def test_a_token_that_is_not_finite_spoils_only_what_follows(what, at, a_head):
     rows, H, G, D, V = [140, 80], 2, 2, 32, 24
     args = operands(rows, H, G, D, V, "mild")
-    for i, t in enumerate((args[1], args[2])):                # a key, a value
-        spoilt = [x.clone() for x in args]
-        spoilt[1 + i][75] = float("nan")
-        out, _ = run(rows, *spoilt, H, G, D, V)
-        assert torch.isfinite(out[:75]).all() and torch.isfinite(out[140:]).all() and not torch.isfinite(out[75:140]).any()
+    args[1 if what == "key" else 2][at] = float("nan")
+    out, _ = run(rows, *args, H, G, D, V, a_head=a_head)
+    assert torch.isfinite(out[:at]).all() and torch.isfinite(out[140:]).all() and not torch.isfinite(out[at:140]).any()
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
