@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256) delta_head_prepare_kernel(const HeadParam
                 const float ld = -expf(p.a_log[h]) * softplus_of(z[h] + p.dt_bias[h]);
                 const int64_t at = (int64_t)t * H + h;
                 decay[at] = expf(ld);
-                log_decay[at] = fmaxf(ld, -100.f);             // (e^-100 is nothing in 32 bits; the bound keeps sums of these, and their differences, sharp)
+                log_decay[at] = ld < -100.f ? -100.f : ld;     // (e^-100 is nothing in 32 bits; the bound keeps sums of these, and their differences, sharp; NaN stays)
                 beta[at] = 1.0f / (1.0f + expf(-z[H + h]));
             }
             continue;

@@ -21,6 +21,8 @@
 
 #define DELTA_MAX_KEY 512    // the longest key: sixteen entries a lane, thirty-two lanes a column
 
+// A log decay for the chunks: none below -100 (e^-100 is nothing in 32 bits), and one that is no number stays none.
+__device__ __forceinline__ float log_bound(float l) { return l < -100.f ? -100.f : l; }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // The convolution's output for channel c (of C) at token t: taps [C, K], last tap on the token itself.
@@ -95,7 +97,7 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int64_t stride,
         const float rate = expf(a_log[i / D]);
         const float l = -rate * softplus_f(low[(int64_t)t * low_stride + i] + dt_bias[i]);
         decay[(int64_t)t * H * D + i] = expf(l);
-        if (log_decay) log_decay[(int64_t)t * H * D + i] = fmaxf(l, -100.f);
+        if (log_decay) log_decay[(int64_t)t * H * D + i] = log_bound(l);
     }
     __syncthreads();                                   // q and k of this token, written above by other warps of the block
     for (int g = warp; g < G; g += nw) {               // k . q per key head: the same for every value column of the recurrence
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(256) delta_prepare_runs_kernel(const T* __rest
                                          -rate * softplus_f(x[i].w + bias.w));
             const int64_t to = (int64_t)(t0 + i) * H * D + at;
             *reinterpret_cast<float4*>(decay + to) = make_float4(expf(l.x), expf(l.y), expf(l.z), expf(l.w));
-            if (log_decay) *reinterpret_cast<float4*>(log_decay + to) = make_float4(fmaxf(l.x, -100.f), fmaxf(l.y, -100.f), fmaxf(l.z, -100.f), fmaxf(l.w, -100.f));
+            if (log_decay) *reinterpret_cast<float4*>(log_decay + to) = make_float4(log_bound(l.x), log_bound(l.y), log_bound(l.z), log_bound(l.w));
         }
         return;
     }
