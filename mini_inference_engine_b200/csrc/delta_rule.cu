@@ -199,19 +199,19 @@ __global__ void __launch_bounds__(256) delta_prepare_runs_kernel(const T* __rest
             if (on) b.step(raw1[i], k);
             float qq = 0.f, kk = 0.f, qk = 0.f;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { qq = fmaf(q[e], q[e], qq); kk = fmaf(k[e], k[e], kk); qk = fmaf(q[e], k[e], qk); }
+            for (int e = 0; e < 4; ++e) { qq = fmaf(q[e], q[e], qq); kk = fmaf(k[e], k[e], kk); }
             qq = warp_sum(qq);
             kk = warp_sum(kk);
-            qk = warp_sum(qk);
             const float qs = q_scale / sqrtf(qq + unit_eps), ks = 1.0f / sqrtf(kk + unit_eps);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { q[e] *= qs; k[e] *= ks; }
+            for (int e = 0; e < 4; ++e) { q[e] *= qs; k[e] *= ks; qk = fmaf(q[e], k[e], qk); }      // (of the vectors as they are written: sums of squares may overflow, which makes those zero)
+            qk = warp_sum(qk);
             const int64_t to = ((int64_t)t * G + unit) * D + at;
             if (on) {
                 *reinterpret_cast<float4*>(qn + to) = make_float4(q[0], q[1], q[2], q[3]);
                 *reinterpret_cast<float4*>(kn + to) = make_float4(k[0], k[1], k[2], k[3]);
             }
-            if (lane == 0) kq[(int64_t)t * G + unit] = qk * qs * ks;
+            if (lane == 0) kq[(int64_t)t * G + unit] = qk;
         }
         return;
     }

@@ -9,14 +9,15 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows", [[1], [1] * 9, [3, 1, 2, 8, 17, 5], [700, 900], [4000]])
 @pytest.mark.parametrize("H,G,D,V", [(2, 2, 128, 128), (4, 2, 64, 32), (3, 1, 20, 12), (16, 16, 128, 128)])
-def test_runs_against_tokens(dt, rows, H, G, D, V):
+@pytest.mark.parametrize("scale", [1.0, 1e20])                  # (1e20: sums of squares overflow, and unit vectors become zeros)
+def test_runs_against_tokens(dt, rows, H, G, D, V, scale):
     from mini_inference_engine_b200.kernels import ops
     g = torch.Generator(device="cuda").manual_seed(len(rows) + H)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     T, C = sum(rows), 2 * G * D + H * V
     if T > 1000 and H == 16:
         rows, T = [300, 260], 560
-    proj, low = rnd(T, -(-(C + H) // 8) * 8).to(dt), rnd(T, H * D + 4)
+    proj, low = (rnd(T, -(-(C + H) // 8) * 8) * scale).to(dt), rnd(T, H * D + 4)
     taps, conv, a_log, bias = rnd(C, 4) * 0.5, rnd(len(rows) + 1, 3, C), rnd(H), rnd(H * D)
     lens = torch.tensor(rows, dtype=torch.int32, device="cuda")
     starts = torch.cumsum(lens, 0, dtype=torch.int32) - lens
