@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "range_check.cuh"
 
+#define MIE_K_ATTENTION_F32 14     // this kernel's number in the range report (csrc/range_check.cuh)
 #define F32_PAIRS 64
 #define F32_KEYS 64
 #define F32_PS 80                 // stride of a row of probabilities: neighbouring rows 16 banks apart
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(THREADS, DT == 64 ? 3 : 2) f32_attention_kerne
     if (r < 0) return;
     const int q_len = p.row_q_len[r], ctx_len = p.row_ctx_len[r], q_start = p.row_q_start[r], pair0 = s_tile * F32_PAIRS;
     if (ctx_len > p.table_stride * p.page_size) {
-        if (threadIdx.x == 0) range_report(p.report, MIE_RANGE_POSITION, MIE_K_ATTENTION_SIMT, r, ctx_len);
+        if (threadIdx.x == 0) range_report(p.report, MIE_RANGE_POSITION, MIE_K_ATTENTION_F32, r, ctx_len);
         return;
     }
     const int lane = threadIdx.x & 31, tx = lane & 15, ty = (threadIdx.x >> 5) * 2 + (lane >> 4);
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(THREADS, DT == 64 ? 3 : 2) f32_attention_kerne
                 const bool on = (key >= k_lo || key < p.keep) && key < k_hi && d < D;
                 const float* src = cache;
                 if (on) {
-                    const int page = checked_page(table[key >> p.page_shift], p.num_pages, p.report, MIE_K_ATTENTION_SIMT, key >> p.page_shift);
+                    const int page = checked_page(table[key >> p.page_shift], p.num_pages, p.report, MIE_K_ATTENTION_F32, key >> p.page_shift);
                     src = cache + (((int64_t)page * p.num_kv_heads + kvh) * p.page_size + (key & (p.page_size - 1))) * D + d;
                 }
                 f32_copy16(dst + jj * stride + d, src, on);

@@ -79,7 +79,7 @@ _RANGE_CODES = {1: "token id outside the vocabulary (or the fed-back tokens)", 2
 _RANGE_KERNELS = {1: "embedding", 2: "rope_cache", 3: "norm", 4: "attention_simt", 5: "attention_decode",
                   6: "attention_prefill", 7: "attention_prefill_tc", 8: "gemm_tcgen05 (q|k|v with rotation)",
                   9: "norm_group", 10: "qk_norm_rope", 11: "hyper_norm", 12: "latent_kv",
-                  13: "sandwich_norm"}
+                  13: "sandwich_norm", 14: "attention_f32"}
 _range_report: torch.Tensor | None = None
 _range_told: set = set()
 

@@ -110,3 +110,21 @@ def test_the_step_takes_it_in_float32():
         ctx = SimpleNamespace(block_tables=[block], row_q_start=starts, row_q_len=lens, row_ctx_len=ctx_lens, num_tokens=T, max_ctx_len=400, host=host)
         got = attention.attention(q, ctx, cache, torch.zeros_like(out), H, G, D, D ** -0.5, 0)
         close(got, want, v)
+
+
+@pytest.mark.parametrize("what", ["page", "context"])
+def test_a_number_out_of_range_is_reported_under_this_kernel_s_name(what):
+    """A page that is not in the pool (page 0 is read in its place), and more positions than the block table covers (the row is left alone)."""
+    from mini_inference_engine_b200.kernels import ops
+    H, G, D, page = 8, 2, 64, 16
+    args, _, out = case([(70, 70)], H, G, D, page)
+    args = list(args)
+    if what == "page":
+        args[4][0, 1] = args[2].shape[0]
+    else:
+        args[7] = args[7] + 1000
+    ops.check_range_errors()
+    ops.attention_f32(*args, out, H, G, D, page, D ** -0.5, 0)
+    torch.cuda.synchronize()
+    with pytest.raises(ops.KernelError, match="attention_f32"):
+        ops.check_range_errors()
