@@ -135,8 +135,13 @@ static int tc_setup() {
         g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
     if (!g_error_host) {
-        cudaError_t e = cudaHostAlloc((void**)&g_error_host, sizeof(int), cudaHostAllocMapped);
+        // A library's first use may fall into a stream capture, which forbids allocations to the thread that captures unless that thread asks for them.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) return (int)e;
+        e = cudaHostAlloc((void**)&g_error_host, sizeof(int), cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) { g_error_host = nullptr; return (int)e; }
         *g_error_host = 0;
         e = cudaHostGetDevicePointer((void**)&g_error_dev, g_error_host, 0);
         if (e != cudaSuccess) return (int)e;

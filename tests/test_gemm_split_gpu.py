@@ -153,3 +153,27 @@ def test_the_runtime_takes_it_for_prompts_in_float32():
     got = linear(x, w, bias, torch.float32)
     assert torch.equal(got, gemm_split.gemm_split(x, w, torch.empty_like(got), bias))
     check(got, x, w, bias)
+
+
+def test_its_first_use_may_fall_into_a_capture():
+    """A process whose first product of this kind is captured (a portion that ran on the CUDA cores is captured at its padded length)."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from mini_inference_engine_b200.kernels import gemm_split, gemm_tc
+x, w, out = torch.randn(32, 256, device="cuda"), torch.randn(512, 256, device="cuda"), torch.empty(32, 512, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    gemm_split.gemm_split(x, w, out)
+graph.replay()
+torch.cuda.synchronize()
+gemm_tc.check_error()
+want = x.double() @ w.double().t()
+assert ((out.double() - want).norm() / want.norm()).item() < 1e-6
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
