@@ -27,8 +27,9 @@ struct DcParams {
     const float* decay; const float* tok_decay;
     float* state; float* states; float* scratch;        // scratch per (chunk, head): P [64, 64], G [64]
     float* out; int H, D, Dv_in, Dv, v_act;
+    int h0, heads;                             // the heads of this pass: states and scratch hold these only
 };
-__device__ __forceinline__ float* dc_scratch(const DcParams& p, int64_t chunk, int h) { return p.scratch + (chunk * p.H + h) * (DC_L * DC_L + DC_L); }
+__device__ __forceinline__ float* dc_scratch(const DcParams& p, int64_t chunk, int h) { return p.scratch + (chunk * p.heads + h - p.h0) * (DC_L * DC_L + DC_L); }
 
 __device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool on) {       // zeros where `on` is false (nothing is read then)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
     const bool mine = dc_find(p, &s_row, &s_chunk);
     pdl_wait();                                        // (a block without work waits too: see common.cuh)
     if (!mine) return;
-    const int h = blockIdx.y, H = p.H, D = p.D, half = blockIdx.z;
+    const int h = p.h0 + blockIdx.y, H = p.H, D = p.D, half = blockIdx.z;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     dc_rows<DT>(K, p.k + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
     if (half == 0) dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
         *at = v;
     }
     // the state's columns, 64 at a time: column 4 ty + c, entries 4 tx + 64 e .. + 3
-    float* to = p.states + ((int64_t)blockIdx.x * H + h) * (int64_t)p.Dv * D;
+    float* to = p.states + ((int64_t)blockIdx.x * p.heads + blockIdx.y) * (int64_t)p.Dv * D;
     constexpr int E = DT / 64;
     const int tiles = (p.Dv_in + 63) / 64, per = (tiles + halves - 1) / halves;
     for (int tile = half * per; tile < min(tiles, (half + 1) * per); ++tile) {
@@ -198,13 +199,13 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
 // A thread four entries of a state; eight chunks' additions are read ahead of the chain.
 __global__ void __launch_bounds__(128) decay_combine_kernel(const DcParams p) {
     pdl_enter();
-    const int64_t per_state = (int64_t)p.H * p.Dv * p.D, e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int64_t per_state = (int64_t)p.heads * p.Dv * p.D, e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int row = blockIdx.y, items = dc_chunks(p.row_q_len[row]);
     if (e >= per_state || items == 0) return;
     int first = 0;
     for (int r = 0; r < row; ++r) first += dc_chunks(p.row_q_len[r]);
-    const int h = (int)(e / ((int64_t)p.Dv * p.D));
-    float* end = p.state + (int64_t)p.state_slots[row] * per_state + e;
+    const int h = p.h0 + (int)(e / ((int64_t)p.Dv * p.D));
+    float* end = p.state + ((int64_t)p.state_slots[row] * p.H + p.h0) * p.Dv * p.D + e;
     float4 cur = *reinterpret_cast<const float4*>(end);
     float* slot = p.states + (int64_t)first * per_state + e;
     const int last = p.row_q_len[row] - (items - 1) * DC_L - 1;
@@ -243,9 +244,9 @@ __global__ void __launch_bounds__(256, 2) decay_output_kernel(const DcParams p) 
     const bool mine = dc_find(p, &s_row, &s_chunk);
     pdl_wait();                                        // (a block without work waits too: see common.cuh)
     if (!mine) return;
-    const int h = blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
+    const int h = p.h0 + blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
-    const float* from = p.states + ((int64_t)blockIdx.x * H + h) * (int64_t)p.Dv * D;
+    const float* from = p.states + ((int64_t)blockIdx.x * p.heads + blockIdx.y) * (int64_t)p.Dv * D;
     const float* pg = dc_scratch(p, blockIdx.x, h);
     const bool ones = blockIdx.z == 0 && p.Dv > p.Dv_in;
     dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
@@ -330,18 +331,17 @@ __global__ void __launch_bounds__(256, 2) decay_output_kernel(const DcParams p) 
 extern "C" int mie_decay_chunk_floats() { return DC_L * DC_L + DC_L; }
 
 // Rows of more than 64 new tokens.  q, k [T, H, D] float32, v [T][v_stride] of `v_tag`'s type; decay [H] or tok_decay [T, H]; state [slots, H, Dv, D],
-// states [chunks, H, Dv, D], scratch [chunks, H, mie_decay_chunk_floats()], `chunks` at least the chunks of those rows; out [T, H, Dv] with Dv = Dv_in or
+// `per_pass` heads at a time, on the same scratch memory: states [chunks, per_pass, Dv, D], scratch [chunks, per_pass, mie_decay_chunk_floats()], `chunks` at least the chunks of those rows; out [T, H, Dv] with Dv = Dv_in or
 // Dv_in + 1 (the last column fed with ones).  D a multiple of 4 up to 128; q, k, state, states 16-byte aligned.
 extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, int v_tag, long long v_stride, const int* row_q_start, const int* row_q_len,
                                 const int* state_slots, int num_rows, const float* decay, const float* tok_decay, float* state, float* states,
-                                float* scratch, int chunks, float* out, int H, int D, int Dv_in, int Dv, int v_act, cudaStream_t stream) {
+                                float* scratch, int chunks, float* out, int H, int D, int Dv_in, int Dv, int v_act, int per_pass, cudaStream_t stream) {
     if (num_rows <= 0 || chunks <= 0) return 0;
-    if (H <= 0 || D < 4 || D > 128 || D % 4 || Dv_in <= 0 || Dv < Dv_in || Dv > Dv_in + 1 || (!decay && !tok_decay)) return MIE_ERR_BAD_ARG;
+    if (H <= 0 || D < 4 || D > 128 || D % 4 || Dv_in <= 0 || Dv < Dv_in || Dv > Dv_in + 1 || (!decay && !tok_decay) || per_pass < 1) return MIE_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(states) |
          reinterpret_cast<uintptr_t>(scratch)) & 15) return MIE_ERR_BAD_ARG;
-    const DcParams p{q, k, v, v_stride, row_q_start, row_q_len, state_slots, num_rows, decay, tok_decay, state, states, scratch, out, H, D, Dv_in, Dv, v_act};
+    DcParams p{q, k, v, v_stride, row_q_start, row_q_len, state_slots, num_rows, decay, tok_decay, state, states, scratch, out, H, D, Dv_in, Dv, v_act, 0, 0};
     const int halves = Dv_in > 64 ? 2 : 1;
-    const int64_t quads = (int64_t)H * Dv * D / 4;
     int rc;
 #define DC_LAUNCH(T, DT)                                                                                                                  \
     {                                                                                                                                     \
@@ -349,11 +349,17 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
         cudaError_t e = cudaFuncSetAttribute(decay_local_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l);             \
         if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_output_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_o);  \
         if (e != cudaSuccess) return (int)e;                                                                                              \
-        rc = launch_kernel(decay_local_kernel<T, DT>, dim3(chunks, H, halves), dim3(256), smem_l, stream, p, halves);                     \
-        if (rc) return rc;                                                                                                                \
-        rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), num_rows), dim3(128), 0, stream, p);               \
-        if (rc) return rc;                                                                                                                \
-        return launch_kernel(decay_output_kernel<T, DT>, dim3(chunks, H, (Dv_in + 63) / 64), dim3(256), smem_o, stream, p);               \
+        for (p.h0 = 0; p.h0 < H; p.h0 += per_pass) {                                                                                      \
+            p.heads = H - p.h0 < per_pass ? H - p.h0 : per_pass;                                                                          \
+            rc = launch_kernel(decay_local_kernel<T, DT>, dim3(chunks, p.heads, halves), dim3(256), smem_l, stream, p, halves);           \
+            if (rc) return rc;                                                                                                            \
+            const int64_t quads = (int64_t)p.heads * Dv * D / 4;                                                                          \
+            rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), num_rows), dim3(128), 0, stream, p);           \
+            if (rc) return rc;                                                                                                            \
+            rc = launch_kernel(decay_output_kernel<T, DT>, dim3(chunks, p.heads, (Dv_in + 63) / 64), dim3(256), smem_o, stream, p);       \
+            if (rc) return rc;                                                                                                            \
+        }                                                                                                                                 \
+        return 0;                                                                                                                         \
     }
     if (v_tag == MIE_F32) { if (D <= 64) DC_LAUNCH(float, 64) else DC_LAUNCH(float, 128) }
     if (v_tag == MIE_BF16) { if (D <= 64) DC_LAUNCH(bf16, 64) else DC_LAUNCH(bf16, 128) }

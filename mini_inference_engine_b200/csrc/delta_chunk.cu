@@ -146,7 +146,7 @@ template <int DT>
 __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
                                                                const float* __restrict__ beta, const float* __restrict__ log_decay,
                                                                const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
-                                                               int num_rows, int min_len, float* __restrict__ scratch, int H, int G, int D) {
+                                                               int num_rows, int min_len, float* __restrict__ scratch, int H, int G, int D, int h0, int heads) {
     extern __shared__ __align__(16) float sm[];
     float* K = sm;                                             // [64][DT + 4]
     float* Q = K + CH * (DT + 4);
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* _
     }
     __syncthreads();
     if (s_row < 0) return;
-    const int g = blockIdx.y, row = s_row;
+    const int g = h0 / (H / G) + blockIdx.y, row = s_row;
     const int t0 = row_q_start[row] + s_chunk * CH, count = min(CH, row_q_len[row] - s_chunk * CH);
     copy_rows<DT>(K, kn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
     copy_rows<DT>(Q, qn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prep_kernel(const float* _
             for (int k = 0; k < 2; ++k) { const int i = lane + 32 * k; be[i] = i < count ? beta[(int64_t)(t0 + i) * H + h] : 0.f; }
         }
         __syncthreads();
-        const ChunkScratch out(scratch, (int64_t)blockIdx.x * H + h);
+        const ChunkScratch out(scratch, (int64_t)blockIdx.x * heads + h - h0);
         if (threadIdx.x < CH) {
             out.eg[threadIdx.x] = expf(lg[threadIdx.x]);
             out.er[threadIdx.x] = expf(lg[CH - 1] - lg[threadIdx.x]);
@@ -261,7 +261,7 @@ template <int DT>
 __global__ void __launch_bounds__(CP_THREADS) delta_channel_prep_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ beta,
                                                                         const float* __restrict__ decay, const float* __restrict__ log_decay,
                                                                         const int* __restrict__ row_q_start, const int* __restrict__ row_q_len, int num_rows,
-                                                                        int min_len, float* __restrict__ scratch, int H, int G, int D) {
+                                                                        int min_len, float* __restrict__ scratch, int H, int G, int D, int h0, int heads) {
     constexpr int DP = DT + 4;
     extern __shared__ __align__(16) float sm[];
     float* K = sm;                                             // [64][DP]; then e^(sum from the block's first token) k
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(CP_THREADS) delta_channel_prep_kernel(const fl
     }
     __syncthreads();
     if (s_row < 0) return;
-    const int h = blockIdx.y, g = h / (H / G);
+    const int h = h0 + blockIdx.y, g = h / (H / G);
     const int t0 = row_q_start[s_row] + s_chunk * CH, count = min(CH, row_q_len[s_row] - s_chunk * CH);
     copy_rows<DT>(K, kn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
     copy_rows<DT>(Q, qn + ((int64_t)t0 * G + g) * D, (int64_t)G * D, D, count);
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(CP_THREADS) delta_channel_prep_kernel(const fl
         (which ? QK : KK)[r * CHP + c] = (r >> 4) == (c >> 4) ? (y[0] + y[2 * CH * 16]) + (y[4 * CH * 16] + y[6 * CH * 16]) : 0.f;
     }
     // sums of log decays; keys and queries with their factors, into scratch memory and, for the products between blocks, in place
-    const ChannelScratch out(scratch, (int64_t)blockIdx.x * H + h, D);
+    const ChannelScratch out(scratch, (int64_t)blockIdx.x * heads + blockIdx.y, D);
     for (int c = threadIdx.x; c < 4 * DT; c += CP_THREADS) {
         float s = 0.f;
 #pragma unroll
@@ -440,7 +440,7 @@ template <int DT, bool CHANNEL>
 __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn,
                                                                const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
                                                                const int* __restrict__ state_slots, int min_len, const float* __restrict__ scratch,
-                                                               float* __restrict__ state, float* __restrict__ out, int H, int G, int D, int Dv) {
+                                                               float* __restrict__ state, float* __restrict__ out, int H, int G, int D, int Dv, int h0, int heads) {
     constexpr int DP = DT + 4;
     extern __shared__ __align__(16) float sm[];
     float* KQ = sm;                                            // two stages of K [64][DP] | Q [64][DP] | V [64][16] | e^G [64] | e^{G_C - G} [64]
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
     float* UE = U + COLS * CHP;                                // U with e^{G_C - G} [16][68]
     __shared__ int s_first;
     pdl_enter();
-    const int row = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * COLS;
+    const int row = blockIdx.x, h = h0 + blockIdx.y, j0 = blockIdx.z * COLS;
     const int n = row_q_len[row], chunks = chunks_of(n, min_len);
     if (chunks == 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
             const int64_t tf = t0 + c * CH;
             const int count = min(CH, n - c * CH);
             if constexpr (CHANNEL) {
-                const ChannelScratch in(const_cast<float*>(scratch), (first + c) * H + h, D);
+                const ChannelScratch in(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y, D);
                 copy_rows<DT>(st, in.kt, D, D, CH);
                 copy_rows<DT>(st + CH * DP, in.qt, D, D, CH);
             } else {
@@ -504,18 +504,18 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
                 copy4(v + i, on ? vn + ((tf + t) * H + h) * Dv + j0 + j : vn, on);
             }
             if constexpr (CHANNEL) {
-                const float* ec = ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).ec;
+                const float* ec = ChannelScratch(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y, D).ec;
                 if (threadIdx.x < DT / 4) copy16(v + CH * COLS + threadIdx.x * 4, threadIdx.x * 4 < D ? ec + threadIdx.x * 4 : ec, threadIdx.x * 4 < D);
             } else if (threadIdx.x < 32) {
-                const float* eg = ChunkScratch(const_cast<float*>(scratch), (first + c) * H + h).eg;      // e^G and e^{G_C - G} lie side by side
+                const float* eg = ChunkScratch(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y).eg;      // e^G and e^{G_C - G} lie side by side
                 copy16(v + CH * COLS + threadIdx.x * 4, eg + threadIdx.x * 4, true);
             }
         }
         copy_commit();
     };
     auto issue_squares = [&](int c) {
-        const float* tb = CHANNEL ? ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).tb
-                                  : ChunkScratch(const_cast<float*>(scratch), (first + c) * H + h).tb;
+        const float* tb = CHANNEL ? ChannelScratch(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y, D).tb
+                                  : ChunkScratch(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y).tb;
         for (int i = threadIdx.x; i < CH * CH / 4; i += 256) {
             const int r = i >> 4, m = (i & 15) * 4;
             copy16(TB + r * CHP + m, tb + i * 4, true);
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
         }
         if constexpr (CHANNEL) {
             __syncthreads();                                   // the keys are done with: those that the state takes come in their place
-            copy_rows<DT>(st, ChannelScratch(const_cast<float*>(scratch), (first + c) * H + h, D).ke, D, D, CH);
+            copy_rows<DT>(st, ChannelScratch(const_cast<float*>(scratch), (first + c) * heads + blockIdx.y, D).ke, D, D, CH);
             copy_commit();
             issue_keys(c + 1);
             copy_wait<2>();
@@ -677,32 +677,32 @@ __global__ void __launch_bounds__(256) delta_chunk_scan_kernel(const float* __re
     }
 }
 
+// The heads of `per_pass` key heads at a time, one pass behind the other on the same scratch memory.
 template <int DT>
 static int launch_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* log_decay, const int* row_q_start,
                          const int* row_q_len, const int* state_slots, float* state, float* out, float* scratch, int max_chunks, int num_rows,
-                         int min_len, int H, int G, int D, int Dv, cudaStream_t stream) {
+                         int min_len, int H, int G, int D, int Dv, int per_pass, cudaStream_t stream) {
     const size_t scan = (size_t)(2 * (2 * CH * (DT + 4) + CH * COLS + 2 * CH) + 2 * CH * CHP + COLS * (DT + 4) + 3 * COLS * CHP) * sizeof(float);
-    const dim3 scan_grid(num_rows, H, (Dv + COLS - 1) / COLS);
-    if (decay) {                                               // a decay per channel
-        const size_t prep = (size_t)(3 * CH * (DT + 4) + 2 * CH * CHP + 4 * DT + 8 * CH * 16) * sizeof(float);
-        cudaError_t e = cudaFuncSetAttribute(delta_channel_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
-        if (e != cudaSuccess) return (int)e;
-        const int rc = launch_kernel(delta_channel_prep_kernel<DT>, dim3(max_chunks, H), dim3(CP_THREADS), prep, stream, qn, kn, beta, decay, log_decay, row_q_start,
-                                     row_q_len, num_rows, min_len, scratch, H, G, D);
-        if (rc) return rc;
-        return launch_kernel(delta_chunk_scan_kernel<DT, true>, scan_grid, dim3(256), scan, stream, qn, kn, vn, row_q_start, row_q_len, state_slots, min_len,
-                             (const float*)scratch, state, out, H, G, D, Dv);
-    }
-    const size_t prep = (size_t)(2 * CH * (DT + 4) + 2 * CH * CHP + 3 * 256) * sizeof(float);      // two blocks on an SM
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
+    // a decay per channel: one block on an SM; one per head: two
+    const size_t prep = decay ? (size_t)(3 * CH * (DT + 4) + 2 * CH * CHP + 4 * DT + 8 * CH * 16) * sizeof(float)
+                              : (size_t)(2 * CH * (DT + 4) + 2 * CH * CHP + 3 * 256) * sizeof(float);
+    auto scan_kernel = decay ? delta_chunk_scan_kernel<DT, true> : delta_chunk_scan_kernel<DT, false>;
+    cudaError_t e = decay ? cudaFuncSetAttribute(delta_channel_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep)
+                          : cudaFuncSetAttribute(delta_chunk_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan);
     if (e != cudaSuccess) return (int)e;
-    const int rc = launch_kernel(delta_chunk_prep_kernel<DT>, dim3(max_chunks, G), dim3(256), prep, stream, qn, kn, beta, log_decay, row_q_start,
-                                 row_q_len, num_rows, min_len, scratch, H, G, D);
-    if (rc) return rc;
-    return launch_kernel(delta_chunk_scan_kernel<DT, false>, scan_grid, dim3(256), scan, stream, qn, kn, vn, row_q_start, row_q_len, state_slots, min_len,
-                         (const float*)scratch, state, out, H, G, D, Dv);
+    for (int g0 = 0; g0 < G; g0 += per_pass) {
+        const int groups = G - g0 < per_pass ? G - g0 : per_pass, h0 = g0 * (H / G), heads = groups * (H / G);
+        int rc = decay ? launch_kernel(delta_channel_prep_kernel<DT>, dim3(max_chunks, heads), dim3(CP_THREADS), prep, stream, qn, kn, beta, decay, log_decay,
+                                       row_q_start, row_q_len, num_rows, min_len, scratch, H, G, D, h0, heads)
+                       : launch_kernel(delta_chunk_prep_kernel<DT>, dim3(max_chunks, groups), dim3(256), prep, stream, qn, kn, beta, log_decay, row_q_start,
+                                       row_q_len, num_rows, min_len, scratch, H, G, D, h0, heads);
+        if (rc) return rc;
+        rc = launch_kernel(scan_kernel, dim3(num_rows, heads, (Dv + COLS - 1) / COLS), dim3(256), scan, stream, qn, kn, vn, row_q_start, row_q_len, state_slots,
+                           min_len, (const float*)scratch, state, out, H, G, D, Dv, h0, heads);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 // Floats of scratch memory for one (chunk, head); tokens a chunk.
@@ -710,18 +710,18 @@ extern "C" int mie_delta_chunk_floats(int per_channel, int D) { return 2 * CH * 
 extern "C" int mie_delta_chunk_tokens(void) { return CH; }
 
 // qn, kn: float32 [T, G, D]; vn, out: [T, H, Dv]; beta [T, H]; log_decay (not positive) [T, H] with `decay` null, or [T, H, D] with `decay` [T, H, D] its
-// exponential; state [slots, H, Dv, D].  D a multiple of 4 up to 128, everything 16-byte aligned.  max_chunks: no fewer than the chunks of all rows with min_len tokens or more; scratch holds
-// max_chunks * H times mie_delta_chunk_floats() floats.
+// exponential; state [slots, H, Dv, D].  D a multiple of 4 up to 128, everything 16-byte aligned.  max_chunks: no fewer than the chunks of all rows with min_len tokens or more; the heads of
+// `per_pass` key heads at a time: scratch holds max_chunks * per_pass * H / G times mie_delta_chunk_floats() floats.
 extern "C" int mie_delta_chunks(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const float* log_decay,
                                 const int* row_q_start, const int* row_q_len, const int* state_slots, float* state, float* out, float* scratch,
-                                int max_chunks, int num_rows, int min_len, int H, int G, int D, int Dv, cudaStream_t stream) {
+                                int max_chunks, int num_rows, int min_len, int H, int G, int D, int Dv, int per_pass, cudaStream_t stream) {
     if (num_rows <= 0 || max_chunks <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || D <= 0 || D % 4 || Dv <= 0 || min_len < 1) return MIE_ERR_BAD_ARG;
+    if (H <= 0 || G <= 0 || H % G || D <= 0 || D % 4 || Dv <= 0 || min_len < 1 || per_pass < 1) return MIE_ERR_BAD_ARG;
     if (D > 128 || H > 65535) return MIE_ERR_TOO_LARGE;
     if (decay && ((reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(log_decay)) & 15)) return MIE_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(scratch)) & 15)
         return MIE_ERR_BAD_ARG;
     if (D <= 64)
-        return launch_chunks<64>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
-    return launch_chunks<128>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, stream);
+        return launch_chunks<64>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, per_pass, stream);
+    return launch_chunks<128>(qn, kn, vn, beta, decay, log_decay, row_q_start, row_q_len, state_slots, state, out, scratch, max_chunks, num_rows, min_len, H, G, D, Dv, per_pass, stream);
 }

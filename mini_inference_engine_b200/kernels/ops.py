@@ -912,6 +912,16 @@ def retention_scan(qkv: torch.Tensor, positions, row_q_start, row_q_len, state_s
                        1.0, k_scale, freq, rot, q_lens)
 
 
+CHUNK_SCRATCH_BYTES = 512 << 20     # what the kernels that go in chunks may hold in scratch memory: a step that needs more has its heads done some at a time.  A step of 8,192
+                                    # tokens and 32 heads of 128 (a decay per channel: 540 MB) goes in two passes, whose chains are as long together as the one's
+
+
+def _heads_a_pass(heads: int, bytes_a_head: int) -> int:
+    """How many of ``heads`` to do at a time, in passes of equal size, so that their scratch memory stays within CHUNK_SCRATCH_BYTES (one at least)."""
+    most = max(1, min(heads, CHUNK_SCRATCH_BYTES // max(1, bytes_a_head)))
+    return -(-heads // -(-heads // most))
+
+
 DECAY_CHUNK_TOKENS = 64        # rows of more new tokens than this go in chunks as matrix products
 
 
@@ -945,12 +955,13 @@ def _decay_rows(rows_in, positions, row_q_start, row_q_len, state_slots, state, 
     if chunked:
         dc = load("decay_chunk")
         chunks = sum(-(-n // chunk) for n in long) if long is not None else 2 * (T // chunk)     # (a row of two chunks has more than 64 tokens)
-        states = torch.empty(chunks * H * dv * D, dtype=torch.float32, device=rows_in.device)
-        work = torch.empty(chunks * H * dc.mie_decay_chunk_floats(), dtype=torch.float32, device=rows_in.device)
+        per_pass = _heads_a_pass(H, 4 * chunks * (dv * D + dc.mie_decay_chunk_floats()))
+        states = torch.empty(chunks * per_pass * dv * D, dtype=torch.float32, device=rows_in.device)
+        work = torch.empty(chunks * per_pass * dc.mie_decay_chunk_floats(), dtype=torch.float32, device=rows_in.device)
         v = rows_in[:, 2 * H * D:]
         _check(dc.mie_decay_chunks(_ptr(qr[0]), _ptr(qr[1]), _ptr(v), tag(v), ctypes.c_longlong(v.stride(0)), _ptr(row_q_start), _ptr(row_q_len),
                                    _ptr(state_slots), rows, _ptr(decay), _ptr(tok_decay), _ptr(state), _ptr(states), _ptr(work), chunks, _ptr(out), H, D,
-                                   vdim, dv, int(act), _stream()), "decay_chunks")
+                                   vdim, dv, int(act), per_pass, _stream()), "decay_chunks")
     return out
 
 
@@ -1420,9 +1431,11 @@ def delta_chunks(qn, kn, vn, beta, log_decay, row_q_start, row_q_len, state_slot
     rows, tokens = work if work is not None else (row_q_len.numel(), T)
     size = lib.mie_delta_chunk_tokens()
     chunks = tokens // size + min(rows, tokens // max(1, min_len))
-    scratch = torch.empty(chunks * H * lib.mie_delta_chunk_floats(int(decay is not None), D), dtype=torch.float32, device=qn.device)
+    a_group = chunks * (H // G) * lib.mie_delta_chunk_floats(int(decay is not None), D)         # floats for the heads of one key head
+    per_pass = _heads_a_pass(G, 4 * a_group)
+    scratch = torch.empty(per_pass * a_group, dtype=torch.float32, device=qn.device)
     _check(lib.mie_delta_chunks(_ptr(qn), _ptr(kn), _ptr(vn), _ptr(beta), _ptr(decay), _ptr(log_decay), _ptr(row_q_start), _ptr(row_q_len), _ptr(state_slots),
-                                _ptr(state), _ptr(out), _ptr(scratch), chunks, row_q_len.numel(), int(min_len), H, G, D, Dv, _stream()), "delta_chunks")
+                                _ptr(state), _ptr(out), _ptr(scratch), chunks, row_q_len.numel(), int(min_len), H, G, D, Dv, per_pass, _stream()), "delta_chunks")
     return out
 
 

@@ -105,6 +105,24 @@ def test_a_token_that_is_not_finite_spoils_only_what_follows(what, at, a_head):
     assert torch.isfinite(out[:at]).all() and torch.isfinite(out[140:]).all() and not torch.isfinite(out[at:140]).any()
 
 
+@pytest.mark.parametrize("a_head", [False, True])
+@pytest.mark.parametrize("H,G", [(5, 5), (6, 3), (4, 1)])
+def test_some_heads_at_a_time(monkeypatch, H, G, a_head):
+    """Scratch memory for one key head's heads, or two, at a time: every number as with all at once."""
+    from mini_inference_engine_b200.kernels import ops
+    rows, D, V = [100, 65, 3], 32, 24
+    args = operands(rows, H, G, D, V, "mixed")
+    whole = run(rows, *args, H, G, D, V, a_head=a_head)
+    sizes, empty = [], torch.empty
+    for key_heads in (1, 2):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_heads_a_pass", lambda heads, bytes_a_head: min(heads, key_heads))
+            m.setattr(ops.torch, "empty", lambda *s, **k: (sizes.append(s[0]), empty(*s, **k))[1])
+            got = run(rows, *args, H, G, D, V, a_head=a_head)
+        assert all(torch.equal(a, b) for a, b in zip(got, whole))
+    assert sizes[0] * G == sizes[1] * G // min(2, G)
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_the_mixer_in_portions_of_any_length(dt):
     """Whole, in long and short portions, and beside decoding rows: the same outputs."""

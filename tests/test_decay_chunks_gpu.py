@@ -82,3 +82,16 @@ def test_preparation_of_rows_that_start_anywhere(monkeypatch, dt):
                            rot=rot, k_scale=0.2, max_q_len=T)
         res.append((out, state))
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("heads", [1, 2, 3])
+def test_some_heads_at_a_time(monkeypatch, heads, known):
+    """Scratch memory for that many heads at a time: every number as with all at once."""
+    from mini_inference_engine_b200.kernels import ops
+    for how in (dict(per_token=True, ones=True), dict(act=True)):
+        whole = scan(monkeypatch, True, ROWS, 5, 68, 70, torch.bfloat16, known=known, **how)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_heads_a_pass", lambda all_heads, bytes_a_head: heads)
+            got = scan(m, True, ROWS, 5, 68, 70, torch.bfloat16, known=known, **how)
+        assert all(torch.equal(a, b) for a, b in zip(got, whole))

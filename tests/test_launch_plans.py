@@ -94,3 +94,13 @@ def test_paired_product_is_chosen_by_the_share_of_its_tiles_that_a_product_fills
     for M, N in loses:
         assert linear.pair_fill(M, N) < linear.PAIR_MIN_FILL, (M, N)
     assert linear.pair_fill(1, 256) < 0.001 and 0.99 < linear.pair_fill(74 * 256, 256) <= 1.0
+
+
+def test_the_scratch_of_chunked_recurrences_is_bounded():
+    for heads in (1, 3, 16, 32, 64):
+        for each in (1, 10 << 20, 100 << 20, 511 << 20, 600 << 20, 3 << 30):
+            n = ops._heads_a_pass(heads, each)
+            assert 1 <= n <= heads and (n == 1 or n * each <= ops.CHUNK_SCRATCH_BYTES)
+            passes = -(-heads // n)
+            assert passes == 1 or (passes - 1) * n < heads                       # none is empty
+    assert ops._heads_a_pass(16, 1 << 20) == 16 and ops._heads_a_pass(32, 17 << 20) == 16
