@@ -147,7 +147,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
     // below that every tile has a block of its own and the longest one is the critical path.
     if (warp == 0) {
         int pair, tiles_r;
-        const int r = warp_find_row(p.row_q_len, p.num_rows, (int)blockIdx.y, [&](int ql) {
+        const int r = warp_find_row(p.row_q_len, p.num_rows, (int)(blockIdx.z * gridDim.y + blockIdx.y), [&](int ql) {
             const int t = ql >= p.min_q_len ? (ql + FA_BM - 1) / FA_BM : 0;
             return p.pair ? (t + 1) / 2 : t;
         }, pair, tiles_r);
@@ -972,8 +972,8 @@ static int launch_fa_tile(const CUtensorMap& mq, const CUtensorMap& mk, const CU
     cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, MODS, KEEP, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     // heads fastest: the longest tiles of all heads start first
-    const dim3 grid(p.num_heads, p.pair ? (tiles + rows + 1) / 2 : tiles);
-    if (grid.y > 65535) return MIE_ERR_TOO_LARGE;
+    const unsigned blocks = p.pair ? (tiles + rows + 1) / 2 : tiles, high = blocks < 32768u ? blocks : 32768u;
+    const dim3 grid(p.num_heads, high, (blocks + high - 1) / high);             // (a grid is at most 65,535 high)
     return launch_kernel(prefill_attention_tc_kernel<D, MODS, KEEP, BN>, grid, dim3(FA_THREADS), smem, stream, mq, mk, mv, p);
 }
 

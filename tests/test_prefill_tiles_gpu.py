@@ -92,3 +92,22 @@ def test_fewer_keys_a_tile_lose_no_precision(n):
         ops.check_tc_errors()
         errors.append((out.view(n, G, times, D)[:, :, 0].double() - want).norm().item())
     assert errors[1] <= errors[0]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_more_rows_than_a_grid_is_high(D):
+    """70,000 portions of two tokens in a step (a tile each) against the CUDA-core kernel."""
+    from mini_inference_engine_b200.kernels import ops
+    rows, page = 70000, 8
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    k, v, q = rnd(rows + 1, 1, page, D), rnd(rows + 1, 1, page, D), rnd(2 * rows, 2 * D)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    args = (q, 2 * D, k, v, torch.randperm(rows, device="cuda").int().add(1).view(rows, 1), torch.arange(0, 2 * rows, 2, **i32), torch.full((rows,), 2, **i32),
+            torch.full((rows,), 5, **i32), 2 * rows)
+    out = [torch.zeros(2 * rows, 2, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    ops.prefill_attention_tc(*args, out[0], 2, 1, D, page, D ** -0.5, 0, work=(rows, 2 * rows))
+    ops.paged_attention(*args, out[1], 2, 1, D, page, D ** -0.5, 0)
+    torch.cuda.synchronize()
+    ops.check_tc_errors()
+    close(*out)
