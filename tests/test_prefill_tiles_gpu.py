@@ -69,13 +69,15 @@ def test_modified_scores_in_large_launches(what):
 
 @pytest.mark.parametrize("n", [300, 800, 1500])
 def test_fewer_keys_a_tile_lose_no_precision(n):
-    """The same heads in a launch of few blocks (128 keys a tile) and, each thirty-two times, in one of many (64 keys): the error against 64 bits is no larger."""
+    """The same heads in a launch of few blocks (128 keys a tile) and, each twice, in one of many (64 keys): the error against 64 bits is no larger.  (Over some 30,000 rows,
+    whose squared errors scatter by one and a half times their mean, the two norms differ by about half a percent by chance: four times that is allowed.  With the
+    sums of unrounded weights the smaller tiles' error is 5 to 8 percent larger.)"""
     from mini_inference_engine_b200.kernels import ops
-    G, D, page, copies = 4, 128, 16, 32
-    g = torch.Generator().manual_seed(n)
+    G, D, page = 288 // -(-n // 128), 128, 16
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     pages = -(-n // page)
-    k, v = (torch.randn(pages, G, page, D, generator=g).bfloat16().cuda() for _ in "kv")
-    q = torch.randn(n, G, D, generator=g).bfloat16().cuda() * 1.5
+    k, v, q = rnd(pages, G, page, D).bfloat16(), rnd(pages, G, page, D).bfloat16(), (rnd(n, G, D) * 1.5).bfloat16()
     i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device="cuda")
     table = torch.arange(pages, dtype=torch.int32, device="cuda").view(1, -1)
     flat = lambda t: t.permute(1, 0, 2, 3).reshape(G, -1, D)[:, :n].double()
@@ -83,7 +85,7 @@ def test_fewer_keys_a_tile_lose_no_precision(n):
     scores = scores.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), -float("inf"))
     want = (torch.softmax(scores, -1) @ flat(v)).permute(1, 0, 2)
     errors = []
-    for times in (1, copies):
+    for times in (1, 2):
         H = G * times
         qs = q.repeat_interleave(times, 1).reshape(n, H * D).contiguous()
         out = torch.empty(n, H, D, device="cuda")
@@ -91,7 +93,8 @@ def test_fewer_keys_a_tile_lose_no_precision(n):
         torch.cuda.synchronize()
         ops.check_tc_errors()
         errors.append((out.view(n, G, times, D)[:, :, 0].double() - want).norm().item())
-    assert errors[1] <= errors[0]
+    print(f"{n} tokens: {errors[1] / errors[0] - 1:+.2%}")
+    assert errors[1] <= 1.02 * errors[0]
 
 
 @pytest.mark.parametrize("D", [64, 128])
