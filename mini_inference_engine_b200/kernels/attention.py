@@ -58,20 +58,30 @@ def rotates_in_decode(dtype, head_dim: int, ctx) -> bool:
             and decode_only(ctx))
 
 
-F32_MIN_PAIRS = 16          # a row with fewer pairs would leave three quarters of a 64-pair tile empty; the other kernel gives each of its pairs a warp
+# float32: tiles of 64 (token, head) pairs against a warp a pair.  A tile takes as long with one pair as with 64, some 0.15 us a key tile more than the warps
+# as long as those have the GPU to themselves; those fill it at about 1,500 pairs.  One row, us, a warp a pair : tiles, 0 / 500 / 2,000 earlier positions --
+# 32 heads of 64 on 4: 8 tokens (256 pairs) 6 : 16 / 64 : 84 / 244 : 315, 32 (1,024) 7 : 16 / 76 : 93 / 282 : 317, 48 (1,536) 13 : 16 / 100 : 95 / 364 : 321,
+# 64 (2,048) 16.6 : 16.8 / 120 : 95 / 426 : 328, 128 (4,096) 38 : 28 / 188 : 110 / 638 : 357; 16 of 64 on 16: 64 tokens (1,024) 11 : 17 / 82 : 96 / 287 : 331, 128 (2,048)
+# 28 : 27 / 144 : 105 / 437 : 339; 32 of 128 on 8: 32 (1,024) 8 : 17 / 100 : 113 / 372 : 392, 48 16 : 18 / 143 : 114 / 521 : 392; 12 of 64 on 4: 128 (1,536) 24 : 26 / 117 : 104 / 389 : 337.
+F32_MIN_WORK = 1536         # (token, head) pairs of the rows that tiles could take, from which they do ...
+F32_MIN_WORK_FRESH = 2048   # ... where no row has more than F32_FRESH positions
+F32_FRESH = 256
+F32_MIN_PAIRS = 16          # pairs of a row on one key head below which it is left to the warps: three quarters of its tile would be empty
 
 
 def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size, scale, window, mods, keep):
-    """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles of 64 pairs, shorter ones one pair a warp.  Where the host does
-    not know the rows' lengths (a captured step) each of the two kernels takes the rows that are its own."""
+    """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles of 64 pairs, shorter ones one pair a warp, as all are in a step of few
+    pairs.  Where the host does not know the rows' lengths (a captured step) each of the two kernels takes the rows that are its own."""
     min_q_len = max(2, -(-F32_MIN_PAIRS // (num_heads // num_kv_heads)))
     q_lens = ctx.host.get("q_len")
     long = None if q_lens is None else [n for n in q_lens if n >= min_q_len]
     sizes = (ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, page_size, scale, window)
+    pairs = (ctx.num_tokens if long is None else sum(long)) * num_heads
+    if pairs < (F32_MIN_WORK_FRESH if ctx.max_ctx_len <= F32_FRESH else F32_MIN_WORK):
+        return ops.paged_attention(*args, *sizes, mods=mods, keep=keep)
     if long is None or len(long) < len(q_lens):
         ops.paged_attention(*args, *sizes, mods=mods, keep=keep, below=min_q_len)
-    if long is None or long:
-        ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)))
+    ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)))
     return out
 
 

@@ -112,6 +112,27 @@ def test_the_step_takes_it_in_float32():
         close(got, want, v)
 
 
+@pytest.mark.parametrize("rows,max_ctx,host,kernels", [([(40, 600)], 600, True, {"paged"}), ([(200, 600)], 600, True, {"tiles"}), ([(200, 600), (1, 50)], 600, True, {"paged", "tiles"}),
+                                                       ([(200, 200)], 200, True, {"paged"}), ([(256, 256)], 256, True, {"tiles"}), ([(150, 600)], 600, False, {"paged"}),
+                                                       ([(250, 600)], 600, False, {"paged", "tiles"}), ([(1, 90)] * 300, 90, True, {"paged"})])
+def test_a_step_of_few_pairs_is_left_to_the_warps(monkeypatch, rows, max_ctx, host, kernels):
+    """Eight heads: 192 tokens are enough beside earlier positions, 256 without."""
+    from types import SimpleNamespace
+    from mini_inference_engine_b200.kernels import attention, ops
+    H, G, D, page = 8, 2, 64, 16
+    args, _, out = case(rows, H, G, D, page)
+    q, stride, k, v, block, starts, lens, ctx_lens, T = args
+    want = ops.paged_attention(*args, out.clone(), H, G, D, page, D ** -0.5)
+    used, paged, tiles = set(), ops.paged_attention, ops.attention_f32
+    monkeypatch.setattr(ops, "paged_attention", lambda *a, **h: (used.add("paged"), paged(*a, **h))[1])
+    monkeypatch.setattr(ops, "attention_f32", lambda *a, **h: (used.add("tiles"), tiles(*a, **h))[1])
+    ctx = SimpleNamespace(block_tables=[block], row_q_start=starts, row_q_len=lens, row_ctx_len=ctx_lens, num_tokens=T, max_ctx_len=max_ctx,
+                          host={"q_len": [n for n, _ in rows] if host else None})
+    got = attention.attention(q, ctx, SimpleNamespace(k=k, v=v, group=0, page_size=page), torch.zeros_like(out), H, G, D, D ** -0.5, 0)
+    close(got, want, v)
+    assert used == kernels
+
+
 @pytest.mark.parametrize("what", ["page", "context"])
 def test_a_number_out_of_range_is_reported_under_this_kernel_s_name(what):
     """A page that is not in the pool (page 0 is read in its place), and more positions than the block table covers (the row is left alone)."""
