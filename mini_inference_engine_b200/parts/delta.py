@@ -18,6 +18,7 @@ import torch
 
 from ..kernels import ops
 from ..kernels.attention import _row_kinds, decode_only
+from ..kernels.device import num_sms
 from ..weights.loader import TensorSpec
 from .attention import _padded_rows
 from .base import Mixer, StateNeed, register_part
@@ -29,8 +30,13 @@ def _singles(ctx, long) -> bool:
     return kinds is not None and kinds[1] == len(long or ())
 
 
-CHANNEL_CHUNKED_FROM = 112      # new tokens from which a row's recurrence goes in chunks (the line of one decay per head, see CHUNKED_FROM: the scans are the same; 1,500 tokens
-                                # in rows of 500 and 1,000, 16 heads of 128 x 128: 427 us token by token, 302 us in chunks, preparation included)
+def channel_chunked_from(num_heads: int, vdim: int) -> int:
+    """New tokens from which a row's recurrence with a decay per channel goes in chunks.  The chunks' scan is a chain of 64 tokens a link in blocks of 16 value columns with an
+    SM each, so it pays later where a row's blocks are more than the SMs and go in two waves.  The layer, us, token by token : in chunks (width 2,048, 16 heads
+    of 128 x 128 = 128 blocks): 96 tokens 67 : 70, 104 69.7 : 70.6, 112 72.6 : 71.1, 128 74.6 : 71.3, 136 80.1 : 80.4, 144 81.3 : 80.9, 160 91 : 80, 256 132 : 95; two rows of 100 92 : 94,
+    of 128 106 : 95, of 144 118 : 113.  Width 4,096, 32 heads (256 blocks): 112 tokens 121 : 126, 128 129 : 129, 129 134 : 145, 160 151 : 141, 193 179 : 165, 256 210 : 168;
+    two rows of 144 205 : 221, of 160 228 : 232, of 192 259 : 238; three of 144 278 : 287, of 160 300 : 292."""
+    return 112 if num_heads * -(-vdim // 16) <= num_sms() else 160
 
 
 class ChannelDelta(Mixer):
@@ -98,9 +104,10 @@ class ChannelDelta(Mixer):
         qn, kn, vn, beta, decay, kq = f32(G * D), f32(G * D), f32(H * Dv), f32(H), f32(H * D), f32(G)
         sizes = dict(num_heads=H, num_kv_heads=G, dim=D, vdim=Dv)
         # (as in HeadDelta: where the host does not know the rows' lengths each of the two kernels takes the rows that are its own)
-        chunked = ops.delta_chunks_take(D) and ctx.max_q_len >= CHANNEL_CHUNKED_FROM
+        line = channel_chunked_from(H, Dv)
+        chunked = ops.delta_chunks_take(D) and ctx.max_q_len >= line
         q_lens = ctx.host.get("q_len")
-        long = [n for n in q_lens if n >= CHANNEL_CHUNKED_FROM] if chunked and q_lens is not None else None
+        long = [n for n in q_lens if n >= line] if chunked and q_lens is not None else None
         log_decay = f32(H * D) if chunked else None
         ops.delta_prepare(proj, low, self.conv, conv_state, ctx.token_row, ctx.row_q_start, ctx.state_slots, self.a_log, self.dt_bias,
                           qn, kn, vn, beta, decay, kq, unit_eps=self.unit_eps, log_decay=log_decay, **sizes)
@@ -109,9 +116,9 @@ class ChannelDelta(Mixer):
         o = f32(H * Dv)
         rows = (ctx.row_q_start, ctx.row_q_len, ctx.state_slots, state, o)
         if chunked:
-            ops.delta_chunks(qn, kn, vn, beta, log_decay, *rows, min_len=CHANNEL_CHUNKED_FROM, work=(len(long), sum(long)) if long else None, decay=decay, **sizes)
+            ops.delta_chunks(qn, kn, vn, beta, log_decay, *rows, min_len=line, work=(len(long), sum(long)) if long else None, decay=decay, **sizes)
         if long is None or len(long) < len(q_lens):
-            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=CHANNEL_CHUNKED_FROM if chunked else 1 << 30, singles=_singles(ctx, long), **sizes)
+            ops.delta_scan(qn, kn, vn, beta, decay, kq, *rows, below=line if chunked else 1 << 30, singles=_singles(ctx, long), **sizes)
         gated = self.rt.empty(T, H * Dv)
         ops.head_norm_gate(o, low[:, H * D:], self.norm, gated, H, Dv, self.eps)
         return self.rt.linear(gated, self.w_o, None, out_dtype=torch.float32)

@@ -104,3 +104,11 @@ def test_the_scratch_of_chunked_recurrences_is_bounded():
             passes = -(-heads // n)
             assert passes == 1 or (passes - 1) * n < heads                       # none is empty
     assert ops._heads_a_pass(16, 1 << 20) == 16 and ops._heads_a_pass(32, 17 << 20) == 16
+
+
+def test_a_recurrence_whose_chunks_go_in_two_waves_takes_them_later():
+    from mini_inference_engine_b200.parts.delta import channel_chunked_from
+    if device.num_sms() != device.B200_SMS:
+        pytest.skip("the expected numbers are for 148 SMs")
+    assert channel_chunked_from(16, 128) == channel_chunked_from(2, 32) == channel_chunked_from(148, 16) == 112
+    assert channel_chunked_from(32, 128) == channel_chunked_from(149, 16) == channel_chunked_from(19, 128) == 160
