@@ -138,22 +138,39 @@ __device__ __noinline__ void sp_again(const SpParams& p, float* sm, int m0, int 
 
 // --------------------------------------------------------------------------- split
 
-// The nearest bfloat16 number (8 bits of the significand); the one towards zero where rounding would leave the range.
-__device__ __forceinline__ float top_part(float v) {
-    const uint32_t u = __float_as_uint(v), r = (u + 0x7fffu + ((u >> 16) & 1u)) & 0xffff0000u;
-    return __uint_as_float((r & 0x7f800000u) == 0x7f800000u ? u & 0xffff0000u : r);
+// A number as its nearest bfloat16 number, the nearest to what is left, and the rest, which is one too: pairs of numbers, the first in the lower halves.
+__device__ __forceinline__ uint32_t nearest2(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
-// A part that is neither zero nor a normal number: bfloat16 may hold less of it than there is (its last bit is 2^-133, float32's 2^-149).
-__device__ __forceinline__ bool too_small(uint32_t u) { return (u & 0x7f800000u) == 0u && (u & 0x007fffffu) != 0u; }
-// A number as its nearest bfloat16 number, the nearest to what is left, and the rest, which is one too; a number that is not finite has no rest.  One so small
-// (below 2^-102) that a part leaves the normal numbers goes on as NaN, and its outputs with it: they are then worked out from the operands.
-__device__ __forceinline__ void cut3(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
+__device__ __forceinline__ void cut3(float v0, float v1, uint32_t& a, uint32_t& b, uint32_t& c) {
+    a = nearest2(v0, v1);
+    const float r0 = v0 - __uint_as_float(a << 16), r1 = v1 - __uint_as_float(a & 0xffff0000u);                // differences are exact
+    b = nearest2(r0, r1);
+    c = nearest2(r0 - __uint_as_float(b << 16), r1 - __uint_as_float(b & 0xffff0000u));                        // (at most 7 bits: nothing is rounded)
+}
+// Zero, or a number whose parts are normal numbers: from 2^-102 on, and below what rounds to infinity.
+__device__ __forceinline__ bool ordinary(float v) {
+    const uint32_t t = __float_as_uint(v) & 0x7fffffffu;
+    return t - 0x0c800000u < 0x7f7f8000u - 0x0c800000u || t == 0u;
+}
+// The others: no rest behind a number that is not finite; the first part towards zero where rounding leaves the range; a number so small that a part leaves
+// the normal numbers (bfloat16's last bit is 2^-133, float32's 2^-149) goes on as NaN, and its outputs with it: they are then worked out from the operands.
+__device__ __noinline__ void cut3_other(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
     const uint32_t u = __float_as_uint(v);
     b = c = 0u;
-    if ((u & 0x7f800000u) == 0x7f800000u) { a = (u & 0x007fffffu) ? 0x7fc00000u : u; return; }
-    const float fa = top_part(v), r = v - fa, fb = top_part(r);            // the differences are exact
-    a = __float_as_uint(fa); b = __float_as_uint(fb); c = __float_as_uint(r - fb);       // (at most 7 bits: c's lower half is zero)
-    if (too_small(a) || too_small(b) || too_small(c)) { a = 0x7fc00000u; b = c = 0u; }
+    a = u >> 16;
+    if ((u & 0x7f800000u) == 0x7f800000u) { if (u & 0x007fffffu) a = 0x7fc0u; return; }
+    if ((u & 0x7fffffffu) >= 0x7f7f8000u) {
+        const float r = v - __uint_as_float(u & 0xffff0000u);
+        b = nearest2(r, 0.f);
+        c = nearest2(r - __uint_as_float(b << 16), 0.f);
+        return;
+    }
+    cut3(v, 0.f, a, b, c);
+    auto too_small = [](uint32_t p) { return (p & 0x7f80u) == 0u && (p & 0x007fu) != 0u; };
+    const float rest = (v - __uint_as_float(a << 16)) - __uint_as_float(b << 16);
+    if (too_small(a) || too_small(b) || too_small(c) || rest != __uint_as_float(c << 16)) { a = 0x7fc0u; b = c = 0u; }
 }
 
 // src [rows, K] -> dst [Kp / 64][row blocks][3 planes][block rows][64]: what one stage of the product reads of one block of rows is one stretch
@@ -176,12 +193,21 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ sr
             for (int i = 0; i < 8; ++i) v[i] = k + i < K ? p[i] : 0.f;
         }
         uint32_t o[3][4];
+        bool plain = true;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            uint32_t a0, b0, c0, a1, b1, c1;
-            cut3(v[2 * i], a0, b0, c0);
-            cut3(v[2 * i + 1], a1, b1, c1);
-            o[0][i] = (a0 >> 16) | a1; o[1][i] = (b0 >> 16) | b1; o[2][i] = (c0 >> 16) | (c1 & 0xffff0000u);
+            cut3(v[2 * i], v[2 * i + 1], o[0][i], o[1][i], o[2][i]);
+            plain = plain && ordinary(v[2 * i]) && ordinary(v[2 * i + 1]);
+        }
+        if (!plain) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t lo[3], hi[3];
+                cut3_other(v[2 * i], lo[0], lo[1], lo[2]);
+                cut3_other(v[2 * i + 1], hi[0], hi[1], hi[2]);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) o[j][i] = lo[j] | hi[j] << 16;
+            }
         }
         const int rb = row / block;
         bf16* d = dst + ((((int64_t)kc * row_blocks + rb) * 3) * block + (row - rb * block)) * SP_BK + piece * 8;
@@ -348,14 +374,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
 
-// The shares of K added up in order: a block 64 columns of 4 V tokens, a thread V columns next to one another.
+// The shares of K added up in order: a block 128 columns of 2 V tokens, a thread V columns next to one another.
 template <int V>
-__global__ void __launch_bounds__(256) split_sum_kernel(const __grid_constant__ SpParams p) {
+__global__ void __launch_bounds__(256, 7) split_sum_kernel(const __grid_constant__ SpParams p) {
     __shared__ float sm[SP_AGAIN_FLOATS];
     pdl_enter();
-    constexpr int TOKENS = 4 * V;
-    const int tiles_n = (p.N + 63) / 64, m0 = (int)(blockIdx.x / tiles_n) * TOKENS, n0 = (int)(blockIdx.x % tiles_n) * 64;
-    const int m = m0 + threadIdx.x / (64 / V), n = n0 + threadIdx.x % (64 / V) * V;
+    constexpr int TOKENS = 2 * V;
+    const int tiles_n = (p.N + 127) / 128, m0 = (int)(blockIdx.x / tiles_n) * TOKENS, n0 = (int)(blockIdx.x % tiles_n) * 128;
+    const int m = m0 + threadIdx.x / (128 / V), n = n0 + threadIdx.x % (128 / V) * V;
     bool fine = true;
     if (m < p.M && n < p.N) {
         const int64_t per = (int64_t)p.M * p.N;
@@ -377,7 +403,7 @@ __global__ void __launch_bounds__(256) split_sum_kernel(const __grid_constant__ 
             p.out[(int64_t)m * p.out_stride + n + i] = v[i];
         }
     }
-    if (__syncthreads_or(!fine)) sp_again(p, sm, m0, TOKENS, n0, 64);
+    if (__syncthreads_or(!fine)) sp_again(p, sm, m0, TOKENS, n0, 128);
 }
 
 // --------------------------------------------------------------------------- host side
@@ -440,9 +466,9 @@ extern "C" int mie_gemm_split(const void* xs, const void* ws, const float* x, co
     p.num_items = p.tiles_m * ((N + 255) / 256) * p.splits;
     rc = bn == 64 ? sp_launch<64>(mw, mx, p, stream) : bn == 128 ? sp_launch<128>(mw, mx, p, stream) : sp_launch<256>(mw, mx, p, stream);
     if (rc || p.splits == 1) return rc;
-    const unsigned tiles_n = (unsigned)((N + 63) / 64);
-    if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3(tiles_n * (unsigned)((M + 15) / 16)), dim3(256), 0, stream, p);
-    return launch_kernel(split_sum_kernel<1>, dim3(tiles_n * (unsigned)((M + 3) / 4)), dim3(256), 0, stream, p);
+    const unsigned tiles_n = (unsigned)((N + 127) / 128);
+    if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3(tiles_n * (unsigned)((M + 7) / 8)), dim3(256), 0, stream, p);
+    return launch_kernel(split_sum_kernel<1>, dim3(tiles_n * (unsigned)((M + 1) / 2)), dim3(256), 0, stream, p);
 }
 
 extern "C" int mie_gemm_split_error(void) { return g_error_host ? *g_error_host : 0; }

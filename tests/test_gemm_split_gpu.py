@@ -99,8 +99,8 @@ def test_numbers_that_are_not_finite_or_overflow(force):
 @pytest.mark.parametrize("what", ["nan", "inf", "overflow", "a column"])
 @pytest.mark.parametrize("force", [(64, 1), (256, 1), (128, 3)])
 def test_many_outputs_that_are_not_finite(what, force):
-    """A step of such numbers is what the CUDA-core product leaves, and takes no more than a few times that product's time (seen: 2.3 to 4 times, and 7 times with
-    tiles that only a third of the SMs have; an output after the other in a thread took many more times)."""
+    """A step of such numbers is what the CUDA-core product leaves, and takes no more than a few times that product's time (seen: 4 to 7 times, the latter with
+    tiles that only a third of the SMs have; with an output after the other in a thread the limit below is passed in every case)."""
     from mini_inference_engine_b200.kernels import gemm_split, gemm_tc, ops
     M, N, K = 640, 2048, 1024
     x, w, bias = operands(M, N, K, 3)
