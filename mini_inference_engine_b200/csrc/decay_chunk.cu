@@ -196,14 +196,20 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
     }
 }
 
-// A thread four entries of a state; eight chunks' additions are read ahead of the chain.
+// A thread four entries of a state; eight chunks' additions are read ahead of the chain.  blockIdx.y counts the rows of two chunks or more only: beside 64
+// single tokens the blocks of rows that have no chunks had cost more than the chunks (a portion of 100 tokens, 16 heads of 128 x 256).
 __global__ void __launch_bounds__(128) decay_combine_kernel(const DcParams p) {
     pdl_enter();
     const int64_t per_state = (int64_t)p.heads * p.Dv * p.D, e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    const int row = blockIdx.y, items = dc_chunks(p.row_q_len[row]);
-    if (e >= per_state || items == 0) return;
-    int first = 0;
-    for (int r = 0; r < row; ++r) first += dc_chunks(p.row_q_len[r]);
+    int within, one;
+    const int row = warp_find_row(p.row_q_len, p.num_rows, (int)blockIdx.y, [](int n) { return dc_chunks(n) > 0 ? 1 : 0; }, within, one);
+    if (row < 0) return;
+    int first = 0;                                     // where the row's chunks begin
+    for (int r = threadIdx.x & 31; r < row; r += 32) first += dc_chunks(p.row_q_len[r]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+    const int items = dc_chunks(p.row_q_len[row]);
+    if (e >= per_state) return;
     const int h = p.h0 + (int)(e / ((int64_t)p.Dv * p.D));
     float* end = p.state + ((int64_t)p.state_slots[row] * p.H + p.h0) * p.Dv * p.D + e;
     float4 cur = *reinterpret_cast<const float4*>(end);
@@ -342,6 +348,7 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
          reinterpret_cast<uintptr_t>(scratch)) & 15) return MIE_ERR_BAD_ARG;
     DcParams p{q, k, v, v_stride, row_q_start, row_q_len, state_slots, num_rows, decay, tok_decay, state, states, scratch, out, H, D, Dv_in, Dv, v_act, 0, 0};
     const int halves = Dv_in > 64 ? 2 : 1;
+    const int long_rows = num_rows < chunks / 2 ? num_rows : chunks / 2 > 0 ? chunks / 2 : 1;      // (each has two chunks at least)
     int rc;
 #define DC_LAUNCH(T, DT)                                                                                                                  \
     {                                                                                                                                     \
@@ -354,7 +361,7 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
             rc = launch_kernel(decay_local_kernel<T, DT>, dim3(chunks, p.heads, halves), dim3(256), smem_l, stream, p, halves);           \
             if (rc) return rc;                                                                                                            \
             const int64_t quads = (int64_t)p.heads * Dv * D / 4;                                                                          \
-            rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), num_rows), dim3(128), 0, stream, p);           \
+            rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), long_rows), dim3(128), 0, stream, p);          \
             if (rc) return rc;                                                                                                            \
             rc = launch_kernel(decay_output_kernel<T, DT>, dim3(chunks, p.heads, (Dv_in + 63) / 64), dim3(256), smem_o, stream, p);       \
             if (rc) return rc;                                                                                                            \
