@@ -10,11 +10,20 @@ import torch
 from . import build, ops
 from .device import num_sms
 
-MIN_TOKENS = 9                        # Device time against the CUDA-core product, L2 flushed, B200, tokens x outputs x K: 8 x 11,264 x 2,048 82 against 75 us (the
-MIN_K = 128                           # row-streaming kernel reads w once for up to eight tokens), 9 x 2,048 x 2,048 27 : 39, 16 x 11,264 x 2,048 82 : 118,
-MIN_WEIGHT = 1 << 14                  # 17 x 2,048 x 2,048 28 : 214, 509 x 11,264 x 2,048 165 : 1,008, 509 x 2,048 x 5,632 90 : 1,195, 1,000 x 2,560 x 2,048 84 : 517,
-                                      # 2,048 x 11,264 x 2,048 415 : 2,707; small matrices: 64 x 256 x 256 15 : 32, 2,000 x 128 x 128 16 : 40,
-                                      # 64 x 2,048 x 128 15 : 18, 2,000 x 64 x 64 15 : 12 (three launches instead of one)
+# Device time against the CUDA-core product, B200, weights from memory (L2 overwritten in front of every product), us, CUDA cores : here, at 9 / 16 / 17 / 32 tokens.
+# Up to 16 tokens its row-streaming kernel runs, which reads w once per eight tokens and is the faster one where w has rows for all SMs many times over, or is small:
+#   1,024 x 128 (outputs x K) 4 : 11 / 4 : 11 / 14 : 11 / 14 : 11    1,024 x 1,024 19 : 15 / 19 : 16 / 102 : 15 / 103 : 16 (w in L2: 9 : 14 up to 16 tokens)
+#   2,048 x 2,048 36 : 23 / 36 : 24 / 209 : 24 / 214 : 24            4,096 x 2,048 45 : 35 / 52 : 36 / 208 : 36 / 217 : 36
+#   11,264 x 2,048 89 : 88 / 115 : 88 / 235 : 88 / 239 : 88          2,048 x 5,632 90 : 46 / 91 : 46 / 583 : 46 / 605 : 47
+#   5,632 x 4,096 119 : 87 / 165 : 88 / 428 : 87 / 433 : 88          32,000 x 2,048 207 : 251 / 228 : 251 / 327 : 251 / 334 : 252
+# (taken with the parts' first form; the present one takes 12 to 14 less for 11,264 x 2,048.)  From 17 tokens on every size from 128 x 128 on: 13 : 11.  More tokens: 509 x 11,264 x 2,048
+# 1,008 : 154, 509 x 2,048 x 5,632 1,195 : 78, 2,048 x 11,264 x 2,048 2,707 : 403; smaller ones: 2,000 x 128 x 128 40 : 16, 2,000 x 64 x 64 12 : 15 (three launches instead of one).
+MIN_TOKENS = 9
+MIN_K = 128
+MIN_WEIGHT = 1 << 14
+FEW_TOKENS = 16                       # up to this many tokens ...
+FEW_MIN_WEIGHT = 1 << 22              # ... from this size on (smaller ones are likely to be in L2) ...
+FEW_MAX_ASPECT = 6                    # ... and up to this many outputs per entry of K
 W_SLAB_BYTES = 144 << 20              # planes of the weight rows that are in scratch at a time (a slab of 23 M numbers: one
                                       # gate|up matrix of 2 x 5,632 x 2,048 in one go)
 X_SLAB_BYTES = 48 << 20
@@ -22,6 +31,8 @@ PARTIAL_BYTES = 48 << 20
 
 
 def takes(M: int, N: int, K: int) -> bool:
+    if M <= FEW_TOKENS and (N * K < FEW_MIN_WEIGHT or N > FEW_MAX_ASPECT * K):
+        return False
     return M >= MIN_TOKENS and K >= MIN_K and N * K >= MIN_WEIGHT
 
 

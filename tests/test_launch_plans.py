@@ -112,3 +112,11 @@ def test_a_recurrence_whose_chunks_go_in_two_waves_takes_them_later():
         pytest.skip("the expected numbers are for 148 SMs")
     assert channel_chunked_from(16, 128) == channel_chunked_from(2, 32) == channel_chunked_from(148, 16) == 112
     assert channel_chunked_from(32, 128) == channel_chunked_from(149, 16) == channel_chunked_from(19, 128) == 160
+
+
+def test_which_float32_products_go_to_the_tensor_cores():
+    from mini_inference_engine_b200.kernels.gemm_split import takes
+    for sizes in [(9, 2048, 2048), (16, 11264, 2048), (9, 2048, 5632), (17, 32000, 2048), (17, 128, 128), (2000, 128, 128), (509, 11264, 2048)]:
+        assert takes(*sizes), sizes
+    for sizes in [(8, 2048, 2048), (16, 1024, 1024), (9, 32000, 2048), (16, 32000, 2048), (2000, 64, 64), (64, 128, 64), (9, 128, 128)]:
+        assert not takes(*sizes), sizes
