@@ -3,10 +3,10 @@
 //
 // A block owns 64 (token, query head) pairs that share a key head -- tokens of one row, the group's heads side by side -- so a tile of
 // 64 keys and values in shared memory serves all heads of the group.  A thread holds 8 (or 4) pairs x 4 keys of the scores and
-// the same pairs x 4 (or 8) entries of the output: 16 wavefronts of shared memory for 128 warp-wide multiply-adds, where a warp that owns one pair
-// reads its keys and values once per pair and is bound by that.  The next tile's keys arrive (cp.async) under the product with the values, the next
-// values under the scores.  Tiles of a row go longest first.  Bound: the CUDA cores' multiply-adds.  A layer of TinyLlama's sizes over 1,000 tokens of two
-// requests, products included: 958 us with the other kernel -> 318 us.
+// the same pairs x 4 (or 8) entries of the output, where a warp that owns one pair reads its keys and values once per pair.  The next tile's keys arrive
+// (cp.async) under the product with the values, the next values under the scores.  Tiles of a row go longest first.  Bound: latencies at three warps a
+// scheduler -- 640 tokens of 32 heads of 64 (156 us under the profiler): a scheduler has an instruction to issue in 45 % of the cycles, the multiply-add pipe is at 32 %
+// of its peak, L1 and shared memory at 30 %.  A layer of TinyLlama's sizes over 1,000 tokens of two requests, products included: 958 us with the other kernel -> 318 us.
 #include "common.cuh"
 #include "range_check.cuh"
 

@@ -154,9 +154,12 @@ static inline int device_sm_count() {
 // What is gained is the launch gap between dependent kernels; what keeps it correct is that no
 // kernel writes global memory, or reads anything that a kernel of the same step writes, before its
 // wait, and that every block of every kernel waits, so "the kernel before me is complete" carries
-// over the whole chain.  Three kernels do read before their wait, and only what is older than the
+// over the whole chain -- a block that finds nothing to do waits before it leaves: a grid whose blocks had all left at once would
+// be complete while the kernel in front of it still runs, and the kernel behind it waits for that grid alone.
+// Some kernels do read before their wait, and only what is older than the
 // step: the tcgen05 product its weights (and, with the rotation epilogue, positions, slots and the
-// cos/sin rows), decode attention the lengths, block tables and every cached row but the newest.  Launched without the
+// cos/sin rows), decode attention the lengths, block tables and every cached row but the newest, and the kernels whose blocks look
+// for their row (warp_find_row) the rows' lengths.  Launched without the
 // attribute (MIE_B200_PDL=0), both instructions do nothing.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

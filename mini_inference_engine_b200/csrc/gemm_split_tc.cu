@@ -6,8 +6,8 @@
 // together, as much as one rounding of a float32 product may lose, and of either sign.  (Parts cut off towards zero would leave out up to 2^-21, always of the
 // product's sign, so that a sum of products of one sign never lost it again.)  The tensor core's own float32 sums are cut off rather than rounded, so
 // a sum stays there for 64 products only (small parts first); every 64-wide chunk of K is taken out of tensor memory and added to a
-// float32 register, rounded to nearest.  Against 64 bits the error is 1.1e-7 at K 2,048 and 1.8e-7 at K 5,632 (2-norm) where one
-// chain of K fused multiply-adds leaves 5.5e-7 and 1.1e-6.
+// float32 register, rounded to nearest.  Against 64 bits the error is 1.04e-7 to 1.31e-7 at K 2,048 (with and without shares of K) and 1.25e-7 at K 5,632
+// (2-norm; parts cut off towards zero 1.42e-7 to 1.63e-7) where one chain of K fused multiply-adds leaves 8.1e-7 and 1.35e-6.
 // A number that is not finite, one too small for its parts, or a sum that overflows on the way makes the sum of the parts infinite or NaN: an output that is not finite is
 // worked out again as one chain of fused multiply-adds from the operands themselves, so it is what the CUDA-core product gives: by the whole block, once its
 // tiles are done and nothing waits for it, 64 x 64 outputs at a time (`sp_again`).
@@ -20,8 +20,8 @@
 //            The pair runs persistently over (tile, share of K) items; shares meet in `partial` and a last small kernel adds them up in order.
 //
 // Bound: the tensor pipe (6 bfloat16 products for one float32 one: a sixth of its rate) for many tokens, memory (4 bytes of w read, 6
-// written and read again) for few.  2,048 x 11,264 x 2,048: 2,707 us on the CUDA cores -> 415 us (228 TFLOP/s, 252 without the split);
-// 509 x 11,264 x 2,048 1,008 -> 165 us; 509 x 2,048 x 5,632 1,195 -> 90 us; 17 x 2,048 x 2,048 210 -> 28 us.  Chunks of 32 in a deeper ring were slower
+// written and read again) for few.  2,048 x 11,264 x 2,048: 2,707 us on the CUDA cores -> 403 us (235 TFLOP/s);
+// 509 x 11,264 x 2,048 1,008 -> 154 us; 509 x 2,048 x 5,632 1,195 -> 78 us; 17 x 2,048 x 2,048, w from memory, 209 -> 24 us.  Chunks of 32 in a deeper ring were slower
 // (550 us at 2,048 tokens): the way from a full accumulator to an empty one costs about 2 us, so what counts is the work per accumulator and their number.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -2,7 +2,7 @@
 // one wide feed-forward.
 //
 //   router     route with the logits computed in the same kernel: z = W_router x in float32 (float32 weights, the token's
-//              input widened), a block per eight tokens, a warp per expert in turn.
+//              input widened), a block per one to eight tokens, a warp per two outputs and stretch of columns in turn, then a warp per token.
 //   route      per token, from float32 router logits z [T, E]: the `top` experts with the largest logits (ties: the lower
 //              index first), weights = softmax over the chosen logits only.  ids [T, top] int32, wts [T, top] float32.
 //   dense_act  with up[t] = [expert 0: F | expert 1: F | ...] the up-projections of ALL experts (one product with the

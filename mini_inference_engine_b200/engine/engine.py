@@ -296,7 +296,8 @@ class LLMEngine:
         ctx = b.to_device(buf, layout, into=static)
         ctx.token_feedback = self._sampled
         tokens = self._sampled[self._portion_slot:self._portion_slot + wanted]
-        # no warm-up run: a step of this shape has run before (kernels built, buffers sized), and running
+        # no warm-up run: a step of this padded length has run before, eagerly and unpadded, so nearly all kernels are built and loaded
+        # (one that only the padded length takes sets itself up inside the capture, which the libraries allow for), and running
         # this one twice would write the request's cache twice -- harmless, but not free
         graph = torch.cuda.CUDAGraph()
         before = ops.launches

@@ -1,7 +1,7 @@
 """The matrix product y = x W^T (+ b) of every projection, by operand type.
 
 * float32 activations (the true 32-bit mode), or a weight the checkpoint holds in 32 bits: the CUDA-core FMA kernel of
-  ``csrc/gemm_simt.cu``; from nine tokens on, where both are float32, the product on the tensor cores with operands
+  ``csrc/gemm_simt.cu``; from nine tokens on (``gemm_split.takes``), where both are float32, the product on the tensor cores with operands
   split into three bfloat16 parts (``csrc/gemm_split_tc.cu``), whose error against 64 bits is the smaller one.
 * bfloat16 activations and weights: a tensor-core product.  The reference calls the vendor library
   for these (F.linear, inference_engine/model.py:172,178,180,181,185).  ``auto`` (the default) uses

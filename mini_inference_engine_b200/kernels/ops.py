@@ -922,7 +922,9 @@ def _heads_a_pass(heads: int, bytes_a_head: int) -> int:
     return -(-heads // -(-heads // most))
 
 
-DECAY_CHUNK_TOKENS = 64        # rows of more new tokens than this go in chunks as matrix products
+DECAY_CHUNK_TOKENS = 64        # rows of more new tokens than this go in chunks as matrix products: what one chunk of the token-by-token kernels takes at most.  The layer, us,
+                               # their chunks : matrix products (8 heads of 128 x 256, width 2,048): 65 tokens 103 : 60, 96 107 : 58, 128 127 : 64, 129 144 : 70, 256 146 : 71, 512 155 : 82;
+                               # 16 heads, width 4,096: 65 137 : 81, 128 171 : 91, 256 179 : 100, 512 234 : 135
 
 
 def decay_chunks_take(dim: int) -> bool:
