@@ -986,8 +986,10 @@ static int fa_keys(int head_dim, int mods, int num_heads, int work_tokens, int w
 // tiles <= tokens / 128 + rows (of the rows that this kernel serves, where the caller knows them).  Whether a block takes one tile or a pair of equal
 // total length, and for heads of 128 how many keys a tile: device time in a graph, one pass after the other, us.
 //   Heads of 64, two blocks on an SM (296 places).  Pairs are all as long as the longest tile and one more, so they pay only where one round of
-//   them fills nearly every place; else tiles alone, longest first, fill the GPU evenly (32 heads, alone : in pairs): 1,152 tokens 22 : 30,
-//   1,400 27 : 33, 1,600 33 : 37, 1,800 40.5 : 40.3, 2,048 44.4 : 42.4, 3,000 85 : 104; rows of 333 and 667 tokens 18 : 25.
+//   them fills nearly every place and rows are long, or where rows are of two to four tiles and those alone are a third more than the places (the second
+//   round's blocks then cost more to set up than they run); else tiles alone, longest first, fill the GPU evenly (32 heads, alone : in pairs): 1,152 tokens 22 : 30,
+//   1,400 27 : 33, 1,600 33 : 37, 1,800 40.5 : 40.3, 2,048 44.4 : 42.4, 3,000 85 : 104; rows of 333 and 667 tokens 18 : 25; two rows of 1,000 32 : 30 (16 heads, four rows
+//   37 : 30), four of 333 21 : 19, six of 200 18.9 : 17.1, three of 500 21.8 : 21.7; but two of 640 19 : 23, four of 500 27 : 33, eight of 200 21 : 28, six of 333 25 : 32.
 //   Heads of 128: tiles of 128 keys with an SM alone are the faster ones (a launch of few blocks waits for its longest), tiles of 64 with two blocks on an
 //   SM the more per second.  More blocks than 296 (32 heads, 128 keys and pairs : 64 keys): 1,500 tokens 71 : 45, 2,048 88 : 65, 8,192 980 : 767, rows of
 //   645 tokens on 1,500 and of 1,292 138 : 73; fewer: 1,000 tokens 29 : 33, 2,048 tokens of 16 heads 45 : 59, 4,096 of 8 heads 76 : 108.
@@ -995,7 +997,7 @@ template <int D, int MODS, bool KEEP>
 static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p, int work_tokens,
                      int work_rows, cudaStream_t stream) {
     const int tiles = (work_tokens + FA_BM - 1) / FA_BM + work_rows;
-    const int64_t sms = device_sm_count(), blocks = (int64_t)((work_tokens + FA_BM - 1) / FA_BM + work_rows - 1) * p.num_heads;
+    const int64_t sms = device_sm_count();
     FaParams pp = p;
     if constexpr (D == 128) {
         if constexpr ((MODS & 3) == 0)
@@ -1004,7 +1006,9 @@ static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     } else if constexpr ((MODS & 3) != 0) {
         pp.pair = (int64_t)tiles * p.num_heads > 2 * sms;          // (these instances have an SM alone)
     } else {
-        pp.pair = work_rows == 1 && blocks <= 4 * sms && blocks * 10 > 33 * sms;
+        const int64_t each = ((work_tokens + work_rows - 1) / work_rows + FA_BM - 1) / FA_BM, alone = each * work_rows * p.num_heads;
+        pp.pair = alone > 2 * sms && (each + 1) / 2 * work_rows * p.num_heads <= 2 * sms &&
+                  (each <= 4 ? alone * 10 <= 27 * sms : each >= 8 && alone * 10 > 33 * sms);
     }
     return launch_fa_tile<D, MODS, KEEP, 128>(mq, mk, mv, pp, tiles, work_rows, stream);
 }
