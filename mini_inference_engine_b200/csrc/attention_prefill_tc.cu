@@ -446,8 +446,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,   // qkv 
                     }
                     float alpha = 1.f, sum = 0.f;
                     // 64 keys a tile: a row's largest score is the reference point, and its weight of 1 free of rounding, half as often as with 128,
-                    // so the output's error grew (0.3 % of a layer's, 1 to 3 % of the kernel's up to 1,500 keys).  There the sum takes the weights as rounded for the
-                    // product with the values: they then add up to one, and the error is below that of 128 keys and exact weights in the sum.
+                    // so the float32 output's error grew (300 / 800 / 1,500 causal keys: by 8 / 6 / 5 %).  There the sum takes the weights as rounded for the product
+                    // with the values: they then add up to one, and the error is 0.3 / 1.4 / 2.0 % below that of 128 keys and unrounded weights in the sum.  (3 to 9 % of
+                    // this kernel's time: 1,500 tokens of 32 heads 45 -> 47 us, 2,048 66 -> 69, 4,096 210 -> 215.)
                     constexpr bool ROUNDED_SUM = BN == 64;
                     auto p_pass = [&](auto mask_tag, float neg_m, float& xmax_out) {
                         constexpr bool MASK = decltype(mask_tag)::value;
@@ -991,8 +992,8 @@ static int fa_keys(int head_dim, int mods, int num_heads, int work_tokens, int w
 //   1,400 27 : 33, 1,600 33 : 37, 1,800 40.5 : 40.3, 2,048 44.4 : 42.4, 3,000 85 : 104; rows of 333 and 667 tokens 18 : 25; two rows of 1,000 32 : 30 (16 heads, four rows
 //   37 : 30), four of 333 21 : 19, six of 200 18.9 : 17.1, three of 500 21.8 : 21.7; but two of 640 19 : 23, four of 500 27 : 33, eight of 200 21 : 28, six of 333 25 : 32.
 //   Heads of 128: tiles of 128 keys with an SM alone are the faster ones (a launch of few blocks waits for its longest), tiles of 64 with two blocks on an
-//   SM the more per second.  More blocks than 296 (32 heads, 128 keys and pairs : 64 keys): 1,500 tokens 71 : 45, 2,048 88 : 65, 8,192 980 : 767, rows of
-//   645 tokens on 1,500 and of 1,292 138 : 73; fewer: 1,000 tokens 29 : 33, 2,048 tokens of 16 heads 45 : 59, 4,096 of 8 heads 76 : 108.
+//   SM the more per second.  More blocks than 296 (32 heads, 128 keys and pairs : 64 keys): 1,153 tokens 62 : 38, 1,500 71 : 47, 2,048 89 : 69, 4,096 300 : 215, nine rows of
+//   128 23 : 15, five of 200 30 : 22; fewer: 1,000 tokens 29 : 33, 2,048 tokens of 16 heads 45 : 59, 4,096 of 8 heads 76 : 108.
 template <int D, int MODS, bool KEEP>
 static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p, int work_tokens,
                      int work_rows, cudaStream_t stream) {
