@@ -987,10 +987,10 @@ static int fa_keys(int head_dim, int mods, int num_heads, int work_tokens, int w
 // tiles <= tokens / 128 + rows (of the rows that this kernel serves, where the caller knows them).  Whether a block takes one tile or a pair of equal
 // total length, and for heads of 128 how many keys a tile: device time in a graph, one pass after the other, us.
 //   Heads of 64, two blocks on an SM (296 places).  Pairs are as long as the longest tile and one more, so one round of them has to replace a round and a good part
-//   of a second of tiles alone, whose blocks cost a set-up each: rows of two to six tiles with a quarter more tiles than places, longer rows with two thirds
-//   more (rows of the mean length; alone : in pairs).  32 heads: 1,000 tokens 21 : 25, 1,400 27 : 34, 1,536 30 : 36, 2,048 45.2 : 43.5, four rows of 256 12 : 18, of 333 20.9 : 18.6,
+//   of a second of tiles alone, whose blocks cost a set-up each: rows of two or three tiles with more tiles than places, of up to six with a quarter more, longer ones
+//   with two thirds more (rows of the mean length; alone : in pairs).  32 heads: 1,000 tokens 21 : 25, 1,400 27 : 34, 1,536 30 : 36, 2,048 45.2 : 43.5, four rows of 256 12 : 18, of 333 20.9 : 18.6,
 //   of 500 26.6 : 21.4, of 700 41 : 44 (pairs do not fit one round), three of 640 27.4 : 23.5, eight of 200 21.0 : 17.4.  16 heads: 2,048 tokens 35 : 40, three rows of 896
-//   21 : 27, of 1,000 27.0 : 28.6, four of 700 26.2 : 24.7, of 1,000 37 : 30.  40 heads: 1,153 tokens 29 : 33, two rows of 500 19.5 : 21.1, of 700 27.7 : 25.1, three of 500 25.4 : 21.8.
+//   21 : 27, of 1,000 27.0 : 28.6, four of 700 26.2 : 24.7, of 1,000 37 : 30.  40 heads: 1,153 tokens 29 : 33, four rows of 200 18.1 : 16.4, three of 333 19.9 : 18.9, two of 500 19.5 : 21.1, of 700 27.7 : 25.1, three of 500 25.4 : 21.8.
 //   Heads of 128: tiles of 128 keys with an SM alone are the faster ones (a launch of few blocks waits for its longest), tiles of 64 with two blocks on an
 //   SM the more per second.  More blocks than 296 (32 heads, 128 keys and pairs : 64 keys): 1,153 tokens 62 : 38, 1,500 71 : 47, 2,048 89 : 69, 4,096 300 : 215, nine rows of
 //   128 23 : 15, five of 200 30 : 22; fewer: 1,000 tokens 29 : 33, 2,048 tokens of 16 heads 45 : 59, 4,096 of 8 heads 76 : 108.
@@ -1008,7 +1008,7 @@ static int launch_fa(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
         pp.pair = (int64_t)tiles * p.num_heads > 2 * sms;          // (these instances have an SM alone)
     } else {
         const int64_t each = ((work_tokens + work_rows - 1) / work_rows + FA_BM - 1) / FA_BM, alone = each * work_rows * p.num_heads;
-        pp.pair = each >= 2 && (each + 1) / 2 * work_rows * p.num_heads <= 2 * sms && alone * 100 >= 2 * sms * (each <= 6 ? 125 : 165);
+        pp.pair = each >= 2 && (each + 1) / 2 * work_rows * p.num_heads <= 2 * sms && alone * 100 > 2 * sms * (each <= 3 ? 100 : each <= 6 ? 124 : 164);
     }
     return launch_fa_tile<D, MODS, KEEP, 128>(mq, mk, mv, pp, tiles, work_rows, stream);
 }
