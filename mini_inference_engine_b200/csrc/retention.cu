@@ -56,7 +56,11 @@ __global__ void retention_prepare_kernel(const T* __restrict__ qkv, int64_t stri
                                          float* __restrict__ kr, int H, int D, int rot, int act, float q_scale,
                                          const float* __restrict__ k_tok) {
     extern __shared__ float cs[];                 // cos [rot/2], sin [rot/2]
-    pdl_enter();
+    // The kernel behind may start once those in front have ended, not before: its blocks, resident while products still hold most SMs, would be packed onto the
+    // others and stay there -- 72 long ones, one chunk and head each, two and more to an SM (a portion of 64 tokens beside 8 single ones, 8 heads of 128 x 256, in a graph:
+    // the layer 101 us, 68 with launches that do not overlap, 73 so)
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x, half = rot >> 1;
     const T* src = qkv + (int64_t)t * stride;
     // a head's work: half / VEC pairs of pieces, then (D - rot) / VEC pieces
