@@ -4,16 +4,22 @@
 //
 // With G_i the product of a chunk's decays up to token i, M_ij the product of those behind token j up to token i and S the state in front of the chunk,
 //   O = diag(G) Q S + (Q K^T * M) V,       what the chunk adds to the state = sum over t of M_{last, t} k_t v_t^T,       S <- G_last S + that,
-// so a token costs 2 D Dv multiply-adds and half a chunk's of Q K^T and P V, out of shared memory in tiles of registers, where token by token it costs
-// 5 D Dv in two passes, with a shared-memory read for every one or two.  Products of decays are products (no logarithms: a decay may be 0).  Float32 on the CUDA cores throughout.
+// so a token costs 2 D Dv multiply-adds and half a chunk's of Q K^T and P V, where token by token it costs
+// 5 D Dv in two passes, with a shared-memory read for every one or two.  Products of decays are products (no logarithms: a decay may be 0).  The products run on the tensor
+// cores with every float32 operand as three bfloat16 parts (triple_mma.cuh); values that are bfloat16 as they come are one part, so that half of the part products fall away.
 //
-//   local    a block per (chunk, head, half of the value columns): P = Q K^T * M (lower triangle) and G into scratch memory, and what the chunk adds to the state -> states[chunk].
+//   local    a block per (chunk, head): P = Q K^T * M (lower triangle) and G into scratch memory, and what the chunk adds to the state -> states[chunk].
 //   combine  per row in order: states[chunk] becomes the state in front of the chunk; the state after the last goes to the request's slot.
-//   output   a block per (chunk, head, 64 value columns).
+//   output   a block per (chunk, head, 128 or 64 value columns).
 //
-// Rows of one chunk are left to retention.cu.  q and k come prepared (rotated or activated, scaled) as float32 from its first kernel.  Bound: the
-// CUDA cores' multiply-adds.
-#include "common.cuh"
+// Numbers without three parts (not finite, or beyond 2^127) make their block do its products one multiply-add after the other, without the zeros of the triangle.
+//
+// Rows of one chunk are left to retention.cu.  q and k come prepared (rotated or activated, scaled) as float32 from its first kernel.
+// Bound: the tensor pipe at 8 cycles an instruction on each quarter of an SM, kept busy for 24 - 30 % of the time (operands' way from memory and the blocks' ends are the
+// rest).  2,048 tokens of 8 heads of 128 x 256 from bfloat16 values, us: local 51.7 -> 30, output 78.7 -> 40 (register tiles on the CUDA cores before); the layer
+// with a decay per head 209 -> 146, of 100 tokens 58 -> 46.  Against 64 bits the outputs are 1.0e-7 to 2.7e-7 off (2-norm; the CUDA cores' 2.1e-7 to 3.5e-7), the states
+// 4.7e-8 to 3.0e-7 (4.8e-8 to 3.1e-7).
+#include "triple_mma.cuh"
 
 #define DC_L 64                // tokens a chunk
 #define DC_P 68                // stride of rows of 64: neighbouring rows four banks apart
@@ -30,21 +36,6 @@ struct DcParams {
     int h0, heads;                             // the heads of this pass: states and scratch hold these only
 };
 __device__ __forceinline__ float* dc_scratch(const DcParams& p, int64_t chunk, int h) { return p.scratch + (chunk * p.heads + h - p.h0) * (DC_L * DC_L + DC_L); }
-
-__device__ __forceinline__ void dc_copy16(float* dst, const float* src, bool on) {       // zeros where `on` is false (nothing is read then)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void dc_wait_all() { asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory"); }
-
-// 64 rows of up to DT entries (the rest zero) into rows of DT + 4
-template <int DT>
-__device__ __forceinline__ void dc_rows(float* dst, const float* src, int64_t stride, int D, int count) {
-    for (int c = threadIdx.x; c < DC_L * (DT / 4); c += blockDim.x) {
-        const int r = c / (DT / 4), d = (c - r * (DT / 4)) * 4;
-        const bool on = r < count && d < D;
-        dc_copy16(dst + r * (DT + 4) + d, on ? src + r * stride + d : src, on);
-    }
-}
 
 template <typename T>
 __device__ __forceinline__ float dc_value(const DcParams& p, int64_t token, int h, int col) {
@@ -63,25 +54,147 @@ __device__ __forceinline__ bool dc_find(const DcParams& p, int* s_row, int* s_ch
     return *s_row >= 0;
 }
 
-template <typename T, int DT>
-__global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, int halves) {
-    constexpr int DP = DT + 4;
-    extern __shared__ __align__(16) float sm[];
-    float* Q = sm;                                     // [64][DP]
-    float* K = Q + DC_L * DP;                          // [64][DP]
-    float* M = K + DC_L * DP;                          // [64][DC_P]: products of decays; then a tile of values [64 tokens][DC_P]
+#define DC_THREADS 256
+#define DC_COLS 64             // value columns of the local kernel at a time
+
+// Eight neighbouring values of a token as they lie in memory, those from `left` on zero; and as numbers (nothing is computed from them where they are asked for, so that
+// nothing waits there).
+template <typename T> struct alignas(16) Eight { T x[8]; };
+template <typename T>
+__device__ __forceinline__ Eight<T> dc_values8(const DcParams& p, int64_t token, int h, int col, int left) {
+    Eight<T> r;
+    const T* at = reinterpret_cast<const T*>(p.v) + token * p.v_stride + (int64_t)h * p.Dv_in + col;
+    uint4* to = reinterpret_cast<uint4*>(r.x);
+    if (left >= 8 && (reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T) / 2; ++i) to[i] = reinterpret_cast<const uint4*>(at)[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r.x[i] = i < left ? at[i] : from_f32<T>(0.f);
+    }
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ void dc_numbers(float (&x)[8], const Eight<T>& r, const DcParams& p) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        x[i] = to_f32<T>(r.x[i]);
+        if (p.v_act) x[i] = x[i] / (1.0f + expf(-x[i]));
+    }
+}
+
+// Left operand (16 columns x 16 rows of the tile) from tiles [64][COLS] whose rows run along the contraction.
+template <int COLS, int PARTS>
+__device__ __forceinline__ void dc_left(uint32_t (&a)[PARTS][4], uint32_t tile, int plane, int m, int k, int lane) {
+    const uint32_t at = tile + tile_at<COLS>(k * 16 + (lane & 7) + ((lane >> 4) << 3), m * 2 + ((lane >> 3) & 1));
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p) ldm4t(a[p][0], a[p][1], a[p][2], a[p][3], at + p * plane);
+}
+// sum[n] += A B_n over 16 of the contraction, one of the two operands a single part.
+template <int N>
+__device__ __forceinline__ void one_left_step(float (*sum)[4], const uint32_t (&a)[1][4], const uint32_t (&b)[3][N][2]) {
+    float t[N][4], h[N][4];
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_zero(t[n], a[0], b[2][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_zero(h[n], a[0], b[0][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_more(t[n], a[0], b[1][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[n][i] = h[n][i] + (sum[n][i] + t[n][i]);
+}
+template <int N>
+__device__ __forceinline__ void one_right_step(float (*sum)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[1][N][2]) {
+    float t[N][4], h[N][4];
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_zero(t[n], a[2], b[0][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_zero(h[n], a[0], b[0][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_more(t[n], a[1], b[0][n]);
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[n][i] = h[n][i] + (sum[n][i] + t[n][i]);
+}
+
+// A lane's eight numbers of the left operand with rows r0, r0 + 8 and columns d, d + 1, d + 8, d + 9 of float32 rows; those beyond the rows or the columns are zero.
+struct DcLeft { float4 v, w; };
+__device__ __forceinline__ DcLeft dc_left_rows(const float* rows, int64_t stride, int r0, int d, int count, int D) {
+    auto two = [&](int r, int c) { return r < count && c < D ? *reinterpret_cast<const float2*>(rows + r * stride + c) : make_float2(0.f, 0.f); };
+    const float2 a = two(r0, d), b = two(r0 + 8, d), e = two(r0, d + 8), f = two(r0 + 8, d + 8);
+    return DcLeft{make_float4(a.x, a.y, b.x, b.y), make_float4(e.x, e.y, f.x, f.y)};
+}
+
+// What a chunk adds to the state, a multiply-add after the other; ww: what is left of each token at the chunk's end.
+template <typename T>
+__device__ __noinline__ void dc_walk_state(const DcParams& p, const float* kp, const float* ww, float* to, int t0, int h, int count, int first, int end) {
+    for (int i = first * p.D + threadIdx.x; i < end * p.D; i += DC_THREADS) {
+        const int col = i / p.D, d = i - col * p.D;
+        float sum = 0.f;
+        for (int t = 0; t < count; ++t) sum = fmaf(col < p.Dv_in ? dc_value<T>(p, t0 + t, h, col) : 1.f, ww[t] * kp[(int64_t)t * p.H * p.D + d], sum);
+        to[i] = sum;
+    }
+}
+__device__ __noinline__ void dc_walk_scores(const DcParams& p, const float* qp, const float* kp, const float* M, float* out, int count) {
+    for (int i = threadIdx.x; i < DC_L * DC_L; i += DC_THREADS) {
+        const int r = i >> 6, c = i & 63;
+        float sum = 0.f;
+        if (c <= r && r < count)
+            for (int d = 0; d < p.D; ++d) sum = fmaf(qp[(int64_t)r * p.H * p.D + d], kp[(int64_t)c * p.H * p.D + d], sum);
+        out[i] = c <= r ? sum * M[r * DC_P + c] : 0.f;
+    }
+}
+
+// ONE: the values are bfloat16 as they come.  blockIdx.z: a share of the value columns -- with fewer (chunk, head) pairs than SMs a pair's columns go to as many blocks as there is
+// room for (the first share makes P too): 100 tokens of 8 heads of 128 x 256, 4 shares, the kernel and the output kernel's narrow blocks, layer 58.6 -> 46.1 us; shares
+// for two blocks an SM instead of one: 1,024 tokens 19.4 -> 18.6 us, 512 tokens 14.6 -> 14.9.
+template <typename T, int DT, bool ONE>
+__global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcParams p, int splits) {
+    constexpr int AHEAD = 3;                           // steps of the contraction that the queries are asked for ahead
+    constexpr int PLANE = DC_L * DT * 2, V_PLANE = DC_L * DC_COLS * 2, PARTS = ONE ? 1 : 3, KS = DT / 16, QUADS = DC_L * DT / 4 / DC_THREADS, STEP = DC_THREADS / (DT / 4);
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint8_t* keys = smem;                              // [64][DT] as parts; then with what is left of them at the chunk's end
+    uint8_t* values = smem + 3 * PLANE;                // two buffers of [64][64]
+    float* M = reinterpret_cast<float*>(values + 2 * PARTS * V_PLANE);     // [64][DC_P]: products of decays
     __shared__ float a[DC_L], G[DC_L];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
     const bool mine = dc_find(p, &s_row, &s_chunk);
     pdl_wait();                                        // (a block without work waits too: see common.cuh)
     if (!mine) return;
-    const int h = p.h0 + blockIdx.y, H = p.H, D = p.D, half = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = p.h0 + blockIdx.y, H = p.H, D = p.D;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
-    dc_rows<DT>(K, p.k + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
-    if (half == 0) dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
+    const int tiles = (p.Dv_in + DC_COLS - 1) / DC_COLS, per = (tiles + splits - 1) / splits, part_no = blockIdx.z;       // this block's share of the value columns
+    const int first_col = part_no * per * DC_COLS, end_col = min((part_no + 1) * per * DC_COLS, p.Dv_in);
+    const float* kp = p.k + ((int64_t)t0 * H + h) * D;
+    const float* qp = p.q + ((int64_t)t0 * H + h) * D;
+    const int64_t stride = (int64_t)H * D;
+    const int kr = threadIdx.x / (DT / 4), kd = (threadIdx.x % (DT / 4)) * 4;
+    uint32_t most = 0;                                 // the largest magnitude of keys (and queries) this thread met
+    float4 key[QUADS];
+#pragma unroll
+    for (int i = 0; i < QUADS; ++i)
+        key[i] = kr + i * STEP < count && kd < D ? *reinterpret_cast<const float4*>(kp + (kr + i * STEP) * stride + kd) : make_float4(0.f, 0.f, 0.f, 0.f);
+    auto put_keys = [&](auto factor) {
+#pragma unroll
+        for (int i = 0; i < QUADS; ++i) {
+            const int r = kr + i * STEP;
+            const float f = factor(r);
+            most = max(most, magnitude(key[i]));
+            uint8_t* at = keys + tile_at<DT>(r, kd >> 3) + (kd & 4) * 2;
+            uint2 part[3];
+            split3(key[i].x * f, key[i].y * f, part[0].x, part[1].x, part[2].x);
+            split3(key[i].z * f, key[i].w * f, part[0].y, part[1].y, part[2].y);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(at + j * PLANE) = part[j];
+        }
+    };
     if (threadIdx.x < DC_L)
         a[threadIdx.x] = threadIdx.x >= count ? 1.f : p.tok_decay ? p.tok_decay[(int64_t)(t0 + threadIdx.x) * H + h] : p.decay[h];
+    put_keys([](int) { return 1.f; });
     __syncthreads();
     if (threadIdx.x < DC_L) {                          // a column of M a thread
         const int j = threadIdx.x;
@@ -96,103 +209,140 @@ __global__ void __launch_bounds__(256, 2) decay_local_kernel(const DcParams p, i
 #pragma unroll 8
         for (int i = 0; i < DC_L; ++i) { run *= a[i]; G[i] = run; }
     }
-    dc_wait_all();
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    if (half == 0) {
-        float* out = dc_scratch(p, blockIdx.x, h);
-        float s[4][4];
+    // values of 64 columns, two runs of eight a thread; those of the next columns are asked for while these are multiplied
+    Eight<T> raw[2];
+    auto ask = [&](int j0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i) {
+            const int t = (threadIdx.x >> 3) + 32 * i, c = j0 + (threadIdx.x & 7) * 8;
+            raw[i] = dc_values8<T>(p, t0 + min(t, count - 1), h, c, t < count ? end_col - c : 0);
+        }
+    };
+    ask(first_col);
+    float* out = dc_scratch(p, blockIdx.x, h);
+    if (part_no == 0) {
+        // Q K^T: 16 rows a warp, every other pair of column tiles up to the diagonal; the queries go straight from memory into operands
+        const int m = warp < 4 ? warp : 7 - warp, odd = warp >> 2, r = m * 16 + (lane >> 2), c0 = (lane & 3) * 2;
+        const uint32_t right = (uint32_t)__cvta_generic_to_shared(keys);
+        float sum[4][4] = {};
+        DcLeft q[AHEAD];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < DT; d += 4) {
-            float4 kk[4];
+        for (int k = 0; k < AHEAD; ++k) q[k] = dc_left_rows(qp, stride, r, k * 16 + c0, count, D);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * DP + d);
+        for (int k = 0; k < KS; ++k) {
+            uint32_t left[3][4];
+            const DcLeft x = q[k % AHEAD];
+            most = max(most, max(magnitude(x.v), magnitude(x.w)));
+            split_left(left, x.v, x.w);
+            if (k + AHEAD < KS) q[k % AHEAD] = dc_left_rows(qp, stride, r, (k + AHEAD) * 16 + c0, count, D);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * DP + d);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (j > i) continue;               // wholly above the diagonal
-                    s[i][j] = fmaf(qq.x, kk[j].x, s[i][j]);
-                    s[i][j] = fmaf(qq.y, kk[j].y, s[i][j]);
-                    s[i][j] = fmaf(qq.z, kk[j].z, s[i][j]);
-                    s[i][j] = fmaf(qq.w, kk[j].w, s[i][j]);
-                }
+            for (int j = 0; j < 2; ++j) {
+                if (odd + 2 * j > m) break;
+                uint32_t b[3][2][2];
+                right_columns<DT>(b, right, PLANE, k, 2 * (odd + 2 * j), lane);
+                triple_step<2>(sum + 2 * j, left, b);
             }
         }
+        __syncthreads();                               // M
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j) {
+            const int c = (odd + 2 * (j >> 1)) * 16 + (j & 1) * 8 + c0;
+            if (odd + 2 * (j >> 1) > m) continue;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int r = ty + 16 * i, c = tx + 16 * j;
-                out[r * DC_L + c] = c <= r ? s[i][j] * M[r * DC_P + c] : 0.f;
+            for (int i = 0; i < 2; ++i) {
+                const int rr = r + 8 * i;
+                const float2 f = *reinterpret_cast<const float2*>(M + rr * DC_P + c);
+                *reinterpret_cast<float2*>(out + rr * DC_L + c) = make_float2(c <= rr ? sum[j][2 * i] * f.x : 0.f, c + 1 <= rr ? sum[j][2 * i + 1] * f.y : 0.f);
             }
+        }
         if (threadIdx.x < DC_L) out[DC_L * DC_L + threadIdx.x] = G[threadIdx.x];
-    }
-    // keys with what is left of them at the chunk's end (in place: the scores are done with them once every thread is here)
-    const float w_mine = M[(count - 1) * DC_P + (threadIdx.x & 63)];
-    __syncthreads();
-    if (threadIdx.x < DC_L) a[threadIdx.x] = threadIdx.x < count ? w_mine : 0.f;
-    __syncthreads();
-    for (int i = threadIdx.x; i < DC_L * (DT / 4); i += 256) {
-        const int r = i / (DT / 4);
-        float4* at = reinterpret_cast<float4*>(K + r * DP + (i - r * (DT / 4)) * 4);
-        float4 v = *at;
-        const float w = a[r];
-        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-        *at = v;
-    }
-    // the state's columns, 64 at a time: column 4 ty + c, entries 4 tx + 64 e .. + 3
+    } else __syncthreads();
+    if (threadIdx.x < DC_L) a[threadIdx.x] = threadIdx.x < count ? M[(count - 1) * DC_P + threadIdx.x] : 0.f;      // what is left of each token at the chunk's end
+    __syncthreads();                                   // (the keys are done with)
+    put_keys([&](int r) { return a[r]; });
     float* to = p.states + ((int64_t)blockIdx.x * p.heads + blockIdx.y) * (int64_t)p.Dv * D;
-    constexpr int E = DT / 64;
-    const int tiles = (p.Dv_in + 63) / 64, per = (tiles + halves - 1) / halves;
-    for (int tile = half * per; tile < min(tiles, (half + 1) * per); ++tile) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < DC_L * 64; i += 256) {
-            const int t = i >> 6, c = i & 63, col = tile * 64 + c;
-            M[t * DC_P + c] = t < count && col < p.Dv_in ? dc_value<T>(p, t0 + t, h, col) : 0.f;
-        }
-        __syncthreads();
-        float s[4][4 * E];
+    bool bad = false;
+    for (int j0 = first_col, buf = 0; j0 < end_col; j0 += DC_COLS, buf ^= 1) {
+        uint8_t* tile = values + buf * PARTS * V_PLANE;
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int i = 0; i < 2; ++i) {
+            uint8_t* at = tile + tile_at<DC_COLS>((threadIdx.x >> 3) + 32 * i, threadIdx.x & 7);
+            uint32_t part[3][4];
+            float x[8];
+            dc_numbers(x, raw[i], p);
 #pragma unroll
-            for (int e = 0; e < 4 * E; ++e) s[c][e] = 0.f;
-#pragma unroll 4
-        for (int t = 0; t < DC_L; ++t) {
-            const float4 vv = *reinterpret_cast<const float4*>(M + t * DC_P + 4 * ty);
-            const float vc[4] = {vv.x, vv.y, vv.z, vv.w};
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const float4 kk = *reinterpret_cast<const float4*>(K + t * DP + 64 * e + 4 * tx);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    s[c][4 * e] = fmaf(vc[c], kk.x, s[c][4 * e]);
-                    s[c][4 * e + 1] = fmaf(vc[c], kk.y, s[c][4 * e + 1]);
-                    s[c][4 * e + 2] = fmaf(vc[c], kk.z, s[c][4 * e + 2]);
-                    s[c][4 * e + 3] = fmaf(vc[c], kk.w, s[c][4 * e + 3]);
+            for (int e = 0; e < 4; ++e) {
+                if (ONE) part[0][e] = nearest2(x[2 * e], x[2 * e + 1]);
+                else {
+                    split3(x[2 * e], x[2 * e + 1], part[0][e], part[1][e], part[2][e]);
+                    bad |= has_no_parts(max(magnitude(x[2 * e]), magnitude(x[2 * e + 1])));
                 }
             }
+#pragma unroll
+            for (int j = 0; j < PARTS; ++j) *reinterpret_cast<uint4*>(at + j * V_PLANE) = make_uint4(part[j][0], part[j][1], part[j][2], part[j][3]);
         }
+        ask(j0 + DC_COLS);
+        __syncthreads();
+        // 32 of the columns (rows of the product) and a quarter of the channels a warp
+        const int cg = warp & 1, d0 = (warp >> 1) * (DT / 4), c = j0 + cg * 32;
+        const uint32_t left = (uint32_t)__cvta_generic_to_shared(tile), right = (uint32_t)__cvta_generic_to_shared(keys);
+        if (c < end_col) {
+            constexpr int NT = DT / 32;                // column tiles of a warp: 4 or 2
+            float sum[2][NT][4] = {};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int col = tile * 64 + 4 * ty + c;
+            for (int k = 0; k < 4; ++k) {
+                uint32_t v[2][PARTS][4];
 #pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int d = 64 * e + 4 * tx;
-                if (col < p.Dv_in && d < D)
-                    *reinterpret_cast<float4*>(to + (int64_t)col * D + d) = make_float4(s[c][4 * e], s[c][4 * e + 1], s[c][4 * e + 2], s[c][4 * e + 3]);
+                for (int m = 0; m < 2; ++m) dc_left<DC_COLS, PARTS>(v[m], left, V_PLANE, cg * 2 + m, k, lane);
+#pragma unroll
+                for (int n = 0; n < NT; n += 2) {
+                    uint32_t b[3][2][2];
+                    right_rows<DT>(b, right, PLANE, k, d0 / 8 + n, lane);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        if constexpr (ONE) one_left_step<2>(sum[m] + n, v[m], b);
+                        else triple_step<2>(sum[m] + n, v[m], b);
+                    }
+                }
             }
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int col = c + m * 16 + (lane >> 2) + 8 * i;
+                    if (col >= end_col) continue;
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        const int d = d0 + n * 8 + (lane & 3) * 2;
+                        if (d < D) *reinterpret_cast<float2*>(to + (int64_t)col * D + d) = make_float2(sum[m][n][2 * i], sum[m][n][2 * i + 1]);
+                    }
+                }
         }
     }
-    if (half == 0 && p.Dv > p.Dv_in && threadIdx.x < D) {      // the column fed with ones: the sum of the keys
+    if (part_no == 0 && p.Dv > p.Dv_in) {              // the column fed with ones: the sum of the keys, from their parts
+        const int d = threadIdx.x % DT, first = threadIdx.x / DT * (DT / 4);
         float sum = 0.f;
-        for (int t = 0; t < DC_L; ++t) sum += K[t * DP + threadIdx.x];
-        to[(int64_t)p.Dv_in * D + threadIdx.x] = sum;
+#pragma unroll 8
+        for (int t = first; t < first + DT / 4; ++t) {
+            const uint8_t* at = keys + tile_at<DT>(t, d >> 3) + (d & 7) * 2;
+            const float h = __bfloat162float(*reinterpret_cast<const bf16*>(at)), m = __bfloat162float(*reinterpret_cast<const bf16*>(at + PLANE)),
+                        l = __bfloat162float(*reinterpret_cast<const bf16*>(at + 2 * PLANE));
+            sum += h + (m + l);
+        }
+        float* part = reinterpret_cast<float*>(values);
+        __syncthreads();                               // (the values are done with)
+        part[threadIdx.x] = sum;
+        __syncthreads();
+        if (threadIdx.x < D) {
+#pragma unroll
+            for (int i = 1; i < DC_THREADS / DT; ++i) sum += part[i * DT + threadIdx.x];
+            to[(int64_t)p.Dv_in * D + threadIdx.x] = sum;
+        }
+    }
+    const bool no_keys = has_no_parts(most);
+    if (__syncthreads_or(bad || no_keys)) {
+        dc_walk_state<T>(p, kp, a, to, t0, h, count, first_col, part_no == splits - 1 ? p.Dv : min(end_col, p.Dv));
+        if (part_no == 0) dc_walk_scores(p, qp, kp, M, out, count);
     }
 }
 
@@ -235,101 +385,187 @@ __global__ void __launch_bounds__(128) decay_combine_kernel(const DcParams p) {
     *reinterpret_cast<float4*>(end) = cur;
 }
 
-template <typename T, int DT>
-__global__ void __launch_bounds__(256, 2) decay_output_kernel(const DcParams p) {
-    constexpr int DP = DT + 4;
-    extern __shared__ __align__(16) float sm[];
-    float* Q = sm;                                     // [64][DP]
-    float* S = Q + DC_L * DP;                          // the state's columns [64][DP]
-    float* P = S + 64 * DP;                            // [64][DC_P]
-    float* VT = P + DC_L * DC_P;                       // values, a column a row [64][DC_P]
+// A block per (chunk, head, 128 or 64 value columns): 16 of them a warp, all of the chunk's tokens.  Q, P and the values as parts in shared memory, the state from memory
+// straight into operands.  ONE: the values are bfloat16 as they come.  WARPS 8; 4 where blocks of 8 would leave half of the SMs without one
+// (512 tokens of 8 heads: 15.4 us by blocks of 8 warps, 16.8 by blocks of 4).  Three blocks an SM in 80 registers each: 44 -> 51 us at 2,048 tokens.
+template <int DT, bool ONE, int WARPS> constexpr int output_bytes() { return (4 * (DT / 16) + 10) * 1536 + (ONE ? 1 : 3) * DC_L * 16 * WARPS * 2; }
+template <typename T, int DT, bool ONE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 2) decay_output_kernel(const DcParams p) {
+    constexpr int KS = DT / 16, PARTS = ONE ? 1 : 3, AHEAD = 4;
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint32_t* left = reinterpret_cast<uint32_t*>(smem); // Q [4 * KS][part][lane][4], then P's tiles up to the diagonal, row by row
+    uint8_t* values = smem + (4 * KS + 10) * 1536;     // [64][16 * WARPS] as parts
+    constexpr int THREADS = 32 * WARPS, WIDE = 16 * WARPS, V_PLANE = DC_L * WIDE * 2;
     __shared__ float G[DC_L];
-    __shared__ __align__(16) float n[DT];
     __shared__ int s_row, s_chunk;
     pdl_launch_dependents();
     const bool mine = dc_find(p, &s_row, &s_chunk);
     pdl_wait();                                        // (a block without work waits too: see common.cuh)
     if (!mine) return;
-    const int h = p.h0 + blockIdx.y, H = p.H, D = p.D, c0 = blockIdx.z * 64;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = p.h0 + blockIdx.y, H = p.H, D = p.D, r0 = lane >> 2, c0 = (lane & 3) * 2;
     const int t0 = p.row_q_start[s_row] + s_chunk * DC_L, count = min(DC_L, p.row_q_len[s_row] - s_chunk * DC_L);
     const float* from = p.states + ((int64_t)blockIdx.x * p.heads + blockIdx.y) * (int64_t)p.Dv * D;
     const float* pg = dc_scratch(p, blockIdx.x, h);
-    const bool ones = blockIdx.z == 0 && p.Dv > p.Dv_in;
-    dc_rows<DT>(Q, p.q + ((int64_t)t0 * H + h) * D, (int64_t)H * D, D, count);
-    dc_rows<DT>(S, from + (int64_t)c0 * D, D, D, min(64, p.Dv_in - c0));
-    for (int i = threadIdx.x; i < DC_L * (DC_L / 4); i += 256) dc_copy16(P + (i >> 4) * DC_P + (i & 15) * 4, pg + i * 4, true);
+    const float* qp = p.q + ((int64_t)t0 * H + h) * D;
+    const int64_t stride = (int64_t)H * D;
+    const int j0 = (blockIdx.z * WARPS + warp) * 16;
+    // the state's 16 channels of two tiles of 8 columns, asked for ahead: they come from L2 at best
+    auto ask = [&](float2 (&x)[4], int k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int col = j0 + (i >> 1) * 8 + r0, d = k * 16 + (i & 1) * 8 + c0;
+            x[i] = col < p.Dv_in && d < D ? *reinterpret_cast<const float2*>(from + (int64_t)col * D + d) : make_float2(0.f, 0.f);
+        }
+    };
+    float2 raw[AHEAD][4];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) ask(raw[k], k);
+    auto diagonal = [](int m) { return m * (m + 1) / 2; };
+    uint32_t most = 0;                                 // the largest magnitude among the queries, the state and the values that this thread met
+    constexpr int RUNS = DC_L * WIDE / 8 / THREADS;         // of eight values a thread
+    Eight<T> run[RUNS];
+#pragma unroll
+    for (int o = 0; o < RUNS; ++o) {
+        const int i = threadIdx.x + o * THREADS, t = i / (WIDE / 8), col = blockIdx.z * WIDE + i % (WIDE / 8) * 8;
+        run[o] = dc_values8<T>(p, t0 + min(t, count - 1), h, col, t < count ? p.Dv_in - col : 0);
+    }
     if (threadIdx.x < DC_L) G[threadIdx.x] = pg[DC_L * DC_L + threadIdx.x];
-    if (ones && threadIdx.x < DT) n[threadIdx.x] = threadIdx.x < D ? from[(int64_t)p.Dv_in * D + threadIdx.x] : 0.f;
-    for (int i = threadIdx.x; i < DC_L * 64; i += 256) {
-        const int t = i >> 6, c = i & 63;
-        VT[c * DC_P + t] = t < count && c0 + c < p.Dv_in ? dc_value<T>(p, t0 + t, h, c0 + c) : 0.f;
-    }
-    dc_wait_all();
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float o[4][4];
+    constexpr int TURNS = (4 * KS + 10 + WARPS - 1) / WARPS, HALF = (TURNS + 1) / 2;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int first = 0; first < TURNS; first += HALF) {        // (half of the operands asked for at a time)
+        DcLeft x[HALF];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
-#pragma unroll 4
-    for (int d = 0; d < DT; d += 4) {
-        float4 ss[4];
+        for (int o = 0; o < HALF; ++o) {
+            const int i = warp + (first + o) * WARPS, j = i - 4 * KS, m = j < 0 ? i / KS : j < 1 ? 0 : j < 3 ? 1 : j < 6 ? 2 : 3;
+            if (j < 0) x[o] = dc_left_rows(qp, stride, m * 16 + r0, (i % KS) * 16 + c0, count, D);
+            else if (j < 10) x[o] = dc_left_rows(pg, DC_L, m * 16 + r0, (j - diagonal(m)) * 16 + c0, DC_L, DC_L);
+        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ss[j] = *reinterpret_cast<const float4*>(S + (tx + 16 * j) * DP + d);
+        for (int o = 0; o < HALF; ++o) {
+            const int i = warp + (first + o) * WARPS;
+            if (i >= 4 * KS + 10) break;
+            uint32_t a[3][4];
+            most = max(most, max(magnitude(x[o].v), magnitude(x[o].w)));
+            split_left(a, x[o].v, x[o].w);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * DP + d);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                o[i][j] = fmaf(qq.x, ss[j].x, o[i][j]);
-                o[i][j] = fmaf(qq.y, ss[j].y, o[i][j]);
-                o[i][j] = fmaf(qq.z, ss[j].z, o[i][j]);
-                o[i][j] = fmaf(qq.w, ss[j].w, o[i][j]);
-            }
+            for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(left + i * 384 + q * 128 + lane * 4) = make_uint4(a[q][0], a[q][1], a[q][2], a[q][3]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float g = G[ty + 16 * i];
+    for (int o = 0; o < RUNS; ++o) {
+        const int i = threadIdx.x + o * THREADS;
+        float x[8];
+        dc_numbers(x, run[o], p);
+        uint8_t* at = values + tile_at<WIDE>(i / (WIDE / 8), i % (WIDE / 8));
+        uint32_t part[3][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] *= g;
+        for (int e = 0; e < 4; ++e) {
+            most = max(most, max(magnitude(x[2 * e]), magnitude(x[2 * e + 1])));
+            if (ONE) part[0][e] = nearest2(x[2 * e], x[2 * e + 1]);
+            else split3(x[2 * e], x[2 * e + 1], part[0][e], part[1][e], part[2][e]);
+        }
+#pragma unroll
+        for (int j = 0; j < PARTS; ++j) *reinterpret_cast<uint4*>(at + j * V_PLANE) = make_uint4(part[j][0], part[j][1], part[j][2], part[j][3]);
     }
-    for (int t = 0; t < DC_L; t += 4) {
-        float4 vv[4];
+    bool bad = __syncthreads_or(has_no_parts(most));
+    auto operand = [&](uint32_t (&a)[3][4], int i) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) vv[j] = *reinterpret_cast<const float4*>(VT + (tx + 16 * j) * DC_P + t);
+        for (int q = 0; q < 3; ++q) {
+            const uint4 v = *reinterpret_cast<const uint4*>(left + i * 384 + q * 128 + lane * 4);
+            a[q][0] = v.x; a[q][1] = v.y; a[q][2] = v.z; a[q][3] = v.w;
+        }
+    };
+    if (j0 < p.Dv_in) {
+        float sum[4][2][4] = {};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = ty + 16 * i;
-            if (t > r) continue;                       // (later tokens: their values, whatever they are, do not enter)
-            const float4 pp = *reinterpret_cast<const float4*>(P + r * DC_P + t);
+        for (int k = 0; k < KS; ++k) {
+            uint32_t b[3][2][2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                o[i][j] = fmaf(pp.x, vv[j].x, o[i][j]);
-                if (t + 1 <= r) o[i][j] = fmaf(pp.y, vv[j].y, o[i][j]);
-                if (t + 2 <= r) o[i][j] = fmaf(pp.z, vv[j].z, o[i][j]);
-                if (t + 3 <= r) o[i][j] = fmaf(pp.w, vv[j].w, o[i][j]);
+            for (int i = 0; i < 4; ++i) {
+                const float2 x = raw[k % AHEAD][i];
+                most = max(most, max(magnitude(x.x), magnitude(x.y)));
+                split3(x.x, x.y, b[0][i >> 1][i & 1], b[1][i >> 1][i & 1], b[2][i >> 1][i & 1]);
+            }
+            if (k + AHEAD < KS) ask(raw[k % AHEAD], k + AHEAD);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                uint32_t a[3][4];
+                operand(a, m * KS + k);
+                triple_step<2>(sum[m], a, b);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float f = G[m * 16 + r0 + 8 * i];
+#pragma unroll
+                for (int n = 0; n < 2; ++n) { sum[m][n][2 * i] *= f; sum[m][n][2 * i + 1] *= f; }
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            uint32_t b[PARTS][2][2];
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(values) + tile_at<WIDE>(k * 16 + (lane & 15), warp * 2 + (lane >> 4));
+#pragma unroll
+            for (int q = 0; q < PARTS; ++q) ldm4t(b[q][0][0], b[q][0][1], b[q][1][0], b[q][1][1], at + q * V_PLANE);
+#pragma unroll
+            for (int m = k; m < 4; ++m) {
+                uint32_t a[3][4];
+                operand(a, 4 * KS + diagonal(m) + k);
+                if constexpr (ONE) one_right_step<2>(sum[m], a, b);
+                else triple_step<2>(sum[m], a, b);
+            }
+        }
+        bad |= __any_sync(0xffffffffu, has_no_parts(most));
+        // (later tokens: their values, whatever they are, do not enter)
+        auto again = [&](int r, int col) {
+            float dot = 0.f;
+            for (int d = 0; d < D; ++d) dot = fmaf(qp[r * stride + d], from[(int64_t)col * D + d], dot);
+            dot *= pg[DC_L * DC_L + r];
+            for (int t = 0; t <= r; ++t) dot = fmaf(pg[r * DC_L + t], dc_value<T>(p, t0 + t, h, col), dot);
+            return dot;
+        };
+        if (!bad) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int r = m * 16 + r0 + 8 * i;
+                    if (r >= count) continue;
+                    float* to = p.out + ((int64_t)(t0 + r) * H + h) * p.Dv;
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int col = j0 + n * 8 + c0 + e;
+                            if (col < p.Dv_in) to[col] = sum[m][n][2 * i + e];
+                        }
+                }
+        } else {
+#pragma unroll 1
+            for (int o = lane; o < count * 16; o += 32) {
+                const int r = o >> 4, col = j0 + (o & 15);
+                if (col < p.Dv_in) p.out[((int64_t)(t0 + r) * H + h) * p.Dv + col] = again(r, col);
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = ty + 16 * i;
-        if (r >= count) continue;
-        float* to = p.out + ((int64_t)(t0 + r) * H + h) * p.Dv;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) if (c0 + tx + 16 * j < p.Dv_in) to[c0 + tx + 16 * j] = o[i][j];
-    }
-    if (ones) {                                        // n . q: four lanes a token
-        const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
-        float dot = 0.f, sum = 0.f;
-        for (int d = part; d < DT; d += 4) dot = fmaf(Q[r * DP + d], n[d], dot);
-        for (int t = part; t <= r; t += 4) sum += P[r * DC_P + t];
-        float v = fmaf(G[r], dot, sum);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if (part == 0 && r < count) p.out[((int64_t)(t0 + r) * H + h) * p.Dv + p.Dv_in] = v;
+    if (blockIdx.z == 0 && p.Dv > p.Dv_in) {           // the column fed with ones, n . q: four lanes a token
+        const float* n = from + (int64_t)p.Dv_in * D;
+        for (int first = 0; first < DC_L; first += THREADS / 4) {
+            const int r = first + (threadIdx.x >> 2), part = threadIdx.x & 3;
+            float dot = 0.f, sum = 0.f;
+            if (r < count) {
+                for (int d = part * 4; d < D; d += 16) {
+                    const float4 x = *reinterpret_cast<const float4*>(qp + r * stride + d), y = *reinterpret_cast<const float4*>(n + d);
+                    dot = fmaf(x.x, y.x, dot); dot = fmaf(x.y, y.y, dot); dot = fmaf(x.z, y.z, dot); dot = fmaf(x.w, y.w, dot);
+                }
+                for (int t = part; t <= r; t += 4) sum += pg[r * DC_L + t];
+            }
+            float v = r < count ? fmaf(pg[DC_L * DC_L + r], dot, sum) : 0.f;
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (part == 0 && r < count) p.out[((int64_t)(t0 + r) * H + h) * p.Dv + p.Dv_in] = v;
+        }
     }
 }
 
@@ -347,29 +583,41 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(states) |
          reinterpret_cast<uintptr_t>(scratch)) & 15) return MIE_ERR_BAD_ARG;
     DcParams p{q, k, v, v_stride, row_q_start, row_q_len, state_slots, num_rows, decay, tok_decay, state, states, scratch, out, H, D, Dv_in, Dv, v_act, 0, 0};
-    const int halves = Dv_in > 64 ? 2 : 1;
+    const int sms = device_sm_count();
     const int long_rows = num_rows < chunks / 2 ? num_rows : chunks / 2 > 0 ? chunks / 2 : 1;      // (each has two chunks at least)
     int rc;
-#define DC_LAUNCH(T, DT)                                                                                                                  \
-    {                                                                                                                                     \
-        const int smem_l = (2 * DC_L * (DT + 4) + DC_L * DC_P) * 4, smem_o = ((DC_L + 64) * (DT + 4) + 2 * DC_L * DC_P) * 4;              \
-        cudaError_t e = cudaFuncSetAttribute(decay_local_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l);             \
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_output_kernel<T, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_o);  \
-        if (e != cudaSuccess) return (int)e;                                                                                              \
-        for (p.h0 = 0; p.h0 < H; p.h0 += per_pass) {                                                                                      \
-            p.heads = H - p.h0 < per_pass ? H - p.h0 : per_pass;                                                                          \
-            rc = launch_kernel(decay_local_kernel<T, DT>, dim3(chunks, p.heads, halves), dim3(256), smem_l, stream, p, halves);           \
-            if (rc) return rc;                                                                                                            \
-            const int64_t quads = (int64_t)p.heads * Dv * D / 4;                                                                          \
-            rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), long_rows), dim3(128), 0, stream, p);          \
-            if (rc) return rc;                                                                                                            \
-            rc = launch_kernel(decay_output_kernel<T, DT>, dim3(chunks, p.heads, (Dv_in + 63) / 64), dim3(256), smem_o, stream, p);       \
-            if (rc) return rc;                                                                                                            \
-        }                                                                                                                                 \
-        return 0;                                                                                                                         \
+#define DC_OUTPUT(T, DT, ONE, WARPS)                                                                                                                      \
+    {                                                                                                                                                     \
+        auto kernel = decay_output_kernel<T, DT, ONE, WARPS>;                                                                                             \
+        constexpr int bytes = output_bytes<DT, ONE, WARPS>();                                                                                             \
+        const cudaError_t f = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);                                            \
+        rc = f != cudaSuccess ? (int)f                                                                                                                    \
+                              : launch_kernel(kernel, dim3(chunks, p.heads, (Dv_in + 16 * WARPS - 1) / (16 * WARPS)), dim3(32 * WARPS), bytes, stream, p); \
     }
-    if (v_tag == MIE_F32) { if (D <= 64) DC_LAUNCH(float, 64) else DC_LAUNCH(float, 128) }
-    if (v_tag == MIE_BF16) { if (D <= 64) DC_LAUNCH(bf16, 64) else DC_LAUNCH(bf16, 128) }
+#define DC_LAUNCH(T, DT, ONE)                                                                                                                             \
+    {                                                                                                                                                     \
+        const int smem_l = 3 * DC_L * DT * 2 + 2 * (ONE ? 1 : 3) * DC_L * DC_COLS * 2 + DC_L * DC_P * 4;                                                   \
+        const cudaError_t e = cudaFuncSetAttribute(decay_local_kernel<T, DT, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l);                   \
+        if (e != cudaSuccess) return (int)e;                                                                                                              \
+        for (p.h0 = 0; p.h0 < H; p.h0 += per_pass) {                                                                                                      \
+            p.heads = H - p.h0 < per_pass ? H - p.h0 : per_pass;                                                                                          \
+            /* a step of few chunks: the value columns in as many shares as the SMs have room for */                                                      \
+            const int items = chunks * p.heads, room = items < sms ? sms / items : 1, tiles = (Dv_in + DC_COLS - 1) / DC_COLS;                             \
+            const int splits = room < tiles ? room : tiles;                                                                                               \
+            rc = launch_kernel(decay_local_kernel<T, DT, ONE>, dim3(chunks, p.heads, splits), dim3(DC_THREADS), smem_l, stream, p, splits);                \
+            if (rc) return rc;                                                                                                                            \
+            const int64_t quads = (int64_t)p.heads * Dv * D / 4;                                                                                          \
+            rc = launch_kernel(decay_combine_kernel, dim3((unsigned)((quads + 127) / 128), long_rows), dim3(128), 0, stream, p);                          \
+            if (rc) return rc;                                                                                                                            \
+            if (items * ((Dv_in + 127) / 128) > sms / 2) DC_OUTPUT(T, DT, ONE, 8) else DC_OUTPUT(T, DT, ONE, 4)                                            \
+            if (rc) return rc;                                                                                                                            \
+        }                                                                                                                                                 \
+        return 0;                                                                                                                                         \
+    }
+    if (v_tag == MIE_F32) { if (D <= 64) DC_LAUNCH(float, 64, false) else DC_LAUNCH(float, 128, false) }
+    if (v_tag == MIE_BF16 && v_act) { if (D <= 64) DC_LAUNCH(bf16, 64, false) else DC_LAUNCH(bf16, 128, false) }
+    if (v_tag == MIE_BF16) { if (D <= 64) DC_LAUNCH(bf16, 64, true) else DC_LAUNCH(bf16, 128, true) }
 #undef DC_LAUNCH
+#undef DC_OUTPUT
     return MIE_ERR_BAD_ARG;
 }

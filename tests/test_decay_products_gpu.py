@@ -1,0 +1,80 @@
+"""The chunked decay recurrence's products as bfloat16 parts: shares of the value columns and narrow blocks of few chunks, whole blocks of many, values that are one part or
+three, values without parts, and how far the results are from 64 bits."""
+import pytest
+import torch
+
+from test_decay_chunks_gpu import close, scan
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,H", [([66], 1), ([128, 70], 3), ([640], 8), ([1000, 900], 6), ([2000], 12)])
+@pytest.mark.parametrize("D,V", [(128, 300), (64, 64), (96, 129), (32, 5)])
+def test_shares_and_blocks_of_every_size(monkeypatch, dt, rows, H, D, V):
+    how = dict(per_token=True, ones=V % 2 == 1, act=dt == torch.bfloat16 and D == 96, seed=D + V + H)
+    close(scan(monkeypatch, True, rows, H, D, V, dt, **how), scan(monkeypatch, False, rows, H, D, V, dt, **how))
+
+
+def run(qkv, tok, k_tok, state, rows, H, D, V):
+    from mini_inference_engine_b200.kernels import ops
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    T = sum(rows)
+    state, out = state.clone(), torch.zeros(T, H * V, device="cuda")
+    ops.decay_scan(qkv, i32([0] * T), i32([sum(rows[:i]) for i in range(len(rows))]), i32(rows), i32([i + 1 for i in range(len(rows))]), state, out, num_heads=H, dim=D, vdim=V,
+                   max_q_len=max(rows), tok_decay=tok, k_tok=k_tok, q_scale=0.125, q_lens=rows)
+    torch.cuda.synchronize()
+    return out.view(T, H, V), state
+
+
+def operands(rows, H, D, V, dt, least, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T = sum(rows)
+    qkv = torch.randn(T, H * (2 * D + V), generator=g, device="cuda").to(dt)
+    tok = least + (1 - least) * torch.rand(T, H, generator=g, device="cuda")
+    return qkv, tok, torch.rand(T, H, generator=g, device="cuda"), torch.randn(len(rows) + 1, H, V, D, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("least", [0.97, 0.5, 0.0])
+def test_as_far_from_64_bits_as_token_by_token(monkeypatch, dt, least):
+    from mini_inference_engine_b200.kernels import ops
+    rows, H, D, V = [200, 130], 2, 128, 80
+    qkv, tok, k_tok, state = operands(rows, H, D, V, dt, least)
+    got = run(qkv, tok, k_tok, state, rows, H, D, V)
+    monkeypatch.setattr(ops, "decay_chunks_take", lambda d: False)
+    ref = run(qkv, tok, k_tok, state, rows, H, D, V)
+    x = qkv.double()
+    q, k, v = x[:, :H * D].view(-1, H, D) * 0.125, x[:, H * D:2 * H * D].view(-1, H, D) * k_tok.double()[:, :, None], x[:, 2 * H * D:].view(-1, H, V)
+    out, end, at = torch.zeros_like(v), state.double().clone(), 0
+    for r, n in enumerate(rows):
+        S = end[r + 1].clone()
+        for t in range(at, at + n):
+            S = tok[t].double()[:, None, None] * S + v[t][:, :, None] * k[t][:, None, :]
+            out[t] = (S * q[t][:, None, :]).sum(-1)
+        end[r + 1] = S
+        at += n
+    for a, b, w in zip(got, ref, (out, end)):
+        off = lambda t: ((t.double() - w).norm() / w.norm()).item()
+        assert off(a) <= 1.5 * off(b) + 2.0 ** -25
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["value", "key", "query"])
+def test_numbers_without_three_parts(monkeypatch, dt, what):
+    """Beyond 2^127 and still finite: as the token-by-token kernel has them, token for token."""
+    from mini_inference_engine_b200.kernels import ops
+    rows, H, D, V = [150], 2, 32, 40
+    qkv, tok, k_tok, state = operands(rows, H, D, V, dt, 0.9)
+    qkv *= 1e-3
+    col = dict(query=3, key=H * D + 3, value=2 * H * D + 3)[what]
+    qkv[70, col] = 3e38
+    got = run(qkv, tok, k_tok, state, rows, H, D, V)
+    monkeypatch.setattr(ops, "decay_chunks_take", lambda d: False)
+    ref = run(qkv, tok, k_tok, state, rows, H, D, V)
+    for a, b in zip(got, ref):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.isfinite(a[:70]).all()
+        ok = torch.isfinite(b)
+        assert ((a - b).abs()[ok] <= 1.5e-5 * b[ok].abs().max()).all()
+        quiet = ok & (b.abs() < 1e30)                          # what the large number does not reach keeps its digits
+        assert ((a - b).abs()[quiet] <= 1.5e-5 * b[quiet].abs().max()).all()
