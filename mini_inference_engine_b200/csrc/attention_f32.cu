@@ -1,19 +1,25 @@
 // Paged causal attention of prompt portions in float32 (the true 32-bit path): rows with many new tokens; csrc/attention_simt.cu serves the
-// others, and every row in bfloat16.  The same rules: masks, kept first keys, score modifiers, sink, range checks; float32 fused multiply-adds throughout.
+// others, and every row in bfloat16.  The same rules: masks, kept first keys, score modifiers, sink, range checks.  Scores and outputs are products on the tensor cores
+// with every operand as three bfloat16 parts (triple_mma.cuh); weights, sums and everything else are float32.
 //
-// A block owns 64 (token, query head) pairs that share a key head -- tokens of one row, the group's heads side by side -- so a tile of
-// 64 keys and values in shared memory serves all heads of the group.  A thread holds 8 (or 4) pairs x 4 keys of the scores and
-// the same pairs x 4 (or 8) entries of the output, where a warp that owns one pair reads its keys and values once per pair.  The next tile's keys arrive
-// (cp.async) under the product with the values, the next values under the scores.  Tiles of a row go longest first.  Bound: latencies at three warps a
-// scheduler -- 640 tokens of 32 heads of 64 (156 us under the profiler): a scheduler has an instruction to issue in 45 % of the cycles, the multiply-add pipe is at 32 %
-// of its peak, L1 and shared memory at 30 %.  A layer of TinyLlama's sizes over 1,000 tokens of two requests, products included: 958 us with the other kernel -> 318 us.
-#include "common.cuh"
+// A block owns 16 (token, query head) pairs a warp that share a key head -- tokens of one row, the group's heads side by side -- so a tile of
+// 64 keys and values in shared memory serves all heads of the group.  Queries, keys and values lie there as parts, split by the threads that fetched them; the scores of a
+// warp's pairs become the left operand of the product with the values where they are.  A walk of keys may be shared out over the blocks of a cluster, every n-th tile a block;
+// their sums meet in shared memory.  The next tile's keys arrive (cp.async) under the product with the
+// values, the values under the scores.  Tiles of a row go longest first, over all heads.
+//
+// A tile with keys or values that have no three parts (not finite, or beyond 2^127) is multiplied number by number, and a weight that does not exist then meets no value.
+//
+// Bound: the tensor pipe while a tile's products run (8.2 cycles an instruction with four warps a scheduler, 8 its rate), about 60 % of the time; the rest are the softmax, the
+// splitting and the blocks' ends.  Kernel, us: 333 tokens on 300 positions beside 667, 32 heads of 64: 177 (register tiles on the CUDA cores) -> 94; 1,024 tokens 128; a layer of
+// TinyLlama's sizes over both rows, products included, 314 -> 230; 200 tokens on 800 positions 320 -> 120.  Against 64 bits the layer is 2.7e-7 off (2-norm), 3.6e-7 before.
+#include <algorithm>
+
 #include "range_check.cuh"
+#include "triple_mma.cuh"
 
 #define MIE_K_ATTENTION_F32 14     // this kernel's number in the range report (csrc/range_check.cuh)
-#define F32_PAIRS 64
 #define F32_KEYS 64
-#define F32_PS 80                 // stride of a row of probabilities: neighbouring rows 16 banks apart
 
 struct F32Params {
     const float* q; int64_t q_stride; const float* k_cache; const float* v_cache;
@@ -27,213 +33,322 @@ __device__ __forceinline__ void f32_copy16(float* dst, const float* src, bool on
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
 
-template <bool B> struct Bool { static constexpr bool value = B; };
+__device__ __noinline__ float f32_dot(const float* q, const float* k, int D, float scale) {
+    float sum = 0.f;
+    for (int d = 0; d < D; ++d) sum = fmaf(q[d] * scale, k[d], sum);
+    return sum;
+}
 
-// DT: entries of a head as the block holds them (head_dim padded with zeros); THREADS 128 or 256; the probabilities take the keys' memory
-// where SHARE (two blocks on an SM at DT 128).
-template <int DT, int THREADS, bool SHARE>
-__global__ void __launch_bounds__(THREADS, DT == 64 ? 3 : 2) f32_attention_kernel(const F32Params p) {
-    constexpr int TY = THREADS / 16, RI = F32_PAIRS / TY, QS = DT + 4, KS = DT + 4, CG = DT / 64;
-    extern __shared__ __align__(16) float sm[];
-    float* Q = sm;                                    // [64][QS]
-    float* K = Q + F32_PAIRS * QS;                    // [64][KS]
-    float* V = K + F32_KEYS * KS;                     // [64][DT]
-    float* P = SHARE ? K : V + F32_KEYS * DT;         // [64][F32_PS]
-    __shared__ int s_row, s_tile;
-    const int D = p.head_dim, G = p.num_heads / p.num_kv_heads, kvh = blockIdx.y;
+// DT: entries of a head as the block holds them (head_dim padded with zeros); WARPS of 16 pairs each.
+template <int DT, int WARPS> constexpr int f32_bytes() { return 3 * 16 * WARPS * DT * 2 + 3 * F32_KEYS * DT * 2 + F32_KEYS * DT * 4; }
+template <int DT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2) f32_attention_kernel(const F32Params p, int splits) {
+    constexpr int GROUP = WARPS == 4 ? 4 : 2;         // column tiles at a time: as many as the registers have room for
+    constexpr int THREADS = 32 * WARPS, PAIRS = 16 * WARPS, Q_PLANE = PAIRS * DT * 2, K_PLANE = F32_KEYS * DT * 2, KS = DT / 16, NT = DT / 8;
+    constexpr int QUADS = F32_KEYS * DT / 4 / THREADS, STEP = THREADS / (DT / 4);
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint8_t* Q = smem;                                // [PAIRS][DT] as parts
+    uint8_t* KV = Q + 3 * Q_PLANE;                    // keys, then values [64][DT]; then weights [16][64] a warp where a tile is multiplied number by number
+    float* raw = reinterpret_cast<float*>(KV + 3 * K_PLANE);       // keys or values on their way [64][DT]: a thread splits what it fetched
+    __shared__ int s_row, s_tile, s_page[2][F32_KEYS];             // the pages of a tile's keys (-1: a key that nobody reads), the next tile's besides
+    const int share = blockIdx.x % splits, item = blockIdx.x / splits;
+    const int D = p.head_dim, G = p.num_heads / p.num_kv_heads, kvh = item % p.num_kv_heads;
     pdl_launch_dependents();
     if (threadIdx.x < 32) {
         int within, items;
-        const int found = warp_find_row(p.row_q_len, p.num_rows, (int)blockIdx.x,
-                                        [&](int n) { return n >= p.min_q_len ? (n * G + F32_PAIRS - 1) / F32_PAIRS : 0; }, within, items);
+        const int found = warp_find_row(p.row_q_len, p.num_rows, item / p.num_kv_heads,
+                                        [&](int n) { return n >= p.min_q_len ? (n * G + PAIRS - 1) / PAIRS : 0; }, within, items);
         if (threadIdx.x == 0) { s_row = found; s_tile = items - 1 - within; }
     }
     __syncthreads();
     const int r = s_row;
     pdl_wait();                                       // (a block without work waits too: see common.cuh)
     if (r < 0) return;
-    const int q_len = p.row_q_len[r], ctx_len = p.row_ctx_len[r], q_start = p.row_q_start[r], pair0 = s_tile * F32_PAIRS;
+    const int q_len = p.row_q_len[r], ctx_len = p.row_ctx_len[r], q_start = p.row_q_start[r], pair0 = s_tile * PAIRS;
     if (ctx_len > p.table_stride * p.page_size) {
         if (threadIdx.x == 0) range_report(p.report, MIE_RANGE_POSITION, MIE_K_ATTENTION_F32, r, ctx_len);
         return;
     }
-    const int lane = threadIdx.x & 31, tx = lane & 15, ty = (threadIdx.x >> 5) * 2 + (lane >> 4);
-    const int pairs = q_len * G, last = min(pair0 + F32_PAIRS, pairs) - 1, base_pos = ctx_len - q_len;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = lane >> 2, c0 = (lane & 3) * 2;
+    const int pairs = q_len * G, last = min(pair0 + PAIRS, pairs) - 1, base_pos = ctx_len - q_len;
     const int first_pos = base_pos + pair0 / G, last_pos = base_pos + last / G;
     const int k_hi = last_pos + 1, k_lo = mask_first_key(first_pos, p.window);
-
-    for (int i = threadIdx.x; i < F32_PAIRS * (DT / 4); i += THREADS) {
-        const int pr = i / (DT / 4), d = (i - pr * (DT / 4)) * 4, at = pair0 + pr;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (at < pairs && d < D) {
-            const int token = q_start + at / G, head = kvh * G + at % G;
-            const float* src = p.q + (int64_t)token * p.q_stride + (int64_t)head * D + d;
-            v = make_float4(src[0] * p.scale, src[1] * p.scale, src[2] * p.scale, src[3] * p.scale);
-        }
-        *reinterpret_cast<float4*>(Q + pr * QS + d) = v;
-    }
-    int pos[RI], head[RI];
-    float m[RI], l[RI], o[RI][4 * CG];
-#pragma unroll
-    for (int i = 0; i < RI; ++i) {
-        const int at = pair0 + ty + TY * i;
-        pos[i] = at < pairs ? base_pos + at / G : -1;              // (a pair that does not exist reads no key)
-        head[i] = kvh * G + at % G;
-        m[i] = -INFINITY;
-        l[i] = 0.f;
-        if (p.mods.sink && at < pairs) { m[i] = p.mods.sink[head[i]]; l[i] = tx == 0 ? 1.f : 0.f; }
-#pragma unroll
-        for (int c = 0; c < 4 * CG; ++c) o[i][c] = 0.f;
-    }
     const int* table = p.block_tables + (int64_t)r * p.table_stride;
     const int kbeg = k_lo & ~(F32_KEYS - 1), kept = mask_kept_tiles(p.keep, kbeg, F32_KEYS);
     const int tiles = kept + (k_hi - kbeg + F32_KEYS - 1) / F32_KEYS;
     auto tile_key = [&](int t) { return t < kept ? t * F32_KEYS : kbeg + (t - kept) * F32_KEYS; };
-    auto issue = [&](const float* cache, float* dst, int stride, int t) {
+    auto in_reach = [&](int key) { return (key >= k_lo || key < p.keep) && key < k_hi; };
+    auto row_in = [&](const float* cache, int page, int key) { return cache + (((int64_t)page * p.num_kv_heads + kvh) * p.page_size + (key & (p.page_size - 1))) * D; };
+    auto page_of = [&](int t) {                       // of this thread's key of a tile
+        const int key = tile_key(t) + (int)threadIdx.x;
+        return t < tiles && threadIdx.x < F32_KEYS && in_reach(key) ? checked_page(table[key >> p.page_shift], p.num_pages, p.report, MIE_K_ATTENTION_F32, key >> p.page_shift) : -1;
+    };
+    const int my_d = (threadIdx.x % (DT / 4)) * 4, my_row = threadIdx.x / (DT / 4);
+    auto issue = [&](const float* cache, int t) {
         if (t < tiles) {
             const int k0 = tile_key(t);
-#pragma unroll 4
-            for (int i = threadIdx.x; i < F32_KEYS * (DT / 4); i += THREADS) {
-                const int jj = i / (DT / 4), d = (i - jj * (DT / 4)) * 4, key = k0 + jj;
-                const bool on = (key >= k_lo || key < p.keep) && key < k_hi && d < D;
-                const float* src = cache;
-                if (on) {
-                    const int page = checked_page(table[key >> p.page_shift], p.num_pages, p.report, MIE_K_ATTENTION_F32, key >> p.page_shift);
-                    src = cache + (((int64_t)page * p.num_kv_heads + kvh) * p.page_size + (key & (p.page_size - 1))) * D + d;
-                }
-                f32_copy16(dst + jj * stride + d, src, on);
+#pragma unroll
+            for (int i = 0; i < QUADS; ++i) {
+                const int jj = my_row + i * STEP, page = s_page[(t / splits) & 1][jj];
+                const bool on = page >= 0 && my_d < D;
+                f32_copy16(raw + jj * DT + my_d, on ? row_in(cache, page, k0 + jj) + my_d : cache, on);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");       // every thread one group, also an empty one
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    const bool plain = !(p.mods.softcap > 0.f) && !p.mods.dist_bias && !p.mods.slope;
-    issue(p.k_cache, K, KS, 0);
-    issue(p.v_cache, V, DT, 0);
-    for (int t = 0; t < tiles; ++t) {
-        const int k0 = tile_key(t);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");       // this tile's keys (its values may still be on the way)
+    auto put = [&](uint8_t* tile, int plane, int row, int d, float4 v) {
+        uint2 part[3];
+        split3(v.x, v.y, part[0].x, part[1].x, part[2].x);
+        split3(v.z, v.w, part[0].y, part[1].y, part[2].y);
+        uint8_t* at = tile + tile_at<DT>(row, d >> 3) + (d & 4) * 2;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(at + j * plane) = part[j];
+        return magnitude(v);
+    };
+    auto split = [&]() {                              // what this thread fetched, once every warp is done with what lay there; whether a number of the block's has no parts
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        float s[RI][4];
+        uint32_t most = 0;
 #pragma unroll
-        for (int i = 0; i < RI; ++i)
+        for (int i = 0; i < QUADS; ++i) {
+            const int jj = my_row + i * STEP;
+            most = max(most, put(KV, K_PLANE, jj, my_d, *reinterpret_cast<const float4*>(raw + jj * DT + my_d)));
+        }
+        return __syncthreads_or(has_no_parts(most)) != 0;
+    };
+    if (threadIdx.x < F32_KEYS) s_page[0][threadIdx.x] = page_of(share);
+    __syncthreads();
+    issue(p.k_cache, share);
+    uint32_t q_most = 0;
+    {
+        constexpr int TURNS = PAIRS * (DT / 4) / THREADS;
+        float4 v[TURNS];                              // (all asked for before the first is split)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 2
-        for (int d = 0; d < DT; d += 4) {
-            float4 kk[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * KS + d);
-#pragma unroll
-            for (int i = 0; i < RI; ++i) {
-                const float4 qq = *reinterpret_cast<const float4*>(Q + (ty + TY * i) * QS + d);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[i][j] = fmaf(qq.x, kk[j].x, s[i][j]);
-                    s[i][j] = fmaf(qq.y, kk[j].y, s[i][j]);
-                    s[i][j] = fmaf(qq.z, kk[j].z, s[i][j]);
-                    s[i][j] = fmaf(qq.w, kk[j].w, s[i][j]);
-                }
+        for (int i = 0; i < TURNS; ++i) {
+            const int at = pair0 + my_row + i * STEP, token = at / G, head = kvh * G + at - token * G;
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (at < pairs && my_d < D) {
+                const float* src = p.q + (int64_t)(q_start + token) * p.q_stride + (int64_t)head * D + my_d;
+                v[i] = make_float4(src[0], src[1], src[2], src[3]);
             }
         }
-        if constexpr (SHARE) __syncthreads();                      // the keys are done with: their memory takes the probabilities
+#pragma unroll
+        for (int i = 0; i < TURNS; ++i)
+            q_most = max(q_most, put(Q, Q_PLANE, my_row + i * STEP, my_d, make_float4(v[i].x * p.scale, v[i].y * p.scale, v[i].z * p.scale, v[i].w * p.scale)));
+    }
+    // this lane's pairs: r0 and r0 + 8 of the warp's sixteen
+    int pos[2], head[2], from[2];                     // (and the first position that each reads beside the kept ones)
+    float m[2], l[2], o[NT][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int at = pair0 + warp * 16 + r0 + 8 * i;
+        pos[i] = at < pairs ? base_pos + at / G : -1;              // (a pair that does not exist reads no key)
+        head[i] = kvh * G + at % G;
+        from[i] = mask_first_key(max(pos[i], 0), p.window);
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+        if (p.mods.sink && at < pairs && share == 0) { m[i] = p.mods.sink[head[i]]; l[i] = c0 == 0 ? 1.f : 0.f; }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
+    const bool plain = !(p.mods.softcap > 0.f) && !p.mods.dist_bias && !p.mods.slope, q_bad = has_no_parts(q_most);
+    const bool block_q_bad = __syncthreads_or(q_bad) != 0;
+    const uint32_t q_at = (uint32_t)__cvta_generic_to_shared(Q), kv_at = (uint32_t)__cvta_generic_to_shared(KV);
+    for (int t = share; t < tiles; t += splits) {
+        const int k0 = tile_key(t);
+        const int next_page = page_of(t + splits);
+        const int* pages = s_page[(t / splits) & 1];
+        const bool k_bad = split() || block_q_bad;
+        issue(p.v_cache, t);
+        float s[8][4];
         // a tile that every pair sees whole needs no mask: all keys at or before the first pair's position, none before the last one's first key
-        const bool whole = k0 + F32_KEYS - 1 <= first_pos && k0 >= mask_first_key(last_pos, p.window) && last - pair0 == F32_PAIRS - 1;
+        const bool whole = k0 + F32_KEYS - 1 <= first_pos && k0 >= mask_first_key(last_pos, p.window) && last - pair0 == PAIRS - 1;
 #pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            float top = -INFINITY;
-            int unseen = 0;
+        for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int key = k0 + tx + 16 * j;
-                if (!plain) s[i][j] = mod_score(s[i][j], p.mods, head[i], p.num_heads, pos[i] - key);
-                if (!whole && !mask_reads(pos[i], key, p.window, p.keep)) { s[i][j] = -INFINITY; unseen |= 1 << j; }
-                top = fmaxf(top, s[i][j]);
+            for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
+        if (!k_bad) {
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+                uint32_t a[3][4];
+                left_rows<DT>(a, q_at, Q_PLANE, warp, k, lane);
+#pragma unroll
+                for (int n = 0; n < 8; n += GROUP) {
+                    uint32_t b[3][GROUP][2];
+#pragma unroll
+                    for (int j = 0; j < GROUP; j += 2) right_columns<DT>(b, j, kv_at, K_PLANE, k, n + j, lane);
+                    triple_step<GROUP>(s + n, a, b);
+                }
             }
+        } else {
 #pragma unroll
-            for (int w = 8; w > 0; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
-            const float m_new = fmaxf(m[i], top);
-            const bool any = m_new > -INFINITY;                    // else every key so far is masked for this pair
-            const float alpha = any ? expf(m[i] - m_new) : 1.f;
+            for (int i = 0; i < 2; ++i) {
+                const float* q = p.q + (int64_t)(q_start + max(pos[i] - base_pos, 0)) * p.q_stride + (int64_t)head[i] * D;
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int key = k0 + n * 8 + c0 + e;
+                        s[n][2 * i + e] = pos[i] >= 0 && pages[key - k0] >= 0 ? f32_dot(q, row_in(p.k_cache, pages[key - k0], key), D, p.scale) : 0.f;
+                    }
+            }
+        }
+        uint32_t unseen = 0;                                       // a bit a score, of keys out of sight
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (!plain)
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) s[n][2 * i + e] = mod_score(s[n][2 * i + e], p.mods, head[i], p.num_heads, pos[i] - (k0 + n * 8 + c0 + e));
+            if (!whole)
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int key = k0 + n * 8 + c0 + e;
+                        if (key > pos[i] || (key < from[i] && key >= p.keep)) { s[n][2 * i + e] = -INFINITY; unseen |= 1u << (4 * n + 2 * i + e); }
+                    }
+            float top = fmaxf(s[0][2 * i], s[0][2 * i + 1]);
+#pragma unroll
+            for (int n = 1; n < 8; ++n) top = fmaxf(top, fmaxf(s[n][2 * i], s[n][2 * i + 1]));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const float m_new = fmaxf(m[i], top), base = m_new > -INFINITY ? m_new : 0.f;
+            if (!(m_new > -INFINITY))                              // every key so far is masked for this pair, or its score no number: no weights
+#pragma unroll
+                for (int n = 0; n < 8; ++n) s[n][2 * i] = s[n][2 * i + 1] = -INFINITY;
+            const float alpha = expf(m[i] - base);
             float sum = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float e = any ? expf(s[i][j] - m_new) : 0.f;
-                sum += e;
-                P[(ty + TY * i) * F32_PS + tx + 16 * j] = (unseen >> j) & 1 ? -1.f : e;
-            }
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float x = expf(s[n][2 * i + e] - base);
+                    sum += x;
+                    s[n][2 * i + e] = x;
+                }
             l[i] = l[i] * alpha + sum;
             m[i] = m_new;
 #pragma unroll
-            for (int c = 0; c < 4 * CG; ++c) o[i][c] *= alpha;
+            for (int n = 0; n < NT; ++n) { o[n][2 * i] *= alpha; o[n][2 * i + 1] *= alpha; }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");       // the values
-        __syncthreads();
-        if constexpr (!SHARE) issue(p.k_cache, K, KS, t + 1);
-        auto add_values = [&](auto masked) {
-#pragma unroll 2
-        for (int kk = 0; kk < F32_KEYS; kk += 4) {
-            float4 pp[RI];
+        if (threadIdx.x < F32_KEYS) s_page[(t / splits + 1) & 1][threadIdx.x] = next_page;
+        const bool v_bad = split();
+        issue(p.k_cache, t + splits);
+        if (!v_bad) {
 #pragma unroll
-            for (int i = 0; i < RI; ++i) pp[i] = *reinterpret_cast<const float4*>(P + (ty + TY * i) * F32_PS + kk);
+            for (int k = 0; k < 4; ++k) {
+                uint32_t a[3][4];
 #pragma unroll
-            for (int c = 0; c < CG; ++c) {
-                float4 v[4];
+                for (int i = 0; i < 4; ++i) split3(s[2 * k + (i >> 1)][2 * (i & 1)], s[2 * k + (i >> 1)][2 * (i & 1) + 1], a[0][i], a[1][i], a[2][i]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const float4*>(V + (kk + e) * DT + 64 * c + 4 * tx);
+                for (int n = 0; n < NT; n += GROUP) {
+                    uint32_t b[3][GROUP][2];
 #pragma unroll
-                for (int i = 0; i < RI; ++i) {
-                    float* oo = o[i] + 4 * c;
-                    const float pe[4] = {pp[i].x, pp[i].y, pp[i].z, pp[i].w};
+                    for (int j = 0; j < GROUP; j += 2) right_rows<DT>(b, j, kv_at, K_PLANE, k, n + j, lane);
+                    triple_step<GROUP>(o + n, a, b);
+                }
+            }
+        } else {
+            float* P = reinterpret_cast<float*>(KV) + warp * 16 * F32_KEYS;        // (the values' parts are not read)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (decltype(masked)::value && pe[e] < 0.f) continue;         // a key out of sight: its value may be anything
-                        oo[0] = fmaf(pe[e], v[e].x, oo[0]);
-                        oo[1] = fmaf(pe[e], v[e].y, oo[1]);
-                        oo[2] = fmaf(pe[e], v[e].z, oo[2]);
-                        oo[3] = fmaf(pe[e], v[e].w, oo[3]);
-                    }
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) P[(r0 + 8 * (i >> 1)) * F32_KEYS + n * 8 + c0 + (i & 1)] = (unseen >> (4 * n + i)) & 1 ? -1.f : s[n][i];
+            __syncwarp();
+#pragma unroll 1
+            for (int j = 0; j < F32_KEYS; ++j) {
+                const int key = k0 + j;
+                if (pages[j] < 0) continue;
+                const float* v = row_in(p.v_cache, pages[j], key);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float w = P[(r0 + 8 * i) * F32_KEYS + j];
+                    if (w < 0.f) continue;                         // a key out of sight: its value may be anything
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            if (n * 8 + c0 + e < D) o[n][2 * i + e] = fmaf(w, v[n * 8 + c0 + e], o[n][2 * i + e]);
                 }
             }
         }
-        };
-        if (whole) add_values(Bool<false>{});
-        else add_values(Bool<true>{});
-        __syncthreads();
-        if constexpr (SHARE) issue(p.k_cache, K, KS, t + 1);
-        issue(p.v_cache, V, DT, t + 1);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < RI; ++i) {
-        float sum = l[i];
+    for (int i = 0; i < 2; ++i) {
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+    }
+    if (splits == 1) {
 #pragma unroll
-        for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
-        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
-        if (pos[i] < 0) continue;
-        float* op = p.out + ((int64_t)(q_start + pos[i] - base_pos) * p.num_heads + head[i]) * D;
+        for (int i = 0; i < 2; ++i) {
+            if (pos[i] < 0) continue;
+            const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+            float* op = p.out + ((int64_t)(q_start + pos[i] - base_pos) * p.num_heads + head[i]) * D;
 #pragma unroll
-        for (int c = 0; c < CG; ++c) {
-            const int d = 64 * c + 4 * tx;
-            if (d < D) *reinterpret_cast<float4*>(op + d) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+            for (int n = 0; n < NT; ++n) {
+                const int d = n * 8 + c0;
+                if (d < D) *reinterpret_cast<float2*>(op + d) = make_float2(o[n][2 * i] * inv, o[n][2 * i + 1] * inv);
+            }
         }
+        return;
     }
+    // the shares of the keys meet: every block of the cluster adds up its part of the pairs
+    constexpr int OS = DT + 4;
+    float* sums = reinterpret_cast<float*>(smem);     // [PAIRS][OS], then the largest scores and the weights' sums
+    float *tops = sums + PAIRS * OS, *weights = tops + PAIRS;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = warp * 16 + r0 + 8 * i;
+        if (c0 == 0) { tops[row] = m[i]; weights[row] = l[i]; }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) *reinterpret_cast<float2*>(sums + row * OS + n * 8 + c0) = make_float2(o[n][2 * i], o[n][2 * i + 1]);
+    }
+    cluster_sync_all();
+    const uint32_t at0 = (uint32_t)__cvta_generic_to_shared(sums), top0 = (uint32_t)__cvta_generic_to_shared(tops), weight0 = (uint32_t)__cvta_generic_to_shared(weights);
+    const int mine = PAIRS / splits;
+    for (int i = threadIdx.x; i < mine * (DT / 4); i += THREADS) {
+        const int row = share * mine + i / (DT / 4), d = (i % (DT / 4)) * 4, at = pair0 + row;
+        if (at >= pairs || d >= D) continue;
+        float top = -INFINITY;
+        for (int j = 0; j < splits; ++j) top = fmaxf(top, ld_cluster_f32(cluster_addr(top0 + row * 4, j)));
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        float weight = 0.f;
+        for (int j = 0; j < splits; ++j) {
+            const float m_j = ld_cluster_f32(cluster_addr(top0 + row * 4, j)), f = m_j > -INFINITY ? expf(m_j - top) : 0.f;
+            const float4 x = ld_cluster_f32x4(cluster_addr(at0 + (row * OS + d) * 4, j));
+            weight = fmaf(f, ld_cluster_f32(cluster_addr(weight0 + row * 4, j)), weight);
+            sum.x = fmaf(f, x.x, sum.x); sum.y = fmaf(f, x.y, sum.y); sum.z = fmaf(f, x.z, sum.z); sum.w = fmaf(f, x.w, sum.w);
+        }
+        const float inv = weight > 0.f ? 1.0f / weight : 0.f;
+        const int token = at / G;
+        *reinterpret_cast<float4*>(p.out + ((int64_t)(q_start + token) * p.num_heads + kvh * G + at - token * G) * D + d) = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv);
+    }
+    cluster_sync_all();                               // (the others may still read this block's memory)
 }
 
-template <int DT, int THREADS, bool SHARE>
-static int f32_launch(const F32Params& p, dim3 grid, cudaStream_t stream) {
-    const int smem = (F32_PAIRS * (DT + 4) + F32_KEYS * (DT + 4) + F32_KEYS * DT + (SHARE ? 0 : F32_PAIRS * F32_PS)) * (int)sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(f32_attention_kernel<DT, THREADS, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+template <int DT, int WARPS>
+static int f32_launch(const F32Params& p, int64_t pairs, int rows, int splits, cudaStream_t stream) {
+    const int64_t blocks = (pairs / (16 * WARPS) + rows) * p.num_kv_heads;          // (every row's last tile may be partly filled)
+    if (blocks * splits > 0x7fffffff) return MIE_ERR_TOO_LARGE;
+    const cudaError_t e = cudaFuncSetAttribute(f32_attention_kernel<DT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_bytes<DT, WARPS>());
     if (e != cudaSuccess) return (int)e;
-    return launch_kernel(f32_attention_kernel<DT, THREADS, SHARE>, grid, dim3(THREADS), smem, stream, p);
+    return launch_kernel_cluster(f32_attention_kernel<DT, WARPS>, dim3((unsigned)(blocks * splits)), dim3(32 * WARPS), f32_bytes<DT, WARPS>(), stream, dim3(splits, 1, 1), p, splits);
 }
 
-// Rows with fewer than `min_q_len` new tokens are left alone; `tiles`: an upper bound of the 64-pair tiles of the others.  Heads of 16 .. 128 in steps
-// of 16, caches and out 16-byte aligned; the rest as mie_paged_attention.
+// Rows with fewer than `min_q_len` new tokens are left alone; `max_ctx`: no row has more positions (it only shapes the launch); `rows`, `pairs`: upper bounds of the others' number and of their (token, head of a group) pairs.  Heads of
+// 16 .. 128 in steps of 16, caches and out 16-byte aligned; the rest as mie_paged_attention.
 extern "C" int mie_attention_f32(const float* q, int64_t q_stride, const float* k_cache, const float* v_cache, const int* block_tables, int table_stride,
-                                 const int* row_q_start, const int* row_q_len, const int* row_ctx_len, int num_rows, int tiles, float* out,
-                                 int num_heads, int num_kv_heads, int head_dim, int page_size, float scale, int window, int keep, int min_q_len,
+                                 const int* row_q_start, const int* row_q_len, const int* row_ctx_len, int num_rows, int rows, long long pairs, float* out,
+                                 int num_heads, int num_kv_heads, int head_dim, int page_size, float scale, int window, int keep, int min_q_len, int max_ctx,
                                  long long num_pages, float softcap, const float* sink, const float* dist_bias, int dist_len, const float* slope,
                                  cudaStream_t stream) {
-    if (num_rows <= 0 || tiles <= 0) return 0;
+    if (num_rows <= 0 || rows <= 0 || pairs <= 0) return 0;
     if (head_dim < 16 || head_dim > 128 || head_dim % 16 || min_q_len < 1 || (dist_bias && dist_len <= 0)) return MIE_ERR_BAD_ARG;
     if (num_kv_heads <= 0 || num_heads % num_kv_heads || page_size < 1 || (page_size & (page_size - 1))) return MIE_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(out)) & 15) return MIE_ERR_BAD_ARG;
@@ -242,6 +357,22 @@ extern "C" int mie_attention_f32(const float* q, int64_t q_stride, const float* 
     const F32Params p{q, q_stride, k_cache, v_cache, block_tables, table_stride, row_q_start, row_q_len, row_ctx_len, num_rows, out, num_heads,
                       num_kv_heads, head_dim, page_size, page_shift, scale, window, keep, min_q_len, (int64_t)num_pages, g_range_report,
                       ScoreMods{softcap, sink, dist_bias, dist_len, slope}};
-    const dim3 grid(tiles, num_kv_heads);
-    return head_dim <= 64 ? f32_launch<64, 128, false>(p, grid, stream) : f32_launch<128, 256, true>(p, grid, stream);
+    // The longest walk, in tiles of keys; blocks of 8 and of 4 warps.  Heads of 64: blocks of 8 warps, two on an SM, where they are as many as the SMs and their walks long (each in two
+    // shares, so that the longest walks do not end alone: 1,024 tokens of 32 heads 147 -> 128 us, 333 on 300 beside 667 109 -> 94; shares of blocks of 4 warps 136 and 115; five rows of 120
+    // on 100 positions 47 us, by blocks of 4 warps 39).  Else blocks of 4 warps, three on an SM, in as many shares as fit beside one another (64 tokens on 900 positions: 1, 2, 4, 8 shares
+    // 109, 61, 35, 25 us; 200 on 800: 110, 71, 52, 73; 100 alone: 17.6, 15.0, 16.0, 27).  Heads of 128 have one block on an SM, so always of 8 warps (1,000 tokens of 32 heads: 207 us, in
+    // two shares 254, by blocks of 4 warps 358; 500 on 300: 170 and 150 in two shares; 100 on 300: 92, 62, 38, 68).
+    using std::max; using std::min;
+    const int reach = window > 0 ? min(max_ctx, window + keep + F32_KEYS) : window < 0 ? min(max_ctx, keep - window) : max_ctx;
+    const int walk = (reach + F32_KEYS - 1) / F32_KEYS, most = max(2 * walk / 3, min(walk + 1, 4));
+    const int64_t wide = (pairs / 128 + rows) * num_kv_heads, narrow = (pairs / 64 + rows) * num_kv_heads;
+    const int sms = device_sm_count();
+    auto shares = [&](int64_t blocks, int room) {
+        int n = 1;
+        while (n < 8 && 2 * n <= most && 2 * n * blocks <= room) n *= 2;
+        return n;
+    };
+    if (head_dim > 64) return f32_launch<128, 8>(p, pairs, rows, shares(wide, 2 * sms), stream);
+    if (pairs / 128 * num_kv_heads >= sms && walk >= 6) return f32_launch<64, 8>(p, pairs, rows, 2, stream);
+    return f32_launch<64, 4>(p, pairs, rows, shares(narrow, 3 * sms), stream);
 }

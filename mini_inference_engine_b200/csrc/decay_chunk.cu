@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
             for (int j = 0; j < 2; ++j) {
                 if (odd + 2 * j > m) break;
                 uint32_t b[3][2][2];
-                right_columns<DT>(b, right, PLANE, k, 2 * (odd + 2 * j), lane);
+                right_columns<DT>(b, 0, right, PLANE, k, 2 * (odd + 2 * j), lane);
                 triple_step<2>(sum + 2 * j, left, b);
             }
         }
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
                     uint32_t b[3][2][2];
-                    right_rows<DT>(b, right, PLANE, k, d0 / 8 + n, lane);
+                    right_rows<DT>(b, 0, right, PLANE, k, d0 / 8 + n, lane);
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
                         if constexpr (ONE) one_left_step<2>(sum[m] + n, v[m], b);

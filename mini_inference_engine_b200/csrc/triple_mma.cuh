@@ -77,17 +77,24 @@ __device__ __forceinline__ void ldm4(uint32_t& r0, uint32_t& r1, uint32_t& r2, u
 __device__ __forceinline__ void ldm4t(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t at) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(at) : "memory");
 }
-// Right operand, two tiles of 8 columns (n, n + 1), from tiles whose rows run along the contraction ...
+// Left operand (16 x 16) from three tiles, `plane` bytes apart, whose rows are its rows.
 template <int COLS>
-__device__ __forceinline__ void right_rows(uint32_t (&b)[3][2][2], uint32_t tile, int plane, int k, int n, int lane) {
+__device__ __forceinline__ void left_rows(uint32_t (&a)[3][4], uint32_t tile, int plane, int m, int k, int lane) {
+    const uint32_t at = tile + tile_at<COLS>(m * 16 + (lane & 15), k * 2 + (lane >> 4));
+#pragma unroll
+    for (int p = 0; p < 3; ++p) ldm4(a[p][0], a[p][1], a[p][2], a[p][3], at + p * plane);
+}
+// Right operand, two tiles of 8 columns (n, n + 1) into b[..][first] and the next, from tiles whose rows run along the contraction ...
+template <int COLS, int N>
+__device__ __forceinline__ void right_rows(uint32_t (&b)[3][N][2], int first, uint32_t tile, int plane, int k, int n, int lane) {
     const uint32_t at = tile + tile_at<COLS>(k * 16 + (lane & 15), n + (lane >> 4));
 #pragma unroll
-    for (int p = 0; p < 3; ++p) ldm4t(b[p][0][0], b[p][0][1], b[p][1][0], b[p][1][1], at + p * plane);
+    for (int p = 0; p < 3; ++p) ldm4t(b[p][first][0], b[p][first][1], b[p][first + 1][0], b[p][first + 1][1], at + p * plane);
 }
 // ... or along its columns.
-template <int COLS>
-__device__ __forceinline__ void right_columns(uint32_t (&b)[3][2][2], uint32_t tile, int plane, int k, int n, int lane) {
+template <int COLS, int N>
+__device__ __forceinline__ void right_columns(uint32_t (&b)[3][N][2], int first, uint32_t tile, int plane, int k, int n, int lane) {
     const uint32_t at = tile + tile_at<COLS>(n * 8 + (lane & 7) + ((lane >> 4) << 3), k * 2 + ((lane >> 3) & 1));
 #pragma unroll
-    for (int p = 0; p < 3; ++p) ldm4(b[p][0][0], b[p][0][1], b[p][1][0], b[p][1][1], at + p * plane);
+    for (int p = 0; p < 3; ++p) ldm4(b[p][first][0], b[p][first][1], b[p][first + 1][0], b[p][first + 1][1], at + p * plane);
 }

@@ -58,30 +58,43 @@ def rotates_in_decode(dtype, head_dim: int, ctx) -> bool:
             and decode_only(ctx))
 
 
-# float32: tiles of 64 (token, head) pairs against a warp a pair.  A tile takes as long with one pair as with 64, some 0.15 us a key tile more than the warps
-# as long as those have the GPU to themselves; those fill it at about 1,500 pairs.  One row, us, a warp a pair : tiles, 0 / 500 / 2,000 earlier positions --
-# 32 heads of 64 on 4: 8 tokens (256 pairs) 6 : 16 / 64 : 84 / 244 : 315, 32 (1,024) 7 : 16 / 76 : 93 / 282 : 317, 48 (1,536) 13 : 16 / 100 : 95 / 364 : 321,
-# 64 (2,048) 16.6 : 16.8 / 120 : 95 / 426 : 328, 128 (4,096) 38 : 28 / 188 : 110 / 638 : 357; 16 of 64 on 16: 64 tokens (1,024) 11 : 17 / 82 : 96 / 287 : 331, 128 (2,048)
-# 28 : 27 / 144 : 105 / 437 : 339; 32 of 128 on 8: 32 (1,024) 8 : 17 / 100 : 113 / 372 : 392, 48 16 : 18 / 143 : 114 / 521 : 392; 12 of 64 on 4: 128 (1,536) 24 : 26 / 117 : 104 / 389 : 337.
+# float32: tiles of (token, head) pairs (csrc/attention_f32.cu) against a warp a pair.  A tile takes as long with one pair as with 64, a walk of keys shared out over up to eight
+# blocks some 15 us a thousand positions; a warp takes 120 us for them, and warps fill the GPU from about 1,500 pairs on.  One row, us, a warp a pair : tiles, 0 / 250 / 500 / 1,000 /
+# 2,000 earlier positions -- 32 heads of 64 on 4: 2 tokens 6 : 12 / 33 : 13 / 64 : 19 / 125 : 19 / 244 : 33, 32 tokens 7 : 14 / 42 : 20 / 76 : 26 / 146 : 28 / 282 : 43, 64 tokens
+# 16.5 : 14.4 / 74 : 21 / 122 : 28 / 222 : 35 / 426 : 50; 16 of 64 on 16: 32 tokens 7 : 14 / 40 : 20 / 73 : 26 / 138 : 29 / 266 : 39; 32 of 128 on 8: 32 tokens 8 : 25 / 55 : 35 / 100 : 48 / 192 : 48 /
+# 372 : 60.  R rows of one token on 250 / 1,000 / 4,000 positions: 32 of 64 on 4, R 1 33 : 12 / 125 : 19 / 481 : 59, 16 36 : 17 / 134 : 47 / 604 : 171, 64 77 : 45 / 304 : 169 / 1,181 : 656;
+# 16 of 64 on 16, 4 30 : 16 / 111 : 47 / 515 : 170, 16 35 : 44 / 148 : 166 / 566 : 644; 32 of 128 on 8, 1 38 : 19 / 143 : 32 / 555 : 107, 4 38 : 20 / 144 : 95 / 724 : 322, 16 48 : 64 / 217 : 215.
 F32_MIN_WORK = 1536         # (token, head) pairs of the rows that tiles could take, from which they do ...
-F32_MIN_WORK_FRESH = 2048   # ... where no row has more than F32_FRESH positions
+F32_MIN_WORK_FRESH = 2048   # ... where no row has more than F32_FRESH positions; any number of pairs ...
 F32_FRESH = 256
+F32_LONG = 640              # ... where a row reaches this many positions: rows of one token too where tiles are faster (F32_FULL_GROUP, F32_FEW)
+F32_LONG_STEP = 128         # the same for a step of rows of one token only
 F32_MIN_PAIRS = 16          # pairs of a row on one key head below which it is left to the warps: three quarters of its tile would be empty
+F32_FULL_GROUP = 8          # query heads on a key head from which a row of one token fills enough of a tile (heads of up to 64) ...
+F32_FEW = 64                # ... or so few such (row, key head) pairs that their tiles run side by side
 
 
 def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size, scale, window, mods, keep):
-    """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles of 64 pairs, shorter ones one pair a warp, as all are in a step of few
-    pairs.  Where the host does not know the rows' lengths (a captured step) each of the two kernels takes the rows that are its own."""
-    min_q_len = max(2, -(-F32_MIN_PAIRS // (num_heads // num_kv_heads)))
+    """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles, shorter ones one pair a warp, as all are in a step of few
+    pairs on few positions; on many positions rows of any length by tiles.  Where the host does not know the rows' lengths (a captured step) each of the two kernels takes the
+    rows that are its own."""
+    group = num_heads // num_kv_heads
+    min_q_len = max(2, -(-F32_MIN_PAIRS // group))
     q_lens = ctx.host.get("q_len")
+    reach = ctx.max_ctx_len if window == 0 else min(ctx.max_ctx_len, abs(window) + keep)
+    singles = ctx.row_q_len.numel() if q_lens is None else q_lens.count(1) if isinstance(q_lens, list) else int((q_lens == 1).sum())
+    if ((reach >= F32_LONG or (reach >= F32_LONG_STEP and decode_only(ctx)))
+            and ((group >= F32_FULL_GROUP and head_dim <= 64) or singles * num_kv_heads <= F32_FEW)):
+        min_q_len = 1
     long = None if q_lens is None else [n for n in q_lens if n >= min_q_len]
     sizes = (ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, page_size, scale, window)
     pairs = (ctx.num_tokens if long is None else sum(long)) * num_heads
-    if pairs < (F32_MIN_WORK_FRESH if ctx.max_ctx_len <= F32_FRESH else F32_MIN_WORK):
+    few = F32_MIN_WORK_FRESH if ctx.max_ctx_len <= F32_FRESH else F32_MIN_WORK if reach < F32_LONG else 1
+    if pairs < few and min_q_len > 1:
         return ops.paged_attention(*args, *sizes, mods=mods, keep=keep)
-    if long is None or len(long) < len(q_lens):
+    if min_q_len > 1 and (long is None or len(long) < len(q_lens)):
         ops.paged_attention(*args, *sizes, mods=mods, keep=keep, below=min_q_len)
-    ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)))
+    ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)), max_ctx=ctx.max_ctx_len)
     return out
 
 

@@ -436,21 +436,21 @@ def attention_f32_takes(q, k_cache, v_cache, out, head_dim: int) -> bool:
 
 def attention_f32(q: torch.Tensor, q_stride: int, k_cache, v_cache, block_tables, row_q_start, row_q_len, row_ctx_len, num_tokens: int,
                   out: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, scale: float, window: int | None = None,
-                  min_q_len: int = 1, mods: ScoreMods | None = None, keep: int = 0, work=None) -> torch.Tensor:
-    """``paged_attention`` in float32 for rows with ``min_q_len`` new tokens or more: 64 (token, head) pairs a block.  ``work`` = (rows, tokens):
-    how many such rows there are and their tokens in sum, where the caller knows."""
+                  min_q_len: int = 1, mods: ScoreMods | None = None, keep: int = 0, work=None, max_ctx: int | None = None) -> torch.Tensor:
+    """``paged_attention`` in float32 for rows with ``min_q_len`` new tokens or more: 64 or 128 (token, head) pairs a block.  ``work`` = (rows, tokens):
+    how many such rows there are and their tokens in sum, ``max_ctx`` = the most positions a row has, where the caller knows (both shape the launch only)."""
     _need(attention_f32_takes(q, k_cache, v_cache, out, head_dim), "attention_f32: float32 operands with 16-byte rows, heads of 16 to 128 in steps of 16")
     _need(num_heads % num_kv_heads == 0, "query heads must be a multiple of kv heads")
     for t, n in ((block_tables, "block_tables"), (row_q_start, "row_q_start"), (row_q_len, "row_q_len"), (row_ctx_len, "row_ctx_len")):
         _i32(t, n)
     _need(out.is_contiguous(), "attention output must be contiguous")
     rows, tokens = work if work is not None else (row_q_len.numel(), num_tokens)
-    tiles = tokens * (num_heads // num_kv_heads) // 64 + rows               # every row's last tile may be partly filled
     lib = load("attention_f32")
     _check(lib.mie_attention_f32(_ptr(q), ctypes.c_int64(q_stride), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), block_tables.shape[1],
-                                 _ptr(row_q_start), _ptr(row_q_len), _ptr(row_ctx_len), row_q_len.numel(), tiles, _ptr(out), num_heads, num_kv_heads,
-                                 head_dim, page_size, ctypes.c_float(scale), int(window or 0), int(keep), int(min_q_len),
-                                 ctypes.c_longlong(k_cache.shape[0]), *(mods or _NO_MODS).args(num_heads), _stream()), "attention_f32")
+                                 _ptr(row_q_start), _ptr(row_q_len), _ptr(row_ctx_len), row_q_len.numel(), rows, ctypes.c_longlong(tokens * (num_heads // num_kv_heads)),
+                                 _ptr(out), num_heads, num_kv_heads, head_dim, page_size, ctypes.c_float(scale), int(window or 0), int(keep), int(min_q_len),
+                                 int(min(max_ctx or 1 << 30, block_tables.shape[1] * page_size)), ctypes.c_longlong(k_cache.shape[0]),
+                                 *(mods or _NO_MODS).args(num_heads), _stream()), "attention_f32")
     return out
 
 
