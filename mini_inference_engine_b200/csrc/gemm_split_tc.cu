@@ -17,11 +17,13 @@
 //            holds its half of both operands' three planes (TMA, 128-byte swizzle), 24 cta_group::2 MMAs of K 16 go into one of
 //            two to four accumulators, and eight warps move a finished one into their registers (a thread a row of w, half of the tokens).
 //            Rows of w on the 128-lane side: what a warp stores for a token is 128 contiguous bytes, and a few tokens waste nothing.
-//            The pair runs persistently over (tile, share of K) items; shares meet in `partial` and a last small kernel adds them up in order.
+//            The pair runs persistently over items: tiles with all of K first, then the shares of K of the remaining tiles, which meet in `partial` and
+//            which a last small kernel adds up in order.  Tiles that are one wave of pairs and a few more would take two waves: as shares the few are spread over
+//            all pairs (509 x 11,264 x 2,048, 88 tiles on 74 pairs: 161 -> 143 us; 1,000 x 2,560 x 2,048, 80 tiles of 128 tokens, 73 -> 66 us).
 //
 // Bound: the tensor pipe (6 bfloat16 products for one float32 one: a sixth of its rate) for many tokens, memory (4 bytes of w read, 6
 // written and read again) for few.  2,048 x 11,264 x 2,048: 2,707 us on the CUDA cores -> 403 us (235 TFLOP/s);
-// 509 x 11,264 x 2,048 1,008 -> 154 us; 509 x 2,048 x 5,632 1,195 -> 78 us; 17 x 2,048 x 2,048, w from memory, 209 -> 24 us.  Chunks of 32 in a deeper ring were slower
+// 509 x 11,264 x 2,048 1,008 -> 140 us; 509 x 2,048 x 5,632 1,195 -> 78 us; 17 x 2,048 x 2,048, w from memory, 209 -> 24 us.  Chunks of 32 in a deeper ring were slower
 // (550 us at 2,048 tokens): the way from a full accumulator to an empty one costs about 2 us, so what counts is the work per accumulator and their number.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -40,9 +42,10 @@ typedef __nv_bfloat16 bf16;
 struct SpParams {
     float* out; int64_t out_stride;              // [M][out_stride], the first column that of w's first row here
     const void* bias; int bias_tag;
-    float* partial;                              // [splits][M][N] when splits > 1
+    float* partial;                              // [splits][M][cols] when splits > 1, less n_shared: indexed by the output's column
     const float* x; const float* w;              // the operands themselves (an output that is not finite)
-    int M, N, K, k_tiles, splits, k_per_split;
+    int M, N, K, k_tiles, splits, k_per_split;   // splits: shares of K of the tiles behind the first `whole` ones, whose rows of w start at n_shared
+    int whole, shared, n_shared, cols;           // (shared: how many tiles those are; cols: how many rows)
     int tiles_m, num_items, stages, blocks_w, blocks_x;      // tiles_m: tiles of tokens; blocks: of 128 rows of w, of BN / 2 tokens
     int* error;
 };
@@ -218,6 +221,21 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ sr
 
 // --------------------------------------------------------------------------- product
 
+// item -> (tile of w, tile of tokens, chunks of K, share); tokens fastest, so that the pairs of a wave share panels of w
+struct SpItem { int tile_w, tile_x, split, k_lo, k_hi; };             // split: -1 for all of K
+__device__ __forceinline__ SpItem sp_item(const SpParams& p, int item) {
+    SpItem t{0, 0, -1, 0, p.k_tiles};
+    if (item >= p.whole) {
+        t.split = (item - p.whole) / p.shared;
+        item -= t.split * p.shared;
+        t.k_lo = t.split * p.k_per_split;
+        t.k_hi = min(p.k_tiles, t.k_lo + p.k_per_split);
+    }
+    t.tile_w = item / p.tiles_m;
+    t.tile_x = item - t.tile_w * p.tiles_m;
+    return t;
+}
+
 template <int BN>
 __global__ void __launch_bounds__(SP_THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ SpParams p) {
@@ -254,17 +272,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tmem_base = tmem_base_slot;
     pdl_wait();
 
-    // item -> (tile of w, tile of tokens, share of K); tokens fastest, so that the pairs of a wave share panels of w
-    const int tiles = p.num_items / p.splits;
     if (warp == 0) {
         int s = 0;
         uint32_t round = 0;
         const uint32_t bar0 = cluster_addr(smem_u32(&full[0]), 0);
         bool ok = true;
         for (int item = pair; item < p.num_items && ok; item += pairs) {
-            const int tile = item % tiles, k_lo = (item / tiles) * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
-            const int block_w = (tile / p.tiles_m) * 2 + (int)rank, block_x = (tile % p.tiles_m) * 2 + (int)rank;
-            for (int kt = k_lo; kt < k_hi; ++kt) {
+            const SpItem t = sp_item(p, item);
+            const int block_w = t.tile_w * 2 + (int)rank, block_x = t.tile_x * 2 + (int)rank;
+            for (int kt = t.k_lo; kt < t.k_hi; ++kt) {
                 if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[s], (round - 1) & 1, abort_p))) { ok = false; break; }
                 if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE);
@@ -286,8 +302,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             uint32_t round = 0, chunk = 0;
             bool ok = true;
             for (int item = pair; item < p.num_items && ok; item += pairs) {
-                const int k_lo = (item / tiles) * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
-                for (int kt = k_lo; kt < k_hi; ++kt, ++chunk) {
+                const SpItem it = sp_item(p, item);
+                for (int kt = it.k_lo; kt < it.k_hi; ++kt, ++chunk) {
                     const uint32_t buf = chunk % ACCS, use = chunk / ACCS;
                     if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use - 1) & 1, abort_p))) { ok = false; break; }
                     if (!__all_sync(0xffffffffu, mbar_wait(&full[s], round & 1, abort_p))) { ok = false; break; }
@@ -318,11 +334,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         uint32_t chunk = 0;
         bool ok = true;
         for (int item = pair; item < p.num_items && ok; item += pairs) {
-            const int tile = item % tiles, split = item / tiles, k_lo = split * p.k_per_split, k_hi = min(p.k_tiles, k_lo + p.k_per_split);
+            const SpItem ks = sp_item(p, item);
+            const uint32_t end = chunk + (uint32_t)(ks.k_hi - ks.k_lo);
             float acc[BNH];
 #pragma unroll
             for (int i = 0; i < BNH; ++i) acc[i] = 0.f;
-            for (int kt = k_lo; kt < k_hi; ++kt, ++chunk) {
+            for (; chunk < end; ++chunk) {
                 const uint32_t buf = chunk % ACCS, use = chunk / ACCS;
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, abort_p))) { ok = false; break; }
                 tc_fence_after();
@@ -338,12 +355,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if (lane == 0) sp_arrive_cluster(acc_empty_leader + buf * 8u);
             }
             if (!ok) break;
-            const int n = (tile / p.tiles_m) * 256 + (int)rank * 128 + q * 32 + lane, m0 = (tile % p.tiles_m) * BN + half * BNH;
+            asm volatile("" : "+r"(item));                        // (worked out again: the loop above has no registers for it)
+            const SpItem t = sp_item(p, item);
+            const int n = t.tile_w * 256 + (int)rank * 128 + q * 32 + lane, m0 = t.tile_x * BN + half * BNH;
             if (n < p.N) {
-                if (p.splits > 1) {
-                    float* o = p.partial + ((int64_t)split * p.M + m0) * p.N + n;
+                if (t.split >= 0) {
+                    float* o = p.partial + ((int64_t)t.split * p.M + m0) * p.cols + n;
 #pragma unroll
-                    for (int i = 0; i < BNH; ++i) if (m0 + i < p.M) o[(int64_t)i * p.N] = acc[i];
+                    for (int i = 0; i < BNH; ++i) if (m0 + i < p.M) o[(int64_t)i * p.cols] = acc[i];
                 } else {
                     const float b = p.bias ? load_tagged(p.bias, n, p.bias_tag) : 0.f;
                     float* o = p.out + (int64_t)m0 * p.out_stride + n;
@@ -366,7 +385,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
     } else if (again) {                                            // (every copy has arrived and every MMA has read it: the stages' memory is free)
         float* sm = reinterpret_cast<float*>(smem_dyn + (base - smem_u32(smem_dyn)));
-        for (int item = pair; item < p.num_items; item += pairs)
+        for (int item = pair; item < p.whole; item += pairs)
             sp_again(p, sm, (item % p.tiles_m) * BN, BN, (item / p.tiles_m) * 256 + (int)rank * 128, 128);
     }
     cluster_sync_all();
@@ -380,12 +399,12 @@ __global__ void __launch_bounds__(256, 7) split_sum_kernel(const __grid_constant
     __shared__ float sm[SP_AGAIN_FLOATS];
     pdl_enter();
     constexpr int TOKENS = 2 * V;
-    const int tiles_n = (p.N + 127) / 128, m0 = (int)(blockIdx.x / tiles_n) * TOKENS, n0 = (int)(blockIdx.x % tiles_n) * 128;
+    const int tiles_n = (p.cols + 127) / 128, m0 = (int)(blockIdx.x / tiles_n) * TOKENS, n0 = p.n_shared + (int)(blockIdx.x % tiles_n) * 128;
     const int m = m0 + threadIdx.x / (128 / V), n = n0 + threadIdx.x % (128 / V) * V;
     bool fine = true;
     if (m < p.M && n < p.N) {
-        const int64_t per = (int64_t)p.M * p.N;
-        const float* src = p.partial + (int64_t)m * p.N + n;
+        const int64_t per = (int64_t)p.M * p.cols;
+        const float* src = p.partial + (int64_t)m * p.cols + n;
         float v[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) v[i] = 0.f;
@@ -443,12 +462,14 @@ static int sp_launch(const CUtensorMap& mw, const CUtensorMap& mx, SpParams& p, 
 }
 
 // y (columns of a matrix with `y_stride` columns) from the planes xs (blocks of bn / 2 rows) and ws (blocks of 128 rows), both an even number of blocks, of
-// x [M, K], w [N, K] float32 row-major.  bn 64, 128 or 256 tokens a tile; splits shares of K (1: no partial); partial [splits][M][N] float32.
+// x [M, K], w [N, K] float32 row-major.  bn 64, 128 or 256 tokens a tile; the first `whole` tiles of 256 rows of w take all of K at once, those behind them
+// `splits` shares of K (1: no partial, and `whole` does not count); partial [splits][M][N - 256 whole] float32.
 extern "C" int mie_gemm_split(const void* xs, const void* ws, const float* x, const float* w, const void* bias, int bias_tag, float* y,
-                              long long y_stride, float* partial, int M, int N, int K, int bn, int splits, cudaStream_t stream) {
+                              long long y_stride, float* partial, int M, int N, int K, int bn, int splits, int whole,
+                              cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     const int chunks = (K + SP_BK - 1) / SP_BK, blocks_w = (N + 255) / 256 * 2, blocks_x = bn > 0 ? (M + bn - 1) / bn * 2 : 0;
-    if (K <= 0 || (bn != 64 && bn != 128 && bn != 256) || splits < 1 || splits > chunks || (splits > 1 && !partial)) return MIE_ERR_BAD_ARG;
+    if (K <= 0 || (bn != 64 && bn != 128 && bn != 256) || splits < 1 || splits > chunks || (splits > 1 && (!partial || whole < 0 || whole >= (N + 255) / 256))) return MIE_ERR_BAD_ARG;
     if (((reinterpret_cast<uintptr_t>(xs) | reinterpret_cast<uintptr_t>(ws)) & 127) || (reinterpret_cast<uintptr_t>(partial) & 15)) return MIE_ERR_BAD_ARG;
     const int64_t rows_w = (int64_t)chunks * blocks_w * 384, rows_x = (int64_t)chunks * blocks_x * 3 * (bn / 2);
     if (rows_w > 0x7fffffff || rows_x > 0x7fffffff) return MIE_ERR_TOO_LARGE;
@@ -463,10 +484,16 @@ extern "C" int mie_gemm_split(const void* xs, const void* ws, const float* x, co
     p.k_per_split = (p.k_tiles + splits - 1) / splits;
     p.splits = (p.k_tiles + p.k_per_split - 1) / p.k_per_split;       // no empty share
     p.tiles_m = (M + bn - 1) / bn;
-    p.num_items = p.tiles_m * ((N + 255) / 256) * p.splits;
+    const int tiles = p.tiles_m * ((N + 255) / 256);
+    p.whole = p.splits > 1 ? whole * p.tiles_m : tiles;
+    p.shared = tiles - p.whole;
+    p.n_shared = p.splits > 1 ? whole * 256 : 0;
+    p.cols = N - p.n_shared;
+    if (partial) p.partial = partial - p.n_shared;
+    p.num_items = p.whole + p.shared * p.splits;
     rc = bn == 64 ? sp_launch<64>(mw, mx, p, stream) : bn == 128 ? sp_launch<128>(mw, mx, p, stream) : sp_launch<256>(mw, mx, p, stream);
     if (rc || p.splits == 1) return rc;
-    const unsigned tiles_n = (unsigned)((N + 127) / 128);
+    const unsigned tiles_n = (unsigned)((p.cols + 127) / 128);
     if (N % 4 == 0) return launch_kernel(split_sum_kernel<4>, dim3(tiles_n * (unsigned)((M + 7) / 8)), dim3(256), 0, stream, p);
     return launch_kernel(split_sum_kernel<1>, dim3(tiles_n * (unsigned)((M + 1) / 2)), dim3(256), 0, stream, p);
 }
