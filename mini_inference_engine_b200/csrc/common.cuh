@@ -224,11 +224,12 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local_addr, uint32_t r
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
     return remote;
 }
-// Plain (not volatile) so that the loads of all ranks are in flight together; ordering against the
-// peers' writes comes from the cluster barrier before the first load.
+// Loads that stay behind the cluster barrier in front of them, which is what orders them against the peers' writes: volatile, and with memory
+// clobbered, since nothing else keeps the compiler from moving one whose address it knows earlier.  (The machine's loads are plain ones: those of all
+// ranks are in flight together.)
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
     float4 v;
-    asm("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
 // A store into another block's shared memory; the cluster barrier after it (release / acquire)
@@ -250,6 +251,6 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float a) {
 }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     float v;
-    asm("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
