@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
     constexpr int QUADS = F32_KEYS * DT / 4 / THREADS, STEP = THREADS / (DT / 4);
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t* Q = smem;                                // [PAIRS][DT] as parts
-    uint8_t* KV = Q + 3 * Q_PLANE;                    // keys, then values [64][DT]; then weights [16][64] a warp where a tile is multiplied number by number
+    uint8_t* KV = Q + 3 * Q_PLANE;                    // keys, then values [64][DT]; then weights [16][32] a warp where a tile is multiplied number by number
     float* raw = reinterpret_cast<float*>(KV + 3 * K_PLANE);       // keys or values on their way [64][DT]: a thread splits what it fetched
     __shared__ int s_row, s_tile, s_page[2][F32_KEYS];             // the pages of a tile's keys (-1: a key that nobody reads), the next tile's besides
     const int share = blockIdx.x % splits, item = blockIdx.x / splits;
@@ -253,26 +253,35 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
                 }
             }
         } else {
-            float* P = reinterpret_cast<float*>(KV) + warp * 16 * F32_KEYS;        // (the values' parts are not read)
-#pragma unroll
-            for (int n = 0; n < 8; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) P[(r0 + 8 * (i >> 1)) * F32_KEYS + n * 8 + c0 + (i & 1)] = (unseen >> (4 * n + i)) & 1 ? -1.f : s[n][i];
-            __syncwarp();
+            // half of the keys at a time: all warps' weights fit the values' parts, which nobody reads now, and stay clear of the next keys that arrive behind them
+            constexpr int HALF = F32_KEYS / 2;
+            static_assert(WARPS * 16 * HALF * (int)sizeof(float) <= 3 * K_PLANE, "weights written over the next keys");
+            float* P = reinterpret_cast<float*>(KV) + warp * 16 * HALF;
 #pragma unroll 1
-            for (int j = 0; j < F32_KEYS; ++j) {
-                const int key = k0 + j;
-                if (pages[j] < 0) continue;
-                const float* v = row_in(p.v_cache, pages[j], key);
+            for (int j0 = 0; j0 < F32_KEYS; j0 += HALF) {
+                __syncwarp();
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float w = P[(r0 + 8 * i) * F32_KEYS + j];
-                    if (w < 0.f) continue;                         // a key out of sight: its value may be anything
+                for (int n = 0; n < 8; ++n) {
+                    if (n / 4 != j0 / HALF) continue;
 #pragma unroll
-                    for (int n = 0; n < NT; ++n)
+                    for (int i = 0; i < 4; ++i) P[(r0 + 8 * (i >> 1)) * HALF + n % 4 * 8 + c0 + (i & 1)] = (unseen >> (4 * n + i)) & 1 ? -1.f : s[n][i];
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (int j = 0; j < HALF; ++j) {
+                    const int key = k0 + j0 + j, page = pages[j0 + j];
+                    if (page < 0) continue;
+                    const float* v = row_in(p.v_cache, page, key);
 #pragma unroll
-                        for (int e = 0; e < 2; ++e)
-                            if (n * 8 + c0 + e < D) o[n][2 * i + e] = fmaf(w, v[n * 8 + c0 + e], o[n][2 * i + e]);
+                    for (int i = 0; i < 2; ++i) {
+                        const float w = P[(r0 + 8 * i) * HALF + j];
+                        if (w < 0.f) continue;                     // a key out of sight: its value may be anything
+#pragma unroll
+                        for (int n = 0; n < NT; ++n)
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                if (n * 8 + c0 + e < D) o[n][2 * i + e] = fmaf(w, v[n * 8 + c0 + e], o[n][2 * i + e]);
+                    }
                 }
             }
         }

@@ -72,3 +72,25 @@ def test_rows_of_one_token_and_long_rows_of_few(monkeypatch, H, G, D, rows, ctx,
     got = attention.attention(q, step, SimpleNamespace(k=k, v=v, group=0, page_size=16), torch.zeros_like(out), H, G, D, D ** -0.5, 0)
     close(got, want, v)
     assert used == kernels
+
+
+@pytest.mark.parametrize("window,keep", [(0, 0), (300, 0), (-256, 70)])
+@pytest.mark.parametrize("what", ["key", "value", "query"])
+@pytest.mark.parametrize("bad", [3e38, float("inf"), float("nan")])
+def test_numbers_without_parts_in_wide_blocks(window, keep, what, bad):
+    """Blocks of eight warps (32 heads on 4, 640 tokens): a number in an early tile, while the next tile's keys are on their way."""
+    H, G, D, page, at = 32, 4, 64, 16, 130
+    args, tables, out = case([(640, 700)], H, G, D, page)
+    if what == "query":
+        args[0][at - 60, 3 * D + 5] = bad                      # the row's first token is at position 60
+    else:
+        args[2 if what == "key" else 3][tables[0][at // page], 1, at % page, 7] = bad
+    a, b = both(args, out, H, G, D, page, window=window, keep=keep)
+    again, _ = both(args, out, H, G, D, page, window=window, keep=keep)
+    assert torch.equal(a.view(torch.int32), again.view(torch.int32))
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(a), kind(b))
+    ok = torch.isfinite(b) & (b.abs() < 1e6)
+    assert ok.float().mean() > 0.5 and ((a - b).abs()[ok] <= 2e-5 * b[ok].abs().max()).all()
+    big = torch.isfinite(b) & (b.abs() >= 1e6)
+    assert ((a - b).abs()[big] <= 1e-4 * b.abs()[big]).all()
