@@ -341,8 +341,11 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
     }
     const bool no_keys = has_no_parts(most);
     if (__syncthreads_or(bad || no_keys)) {
-        dc_walk_state<T>(p, kp, a, to, t0, h, count, first_col, part_no == splits - 1 ? p.Dv : min(end_col, p.Dv));
-        if (part_no == 0) dc_walk_scores(p, qp, kp, M, out, count);
+        dc_walk_state<T>(p, kp, a, to, t0, h, count, first_col, end_col);
+        if (part_no == 0) {                            // (the column of ones is the first share's, like P)
+            dc_walk_state<T>(p, kp, a, to, t0, h, count, p.Dv_in, p.Dv);
+            dc_walk_scores(p, qp, kp, M, out, count);
+        }
     }
 }
 
@@ -603,7 +606,7 @@ extern "C" int mie_decay_chunks(const float* q, const float* k, const void* v, i
             p.heads = H - p.h0 < per_pass ? H - p.h0 : per_pass;                                                                                          \
             /* a step of few chunks: the value columns in as many shares as the SMs have room for */                                                      \
             const int items = chunks * p.heads, room = items < sms ? sms / items : 1, tiles = (Dv_in + DC_COLS - 1) / DC_COLS;                             \
-            const int splits = room < tiles ? room : tiles;                                                                                               \
+            const int per_share = (tiles + room - 1) / room, splits = (tiles + per_share - 1) / per_share;                 /* (no empty share) */          \
             rc = launch_kernel(decay_local_kernel<T, DT, ONE>, dim3(chunks, p.heads, splits), dim3(DC_THREADS), smem_l, stream, p, splits);                \
             if (rc) return rc;                                                                                                                            \
             const int64_t quads = (int64_t)p.heads * Dv * D / 4;                                                                                          \

@@ -16,23 +16,24 @@ def test_shares_and_blocks_of_every_size(monkeypatch, dt, rows, H, D, V):
     close(scan(monkeypatch, True, rows, H, D, V, dt, **how), scan(monkeypatch, False, rows, H, D, V, dt, **how))
 
 
-def run(qkv, tok, k_tok, state, rows, H, D, V):
+def run(qkv, tok, k_tok, state, rows, H, D, V, ones=False):
     from mini_inference_engine_b200.kernels import ops
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     T = sum(rows)
-    state, out = state.clone(), torch.zeros(T, H * V, device="cuda")
+    dv = V + int(ones)
+    state, out = state.clone(), torch.zeros(T, H * dv, device="cuda")
     ops.decay_scan(qkv, i32([0] * T), i32([sum(rows[:i]) for i in range(len(rows))]), i32(rows), i32([i + 1 for i in range(len(rows))]), state, out, num_heads=H, dim=D, vdim=V,
-                   max_q_len=max(rows), tok_decay=tok, k_tok=k_tok, q_scale=0.125, q_lens=rows)
+                   max_q_len=max(rows), tok_decay=tok, k_tok=k_tok, q_scale=0.125, q_lens=rows, ones=ones)
     torch.cuda.synchronize()
-    return out.view(T, H, V), state
+    return out.view(T, H, dv), state
 
 
-def operands(rows, H, D, V, dt, least, seed=0):
+def operands(rows, H, D, V, dt, least, seed=0, ones=False):
     g = torch.Generator(device="cuda").manual_seed(seed)
     T = sum(rows)
     qkv = torch.randn(T, H * (2 * D + V), generator=g, device="cuda").to(dt)
     tok = least + (1 - least) * torch.rand(T, H, generator=g, device="cuda")
-    return qkv, tok, torch.rand(T, H, generator=g, device="cuda"), torch.randn(len(rows) + 1, H, V, D, generator=g, device="cuda")
+    return qkv, tok, torch.rand(T, H, generator=g, device="cuda"), torch.randn(len(rows) + 1, H, V + int(ones), D, generator=g, device="cuda")
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
@@ -78,3 +79,28 @@ def test_numbers_without_three_parts(monkeypatch, dt, what):
         assert ((a - b).abs()[ok] <= 1.5e-5 * b[ok].abs().max()).all()
         quiet = ok & (b.abs() < 1e30)                          # what the large number does not reach keeps its digits
         assert ((a - b).abs()[quiet] <= 1.5e-5 * b[quiet].abs().max()).all()
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what,bad", [("key", 3e38), ("key", float("inf")), ("key", float("nan")), ("value", 3e38)])
+@pytest.mark.parametrize("H,V", [(12, 300), (2, 300), (9, 130), (1, 64)])
+def test_column_of_ones_with_numbers_without_parts(monkeypatch, dt, what, bad, H, V):
+    """Five tiles of value columns in three or five shares, three in three, one: the column of ones has one owner, whatever a share meets."""
+    from mini_inference_engine_b200.kernels import ops
+    rows, D = [150], 32
+    qkv, tok, k_tok, state = operands(rows, H, D, V, dt, 0.9, ones=True)
+    qkv *= 1e-3
+    qkv[70, H * D + 3 if what == "key" else 2 * H * D + H * V - 1] = bad
+    first = run(qkv, tok, k_tok, state, rows, H, D, V, ones=True)
+    for _ in range(4):
+        for a, b in zip(first, run(qkv, tok, k_tok, state, rows, H, D, V, ones=True)):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    monkeypatch.setattr(ops, "decay_chunks_take", lambda d: False)
+    ref = run(qkv, tok, k_tok, state, rows, H, D, V, ones=True)
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(first[1]), kind(ref[1]))
+    assert torch.isfinite(first[0][:70]).all()
+    for a, b in zip(first, ref):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b))
+        for some in (torch.isfinite(b) & (b.abs() < 1e30), torch.isfinite(b) & (b.abs() >= 1e30)):
+            assert not some.any() or ((a - b).abs()[some] <= 1.5e-5 * b[some].abs().max()).all()
