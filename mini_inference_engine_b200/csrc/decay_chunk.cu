@@ -173,17 +173,19 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
     const float* qp = p.q + ((int64_t)t0 * H + h) * D;
     const int64_t stride = (int64_t)H * D;
     const int kr = threadIdx.x / (DT / 4), kd = (threadIdx.x % (DT / 4)) * 4;
-    uint32_t most = 0;                                 // the largest magnitude of keys (and queries) this thread met
+    uint32_t most = 0;                                 // the largest magnitude of keys, queries and values this thread met
     float4 key[QUADS];
 #pragma unroll
     for (int i = 0; i < QUADS; ++i)
         key[i] = kr + i * STEP < count && kd < D ? *reinterpret_cast<const float4*>(kp + (kr + i * STEP) * stride + kd) : make_float4(0.f, 0.f, 0.f, 0.f);
     auto put_keys = [&](auto factor) {
+        uint32_t f_most = 0;
 #pragma unroll
         for (int i = 0; i < QUADS; ++i) {
             const int r = kr + i * STEP;
             const float f = factor(r);
             most = max(most, magnitude(key[i]));
+            f_most = max(f_most, magnitude(f));
             uint8_t* at = keys + tile_at<DT>(r, kd >> 3) + (kd & 4) * 2;
             uint2 part[3];
             split3(key[i].x * f, key[i].y * f, part[0].x, part[1].x, part[2].x);
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
 #pragma unroll
             for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(at + j * PLANE) = part[j];
         }
+        most = max(most, magnitude(__uint_as_float(most) * __uint_as_float(f_most)));      // (a decay may be infinite, or beyond 1)
     };
     if (threadIdx.x < DC_L)
         a[threadIdx.x] = threadIdx.x >= count ? 1.f : p.tok_decay ? p.tok_decay[(int64_t)(t0 + threadIdx.x) * H + h] : p.decay[h];
@@ -261,7 +264,6 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
     __syncthreads();                                   // (the keys are done with)
     put_keys([&](int r) { return a[r]; });
     float* to = p.states + ((int64_t)blockIdx.x * p.heads + blockIdx.y) * (int64_t)p.Dv * D;
-    bool bad = false;
     for (int j0 = first_col, buf = 0; j0 < end_col; j0 += DC_COLS, buf ^= 1) {
         uint8_t* tile = values + buf * PARTS * V_PLANE;
 #pragma unroll
@@ -273,10 +275,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 if (ONE) part[0][e] = nearest2(x[2 * e], x[2 * e + 1]);
-                else {
-                    split3(x[2 * e], x[2 * e + 1], part[0][e], part[1][e], part[2][e]);
-                    bad |= has_no_parts(max(magnitude(x[2 * e]), magnitude(x[2 * e + 1])));
-                }
+                else split3(x[2 * e], x[2 * e + 1], part[0][e], part[1][e], part[2][e]);
+                most = max(most, max(magnitude(x[2 * e]), magnitude(x[2 * e + 1])));       // (one part too: an infinite value must not meet parts of a key that are zero)
             }
 #pragma unroll
             for (int j = 0; j < PARTS; ++j) *reinterpret_cast<uint4*>(at + j * V_PLANE) = make_uint4(part[j][0], part[j][1], part[j][2], part[j][3]);
@@ -339,8 +339,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_local_kernel(const DcPara
             to[(int64_t)p.Dv_in * D + threadIdx.x] = sum;
         }
     }
-    const bool no_keys = has_no_parts(most);
-    if (__syncthreads_or(bad || no_keys)) {
+    if (__syncthreads_or(has_no_parts(most))) {
         dc_walk_state<T>(p, kp, a, to, t0, h, count, first_col, end_col);
         if (part_no == 0) {                            // (the column of ones is the first share's, like P)
             dc_walk_state<T>(p, kp, a, to, t0, h, count, p.Dv_in, p.Dv);

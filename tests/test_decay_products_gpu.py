@@ -16,14 +16,14 @@ def test_shares_and_blocks_of_every_size(monkeypatch, dt, rows, H, D, V):
     close(scan(monkeypatch, True, rows, H, D, V, dt, **how), scan(monkeypatch, False, rows, H, D, V, dt, **how))
 
 
-def run(qkv, tok, k_tok, state, rows, H, D, V, ones=False):
+def run(qkv, tok, k_tok, state, rows, H, D, V, ones=False, act=False):
     from mini_inference_engine_b200.kernels import ops
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     T = sum(rows)
     dv = V + int(ones)
     state, out = state.clone(), torch.zeros(T, H * dv, device="cuda")
     ops.decay_scan(qkv, i32([0] * T), i32([sum(rows[:i]) for i in range(len(rows))]), i32(rows), i32([i + 1 for i in range(len(rows))]), state, out, num_heads=H, dim=D, vdim=V,
-                   max_q_len=max(rows), tok_decay=tok, k_tok=k_tok, q_scale=0.125, q_lens=rows, ones=ones)
+                   max_q_len=max(rows), tok_decay=tok, k_tok=k_tok, q_scale=0.125, q_lens=rows, ones=ones, act=act)
     torch.cuda.synchronize()
     return out.view(T, H, dv), state
 
@@ -102,5 +102,36 @@ def test_column_of_ones_with_numbers_without_parts(monkeypatch, dt, what, bad, H
     assert torch.isfinite(first[0][:70]).all()
     for a, b in zip(first, ref):
         assert torch.equal(torch.isfinite(a), torch.isfinite(b))
+        for some in (torch.isfinite(b) & (b.abs() < 1e30), torch.isfinite(b) & (b.abs() >= 1e30)):
+            assert not some.any() or ((a - b).abs()[some] <= 1.5e-5 * b[some].abs().max()).all()
+
+
+@pytest.mark.parametrize("dt,act", [(torch.float32, False), (torch.bfloat16, False), (torch.bfloat16, True)])
+@pytest.mark.parametrize("what,bad", [("value", float("inf")), ("value", -float("inf")), ("value", float("nan")), ("value", 3.2e38), ("decay", float("inf")), ("decay", 3.4e38 / 2.0 ** 46)])
+@pytest.mark.parametrize("D", [32, 128])
+def test_infinite_values_and_decays_meet_no_parts(monkeypatch, dt, act, what, bad, D):
+    """Keys of 1 have two parts of zero: a number that is not finite must not meet them.  States sign for sign as the token-by-token kernel has them; the keys in front of a
+    large decay outgrow three parts only once it is multiplied in (3.4e38: finite, its nearest bfloat16 is not)."""
+    from mini_inference_engine_b200.kernels import ops
+    rows, H, V = [150], 2, 40
+    qkv, tok, _, state = operands(rows, H, D, V, dt, 0.9)
+    k_tok = torch.ones_like(tok)
+    qkv[:, :H * D] *= 1e-3
+    qkv[:, H * D:2 * H * D] = 1.0
+    if what == "value":
+        qkv[70, 2 * H * D + 3], tok[64:128] = bad, 1.0
+    else:
+        qkv[:, H * D:2 * H * D] = 2.0 ** 46
+        qkv[:, 2 * H * D:] = qkv[:, 2 * H * D:].clamp(0.5, 1.0) * 1e-3
+        state.abs_()
+        tok[100], tok[101:128] = bad, 1.0
+    how = dict(act=act)
+    got = run(qkv, tok, k_tok, state, rows, H, D, V, **how)
+    monkeypatch.setattr(ops, "decay_chunks_take", lambda d: False)
+    ref = run(qkv, tok, k_tok, state, rows, H, D, V, **how)
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(got[1]), kind(ref[1])), kind
+    assert torch.equal(torch.isfinite(got[0]), torch.isfinite(ref[0]))
+    for a, b in zip(got, ref):
         for some in (torch.isfinite(b) & (b.abs() < 1e30), torch.isfinite(b) & (b.abs() >= 1e30)):
             assert not some.any() or ((a - b).abs()[some] <= 1.5e-5 * b[some].abs().max()).all()
