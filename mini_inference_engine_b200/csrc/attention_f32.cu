@@ -5,7 +5,8 @@
 // A block owns 16 (token, query head) pairs a warp that share a key head -- tokens of one row, the group's heads side by side -- so a tile of
 // 64 keys and values in shared memory serves all heads of the group.  Queries, keys and values lie there as parts, split by the threads that fetched them; the scores of a
 // warp's pairs become the left operand of the product with the values where they are.  A walk of keys may be shared out over the blocks of a cluster, every n-th tile a block;
-// their sums meet in shared memory.  The next tile's keys arrive (cp.async) under the product with the
+// their sums meet in shared memory.  A tile whose scores in sight are all NaN counts as out of sight for a pair that has met no number yet and makes its output NaN behind the
+// first number; so that the shares decide as one walk does, each keeps the first tile where a pair met a number and the last one that it passed over.  The next tile's keys arrive (cp.async) under the product with the
 // values, the values under the scores.  Tiles of a row go longest first, over all heads.
 //
 // A tile with keys or values that have no three parts (not finite, or beyond 2^127) is multiplied number by number, and a weight that does not exist then meets no value.
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
     uint8_t* KV = Q + 3 * Q_PLANE;                    // keys, then values [64][DT]; then weights [16][32] a warp where a tile is multiplied number by number
     float* raw = reinterpret_cast<float*>(KV + 3 * K_PLANE);       // keys or values on their way [64][DT]: a thread splits what it fetched
     __shared__ int s_row, s_tile, s_page[2][F32_KEYS];             // the pages of a tile's keys (-1: a key that nobody reads), the next tile's besides
+    __shared__ int s_number[PAIRS], s_none[PAIRS];                 // a pair's first tile with a number; the last one of NaN that it passed over
     const int share = blockIdx.x % splits, item = blockIdx.x / splits;
     const int D = p.head_dim, G = p.num_heads / p.num_kv_heads, kvh = item % p.num_kv_heads;
     pdl_launch_dependents();
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
         m[i] = -INFINITY;
         l[i] = 0.f;
         if (p.mods.sink && at < pairs && share == 0) { m[i] = p.mods.sink[head[i]]; l[i] = c0 == 0 ? 1.f : 0.f; }
+        if (c0 == 0) { s_number[at - pair0] = m[i] > -INFINITY ? -1 : 0x7fffffff; s_none[at - pair0] = -1; }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -217,9 +220,15 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
             const float m_new = fmaxf(m[i], top), base = m_new > -INFINITY ? m_new : 0.f;
-            if (!(m_new > -INFINITY))                              // every key so far is masked for this pair, or its score no number: no weights
+            if (!(m_new > -INFINITY)) {                            // every key so far is masked for this pair, or its score no number: no weights
+                bool none = false;
 #pragma unroll
-                for (int n = 0; n < 8; ++n) s[n][2 * i] = s[n][2 * i + 1] = -INFINITY;
+                for (int n = 0; n < 8; ++n) {
+                    none |= isnan(s[n][2 * i]) || isnan(s[n][2 * i + 1]);
+                    s[n][2 * i] = s[n][2 * i + 1] = -INFINITY;
+                }
+                if (none) s_none[warp * 16 + r0 + 8 * i] = t;
+            } else if (!(m[i] > -INFINITY)) s_number[warp * 16 + r0 + 8 * i] = t;
             const float alpha = expf(m[i] - base);
             float sum = 0.f;
 #pragma unroll
@@ -308,32 +317,39 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
     }
     // the shares of the keys meet: every block of the cluster adds up its part of the pairs
     constexpr int OS = DT + 4;
-    float* sums = reinterpret_cast<float*>(smem);     // [PAIRS][OS], then the largest scores and the weights' sums
-    float *tops = sums + PAIRS * OS, *weights = tops + PAIRS;
+    float* sums = reinterpret_cast<float*>(smem);     // [PAIRS][OS], then a pair's largest score, sum of weights, first tile with a number, last one of NaN passed over
+    float4* ends = reinterpret_cast<float4*>(sums + PAIRS * OS);
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int row = warp * 16 + r0 + 8 * i;
-        if (c0 == 0) { tops[row] = m[i]; weights[row] = l[i]; }
+        if (c0 == 0) ends[row] = make_float4(m[i], l[i], __int_as_float(s_number[row]), __int_as_float(s_none[row]));
 #pragma unroll
         for (int n = 0; n < NT; ++n) *reinterpret_cast<float2*>(sums + row * OS + n * 8 + c0) = make_float2(o[n][2 * i], o[n][2 * i + 1]);
     }
     cluster_sync_all();
-    const uint32_t at0 = (uint32_t)__cvta_generic_to_shared(sums), top0 = (uint32_t)__cvta_generic_to_shared(tops), weight0 = (uint32_t)__cvta_generic_to_shared(weights);
+    const uint32_t at0 = (uint32_t)__cvta_generic_to_shared(sums), end0 = (uint32_t)__cvta_generic_to_shared(ends);
     const int mine = PAIRS / splits;
     for (int i = threadIdx.x; i < mine * (DT / 4); i += THREADS) {
         const int row = share * mine + i / (DT / 4), d = (i % (DT / 4)) * 4, at = pair0 + row;
         if (at >= pairs || d >= D) continue;
         float top = -INFINITY;
-        for (int j = 0; j < splits; ++j) top = fmaxf(top, ld_cluster_f32(cluster_addr(top0 + row * 4, j)));
+        int number = 0x7fffffff, none = -1;
+        for (int j = 0; j < splits; ++j) {
+            const float4 end = ld_cluster_f32x4(cluster_addr(end0 + row * 16, j));
+            top = fmaxf(top, end.x);
+            number = min(number, __float_as_int(end.z));
+            none = max(none, __float_as_int(end.w));
+        }
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
         float weight = 0.f;
         for (int j = 0; j < splits; ++j) {
-            const float m_j = ld_cluster_f32(cluster_addr(top0 + row * 4, j)), f = m_j > -INFINITY ? expf(m_j - top) : 0.f;
-            const float4 x = ld_cluster_f32x4(cluster_addr(at0 + (row * OS + d) * 4, j));
-            weight = fmaf(f, ld_cluster_f32(cluster_addr(weight0 + row * 4, j)), weight);
+            const float4 end = ld_cluster_f32x4(cluster_addr(end0 + row * 16, j)), x = ld_cluster_f32x4(cluster_addr(at0 + (row * OS + d) * 4, j));
+            const float f = end.x > -INFINITY ? expf(end.x - top) : 0.f;
+            weight = fmaf(f, end.y, weight);
             sum.x = fmaf(f, x.x, sum.x); sum.y = fmaf(f, x.y, sum.y); sum.z = fmaf(f, x.z, sum.z); sum.w = fmaf(f, x.w, sum.w);
         }
+        if (none > number) sum = make_float4(NAN, NAN, NAN, NAN);
         const float inv = weight > 0.f ? 1.0f / weight : 0.f;
         const int token = at / G;
         *reinterpret_cast<float4*>(p.out + ((int64_t)(q_start + token) * p.num_heads + kvh * G + at - token * G) * D + d) = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv);

@@ -94,3 +94,30 @@ def test_numbers_without_parts_in_wide_blocks(window, keep, what, bad):
     assert ok.float().mean() > 0.5 and ((a - b).abs()[ok] <= 2e-5 * b[ok].abs().max()).all()
     big = torch.isfinite(b) & (b.abs() >= 1e6)
     assert ((a - b).abs()[big] <= 1e-4 * b.abs()[big]).all()
+
+
+@pytest.mark.parametrize("H,G,D", [(8, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("n,ctx,first,end", [(100, 100, 64, 65), (150, 150, 128, 129), (1, 129, 128, 129), (1, 129, 64, 129), (300, 520, 192, 256), (300, 520, 0, 64), (300, 520, 0, 448),
+                                             (300, 520, 64, 520), (5, 700, 0, 700)])
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("window,keep", [(0, 0), (150, 0), (-128, 70)])
+def test_shares_of_scores_that_are_no_numbers(H, G, D, n, ctx, first, end, sink, window, keep):
+    """Keys that are NaN from position ``first`` up to ``end``: whatever share of a walk meets them, the outputs are no numbers where the walk in one share has none."""
+    from mini_inference_engine_b200.kernels import ops
+    args, tables, out = case([(n, ctx), (70, 700)], H, G, D, 16)
+    for at in range(first, end):
+        args[2][tables[0][at // 16], 1, at % 16] = float("nan")
+    mods = ops.ScoreMods(0.0, torch.linspace(-2.0, 3.0, H).cuda(), None, None) if sink else None
+    res = [ops.attention_f32(*args, out.clone(), H, G, D, 16, D ** -0.5, window, keep=keep, mods=mods, max_ctx=c) for c in (64, 128, 200, 700, 1 << 20)]
+    warps = ops.paged_attention(*args, out.clone(), H, G, D, 16, D ** -0.5, window, keep=keep, mods=mods)
+    torch.cuda.synchronize()
+    for a in res[1:]:
+        assert torch.equal(torch.isnan(a), torch.isnan(res[0]))
+        ok = ~torch.isnan(a)
+        assert ((a - res[0]).abs()[ok] <= 2e-5 * args[3].abs().max()).all()
+    heads = slice(0, H // G)
+    assert torch.isfinite(res[0][:, heads]).all() and torch.isfinite(res[0][n:]).all()        # (the other key head, the other row)
+    if first % 64:                                             # (a tile of 64 keys that are all NaN counts as out of sight in front of the first number; the other kernel's are 32)
+        return
+    if end - first <= 64 and first > 0 and not window:
+        assert torch.equal(torch.isnan(warps), torch.isnan(res[0]))
