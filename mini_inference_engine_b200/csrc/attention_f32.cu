@@ -357,13 +357,45 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
     cluster_sync_all();                               // (the others may still read this block's memory)
 }
 
+// The launch: blocks of 8 or 4 warps, shares of a walk, and (tile of pairs, key head) items.
+// Heads of 64: blocks of 8 warps, two on an SM, where they are as many as the SMs and their walks long (each in two
+// shares, so that the longest walks do not end alone: 1,024 tokens of 32 heads 147 -> 128 us, 333 on 300 beside 667 109 -> 94; shares of blocks of 4 warps 136 and 115; five rows of 120
+// on 100 positions 47 us, by blocks of 4 warps 39).  Else blocks of 4 warps, three on an SM, in as many shares as fit beside one another (64 tokens on 900 positions: 1, 2, 4, 8 shares
+// 109, 61, 35, 25 us; 200 on 800: 110, 71, 52, 73; 100 alone: 17.6, 15.0, 16.0, 27).  Heads of 128 have one block on an SM, so always of 8 warps (1,000 tokens of 32 heads: 207 us, in
+// two shares 254, by blocks of 4 warps 358; 500 on 300: 170 and 150 in two shares; 100 on 300: 92, 62, 38, 68): two shares may wait for one another's place, since portions' walks
+// differ, more must fit beside one another.  Clusters fill a B200's SMs less the larger they are, since one lies within a part of the chip: of blocks that have an SM to themselves 148, 148, 132
+// and 120 run at once in clusters of 1, 2, 4 and 8, of three to an SM 444, 444, 416 and 384; one cluster more costs a whole round (32 heads of 128 on 8, us, as many shares as blocks fit twice : as here -- 4
+// rows of one token on 256 positions planned for 960 58 : 21, 8 rows on 500 66 : 59, 100 tokens on 250 68 : 37; 100 tokens of 32 heads of 64, eight shares 27, four 17).
+struct F32Plan { int warps, shares; int64_t items; };
+static F32Plan f32_plan(int64_t pairs, int rows, int num_heads, int num_kv_heads, int head_dim, int window, int keep, int max_ctx, int sms) {
+    using std::max; using std::min;
+    const int reach = window > 0 ? min(max_ctx, window + keep + F32_KEYS) : window < 0 ? min(max_ctx, keep - window) : max_ctx;
+    const int walk = (reach + F32_KEYS - 1) / F32_KEYS, most = max(2 * walk / 3, min(walk + 1, 4));         // (walk: the longest one, in tiles of keys)
+    // tiles of `per` pairs: a row's pairs are a multiple of the group's heads, so its last tile lacks at most per - gcd(per, heads)
+    const int group = num_heads / num_kv_heads, fits = group & -group;
+    auto items = [&](int per) { return (pairs + (int64_t)rows * (per - min(per, fits))) / per * num_kv_heads; };
+    auto shares = [&](int64_t blocks, int two, int four, int eight) {         // places for blocks in so many shares
+        int n = 1;
+        while (n < 8 && 2 * n <= most && 2 * n * blocks <= (n == 1 ? two : n == 2 ? four : eight)) n *= 2;
+        return n;
+    };
+    if (head_dim > 64) return {8, shares(items(128), 2 * sms, sms * 8 / 9, sms * 13 / 16), items(128)};
+    if (pairs / 128 * num_kv_heads >= sms && walk >= 6) return {8, 2, items(128)};
+    return {4, shares(items(64), 3 * sms, 3 * sms * 15 / 16, 3 * sms * 13 / 16), items(64)};
+}
+// The plan, for tests on the host: 256 x items + 16 x shares + warps.
+extern "C" long long mie_attention_f32_plan(long long pairs, int rows, int num_heads, int num_kv_heads, int head_dim, int window, int keep, int max_ctx, int sms) {
+    const F32Plan plan = f32_plan(pairs, rows, num_heads, num_kv_heads, head_dim, window, keep, max_ctx, sms);
+    return 256 * plan.items + 16 * plan.shares + plan.warps;
+}
+
 template <int DT, int WARPS>
-static int f32_launch(const F32Params& p, int64_t pairs, int rows, int splits, cudaStream_t stream) {
-    const int64_t blocks = (pairs / (16 * WARPS) + rows) * p.num_kv_heads;          // (every row's last tile may be partly filled)
-    if (blocks * splits > 0x7fffffff) return MIE_ERR_TOO_LARGE;
+static int f32_launch(const F32Params& p, const F32Plan& plan, cudaStream_t stream) {
+    const int splits = plan.shares;
+    if (plan.items * splits > 0x7fffffff) return MIE_ERR_TOO_LARGE;
     const cudaError_t e = cudaFuncSetAttribute(f32_attention_kernel<DT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_bytes<DT, WARPS>());
     if (e != cudaSuccess) return (int)e;
-    return launch_kernel_cluster(f32_attention_kernel<DT, WARPS>, dim3((unsigned)(blocks * splits)), dim3(32 * WARPS), f32_bytes<DT, WARPS>(), stream, dim3(splits, 1, 1), p, splits);
+    return launch_kernel_cluster(f32_attention_kernel<DT, WARPS>, dim3((unsigned)(plan.items * splits)), dim3(32 * WARPS), f32_bytes<DT, WARPS>(), stream, dim3(splits, 1, 1), p, splits);
 }
 
 // Rows with fewer than `min_q_len` new tokens are left alone; `max_ctx`: no row has more positions (it only shapes the launch); `rows`, `pairs`: upper bounds of the others' number and of their (token, head of a group) pairs.  Heads of
@@ -382,22 +414,6 @@ extern "C" int mie_attention_f32(const float* q, int64_t q_stride, const float* 
     const F32Params p{q, q_stride, k_cache, v_cache, block_tables, table_stride, row_q_start, row_q_len, row_ctx_len, num_rows, out, num_heads,
                       num_kv_heads, head_dim, page_size, page_shift, scale, window, keep, min_q_len, (int64_t)num_pages, g_range_report,
                       ScoreMods{softcap, sink, dist_bias, dist_len, slope}};
-    // The longest walk, in tiles of keys; blocks of 8 and of 4 warps.  Heads of 64: blocks of 8 warps, two on an SM, where they are as many as the SMs and their walks long (each in two
-    // shares, so that the longest walks do not end alone: 1,024 tokens of 32 heads 147 -> 128 us, 333 on 300 beside 667 109 -> 94; shares of blocks of 4 warps 136 and 115; five rows of 120
-    // on 100 positions 47 us, by blocks of 4 warps 39).  Else blocks of 4 warps, three on an SM, in as many shares as fit beside one another (64 tokens on 900 positions: 1, 2, 4, 8 shares
-    // 109, 61, 35, 25 us; 200 on 800: 110, 71, 52, 73; 100 alone: 17.6, 15.0, 16.0, 27).  Heads of 128 have one block on an SM, so always of 8 warps (1,000 tokens of 32 heads: 207 us, in
-    // two shares 254, by blocks of 4 warps 358; 500 on 300: 170 and 150 in two shares; 100 on 300: 92, 62, 38, 68).
-    using std::max; using std::min;
-    const int reach = window > 0 ? min(max_ctx, window + keep + F32_KEYS) : window < 0 ? min(max_ctx, keep - window) : max_ctx;
-    const int walk = (reach + F32_KEYS - 1) / F32_KEYS, most = max(2 * walk / 3, min(walk + 1, 4));
-    const int64_t wide = (pairs / 128 + rows) * num_kv_heads, narrow = (pairs / 64 + rows) * num_kv_heads;
-    const int sms = device_sm_count();
-    auto shares = [&](int64_t blocks, int room) {
-        int n = 1;
-        while (n < 8 && 2 * n <= most && 2 * n * blocks <= room) n *= 2;
-        return n;
-    };
-    if (head_dim > 64) return f32_launch<128, 8>(p, pairs, rows, shares(wide, 2 * sms), stream);
-    if (pairs / 128 * num_kv_heads >= sms && walk >= 6) return f32_launch<64, 8>(p, pairs, rows, 2, stream);
-    return f32_launch<64, 4>(p, pairs, rows, shares(narrow, 3 * sms), stream);
+    const F32Plan plan = f32_plan(pairs, rows, num_heads, num_kv_heads, head_dim, window, keep, max_ctx, device_sm_count());
+    return head_dim > 64 ? f32_launch<128, 8>(p, plan, stream) : plan.warps == 8 ? f32_launch<64, 8>(p, plan, stream) : f32_launch<64, 4>(p, plan, stream);
 }
