@@ -20,7 +20,8 @@ class EngineConfig:
     use_cuda_graphs: bool = True
     cuda_graph_batch_sizes: tuple = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 224, 256)
     graph_context_bounds: tuple = (960,)    # decode graphs are captured once per bucket for each of these context bounds
-                                            # below max_model_len, and once for max_model_len: kernels that plan by the
+                                            # below max_model_len (float32: and for a short one, whose rows another
+                                            # attention kernel serves), and once for max_model_len: kernels that plan by the
                                             # longest context a launch may meet (decode attention cuts long contexts into
                                             # parts) then get a plan that fits the requests a step really holds
     num_blocks: int | None = None           # explicit pool size in pages (page 0 included); None = from memory

@@ -19,6 +19,7 @@ import torch
 
 from ..config import EngineConfig, load_config
 from ..kernels import gemm_tc, ops
+from ..kernels.attention import captured_context_bounds
 from ..models.decoder import DecoderModel
 from ..parts.base import Runtime
 from ..sampling.params import SamplingParams
@@ -85,6 +86,7 @@ class LLMEngine:
         self.cfg.max_model_len = min(self.cfg.max_model_len, spec.max_position)      # inference_engine/engine.py:42
         self.eos_token_id = spec.eos_token_id
         self.vocab_size = spec.vocab_size
+        self.dtype = dtype
         rt = Runtime(self.device, dtype)
         self.model = DecoderModel(spec, read_model_folder(model), rt, where=model)
         torch.cuda.empty_cache()
@@ -134,7 +136,7 @@ class LLMEngine:
         self.num_steps = 0
         self.num_graph_steps = 0
         self.num_portion_graph_steps = 0
-        self._portion_graphs: dict = {}          # (tokens, wanted logits) -> captured step of one prompt portion
+        self._portion_graphs: dict = {}          # (tokens, whether none of them pads, wanted logits, context bound) -> captured step of one prompt portion
         self._portion_seen: dict = {}
         self._graph_pool = None
         self._capture_stream = None
@@ -180,8 +182,8 @@ class LLMEngine:
     @torch.inference_mode()
     def _capture_cuda_graphs(self):
         """One graph per batch-size bucket, largest first so the smaller ones share its memory
-        pool (inference_engine/engine.py:76-104), and per context bound (``graph_context_bounds`` and
-        ``max_model_len``): a step replays the graph of the smallest bound that covers its longest
+        pool (inference_engine/engine.py:76-104), and per context bound (``graph_context_bounds``, those that the
+        attention kernels of the compute type ask for, and ``max_model_len``): a step replays the graph of the smallest bound that covers its longest
         request.  A graph covers the whole step including the sampling kernel; its inputs live in one
         static device buffer that a step overwrites with one copy.  Rows that pad a batch up to its
         bucket are scratch rows: one token at position 0 of page 0, context length 1."""
@@ -191,7 +193,8 @@ class LLMEngine:
             return
         b = self.runner.builder
         pool = None
-        bounds = sorted({c for c in self.cfg.graph_context_bounds if c < self.cfg.max_model_len} | {self.cfg.max_model_len})
+        asked = {*self.cfg.graph_context_bounds, *captured_context_bounds(self.dtype)}
+        bounds = sorted({c for c in asked if c < self.cfg.max_model_len} | {self.cfg.max_model_len})
         for bs in reversed(sizes):
             static = None
             for bound in reversed(bounds):
@@ -273,11 +276,14 @@ class LLMEngine:
         cut by what is left of the token budget, so their lengths are rounded up (``_padded_length``) for
         shapes to repeat.  What differs between replays -- tokens, positions, block table, the split between
         the portion and its padding, sampling inputs -- lives in the graph's static input buffer; the context
-        bound that kernels plan by is the model's longest.  At most ``graph_prompt_portions`` graphs are kept
+        bound that kernels plan by is the model's longest, or a shorter one that the attention kernels of the
+        compute type ask for (a graph of its own).  At most ``graph_prompt_portions`` graphs are kept
         (the least recently used one goes).  The reference launches such steps eagerly."""
         n = len(row.tokens)
         padded = self._padded_length(n)
-        key = (padded, padded == n, wanted)
+        longest = self.cfg.max_model_len
+        bound = min((c for c in captured_context_bounds(self.dtype) if c >= row.pos0 + n), default=longest)
+        key = (padded, padded == n, wanted, min(bound, longest))
         g = self._portion_graphs.get(key)
         if g is not None:
             self._portion_graphs[key] = self._portion_graphs.pop(key)        # most recently used last
@@ -289,7 +295,7 @@ class LLMEngine:
             return None
         b = self.runner.builder
         buf, layout = b.pack(self._portion_rows(row, padded), table_width=self.max_blocks_per_seq, extras=extras)
-        layout["max_ctx_len"] = self.cfg.max_model_len
+        layout["max_ctx_len"] = key[3]
         layout["q_len"] = None              # the split between portion and padding changes from replay to replay
         layout["few_single_rows"] = True    # (a padding of one token is a row like a decoding one: the kernel for portions serves it)
         static = torch.zeros(layout["size"], dtype=torch.int32, device=self.device)

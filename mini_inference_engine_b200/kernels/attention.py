@@ -74,6 +74,13 @@ F32_FULL_GROUP = 8          # query heads on a key head from which a row of one 
 F32_FEW = 64                # ... or so few such (row, key head) pairs that their tiles run side by side
 
 
+def captured_context_bounds(dtype) -> tuple:
+    """Context bounds, beside the longest one, that a captured step is worth planning for: the choice of kernel above goes by the bound, since a captured step's positions change.
+    float32, few rows: planned for 960 positions or more a row of one token takes a tile, some 12 us on 10 positions too, where a warp a pair takes 6 (32 heads of 64 on 4);
+    a portion of 32 tokens 14 against 7."""
+    return (F32_LONG_STEP - 1,) if dtype == torch.float32 else ()
+
+
 def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size, scale, window, mods, keep):
     """float32: rows with at least F32_MIN_PAIRS (token, head of a group) pairs by tiles, shorter ones one pair a warp, as all are in a step of few
     pairs on few positions; on many positions rows of any length by tiles.  Where the host does not know the rows' lengths (a captured step) each of the two kernels takes the

@@ -317,6 +317,36 @@ def test_decode_graphs_by_context_bound(model_folders):
     assert eng.num_graph_steps > 30
 
 
+def test_float32_graphs_for_short_contexts(tmp_path, monkeypatch):
+    """float32 attention chooses its kernel by the longest context that a captured step is planned for: steps on short contexts have graphs of their own, for decoding and for prompt
+    portions, in which rows of a few tokens go by a warp a (token, head) pair; the others take tiles.  The tokens are those of an engine without graphs."""
+    from mini_inference_engine_b200 import SamplingParams
+    from mini_inference_engine_b200.config import load_config
+    from mini_inference_engine_b200.kernels import ops
+    from mini_inference_engine_b200.weights import write_model_folder
+    folder = str(tmp_path / "long")
+    write_model_folder(folder, load_config(dict(
+        vocab_size=256, hidden_size=128, intermediate_size=160, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=32, rms_norm_eps=1e-5,
+        rope_theta=10000.0, max_position_embeddings=1024, tie_word_embeddings=True, architectures=["LlamaForCausalLM"])), seed=22)
+    tiles, plain, seen = [], ops.attention_f32, []
+    monkeypatch.setattr(ops, "attention_f32", lambda *a, **k: (tiles.append(k["max_ctx"]), plain(*a, **k))[1])
+    rng = random.Random(5)
+    prompts = [[rng.randrange(256) for _ in range(n)] for n in (90, 8, 9, 20, 7, 110)]
+    outs = []
+    for graphs in (True, False):
+        eng = engine_for(folder, torch.float32, max_model_len=1024, max_num_batched_tokens=24, max_num_seqs=2, use_cuda_graphs=graphs)
+        if graphs:
+            assert eng.graph_bounds == [127, 960, 1024] and eng.decode_graph(1, 127).layout["max_ctx_len"] == 127
+            assert set(tiles) == {960, 1024}, set(tiles)
+            tiles.clear()
+        outs.append([o.output_ids for o in eng.generate(prompts, SamplingParams(max_tokens=40, ignore_eos=True))])
+        if graphs:
+            seen = {key[3]: g.layout["max_ctx_len"] for key, g in eng._portion_graphs.items()}
+            assert eng.num_portion_graph_steps > 0 and 127 in seen and all(a == b for a, b in seen.items()), seen
+            assert 127 not in tiles
+    assert outs[0] == outs[1]
+
+
 def test_long_contexts_cut_into_parts_under_graphs(tmp_path):
     """48 requests x 4 kv heads with a context bound of 1,600 keys: the decode graphs' attention launches are
     laid out for three parts merged through scratch memory (a cluster would take two), and every row is cut by its
