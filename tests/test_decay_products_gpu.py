@@ -57,7 +57,8 @@ def test_as_far_from_64_bits_as_token_by_token(monkeypatch, dt, least):
         at += n
     for a, b, w in zip(got, ref, (out, end)):
         off = lambda t: ((t.double() - w).norm() / w.norm()).item()
-        assert off(a) <= 1.5 * off(b) + 2.0 ** -25
+        # measured over four seeds: outputs 0.93 to 1.13 times as far, states 0.90 to 1.13, with decays down to 0 (few terms a sum) 1.15 to 1.29
+        assert off(a) <= 1.35 * off(b)
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])

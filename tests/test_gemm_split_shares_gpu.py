@@ -36,4 +36,5 @@ def test_sizes_whose_plan_has_both(M, N, K):
     out = gemm_split.gemm_split(x, w, torch.empty(M, N, device="cuda"), bias)
     check(out, x, w, bias)
     off = lambda t: ((t.double() - (x.double() @ w.double().t() + bias.double())).norm() / t.double().norm()).item()
-    print(f"{M} x {N} x {K}: {off(out):.3g}, all tiles whole {off(gemm_split.gemm_split(x, w, torch.empty_like(out), bias, force=(128, 1))):.3g}")
+    # as far from 64 bits as one chain of chunks (measured 0.98 to 0.99 times as far: a share's sums are shorter)
+    assert off(out) <= 1.05 * off(gemm_split.gemm_split(x, w, torch.empty_like(out), bias, force=(128, 1)))
