@@ -1,5 +1,5 @@
-// Paged causal attention of prompt portions in float32 (the true 32-bit path): rows with many new tokens; csrc/attention_simt.cu serves the
-// others, and every row in bfloat16.  The same rules: masks, kept first keys, score modifiers, sink, range checks.  Scores and outputs are products on the tensor cores
+// Paged causal attention in float32 (the true 32-bit path) by tiles of (token, head) pairs: rows with many new tokens, and on long contexts rows of a few and of one (the line is
+// drawn in kernels/attention.py); csrc/attention_simt.cu, a warp a pair, serves the others, and every row in bfloat16.  The same rules: masks, kept first keys, score modifiers, sink, range checks.  Scores and outputs are products on the tensor cores
 // with every operand as three bfloat16 parts (triple_mma.cuh); weights, sums and everything else are float32.
 //
 // A block owns 16 (token, query head) pairs a warp that share a key head -- tokens of one row, the group's heads side by side -- so a tile of
@@ -15,6 +15,7 @@
 // splitting and the blocks' ends.  Kernel, us: 333 tokens on 300 positions beside 667, 32 heads of 64: 177 (register tiles on the CUDA cores) -> 94; 1,024 tokens 128; a layer of
 // TinyLlama's sizes over both rows, products included, 314 -> 230; 200 tokens on 800 positions 320 -> 120.  Against 64 bits the layer is 2.7e-7 off (2-norm), 3.6e-7 before.
 #include <algorithm>
+#include <cmath>
 
 #include "range_check.cuh"
 #include "triple_mma.cuh"
@@ -41,10 +42,13 @@ __device__ __noinline__ float f32_dot(const float* q, const float* k, int D, flo
 }
 
 // DT: entries of a head as the block holds them (head_dim padded with zeros); WARPS of 16 pairs each.
-template <int DT, int WARPS> constexpr int f32_bytes() { return 3 * 16 * WARPS * DT * 2 + 3 * F32_KEYS * DT * 2 + F32_KEYS * DT * 4; }
+// Blocks of 4 warps over heads of 65 to 128 have no memory for keys on their way if two are to fit on an SM: they fetch a tile when they split it, from L2 (asked for ahead), under
+// the other block's products.
+template <int DT, int WARPS> constexpr bool f32_direct = DT == 128 && WARPS == 4;
+template <int DT, int WARPS> constexpr int f32_bytes() { return 3 * 16 * WARPS * DT * 2 + 3 * F32_KEYS * DT * 2 + (f32_direct<DT, WARPS> ? 0 : F32_KEYS * DT * 4); }
 template <int DT, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2) f32_attention_kernel(const F32Params p, int splits) {
-    constexpr int GROUP = WARPS == 4 ? 4 : 2;         // column tiles at a time: as many as the registers have room for
+__global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 8 / WARPS : WARPS == 4 ? 3 : 2) f32_attention_kernel(const F32Params p, int splits) {
+    constexpr int GROUP = WARPS == 4 && DT == 64 ? 4 : 2;         // column tiles at a time: as many as the registers have room for
     constexpr int THREADS = 32 * WARPS, PAIRS = 16 * WARPS, Q_PLANE = PAIRS * DT * 2, K_PLANE = F32_KEYS * DT * 2, KS = DT / 16, NT = DT / 8;
     constexpr int QUADS = F32_KEYS * DT / 4 / THREADS, STEP = THREADS / (DT / 4);
     extern __shared__ __align__(16) uint8_t smem[];
@@ -93,7 +97,9 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
             for (int i = 0; i < QUADS; ++i) {
                 const int jj = my_row + i * STEP, page = s_page[(t / splits) & 1][jj];
                 const bool on = page >= 0 && my_d < D;
-                f32_copy16(raw + jj * DT + my_d, on ? row_in(cache, page, k0 + jj) + my_d : cache, on);
+                if constexpr (f32_direct<DT, WARPS>) {
+                    if (on && (my_d & 31) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(row_in(cache, page, k0 + jj) + my_d));
+                } else f32_copy16(raw + jj * DT + my_d, on ? row_in(cache, page, k0 + jj) + my_d : cache, on);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -107,10 +113,27 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
         for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(at + j * plane) = part[j];
         return magnitude(v);
     };
-    auto split = [&]() {                              // what this thread fetched, once every warp is done with what lay there; whether a number of the block's has no parts
+    auto split = [&](const float* cache, int t) {     // what this thread fetched, once every warp is done with what lay there; whether a number of the block's has no parts
+        uint32_t most = 0;
+        if constexpr (f32_direct<DT, WARPS>) {
+            constexpr int AHEAD = 8;                  // quads asked for before the first is split
+            __syncthreads();
+            const int k0 = tile_key(t);
+#pragma unroll
+            for (int first = 0; first < QUADS; first += AHEAD) {
+                float4 v[AHEAD];
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) {
+                    const int jj = my_row + (first + i) * STEP, page = s_page[(t / splits) & 1][jj];
+                    v[i] = page >= 0 && my_d < D ? *reinterpret_cast<const float4*>(row_in(cache, page, k0 + jj) + my_d) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) most = max(most, put(KV, K_PLANE, my_row + (first + i) * STEP, my_d, v[i]));
+            }
+            return __syncthreads_or(has_no_parts(most)) != 0;
+        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        uint32_t most = 0;
 #pragma unroll
         for (int i = 0; i < QUADS; ++i) {
             const int jj = my_row + i * STEP;
@@ -163,7 +186,7 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
         const int k0 = tile_key(t);
         const int next_page = page_of(t + splits);
         const int* pages = s_page[(t / splits) & 1];
-        const bool k_bad = split() || block_q_bad;
+        const bool k_bad = split(p.k_cache, t) || block_q_bad;
         issue(p.v_cache, t);
         float s[8][4];
         // a tile that every pair sees whole needs no mask: all keys at or before the first pair's position, none before the last one's first key
@@ -245,7 +268,7 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
             for (int n = 0; n < NT; ++n) { o[n][2 * i] *= alpha; o[n][2 * i + 1] *= alpha; }
         }
         if (threadIdx.x < F32_KEYS) s_page[(t / splits + 1) & 1][threadIdx.x] = next_page;
-        const bool v_bad = split();
+        const bool v_bad = split(p.v_cache, t);
         issue(p.k_cache, t + splits);
         if (!v_bad) {
 #pragma unroll
@@ -361,16 +384,19 @@ __global__ void __launch_bounds__(32 * WARPS, DT == 128 ? 1 : WARPS == 4 ? 3 : 2
 // Heads of 64: blocks of 8 warps, two on an SM, where they are as many as the SMs and their walks long (each in two
 // shares, so that the longest walks do not end alone: 1,024 tokens of 32 heads 147 -> 128 us, 333 on 300 beside 667 109 -> 94; shares of blocks of 4 warps 136 and 115; five rows of 120
 // on 100 positions 47 us, by blocks of 4 warps 39).  Else blocks of 4 warps, three on an SM, in as many shares as fit beside one another (64 tokens on 900 positions: 1, 2, 4, 8 shares
-// 109, 61, 35, 25 us; 200 on 800: 110, 71, 52, 73; 100 alone: 17.6, 15.0, 16.0, 27).  Heads of 128 have one block on an SM, so always of 8 warps (1,000 tokens of 32 heads: 207 us, in
-// two shares 254, by blocks of 4 warps 358; 500 on 300: 170 and 150 in two shares; 100 on 300: 92, 62, 38, 68): two shares may wait for one another's place, since portions' walks
-// differ, more must fit beside one another.  Clusters fill a B200's SMs less the larger they are, since one lies within a part of the chip: of blocks that have an SM to themselves 148, 148, 132
-// and 120 run at once in clusters of 1, 2, 4 and 8, of three to an SM 444, 444, 416 and 384; one cluster more costs a whole round (32 heads of 128 on 8, us, as many shares as blocks fit twice : as here -- 4
-// rows of one token on 256 positions planned for 960 58 : 21, 8 rows on 500 66 : 59, 100 tokens on 250 68 : 37; 100 tokens of 32 heads of 64, eight shares 27, four 17).
+// 109, 61, 35, 25 us; 200 on 800: 110, 71, 52, 73; 100 alone: 17.6, 15.0, 16.0, 27).  A walk of one tile has no shares: the second would have nothing and
+// the meeting costs 4 to 6 us (64 tokens alone 14.1 -> 10.7).
+// Heads of 65 to 128: blocks of 8 warps have an SM to themselves, those of 4 share it in twos (f32_direct), so that a block too many costs a whole round: the width and the number of shares that take
+// the least estimated time.  Measured, us: a block of 8 warps 6.7 and 12.5 for every tile of its walk, of 4 warps 8.4 and 13.1 (16.9 where two share an SM), the meeting of two, four and eight shares
+// 6.7, 4.1 and 4.4 (6.3, 3.5 and 4.0); clusters of four and eight fill the SMs but for a ninth and a quarter (1/36 and an eighth), since one lies within a part of the chip.  Rows' tiles have
+// walks of different lengths, longest first: beyond one round the places fill up, and the last and shortest end three quarters of a block later; where all are alike it is whole rounds.  Over 468 steps
+// of 1 to 32 rows, 32 heads on 8, 16 on 2, 16 on 16 and 8 on 8, within 0.5 % of the best plan on average.  Us, as many shares of blocks of 8 warps as fit : as here -- 32 heads on 8: 8 rows of 40 tokens
+// 50 : 20, 4 of 100 51 : 32, 4 of 100 on 300 121 : 95, 2 of 64 on 1,000 126 : 75, 16 rows of one token on 400 116 : 73; 16 heads of 96 on 16, 32 rows of 64 tokens 73 : 53, of 64 on 130 224 : 152.
 struct F32Plan { int warps, shares; int64_t items; };
 static F32Plan f32_plan(int64_t pairs, int rows, int num_heads, int num_kv_heads, int head_dim, int window, int keep, int max_ctx, int sms) {
     using std::max; using std::min;
     const int reach = window > 0 ? min(max_ctx, window + keep + F32_KEYS) : window < 0 ? min(max_ctx, keep - window) : max_ctx;
-    const int walk = (reach + F32_KEYS - 1) / F32_KEYS, most = max(2 * walk / 3, min(walk + 1, 4));         // (walk: the longest one, in tiles of keys)
+    const int walk = (reach + F32_KEYS - 1) / F32_KEYS, most = walk > 1 ? max(2 * walk / 3, min(walk + 1, 4)) : 1;      // (walk: the longest one, in tiles of keys)
     // tiles of `per` pairs: a row's pairs are a multiple of the group's heads, so its last tile lacks at most per - gcd(per, heads)
     const int group = num_heads / num_kv_heads, fits = group & -group;
     auto items = [&](int per) { return (pairs + (int64_t)rows * (per - min(per, fits))) / per * num_kv_heads; };
@@ -379,7 +405,28 @@ static F32Plan f32_plan(int64_t pairs, int rows, int num_heads, int num_kv_heads
         while (n < 8 && 2 * n <= most && 2 * n * blocks <= (n == 1 ? two : n == 2 ? four : eight)) n *= 2;
         return n;
     };
-    if (head_dim > 64) return {8, shares(items(128), 2 * sms, sms * 8 / 9, sms * 13 / 16), items(128)};
+    if (head_dim > 64) {
+        const double tokens = (double)pairs / group / rows;        // of a row, as if they were alike
+        F32Plan best{8, 1, 0};
+        double least = 0;
+        for (int warps = 8; warps >= 4; warps -= 4) {
+            const int per = 16 * warps;
+            const double first = max(1.0, min((double)walk, std::ceil((max_ctx - tokens + (double)per / group) / F32_KEYS)));
+            const double shortest = window ? walk : first, mean = (walk + shortest) / 2;           // walks of a row's tiles
+            const int64_t tiles = (int64_t)rows * (int64_t)std::ceil((double)pairs / rows / per) * num_kv_heads;
+            const int wide[] = {sms, sms, sms * 8 / 9, sms * 3 / 4}, narrow[] = {2 * sms, 2 * sms, sms * 35 / 18, sms * 7 / 4};
+            const double meet_wide[] = {0, 6.7, 4.1, 4.4}, meet_narrow[] = {0, 6.3, 3.5, 4.0};
+            for (int n = 1, i = 0; n <= 8 && (n == 1 || walk > 1); n *= 2, ++i) {
+                const double blocks = (double)(tiles * n), rounds = blocks / max(1, warps == 8 ? wide[i] : narrow[i]);
+                const double start = warps == 8 ? 6.7 + meet_wide[i] : 8.4 + meet_narrow[i], step = warps == 8 ? 12.5 : 13.1 + 3.8 * (max(1.0, min(2.0, blocks / sms)) - 1);
+                const double longest = start + step * ((walk + n - 1) / n), usual = start + step * max(1.0, mean / n), last = start + step * max(1.0, shortest / n);
+                const double us = rounds <= 1 ? longest : max(longest, min(std::ceil(rounds) * longest, rounds * usual + 0.75 * last));
+                if (least == 0 || us < least) { best = {warps, n, 0}; least = us; }
+            }
+        }
+        best.items = items(16 * best.warps);
+        return best;
+    }
     if (pairs / 128 * num_kv_heads >= sms && walk >= 6) return {8, 2, items(128)};
     return {4, shares(items(64), 3 * sms, 3 * sms * 15 / 16, 3 * sms * 13 / 16), items(64)};
 }
@@ -415,5 +462,6 @@ extern "C" int mie_attention_f32(const float* q, int64_t q_stride, const float* 
                       num_kv_heads, head_dim, page_size, page_shift, scale, window, keep, min_q_len, (int64_t)num_pages, g_range_report,
                       ScoreMods{softcap, sink, dist_bias, dist_len, slope}};
     const F32Plan plan = f32_plan(pairs, rows, num_heads, num_kv_heads, head_dim, window, keep, max_ctx, device_sm_count());
-    return head_dim > 64 ? f32_launch<128, 8>(p, plan, stream) : plan.warps == 8 ? f32_launch<64, 8>(p, plan, stream) : f32_launch<64, 4>(p, plan, stream);
+    if (head_dim > 64) return plan.warps == 8 ? f32_launch<128, 8>(p, plan, stream) : f32_launch<128, 4>(p, plan, stream);
+    return plan.warps == 8 ? f32_launch<64, 8>(p, plan, stream) : f32_launch<64, 4>(p, plan, stream);
 }

@@ -32,13 +32,16 @@ def test_items_for_every_tile(group, head_dim):
 def test_more_than_two_shares_fit_beside_one_another(group, kv_heads, max_ctx, head_dim):
     for rows, tokens in [(1, 1), (4, 4), (8, 8), (16, 16), (64, 64), (1, 47), (1, 100), (2, 300), (1, 2000)]:
         warps, shares, items = plan(tokens * group, rows, group * kv_heads, kv_heads, head_dim, max_ctx)
-        assert shares in (1, 2, 4, 8) and shares <= max(1, 2 * -(-max_ctx // 64))
-        # what a B200 runs at once in clusters of four and eight (a block of eight warps over heads of 128 has an SM to itself, of four over heads of 64 a third)
-        places = {4: 132, 8: 120} if head_dim == 128 else {4: 416, 8: 384}
-        assert shares <= 2 or shares * items <= places[shares], (rows, tokens, warps, shares)
+        assert shares in (1, 2, 4, 8) and (max_ctx > 64 or shares == 1) and shares <= 2 * -(-max_ctx // 64)
+        # what a B200 runs at once in clusters of four and eight: blocks of four warps over heads of 64 have a third of an SM
+        if head_dim == 64:
+            assert shares <= 2 or shares * items <= {4: 416, 8: 384}[shares], (rows, tokens, warps, shares)
 
 
-def test_decoding_rows_and_portions_of_heads_of_128():
-    # 32 heads on 8: 1, 4, 8 rows of one token on up to 960 positions; one row of 32 and of 100 tokens
-    assert [plan(r * 4, r, 32, 8, 128, 960)[:2] for r in (1, 4, 8)] == [(8, 8), (8, 4), (8, 2)]
-    assert [plan(n * 4, 1, 32, 8, 128, 2048)[:2] for n in (32, 100)] == [(8, 8), (8, 4)]
+@pytest.mark.parametrize("rows,tokens,ctx,heads,kv_heads,best", [
+    (1, 64, 64, 32, 8, (8, 1)), (8, 40, 40, 32, 8, (8, 1)), (32, 20, 20, 16, 2, (8, 1)), (4, 100, 100, 32, 8, (8, 1)), (4, 100, 400, 32, 8, (8, 1)), (1, 100, 230, 32, 8, (8, 4)),
+    (2, 64, 364, 32, 8, (8, 4)), (2, 64, 1064, 32, 8, (8, 4)), (1, 500, 800, 32, 8, (8, 2)), (32, 40, 40, 16, 16, (4, 1)), (32, 64, 194, 16, 16, (4, 1)), (16, 64, 64, 16, 16, (4, 1)),
+    (16, 1, 400, 32, 8, (4, 2)), (8, 1, 400, 32, 8, (4, 4)), (16, 1, 400, 16, 16, (4, 1))])
+def test_heads_of_128_by_the_plan_that_took_least(rows, tokens, ctx, heads, kv_heads, best):
+    """As measured on a B200 by every width and number of shares."""
+    assert plan(rows * tokens * heads // kv_heads, rows, heads, kv_heads, 128, ctx)[:2] == best

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 LONG = [(3, 1200), (1, 1100), (17, 700), (1, 5), (64, 64), (2, 513)]
 
 
-@pytest.mark.parametrize("H,G,D", [(16, 2, 64), (4, 4, 48), (8, 2, 128), (3, 1, 96)])
+@pytest.mark.parametrize("H,G,D", [(16, 2, 64), (4, 4, 48), (8, 2, 128), (3, 1, 96), (20, 20, 80)])
 @pytest.mark.parametrize("window,keep", [(0, 0), (300, 0), (-256, 70)])
 @pytest.mark.parametrize("max_ctx", [None, 64, 1200])
 def test_walks_in_one_to_eight_shares(H, G, D, window, keep, max_ctx):
@@ -36,7 +36,7 @@ def test_wide_blocks(rows, sink):
     close(*both(args, out, H, G, D, 16, mods=mods), args[3])
 
 
-@pytest.mark.parametrize("H,G,D", [(8, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("H,G,D", [(8, 2, 64), (8, 2, 128), (10, 10, 128)])          # (the last: blocks of four warps without memory for keys on their way)
 @pytest.mark.parametrize("what", ["key", "value", "query"])
 @pytest.mark.parametrize("bad", [3e38, float("inf"), float("nan")])
 def test_numbers_without_parts_reach_what_they_reach_one_by_one(H, G, D, what, bad):
@@ -96,7 +96,7 @@ def test_numbers_without_parts_in_wide_blocks(window, keep, what, bad):
     assert ((a - b).abs()[big] <= 1e-4 * b.abs()[big]).all()
 
 
-@pytest.mark.parametrize("H,G,D", [(8, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("H,G,D", [(8, 2, 64), (8, 2, 128), (10, 10, 128)])          # (the last: blocks of four warps without memory for keys on their way)
 @pytest.mark.parametrize("n,ctx,first,end", [(100, 100, 64, 65), (150, 150, 128, 129), (1, 129, 128, 129), (1, 129, 64, 129), (300, 520, 192, 256), (300, 520, 0, 64), (300, 520, 0, 448),
                                              (300, 520, 64, 520), (5, 700, 0, 700)])
 @pytest.mark.parametrize("sink", [False, True])
