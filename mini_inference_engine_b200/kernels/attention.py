@@ -94,14 +94,20 @@ def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size,
             and ((group >= F32_FULL_GROUP and head_dim <= 64) or singles * num_kv_heads <= F32_FEW)):
         min_q_len = 1
     long = None if q_lens is None else [n for n in q_lens if n >= min_q_len]
+    longest, c_lens = ctx.max_ctx_len, ctx.host.get("ctx_len")
+    if long and len(long) < len(q_lens) and c_lens is not None and len(c_lens) == len(q_lens) and max(c_lens) == longest:
+        # the rows that tiles would take, not those beside them, decide (captured steps are planned for more than the host's numbers say).  Us, 20 tokens on 50 positions of 16 heads of
+        # 64 on 16 beside 8 rows of one token on 700: a launch of tiles for that portion alone 99, all rows by warps 82
+        longest = max(c for n, c in zip(q_lens, c_lens) if n >= min_q_len)
+        reach = longest if window == 0 else min(longest, abs(window) + keep)
     sizes = (ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, page_size, scale, window)
     pairs = (ctx.num_tokens if long is None else sum(long)) * num_heads
-    few = F32_MIN_WORK_FRESH if ctx.max_ctx_len <= F32_FRESH else F32_MIN_WORK if reach < F32_LONG else 1
+    few = F32_MIN_WORK_FRESH if longest <= F32_FRESH else F32_MIN_WORK if reach < F32_LONG else 1
     if pairs < few and min_q_len > 1:
         return ops.paged_attention(*args, *sizes, mods=mods, keep=keep)
     if min_q_len > 1 and (long is None or len(long) < len(q_lens)):
         ops.paged_attention(*args, *sizes, mods=mods, keep=keep, below=min_q_len)
-    ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)), max_ctx=ctx.max_ctx_len)
+    ops.attention_f32(*args, *sizes, min_q_len=min_q_len, mods=mods, keep=keep, work=None if long is None else (len(long), sum(long)), max_ctx=longest)
     return out
 
 

@@ -59,7 +59,7 @@ def test_numbers_without_parts_reach_what_they_reach_one_by_one(H, G, D, what, b
 @pytest.mark.parametrize("H,G,D,rows,ctx,kernels", [(8, 1, 64, [(1, 128)] * 70, 128, {"tiles"}), (8, 1, 64, [(1, 127)] * 3, 127, {"paged"}), (4, 4, 64, [(1, 300)] * 16, 300, {"tiles"}),
                                                     (4, 4, 64, [(1, 300)] * 17, 300, {"paged"}), (16, 2, 128, [(1, 300)] * 33, 300, {"paged"}),
                                                     (8, 1, 64, [(2, 640), (1, 30)], 640, {"tiles"}), (4, 4, 64, [(20, 640)] + [(1, 30)] * 17, 640, {"tiles", "paged"}),
-                                                    (4, 4, 64, [(9, 640)] + [(1, 30)] * 17, 640, {"paged"}), (8, 1, 64, [(2, 639), (1, 30)], 639, {"paged"})])
+                                                    (4, 4, 64, [(20, 70)] + [(1, 640)] * 17, 640, {"paged"}), (4, 4, 64, [(9, 640)] + [(1, 30)] * 17, 640, {"paged"}), (8, 1, 64, [(2, 639), (1, 30)], 639, {"paged"})])
 def test_rows_of_one_token_and_long_rows_of_few(monkeypatch, H, G, D, rows, ctx, kernels):
     from mini_inference_engine_b200.kernels import attention, ops
     args, _, out = case(rows, H, G, D, 16)
@@ -68,7 +68,8 @@ def test_rows_of_one_token_and_long_rows_of_few(monkeypatch, H, G, D, rows, ctx,
     used, paged, tiles = set(), ops.paged_attention, ops.attention_f32
     monkeypatch.setattr(ops, "paged_attention", lambda *a, **h: (used.add("paged"), paged(*a, **h))[1])
     monkeypatch.setattr(ops, "attention_f32", lambda *a, **h: (used.add("tiles"), tiles(*a, **h))[1])
-    step = SimpleNamespace(block_tables=[block], row_q_start=starts, row_q_len=lens, row_ctx_len=ctx_lens, num_tokens=T, max_ctx_len=ctx, host={"q_len": [n for n, _ in rows]})
+    step = SimpleNamespace(block_tables=[block], row_q_start=starts, row_q_len=lens, row_ctx_len=ctx_lens, num_tokens=T, max_ctx_len=ctx,
+                           host={"q_len": [n for n, _ in rows], "ctx_len": [c for _, c in rows]})
     got = attention.attention(q, step, SimpleNamespace(k=k, v=v, group=0, page_size=16), torch.zeros_like(out), H, G, D, D ** -0.5, 0)
     close(got, want, v)
     assert used == kernels
