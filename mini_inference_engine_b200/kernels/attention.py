@@ -1,7 +1,8 @@
 """Chooses the attention kernels for a step.
 
-float32 (the true 32-bit path): two CUDA-core kernels, one for rows with many new tokens and heads of up to 128
-(``csrc/attention_f32.cu``), one for the rest.
+float32 (the true 32-bit path): tiles of (token, head) pairs whose products run on the tensor cores with every operand as three
+bfloat16 parts (``csrc/attention_f32.cu``, heads of up to 128) for rows with many new tokens and, on long contexts, for rows of a few and
+of one; a warp a pair on the CUDA cores (``csrc/attention_simt.cu``) for the rest.
 bfloat16: rows with one new token go to the tensor-core decode kernel (context split across
 blocks), rows with more go to a prefill kernel -- the tcgen05 one for head sizes 64 and 128, the
 mma.sync one for the other multiples of 16 up to 128; head sizes beyond those kernels fall back to
@@ -12,6 +13,7 @@ from __future__ import annotations
 import torch
 
 from . import ops
+from .device import num_sms
 
 _backend = "auto"
 _prefill_backend = "tcgen05"
@@ -60,15 +62,17 @@ def rotates_in_decode(dtype, head_dim: int, ctx) -> bool:
 
 # float32: tiles of (token, head) pairs (csrc/attention_f32.cu) against a warp a pair.  A tile takes as long with one pair as with 64, a walk of keys shared out over up to eight
 # blocks some 15 us a thousand positions; a warp takes 120 us for them, and warps fill the GPU from about 1,500 pairs on.  One row, us, a warp a pair : tiles, 0 / 250 / 500 / 1,000 /
-# 2,000 earlier positions -- 32 heads of 64 on 4: 2 tokens 6 : 12 / 33 : 13 / 64 : 19 / 125 : 19 / 244 : 33, 32 tokens 7 : 14 / 42 : 20 / 76 : 26 / 146 : 28 / 282 : 43, 64 tokens
-# 16.5 : 14.4 / 74 : 21 / 122 : 28 / 222 : 35 / 426 : 50; 16 of 64 on 16: 32 tokens 7 : 14 / 40 : 20 / 73 : 26 / 138 : 29 / 266 : 39; 32 of 128 on 8: 32 tokens 8 : 25 / 55 : 35 / 100 : 48 / 192 : 48 /
+# 2,000 earlier positions -- 32 heads of 64 on 4: 2 tokens 6 : 10 / 33 : 13 / 64 : 19 / 125 : 19 / 244 : 33, 32 tokens 7 : 10 / 42 : 20 / 76 : 26 / 146 : 28 / 282 : 43, 64 tokens
+# 13.4 : 10.7 / 74 : 21 / 122 : 28 / 222 : 35 / 426 : 50; 16 of 64 on 16: 32 tokens 7 : 10 / 40 : 20 / 73 : 26 / 138 : 29 / 266 : 39; 32 of 128 on 8: 32 tokens 8 : 19 / 55 : 24 / 100 : 35 / 192 : 48 /
 # 372 : 60.  R rows of one token on 250 / 1,000 / 4,000 positions: 32 of 64 on 4, R 1 33 : 12 / 125 : 19 / 481 : 59, 16 36 : 17 / 134 : 47 / 604 : 171, 64 77 : 45 / 304 : 169 / 1,181 : 656;
-# 16 of 64 on 16, 4 30 : 16 / 111 : 47 / 515 : 170, 16 35 : 44 / 148 : 166 / 566 : 644; 32 of 128 on 8, 1 38 : 19 / 143 : 32 / 555 : 107, 4 38 : 20 / 144 : 95 / 724 : 322, 16 48 : 64 / 217 : 215.
+# 16 of 64 on 16, 4 30 : 16 / 111 : 47 / 515 : 170, 16 35 : 44 / 148 : 166 / 566 : 644; 32 of 128 on 8, 1 38 : 19 / 143 : 32 / 555 : 107, 4 38 : 20 / 144 : 44, 16 48 : 67 / 217 : 245.
 F32_MIN_WORK = 1536         # (token, head) pairs of the rows that tiles could take, from which they do ...
 F32_MIN_WORK_FRESH = 2048   # ... where no row has more than F32_FRESH positions; any number of pairs ...
 F32_FRESH = 256
 F32_LONG = 640              # ... where a row reaches this many positions: rows of one token too where tiles are faster (F32_FULL_GROUP, F32_FEW)
 F32_LONG_STEP = 128         # the same for a step of rows of one token only
+F32_WIDE_WORK = 135_000     # heads above 64: pairs times positions for every round of tiles up to which warps take less (32 heads of 128 on 8, us, a warp a pair : tiles -- 64 tokens
+                            # alone 17 : 20, 64 on 30 23 : 26, two rows of 40 18 : 20, four 27 : 20; 16 of 96 on 16, 16 rows of 20 tokens 20 : 23, 32 33 : 47, 16 rows of 40 40 : 25)
 F32_MIN_PAIRS = 16          # pairs of a row on one key head below which it is left to the warps: three quarters of its tile would be empty
 F32_FULL_GROUP = 8          # query heads on a key head from which a row of one token fills enough of a tile (heads of up to 64) ...
 F32_FEW = 64                # ... or so few such (row, key head) pairs that their tiles run side by side
@@ -103,6 +107,9 @@ def _attention_f32(args, ctx, out, num_heads, num_kv_heads, head_dim, page_size,
     sizes = (ctx.num_tokens, out, num_heads, num_kv_heads, head_dim, page_size, scale, window)
     pairs = (ctx.num_tokens if long is None else sum(long)) * num_heads
     few = F32_MIN_WORK_FRESH if longest <= F32_FRESH else F32_MIN_WORK if reach < F32_LONG else 1
+    if head_dim > 64 and long and min_q_len > 1 and reach < F32_LONG:
+        rounds = sum(-(-n * group // 128) for n in long) * num_kv_heads / num_sms()
+        few = max(few, F32_WIDE_WORK * max(1.0, rounds) / longest)
     if pairs < few and min_q_len > 1:
         return ops.paged_attention(*args, *sizes, mods=mods, keep=keep)
     if min_q_len > 1 and (long is None or len(long) < len(q_lens)):

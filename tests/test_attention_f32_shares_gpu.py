@@ -59,7 +59,9 @@ def test_numbers_without_parts_reach_what_they_reach_one_by_one(H, G, D, what, b
 @pytest.mark.parametrize("H,G,D,rows,ctx,kernels", [(8, 1, 64, [(1, 128)] * 70, 128, {"tiles"}), (8, 1, 64, [(1, 127)] * 3, 127, {"paged"}), (4, 4, 64, [(1, 300)] * 16, 300, {"tiles"}),
                                                     (4, 4, 64, [(1, 300)] * 17, 300, {"paged"}), (16, 2, 128, [(1, 300)] * 33, 300, {"paged"}),
                                                     (8, 1, 64, [(2, 640), (1, 30)], 640, {"tiles"}), (4, 4, 64, [(20, 640)] + [(1, 30)] * 17, 640, {"tiles", "paged"}),
-                                                    (4, 4, 64, [(20, 70)] + [(1, 640)] * 17, 640, {"paged"}), (4, 4, 64, [(9, 640)] + [(1, 30)] * 17, 640, {"paged"}), (8, 1, 64, [(2, 639), (1, 30)], 639, {"paged"})])
+                                                    (4, 4, 64, [(20, 70)] + [(1, 640)] * 17, 640, {"paged"}), (4, 4, 64, [(9, 640)] + [(1, 30)] * 17, 640, {"paged"}), (8, 1, 64, [(2, 639), (1, 30)], 639, {"paged"}),
+                                                    (32, 8, 128, [(64, 64)], 64, {"paged"}), (32, 8, 128, [(64, 64)] * 2, 64, {"tiles"}), (16, 16, 96, [(20, 20)] * 32, 20, {"paged"}),
+                                                    (16, 16, 96, [(40, 40)] * 16, 40, {"tiles"}), (32, 8, 128, [(64, 64)] * 2 + [(1, 90)] * 9, 90, {"tiles", "paged"})])
 def test_rows_of_one_token_and_long_rows_of_few(monkeypatch, H, G, D, rows, ctx, kernels):
     from mini_inference_engine_b200.kernels import attention, ops
     args, _, out = case(rows, H, G, D, 16)
