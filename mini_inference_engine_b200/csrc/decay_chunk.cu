@@ -17,7 +17,8 @@
 // Rows of one chunk are left to retention.cu.  q and k come prepared (rotated or activated, scaled) as float32 from its first kernel.
 // Bound: the tensor pipe at 8 cycles an instruction on each quarter of an SM, kept busy for 24 - 30 % of the time (operands' way from memory and the blocks' ends are the
 // rest).  2,048 tokens of 8 heads of 128 x 256 from bfloat16 values, us: local 51.7 -> 30, output 78.7 -> 40 (register tiles on the CUDA cores before); the layer
-// with a decay per head 209 -> 146, of 100 tokens 58 -> 46.  Against 64 bits the outputs are 1.0e-7 to 2.7e-7 off (2-norm; the CUDA cores' 2.1e-7 to 3.5e-7), the states
+// with a decay per head 209 -> 146, of 100 tokens 58 -> 46.  float32 values, or bfloat16 ones behind an activation, in heads above 64 (three
+// parts, 117 KB, so one block of `local` on an SM where two of bfloat16 values fit): the whole scan of those sizes 159 -> 107 and 172 -> 122 us, 512 tokens 58 -> 46 and 64 -> 50, 100 tokens 43 -> 31 and 50 -> 37.  Against 64 bits the outputs are 1.0e-7 to 2.7e-7 off (2-norm; the CUDA cores' 2.1e-7 to 3.5e-7), the states
 // 4.7e-8 to 3.0e-7 (4.8e-8 to 3.1e-7).
 #include "triple_mma.cuh"
 

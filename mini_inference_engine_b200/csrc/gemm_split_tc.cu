@@ -19,11 +19,11 @@
 //            Rows of w on the 128-lane side: what a warp stores for a token is 128 contiguous bytes, and a few tokens waste nothing.
 //            The pair runs persistently over items: tiles with all of K first, then the shares of K of the remaining tiles, which meet in `partial` and
 //            which a last small kernel adds up in order.  Tiles that are one wave of pairs and a few more would take two waves: as shares the few are spread over
-//            all pairs (509 x 11,264 x 2,048, 88 tiles on 74 pairs: 161 -> 143 us; 1,000 x 2,560 x 2,048, 80 tiles of 128 tokens, 73 -> 66 us).
+//            all pairs (509 x 11,264 x 2,048, 88 tiles on 74 pairs: 161 -> 140 - 143 us; 1,000 x 2,560 x 2,048, 80 tiles of 128 tokens, 73 -> 66 us).
 //
 // Bound: the tensor pipe (6 bfloat16 products for one float32 one: a sixth of its rate) for many tokens, memory (4 bytes of w read, 6
 // written and read again) for few.  2,048 x 11,264 x 2,048: 2,707 us on the CUDA cores -> 403 us (235 TFLOP/s);
-// 509 x 11,264 x 2,048 1,008 -> 140 us; 509 x 2,048 x 5,632 1,195 -> 78 us; 17 x 2,048 x 2,048, w from memory, 209 -> 24 us.  Chunks of 32 in a deeper ring were slower
+// 509 x 11,264 x 2,048 1,008 -> 140 - 143 us; 509 x 2,048 x 5,632 1,195 -> 78 us; 17 x 2,048 x 2,048, w from memory, 209 -> 24 us.  Chunks of 32 in a deeper ring were slower
 // (550 us at 2,048 tokens): the way from a full accumulator to an empty one costs about 2 us, so what counts is the work per accumulator and their number.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -17,7 +17,7 @@ from .device import num_sms
 #   11,264 x 2,048 89 : 88 / 115 : 88 / 235 : 88 / 239 : 88          2,048 x 5,632 90 : 46 / 91 : 46 / 583 : 46 / 605 : 47
 #   5,632 x 4,096 119 : 87 / 165 : 88 / 428 : 87 / 433 : 88          32,000 x 2,048 207 : 251 / 228 : 251 / 327 : 251 / 334 : 252
 # (taken with the parts' first form; the present one takes 12 to 14 less for 11,264 x 2,048.)  From 17 tokens on every size from 128 x 128 on: 13 : 11.  More tokens: 509 x 11,264 x 2,048
-# 1,008 : 140, 509 x 2,048 x 5,632 1,195 : 78, 2,048 x 11,264 x 2,048 2,707 : 403; smaller ones: 2,000 x 128 x 128 40 : 16, 2,000 x 64 x 64 12 : 15 (three launches instead of one).
+# 1,008 : 140 - 143, 509 x 2,048 x 5,632 1,195 : 78, 2,048 x 11,264 x 2,048 2,707 : 403; smaller ones: 2,000 x 128 x 128 40 : 16, 2,000 x 64 x 64 12 : 15 (three launches instead of one).
 MIN_TOKENS = 9
 MIN_K = 128
 MIN_WEIGHT = 1 << 14
@@ -43,7 +43,7 @@ def plan(M: int, N: int, K: int, only: int = 0) -> tuple:
     with 256 tokens only two accumulators fit tensor memory, and the way from a full one to an empty one is as long as the MMAs); an item's start and
     end 3,000; shares of K write and read M x (rows they cover) partial sums each at some 2,500 bytes a cycle, in a launch more.  The tiles in front
     fill whole waves of pairs; those behind them would leave most pairs idle, so it is they that are worth shares (all tiles whole : with shares behind, us,
-    B200, tokens x outputs x K: 509 x 11,264 x 2,048 161 : 143; 1,000 x 5,632 x 2,048 146 : 127; 1,000 x 2,560 x 2,048 73 : 66; 700 x 32,000 x 2,048 545 : 501)."""
+    B200, tokens x outputs x K: 509 x 11,264 x 2,048 161 : 140 - 143; 1,000 x 5,632 x 2,048 146 : 127; 1,000 x 2,560 x 2,048 73 : 66; 700 x 32,000 x 2,048 545 : 501)."""
     pairs = max(1, num_sms() // 2)
     chunks, tiles_n = -(-K // 64), -(-N // 256)
     best = None
