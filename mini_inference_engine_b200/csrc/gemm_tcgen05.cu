@@ -613,10 +613,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,     // the 128-row ope
                 else { rr = r_lo + idx / (BN / 4); c = (idx % (BN / 4)) * 4; }             // neighbours: consecutive columns
                 const uint32_t off = (uint32_t)(rr * RED_LD + c) * 4u;
                 float4 part[8];
+                if (push) {
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    if (s < S) part[s] = push ? *reinterpret_cast<const float4*>(recv + (s * rows_per + li) * RED_LD + c)
-                                              : ld_cluster_f32x4(peer[s] + off);
+                    for (int s = 0; s < 8; ++s)
+                        if (s < S) part[s] = *reinterpret_cast<const float4*>(recv + (s * rows_per + li) * RED_LD + c);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 8; ++s)
+                        if (s < S) part[s] = ld_cluster_f32x4(peer[s] + off);
+                }
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int s = 0; s < 8; ++s)
